@@ -410,8 +410,27 @@ int qtqp_mlp_colsum(const float* d_d, int32_t rows, int32_t cols, float* d_db,
 /* dy = 2 (y - t) / count and *d_loss = sum (y - t)^2 (overwritten). */
 int qtqp_mlp_mse_grad(const float* d_y, const float* d_t, int64_t count,
                       float* d_dy, double* d_loss, void* stream);
+/* One training step's forward and backward pass of the network x (batch x
+ * dim) -> relu(x W1 + b1) -> relu(. W2 + b2) -> y = . W3 + b3 (batch x out),
+ * all matrices row-major FP32 on the device, W1 dim x hidden, W2 hidden x
+ * hidden, W3 hidden x out.
+ * qtqp_mlp_forward_loss: h1, h2, y, dy = 2 (y - target) / (batch out) and
+ * *loss = sum (y - target)^2 (overwritten).
+ * qtqp_mlp_backward: from dy (and h1, h2), the hidden gradients dh1, dh2 and
+ * the gradients g1, gb1, ... of W1, b1, ...; qtqp_mlp_hinge_grad may change dy
+ * between the two. */
+typedef struct qtqp_mlp_step {
+  int32_t batch, dim, hidden, out;
+  const float *x, *target;
+  const float *w1, *b1, *w2, *b2, *w3, *b3;
+  float *h1, *h2, *y, *dy, *dh1, *dh2;
+  float *g1, *gb1, *g2, *gb2, *g3, *gb3;
+  double* loss;
+} qtqp_mlp_step;
+int qtqp_mlp_forward_loss(const qtqp_mlp_step* step, void* stream);
+int qtqp_mlp_backward(const qtqp_mlp_step* step, void* stream);
 /* Hinge term on the sign of the inequality outputs, added to d_dy (after
- * qtqp_mlp_mse_grad on the same buffers): columns [col0, cols) of the
+ * qtqp_mlp_mse_grad or qtqp_mlp_forward_loss on the same buffers): columns [col0, cols) of the
  * rows x cols output; d_zero[j - col0] is the column's decision point (the
  * standardised value of y_i - s_i = 0); the target's side of it gives the
  * sign s = +-1.  Adds weight * mean(relu(margin - s (y - zero))) to *d_loss

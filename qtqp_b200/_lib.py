@@ -57,6 +57,8 @@ EXPORTS = (
     "qtqp_mlp_colsum",
     "qtqp_mlp_mse_grad",
     "qtqp_mlp_hinge_grad",
+    "qtqp_mlp_forward_loss",
+    "qtqp_mlp_backward",
     "qtqp_mlp_gemm_bf16",
     "qtqp_mlp_to_bf16",
     "qtqp_mlp_adam",
@@ -133,6 +135,13 @@ class Result(ctypes.Structure):
       ("dres", ctypes.c_double),
       ("gap", ctypes.c_double),
   ]
+
+
+class MlpStep(ctypes.Structure):
+  _fields_ = ([(k, ctypes.c_int32) for k in ("batch", "dim", "hidden", "out")] +
+              [(k, ctypes.c_void_p) for k in (
+                  "x", "target", "w1", "b1", "w2", "b2", "w3", "b3", "h1", "h2", "y", "dy",
+                  "dh1", "dh2", "g1", "gb1", "g2", "gb2", "g3", "gb3", "loss")])
 
 
 MAX_GROUPS = 8
@@ -222,6 +231,8 @@ def load() -> ctypes.CDLL:
     lib.qtqp_mlp_colsum.argtypes = [vp, i32, i32, vp, vp]
     lib.qtqp_mlp_mse_grad.argtypes = [vp, vp, i64, vp, vp, vp]
     lib.qtqp_mlp_hinge_grad.argtypes = [vp, vp, i32, i32, i32, vp, f32, f32, vp, vp, vp]
+    lib.qtqp_mlp_forward_loss.argtypes = [vp, vp]
+    lib.qtqp_mlp_backward.argtypes = [vp, vp]
     lib.qtqp_mlp_gemm_bf16.argtypes = [i32, i32, i32, vp, vp, vp, i32, vp, i32, vp, i32, vp, vp]
     lib.qtqp_mlp_to_bf16.argtypes = [vp, i32, i32, i32, vp, vp]
     lib.qtqp_mlp_adam.argtypes = [vp, vp, vp, vp, i64, f32, f32, f32, f32, i32, vp]

@@ -3,6 +3,8 @@
 // gradients), the MSE gradient with its loss, the hinge term on the sign of
 // the inequality outputs, Adam, and the decoder that
 // turns network outputs into per-instance warm starts for the banded solver.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 
@@ -10,88 +12,233 @@
 
 namespace qtqp {
 
-constexpr int kTile = 64;         // C tile is kTile x kTile
-constexpr int kTk = 16;           // K slice staged in shared memory
-constexpr int kGemmThreads = 256; // 16 x 16 threads, 4 x 4 outputs each
+constexpr int kTile = 64;          // C tile is kTile x kTile
+constexpr int kTk = 16;            // K slice staged in shared memory
+constexpr int kGemmThreads = 256;  // 16 x 16 threads, 4 x 4 outputs each
+constexpr int kGemmPitch = kTile + 4;  // float4-aligned rows, 2-way store conflicts at most
+constexpr int kGemmMaxSplit = 16;  // CTAs of one cluster sharing a tile's K
 
-// C = alpha op(A) op(B) + beta C (+ bias[col]) (ReLU).  op(A)(r, k) is
-// A[r * lda + k], or A[k * lda + r] when trans_a; op(B)(k, c) is
-// B[k * ldb + c], or B[c * ldb + k] when trans_b.  Both operand slices are
-// staged k-major in shared memory, so the inner product reads two float4
-// rows per k.
-__global__ void __launch_bounds__(kGemmThreads)
-gemm_kernel(int M, int N, int K, float alpha, const float* __restrict__ a, int lda, int ta,
-            const float* __restrict__ b, int ldb, int tb, float beta, float* __restrict__ c,
-            int ldc, const float* __restrict__ bias, int relu) {
-  __shared__ __align__(16) float as[kTk][kTile];
-  __shared__ __align__(16) float bs[kTk][kTile];
+// C = alpha op(A) op(B) + beta C (+ bias[col]) (ReLU), and what a training
+// step does to C or op(B) while they are at hand:
+//   mask:   C_ij = 0 where !(mask_ij > 0) (the ReLU backward), laid out like C;
+//   colsum: the column sums of op(B) (the bias gradient when B is dY);
+//   dy:     dy_ij = dscale (C_ij - target_ij), *loss += sum (C - target)^2.
+struct GemmArgs {
+  int M, N, K;
+  float alpha;
+  const float* a;
+  int lda;
+  const float* b;
+  int ldb;
+  float beta;
+  float* c;
+  int ldc;
+  const float* bias;
+  int relu;
+  const float* mask;
+  float* colsum;
+  const float* target;
+  float* dy;
+  float dscale;
+  double* loss;
+};
+
+// op(A)(r, k) is A[r * lda + k], or A[k * lda + r] when TA; op(B)(k, c) is
+// B[k * ldb + c], or B[c * ldb + k] when TB.  Both operand slices are staged
+// k-major in two shared-memory buffers; the next slice's loads are in flight
+// (registers) while the current one is multiplied, one barrier per slice.
+//
+// The gridDim.z CTAs of a cluster share one tile: each takes a contiguous
+// part of the K slices, and the partial tiles are summed over distributed
+// shared memory in part order (no workspace, no atomics, the same sum on
+// every run).  Without the split a weight-sized product with a long K (dH =
+// dY W^T of a 256-wide layer under 11000 outputs: 16 tiles, 688 slices) ran on
+// 16 of 148 SMs and took about half of the step.
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kGemmThreads) gemm_kernel(const GemmArgs g) {
+  namespace cg = cooperative_groups;
+  __shared__ __align__(16) float sm[2 * 2 * kTk * kGemmPitch];
+  static_assert(2 * 2 * kTk * kGemmPitch >= kTile * kTile + kTile, "partial tile + column sums");
+  __shared__ double lpart[kGemmThreads / 32];
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
   const int row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+  const int parts = gridDim.z, part = blockIdx.z;
+  const int ns = (g.K + kTk - 1) / kTk;
+  const int q0 = int(int64_t(ns) * part / parts), q1 = int(int64_t(ns) * (part + 1) / parts);
+  const bool sums = g.colsum != nullptr && blockIdx.y == 0;
+  float* const as = sm;
+  float* const bs = sm + 2 * kTk * kGemmPitch;
+  // Element t of this thread in a slice: (row ar + t dr, k ka + t dk) of
+  // op(A), (column bc + t dc, k kb + t dk2) of op(B); the fast index is the
+  // contiguous one, so a warp reads whole 64- or 128-byte pieces.
+  constexpr int E = kTile * kTk / kGemmThreads;
+  constexpr int adr = TA ? 0 : kGemmThreads / kTk, adk = TA ? kGemmThreads / kTile : 0;
+  constexpr int bdc = TB ? kGemmThreads / kTk : 0, bdk = TB ? 0 : kGemmThreads / kTile;
+  const int ar = TA ? (tid & 63) : (tid >> 4), ka = TA ? (tid >> 6) : (tid & 15);
+  const int bc = TB ? (tid >> 4) : (tid & 63), kb = TB ? (tid & 15) : (tid >> 6);
+  const float* pa = g.a + (TA ? size_t(q0 * kTk + ka) * g.lda + row0 + ar
+                              : size_t(row0 + ar) * g.lda + q0 * kTk + ka);
+  const float* pb = g.b + (TB ? size_t(col0 + bc) * g.ldb + q0 * kTk + kb
+                              : size_t(q0 * kTk + kb) * g.ldb + col0 + bc);
+  const size_t astep = TA ? size_t(adk) * g.lda : size_t(adr) * g.lda;
+  const size_t bstep = TB ? size_t(bdc) * g.ldb : size_t(bdk) * g.ldb;
+  float ra[E], rb[E];
+  auto fetch = [&](int q) {
+    const int k0 = q * kTk;
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+      const bool va = row0 + ar + t * adr < g.M && k0 + ka + t * adk < g.K;
+      ra[t] = va ? pa[t * astep] : 0.0f;
+      const bool vb = col0 + bc + t * bdc < g.N && k0 + kb + t * bdk < g.K;
+      rb[t] = vb ? pb[t * bstep] : 0.0f;
+    }
+    pa += TA ? size_t(kTk) * g.lda : size_t(kTk);
+    pb += TB ? size_t(kTk) : size_t(kTk) * g.ldb;
+  };
+  auto put = [&](int buf) {
+    float* a0 = as + (buf * kTk + ka) * kGemmPitch + ar;
+    float* b0 = bs + (buf * kTk + kb) * kGemmPitch + bc;
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+      a0[t * (adk * kGemmPitch + adr)] = ra[t];
+      b0[t * (bdk * kGemmPitch + bdc)] = rb[t];
+    }
+  };
   float acc[4][4];
+  float csum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  for (int k0 = 0; k0 < K; k0 += kTk) {
-    // 64 x 16 elements of each operand, 4 per thread.
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int e = tid + t * kGemmThreads;  // 0 .. 1023
-      int r, kk;
-      if (ta) {  // consecutive threads walk r (contiguous in A)
-        r = e & 63;
-        kk = e >> 6;
-      } else {   // consecutive threads walk k (contiguous in A)
-        kk = e & 15;
-        r = e >> 4;
-      }
-      const int gr = row0 + r, gk = k0 + kk;
-      float v = 0.0f;
-      if (gr < M && gk < K) v = ta ? a[size_t(gk) * lda + gr] : a[size_t(gr) * lda + gk];
-      as[kk][r] = v;
-      int cc, kb;
-      if (tb) {
-        kb = e & 15;
-        cc = e >> 4;
-      } else {
-        cc = e & 63;
-        kb = e >> 6;
-      }
-      const int gc = col0 + cc, gkb = k0 + kb;
-      float w = 0.0f;
-      if (gc < N && gkb < K) w = tb ? b[size_t(gc) * ldb + gkb] : b[size_t(gkb) * ldb + gc];
-      bs[kb][cc] = w;
-    }
-    __syncthreads();
+  if (q0 < q1) {
+    fetch(q0);
+    put(0);
+  }
+  __syncthreads();
+  for (int q = q0; q < q1; ++q) {
+    const int buf = (q - q0) & 1;
+    if (q + 1 < q1) fetch(q + 1);
+    const float* sa = as + buf * kTk * kGemmPitch + ty * 4;
+    const float* sb = bs + buf * kTk * kGemmPitch + tx * 4;
 #pragma unroll
     for (int kk = 0; kk < kTk; ++kk) {
-      const float4 av = *reinterpret_cast<const float4*>(&as[kk][ty * 4]);
-      const float4 bv = *reinterpret_cast<const float4*>(&bs[kk][tx * 4]);
-      const float ar[4] = {av.x, av.y, av.z, av.w};
+      const float4 a0 = *reinterpret_cast<const float4*>(sa + kk * kGemmPitch);
+      const float4 bv = *reinterpret_cast<const float4*>(sb + kk * kGemmPitch);
+      const float av[4] = {a0.x, a0.y, a0.z, a0.w};
       const float br[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], br[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], br[j], acc[i][j]);
+      if (sums) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) csum[j] += br[j];
+      }
     }
+    // The other buffer's readers passed the barrier that ended slice q - 1.
+    if (q + 1 < q1) put(buf ^ 1);
     __syncthreads();
   }
+  // The partial tile (and column sums) into shared memory, summed over the
+  // cluster, then the epilogue row by row (coalesced stores).
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = row0 + ty * 4 + i;
-    if (r >= M) continue;
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4*>(&sm[(ty * 4 + i) * kTile + tx * 4]) =
+        make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  if (sums && ty == 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int cc = col0 + tx * 4 + j;
-      if (cc >= N) continue;
-      float v = alpha * acc[i][j];
-      if (beta != 0.0f) v = fmaf(beta, c[size_t(r) * ldc + cc], v);
-      if (bias != nullptr) v += bias[cc];
-      if (relu) v = fmaxf(v, 0.0f);
-      c[size_t(r) * ldc + cc] = v;
+    for (int j = 0; j < 4; ++j) sm[kTile * kTile + tx * 4 + j] = csum[j];
+  }
+  if (parts > 1) {
+    cg::this_cluster().sync();
+  } else {
+    __syncthreads();
+  }
+  auto total = [&](int idx) {
+    if (parts == 1) return sm[idx];
+    float v = 0.0f;
+    for (int p = 0; p < parts; ++p) v += cg::this_cluster().map_shared_rank(sm, p)[idx];
+    return v;
+  };
+  const int rows = kTile / parts;  // parts is a power of two, at most 16
+  double lacc = 0.0;
+  for (int e = tid; e < rows * kTile; e += kGemmThreads) {
+    const int rl = part * rows + (e >> 6), cl = e & 63;
+    const int r = row0 + rl, cc = col0 + cl;
+    if (r >= g.M || cc >= g.N) continue;
+    const size_t o = size_t(r) * g.ldc + cc;
+    float v = g.alpha * total(rl * kTile + cl);
+    if (g.beta != 0.0f) v = fmaf(g.beta, g.c[o], v);
+    if (g.bias != nullptr) v += g.bias[cc];
+    if (g.relu) v = fmaxf(v, 0.0f);
+    if (g.mask != nullptr && !(g.mask[o] > 0.0f)) v = 0.0f;
+    g.c[o] = v;
+    if (g.dy != nullptr) {
+      const float d = v - g.target[o];
+      g.dy[o] = g.dscale * d;
+      lacc += double(d) * double(d);
     }
   }
+  if (sums && part == 0 && tid < kTile && col0 + tid < g.N)
+    g.colsum[col0 + tid] = total(kTile * kTile + tid);
+  if (g.dy != nullptr) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) lacc += __shfl_xor_sync(0xffffffffu, lacc, off);
+    if ((tid & 31) == 0) lpart[tid >> 5] = lacc;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kGemmThreads / 32; ++w) lacc += lpart[w];
+      atomicAdd(g.loss, lacc);
+    }
+  }
+  if (parts > 1) cg::this_cluster().sync();  // peers may still read this CTA's partial
+}
+
+// The CTAs that share a tile's K: enough to give every SM about two, each
+// with at least four slices.  The training step of a 32-256-256-11000 network
+// at batch 256 (forward_loss + backward, 8 launches) takes 275 us against
+// 1539 us with one CTA per tile and separate passes for the error, the masks
+// and the bias gradients (14 launches); its 4.4 GFLOP take 60 us at the FP32
+// peak.  The three 11000-wide products take 60-92 us each, bound by the
+// issue slots of the 4 x 4 tiles (FMA pipe half busy); 8 x 4 tiles with 128
+// threads measured 292 us for the step, a four-stage cp.async ring 280 us.
+static int gemm_split(int M, int N, int K) {
+  const int tiles = ((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
+  const int slices = (K + kTk - 1) / kTk;
+  int s = 1;
+  while (s < kGemmMaxSplit && 2 * s * tiles <= 2 * 148 && slices >= 4 * 2 * s) s *= 2;
+  return s;
+}
+
+template <bool TA, bool TB>
+static int launch_gemm_as(const GemmArgs& g, cudaStream_t stream) {
+  const int split = gemm_split(g.M, g.N, g.K);
+  if (split > 8) {  // beyond the portable cluster size
+    const int rc = cuda_check(
+        cudaFuncSetAttribute(gemm_kernel<TA, TB>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                             1),
+        "cudaFuncSetAttribute(gemm_kernel)");
+    if (rc) return rc;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((g.N + kTile - 1) / kTile, (g.M + kTile - 1) / kTile, split);
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = split;
+  cfg.attrs = at;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  return cuda_check(cudaLaunchKernelEx(&cfg, gemm_kernel<TA, TB>, g), "gemm_kernel launch");
+}
+
+static int launch_gemm(const GemmArgs& g, bool ta, bool tb, cudaStream_t stream) {
+  if (g.M == 0 || g.N == 0) return QTQP_OK;
+  if (ta) return tb ? launch_gemm_as<true, true>(g, stream) : launch_gemm_as<true, false>(g, stream);
+  return tb ? launch_gemm_as<false, true>(g, stream) : launch_gemm_as<false, false>(g, stream);
 }
 
 __global__ void relu_grad_kernel(float* __restrict__ dh, const float* __restrict__ h,
@@ -228,11 +375,105 @@ extern "C" int qtqp_mlp_gemm(int32_t M, int32_t N, int32_t K, float alpha, const
   if (M < 0 || N < 0 || K < 0 || d_a == nullptr || d_b == nullptr || d_c == nullptr ||
       ldc < N || lda < (trans_a ? M : K) || ldb < (trans_b ? K : N))
     return fail(QTQP_ERR_BAD_ARG, "qtqp_mlp_gemm: bad sizes, leading dimensions or pointers");
-  if (M == 0 || N == 0) return QTQP_OK;
-  dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  gemm_kernel<<<grid, kGemmThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      M, N, K, alpha, d_a, lda, trans_a, d_b, ldb, trans_b, beta, d_c, ldc, d_bias, relu);
-  return cuda_check(cudaGetLastError(), "gemm_kernel launch");
+  GemmArgs g = {};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.alpha = alpha;
+  g.a = d_a;
+  g.lda = lda;
+  g.b = d_b;
+  g.ldb = ldb;
+  g.beta = beta;
+  g.c = d_c;
+  g.ldc = ldc;
+  g.bias = d_bias;
+  g.relu = relu;
+  return launch_gemm(g, trans_a != 0, trans_b != 0, static_cast<cudaStream_t>(stream));
+}
+
+// The network of one training step: the layer sizes dim -> hidden -> hidden
+// -> out and a batch of rows.
+static int step_args(const qtqp_mlp_step* s, const char* who) {
+  if (s == nullptr || s->batch < 1 || s->dim < 1 || s->hidden < 1 || s->out < 1)
+    return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": null step or sizes below 1");
+  for (const void* p : {(const void*)s->x, (const void*)s->target, (const void*)s->w1,
+                        (const void*)s->b1, (const void*)s->w2, (const void*)s->b2,
+                        (const void*)s->w3, (const void*)s->b3, (const void*)s->h1,
+                        (const void*)s->h2, (const void*)s->y, (const void*)s->dy,
+                        (const void*)s->dh1, (const void*)s->dh2, (const void*)s->g1,
+                        (const void*)s->gb1, (const void*)s->g2, (const void*)s->gb2,
+                        (const void*)s->g3, (const void*)s->gb3, (const void*)s->loss})
+    if (p == nullptr) return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": null pointer");
+  return QTQP_OK;
+}
+
+static GemmArgs gemm_of(int M, int N, int K, const float* a, int lda, const float* b, int ldb,
+                        float* c) {
+  GemmArgs g = {};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.alpha = 1.0f;
+  g.a = a;
+  g.lda = lda;
+  g.b = b;
+  g.ldb = ldb;
+  g.c = c;
+  g.ldc = N;
+  return g;
+}
+
+// Forward pass with the squared error and its gradient formed in the last
+// product's epilogue: three launches (the error and gradient were a fourth
+// pass over y and the target).
+extern "C" int qtqp_mlp_forward_loss(const qtqp_mlp_step* s, void* stream) {
+  int rc = step_args(s, "qtqp_mlp_forward_loss");
+  if (rc) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  rc = cuda_check(cudaMemsetAsync(s->loss, 0, sizeof(double), st), "cudaMemsetAsync");
+  if (rc) return rc;
+  const int B = s->batch, H = s->hidden;
+  GemmArgs g = gemm_of(B, H, s->dim, s->x, s->dim, s->w1, H, s->h1);
+  g.bias = s->b1;
+  g.relu = 1;
+  if ((rc = launch_gemm(g, false, false, st))) return rc;
+  g = gemm_of(B, H, H, s->h1, H, s->w2, H, s->h2);
+  g.bias = s->b2;
+  g.relu = 1;
+  if ((rc = launch_gemm(g, false, false, st))) return rc;
+  g = gemm_of(B, s->out, H, s->h2, H, s->w3, s->out, s->y);
+  g.bias = s->b3;
+  g.target = s->target;
+  g.dy = s->dy;
+  g.dscale = 2.0f / float(int64_t(B) * s->out);
+  g.loss = s->loss;
+  return launch_gemm(g, false, false, st);
+}
+
+// Backward pass from dy: five launches.  The weight gradients' products also
+// give the bias gradients (the column sums of their right operand), and the
+// hidden gradients' products apply the ReLU mask as they store.
+extern "C" int qtqp_mlp_backward(const qtqp_mlp_step* s, void* stream) {
+  int rc = step_args(s, "qtqp_mlp_backward");
+  if (rc) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int B = s->batch, H = s->hidden, out = s->out;
+  GemmArgs g = gemm_of(H, out, B, s->h2, H, s->dy, out, s->g3);  // dW3 = H2^T dY
+  g.colsum = s->gb3;
+  if ((rc = launch_gemm(g, true, false, st))) return rc;
+  g = gemm_of(B, H, out, s->dy, out, s->w3, out, s->dh2);  // dH2 = dY W3^T
+  g.mask = s->h2;
+  if ((rc = launch_gemm(g, false, true, st))) return rc;
+  g = gemm_of(H, H, B, s->h1, H, s->dh2, H, s->g2);  // dW2 = H1^T dH2
+  g.colsum = s->gb2;
+  if ((rc = launch_gemm(g, true, false, st))) return rc;
+  g = gemm_of(B, H, H, s->dh2, H, s->w2, H, s->dh1);  // dH1 = dH2 W2^T
+  g.mask = s->h1;
+  if ((rc = launch_gemm(g, false, true, st))) return rc;
+  g = gemm_of(s->dim, H, B, s->x, s->dim, s->dh1, H, s->g1);  // dW1 = X^T dH1
+  g.colsum = s->gb1;
+  return launch_gemm(g, true, false, st);
 }
 
 extern "C" int qtqp_mlp_relu_grad(float* d_dh, const float* d_h, int64_t count, void* stream) {

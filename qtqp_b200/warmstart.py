@@ -22,6 +22,7 @@ next layer's BF16 input); training keeps FP32 weights and gradients.
 
 from __future__ import annotations
 
+import ctypes
 import dataclasses
 
 import numpy as np
@@ -161,25 +162,17 @@ class WarmStartMLP:
     dh1 = dh1 if dh1 is not None else torch.empty((batch, self.hidden), **f32)
     if loss_buf is None:
       loss_buf = torch.zeros(1, dtype=torch.float64, device=self.device)
-    h1, h2, y = self._forward(xb, batch)
-    _lib.check(lib.qtqp_mlp_mse_grad(y.data_ptr(), tb.data_ptr(), y.numel(), dy.data_ptr(),
-                                     loss_buf.data_ptr(), st))
+    h1 = torch.empty((batch, self.hidden), **f32)
+    h2 = torch.empty_like(h1)
+    y = torch.empty((batch, self.out), **f32)
+    step = _lib.MlpStep(batch, self.dim, self.hidden, self.out, *(t.data_ptr() for t in (
+        xb, tb, *self.params, h1, h2, y, dy, dh1, dh2, *self.grads, loss_buf)))
+    _lib.check(lib.qtqp_mlp_forward_loss(ctypes.byref(step), st))
     if hinge_weight > 0.0 and self.m > self.z:
       _lib.check(lib.qtqp_mlp_hinge_grad(y.data_ptr(), tb.data_ptr(), batch, self.out,
                                          self.n + self.z, zero.data_ptr(), hinge_weight,
                                          hinge_margin, dy.data_ptr(), loss_buf.data_ptr(), st))
-    _, _, w2, _, w3, _ = self.params
-    g1, gb1, g2, gb2, g3, gb3 = self.grads
-    self._gemm(h2, dy, g3, self.hidden, self.out, batch, ta=1)        # dW3 = H2^T dY
-    _lib.check(lib.qtqp_mlp_colsum(dy.data_ptr(), batch, self.out, gb3.data_ptr(), st))
-    self._gemm(dy, w3, dh2, batch, self.hidden, self.out, tb=1)      # dH2 = dY W3^T
-    _lib.check(lib.qtqp_mlp_relu_grad(dh2.data_ptr(), h2.data_ptr(), dh2.numel(), st))
-    self._gemm(h1, dh2, g2, self.hidden, self.hidden, batch, ta=1)    # dW2 = H1^T dH2
-    _lib.check(lib.qtqp_mlp_colsum(dh2.data_ptr(), batch, self.hidden, gb2.data_ptr(), st))
-    self._gemm(dh2, w2, dh1, batch, self.hidden, self.hidden, tb=1)  # dH1 = dH2 W2^T
-    _lib.check(lib.qtqp_mlp_relu_grad(dh1.data_ptr(), h1.data_ptr(), dh1.numel(), st))
-    self._gemm(xb, dh1, g1, self.dim, self.hidden, batch, ta=1)       # dW1 = X^T dH1
-    _lib.check(lib.qtqp_mlp_colsum(dh1.data_ptr(), batch, self.hidden, gb1.data_ptr(), st))
+    _lib.check(lib.qtqp_mlp_backward(ctypes.byref(step), st))
     return y
 
   # -- public ----------------------------------------------------------------
