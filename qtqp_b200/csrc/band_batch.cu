@@ -8,7 +8,14 @@
 
 namespace qtqp {
 
-constexpr int kBandThreads = 128;
+// Threads per block: 512 while every QP gets an SM of its own, 256 (two
+// blocks per SM) for more QPs than SMs.  One set of 148 T = 50 MPC QPs takes
+// 545 ms with 512 threads and 906 ms with 256 (another set 162 ms, against
+// 497 ms with 128 threads, a thread per Gram column and 8-column solve
+// blocks): the sparse products and the window updates are latency-bound and
+// spread over the threads.
+constexpr int kBandThreadsWide = 512;
+constexpr int kBandThreads = 256;
 constexpr size_t kBandHeader = 256;
 constexpr int kBandMaxBlocksPerSm = 8;
 
@@ -36,8 +43,9 @@ struct BandParams {
   qtqp_options opt;
 };
 
-__global__ void __launch_bounds__(kBandThreads) band_batch_kernel(const BandParams p) {
-  __shared__ double red[2 * (kBandThreads / 32) * kRedMax];
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) band_batch_kernel(const BandParams p) {
+  __shared__ double red[2 * (NT / 32) * kRedMax];
   extern __shared__ double bwin[];  // window of the banded factorisation (win_bytes)
   __shared__ qtqp_options sopt;
   __shared__ int next_idx;
@@ -49,7 +57,7 @@ __global__ void __launch_bounds__(kBandThreads) band_batch_kernel(const BandPara
   while (idx < p.count) {
     const int id = p.order[idx];
     const qtqp_band_instance d = p.inst[id];
-    Ipm<kBandThreads, kFmtBand> s;
+    Ipm<NT, kFmtBand> s;
     s.bind_band(d.n, d.m, d.bw, d.nnz_a, d.nnz_p, slot);
     s.z = d.z;
     s.has_p = d.has_p != 0;
@@ -68,10 +76,10 @@ __global__ void __launch_bounds__(kBandThreads) band_batch_kernel(const BandPara
     s.red = red;
     s.phase = 0;
     s.o = &sopt;
-    s.bwin = (p.win_bytes > 0 && d.bw <= kBandWinMaxBw &&
-              band_win_bytes(d.bw, kBandThreads) <= p.win_bytes)
+    s.bwin = (p.win_bytes > 0 && d.bw <= kBandWinMaxBw && band_win_bytes(d.bw, NT) <= p.win_bytes)
                  ? bwin
                  : nullptr;
+    s.bwin_bytes = p.win_bytes;
     double* st = p.stats ? reinterpret_cast<double*>(p.stats + d.st_off) : nullptr;
     if (p.warm_act != nullptr) {
       s.solve(p.results + id, st, p.x_pool + d.n_off, p.y_pool + d.m_off, p.s_pool + d.m_off,
@@ -84,6 +92,25 @@ __global__ void __launch_bounds__(kBandThreads) band_batch_kernel(const BandPara
     __syncthreads();
     idx = next_idx;
   }
+}
+
+template <int NT>
+static int launch_band(BandParams& p, int slots, cudaStream_t st) {
+  auto kern = band_batch_kernel<NT>;
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           int(p.win_bytes)),
+                      "cudaFuncSetAttribute(band_batch_kernel)");
+  if (rc) return rc;
+  rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, p.win_bytes),
+                  "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+  if (rc) return rc;
+  const int grid = std::max(1, std::min({p.count, slots, sms * std::max(per_sm, 1)}));
+  p.num_slots = grid;
+  kern<<<grid, NT, p.win_bytes, st>>>(p);
+  return cuda_check(cudaGetLastError(), "band_batch_kernel launch");
 }
 
 static double band_cost(const qtqp_band_instance& d) {
@@ -116,17 +143,18 @@ extern "C" int qtqp_band_batch_plan(qtqp_band_instance* h_inst, int32_t count,
   std::copy(ord.begin(), ord.end(), h_order);
   const int sms = num_sms > 0 ? num_sms : 148;
   const int slots = std::max(1, std::min(count, sms * kBandMaxBlocksPerSm));
+  const int nt = count <= sms ? kBandThreadsWide : kBandThreads;
   size_t win = 0;  // the widest band that still fits the shared-memory window
   for (int i = 0; i < count; ++i)
     if (h_inst[i].bw <= kBandWinMaxBw)
-      win = std::max(win, band_win_bytes(std::min(h_inst[i].bw, h_inst[i].n - 1), kBandThreads));
+      win = std::max(win, band_win_bytes(std::min(h_inst[i].bw, h_inst[i].n - 1), nt));
   *plan = qtqp_batch_plan{};
   if (count == 0) return QTQP_OK;
   plan->num_groups = 1;
   qtqp_launch_group& g = plan->groups[0];
   g.begin = 0;
   g.count = count;
-  g.block_threads = kBandThreads;
+  g.block_threads = nt;
   g.smem_bytes = int32_t(win);
   g.slots = slots;
   g.slot_off = kBandHeader;
@@ -154,6 +182,9 @@ extern "C" int qtqp_band_batch_solve(const qtqp_band_instance* d_inst, const int
       d_s_pool == nullptr || d_results == nullptr || d_workspace == nullptr)
     return fail(QTQP_ERR_BAD_ARG, "qtqp_band_batch_solve: null argument");
   const qtqp_launch_group& G = plan->groups[0];
+  if (G.block_threads != kBandThreadsWide && G.block_threads != kBandThreads)
+    return fail(QTQP_ERR_BAD_ARG, "qtqp_band_batch_solve: the plan's block_threads must be 256 "
+                                  "or 512");
   if (G.slots < 1 || workspace_bytes < plan->workspace_bytes ||
       plan->workspace_bytes < G.slot_off + size_t(G.slots) * G.slot_bytes)
     return fail(QTQP_ERR_BAD_ARG, "qtqp_band_batch_solve: workspace smaller than the plan's");
@@ -166,18 +197,6 @@ extern "C" int qtqp_band_batch_solve(const qtqp_band_instance* d_inst, const int
     return fail(QTQP_ERR_BAD_ARG, "qtqp_band_batch_solve: warm_corrections must be in [0, 64]");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc = cuda_check(cudaMemsetAsync(d_workspace, 0, kBandHeader, st), "cudaMemsetAsync");
-  if (rc) return rc;
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const size_t win = size_t(std::max(G.smem_bytes, 0));
-  rc = cuda_check(cudaFuncSetAttribute(band_batch_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(win)),
-                  "cudaFuncSetAttribute(band_batch_kernel)");
-  if (rc) return rc;
-  rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, band_batch_kernel,
-                                                                kBandThreads, win),
-                  "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
   if (rc) return rc;
   BandParams p;
   p.inst = d_inst;
@@ -195,13 +214,11 @@ extern "C" int qtqp_band_batch_solve(const qtqp_band_instance* d_inst, const int
   p.slots = static_cast<char*>(d_workspace) + G.slot_off;
   p.slot_bytes = G.slot_bytes;
   p.counter = static_cast<int*>(d_workspace);
-  p.win_bytes = win;
+  p.win_bytes = size_t(std::max(G.smem_bytes, 0));
   p.warm_x = d_warm_x;
   p.warm_y = d_warm_y;
   p.warm_act = d_warm_active;
   p.opt = *opt;
-  const int grid = std::max(1, std::min({G.count, G.slots, sms * std::max(per_sm, 1)}));
-  p.num_slots = grid;
-  band_batch_kernel<<<grid, kBandThreads, win, st>>>(p);
-  return cuda_check(cudaGetLastError(), "band_batch_kernel launch");
+  return G.block_threads == kBandThreadsWide ? launch_band<kBandThreadsWide>(p, G.slots, st)
+                                             : launch_band<kBandThreads>(p, G.slots, st);
 }

@@ -76,7 +76,7 @@ static int check_inst(const qtqp_band_instance* h, int parts, const char* who) {
       d.nnz_a < 0 || d.nnz_p < 0)
     return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": needs n >= 2, m >= 1, 0 <= z < m, "
                                                      "1 <= bw < n");
-  if (d.bw > kBandWinMaxBw || band_grid_smem_need(d.bw) > kBandGridSmemCap)
+  if (d.bw > kBandWinMaxBw || band_grid_smem_bytes(d.bw) > kBandGridSmemCap)
     return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": half-bandwidth " + std::to_string(d.bw) +
                                       " is too wide for the partitioned factorisation");
   if (parts < 1 || parts > kBandGridBlocks || parts > band_grid_max_parts(d.n, d.bw))

@@ -81,29 +81,20 @@ __host__ __device__ inline int band_grid_max_parts(int n, int bw) {
 __host__ __device__ inline int sep_pitch(int bw) { return bw | 1; }
 
 // Dynamic shared memory of one block (sized for FP64): the largest of the
-// band window (band_chol_window_range), the spike window, the products'
-// staging, the separator reduction, and the solve rings; plus the
-// per-thread Gram columns when they also fit.
-__host__ __device__ inline size_t band_grid_smem_need(int bw) {
+// band window, solves and Gram columns (band_win_bytes), the spike window, the
+// products' staging, the separator reduction, and the solves' extra scratch.
+__host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
   const size_t e = sizeof(double);
-  const size_t B = size_t(bw) + 2;
-  size_t need = ((B * B * e + 7) & ~size_t(7)) + size_t(bw) * (bw + 1) / 2 * 4;
-  if (band_panel_bytes(bw) > need) need = band_panel_bytes(bw);
+  size_t need = band_win_bytes(bw, kGridBT);
   const size_t spike = (size_t(bw) + 1) * bw * e + 256 * e;
   const size_t prod = size_t(bw) * bw * e + 32 * 4 * ((size_t(bw) + 3) / 4) * e;
   const size_t chain = (2 * (size_t(bw) * sep_pitch(bw) + 4) + 3 * 128 + 256 + 2 * 16) * e;
-  const size_t solve = (kBandSolveElems + 512) * e;
+  const size_t solve = (band_solve_elems(bw) + 512) * e;
   if (spike > need) need = spike;
   if (prod > need) need = prod;
   if (chain > need) need = chain;
   if (solve > need) need = solve;
   return (need + 15) & ~size_t(15);
-}
-__host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
-  size_t need = band_grid_smem_need(bw);
-  const size_t cols = size_t(kGridBT) * (size_t(bw) + 1) * sizeof(double);
-  if (cols > need && cols <= kBandGridSmemCap) need = cols;
-  return need;
 }
 
 // Global workspace of the grid solve: barrier / reduction state, the
@@ -625,9 +616,7 @@ __device__ int bandp_factorize(S& s) {
   const BandParts bp(s.n, bw, s.nparts);
   volatile int* info = s.linfo;
   if (s.tid == 0) *info = 0;
-  const bool smem_cols = size_t(kGridBT) * (size_t(bw) + 1) * sizeof(T) <= s.bwin_bytes;
-  s.template band_gram<T>(smem_cols ? reinterpret_cast<T*>(s.bwin) + size_t(threadIdx.x) * (bw + 1)
-                                    : nullptr);
+  s.template band_gram<T>(reinterpret_cast<T*>(s.bwin));
   QTQP_TOC(kPhGram);
   QTQP_RETIC();
   const int k = blockIdx.x;
@@ -644,6 +633,9 @@ __device__ int bandp_factorize(S& s) {
       bandp_spike<T>(s, bp, k);
       bandp_products<T>(s, bp, k);
     }
+    // The spike has used the factor's diagonal blocks; the solves use their
+    // inverses.
+    if (bad == 0) s.template band_invert_diag<T, kGridBT>(lo, li);
   }
   s.sync();
   QTQP_TOC(kPhBpInterior);
@@ -703,7 +695,7 @@ __device__ void bandp_solve(S& s, T* v, T* w) {
             warp = lt >> 5;
   constexpr int kNW = kGridBT / 32;
   // Scratch after the blocked band solves' window and staging.
-  T* scr = reinterpret_cast<T*>(s.bwin) + kBandSolveElems;
+  T* scr = reinterpret_cast<T*>(s.bwin) + band_solve_elems(bw);
   QTQP_TIC();
   // Forward per interior; the spike term W_L^T y of interior k for
   // separator k - 1.

@@ -283,6 +283,13 @@ __device__ __forceinline__ void cp_async4z(void* dst, const void* src, bool vali
                "l"(src), "r"(valid ? 4 : 0)
                : "memory");
 }
+// 16 bytes, both addresses 16-byte aligned.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
 // Element copy of T (double or float), zero-filled when !valid.
 template <typename T>
 __device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool valid) {

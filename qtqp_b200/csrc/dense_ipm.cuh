@@ -102,31 +102,41 @@ __host__ __device__ inline BandLayout plan_band_layout(int n, int m, int bw, int
 }
 
 // Shared-memory window of the banded factorisation / solves: bands up to
-// kBandWinMaxBw use it (the (bw+2)^2 window, the per-thread Gram columns and
-// the 128-slot solve window must fit).
+// kBandWinMaxBw use it (a panel has one row per thread of a 256-thread block;
+// 190 window slots of the solves are live at once, of 256).
 constexpr int kBandWinMaxBw = 126;
-// Shared-memory elements reserved for the blocked band solves: 256 window
-// slots, two staged blocks of factor entries (forward: 2 x 8 x (bw + 1);
-// backward: 2 x (bw + 8) x 8, bw <= 126) and the block's 8 values.
-constexpr int kBandSolveElems = 256 + 2 * (126 + 8) * 8 + 16;
+// Columns per block of the blocked band solves: the largest power of two up
+// to 32 whose inverted lower-triangular diagonal block fits inside the band.
+__host__ __device__ inline int band_solve_block(int bw) {
+  int kb = 1;
+  while (kb < 32 && 2 * kb <= bw + 1) kb *= 2;
+  return kb;
+}
+// Shared-memory elements of the blocked band solves: 256 window slots, two
+// staged blocks of factor columns and the block's values.
+__host__ __device__ inline size_t band_solve_elems(int bw) {
+  return 256 + 2 * size_t(band_solve_block(bw)) * (size_t(bw) + 1) + 32;
+}
 constexpr int kBandPanel = 8;  // columns per panel of the blocked band Cholesky
 // Shared memory of the blocked band Cholesky (band_chol_panel_range): the
-// circular (bw + kBandPanel)^2 window, the panel rows, the publish slots
-// and the 16-bit trailing-update offsets.
+// circular (bw + kBandPanel)^2 window, the panel rows and the list of the
+// window's lower 8 x 8 tiles.
 __host__ __device__ inline size_t band_panel_bytes(int bw) {
-  const size_t B = size_t(bw) + kBandPanel;
-  const size_t elems = B * B + (size_t(bw) + kBandPanel) * (kBandPanel + 1) + 2 * kBandPanel;
-  return elems * sizeof(double) + size_t(bw) * (size_t(bw) + 1) / 2 * sizeof(uint16_t);
+  const size_t B = size_t(bw) + kBandPanel, nt8 = (size_t(bw) + 7) / 8;
+  return (B * B + B * (kBandPanel + 1)) * sizeof(double) +
+         nt8 * (nt8 + 1) / 2 * sizeof(uint16_t);
 }
+// The shared memory a band needs in a block of nt threads: the Cholesky, the
+// solves, one Gram column per warp, one diagonal block to invert.
 __host__ __device__ inline size_t band_win_bytes(int bw, int nt) {
-  const size_t b2 = (size_t(bw) + 2) * (size_t(bw) + 2) * sizeof(double);
-  const size_t pairs = size_t(bw) * (size_t(bw) + 1) / 2 * sizeof(uint32_t);
-  const size_t cols = size_t(nt) * (size_t(bw) + 1) * sizeof(double);
-  const size_t solve = size_t(kBandSolveElems) * sizeof(double);
-  size_t e = b2 + pairs;
-  if (bw + kBandPanel <= nt && band_panel_bytes(bw) > e) e = band_panel_bytes(bw);
+  size_t e = band_panel_bytes(bw);
+  const size_t kb = band_solve_block(bw);
+  const size_t cols = size_t(nt / 32) * (size_t(bw) + 1) * sizeof(double);
+  const size_t solve = band_solve_elems(bw) * sizeof(double);
+  const size_t inv = kb * (kb + 1) * sizeof(double);
   if (cols > e) e = cols;
   if (solve > e) e = solve;
+  if (inv > e) e = inv;
   return (e + 15) & ~size_t(15);
 }
 
@@ -2469,9 +2479,9 @@ struct Ipm {
   // sum_{q0 <= q < q1} val[q] v[voff + idx[q]]: indices and values are
   // loaded 8 at a time, then the 8 gathers, so that several loads are in
   // flight per thread (these sparse dots are latency-bound).
+  template <typename V>
   __device__ __forceinline__ static double sparse_dot(const int* idx, const double* val,
-                                                      const double* v, int voff, int q0,
-                                                      int q1) {
+                                                      const V* v, int voff, int q0, int q1) {
     double t0 = 0.0, t1 = 0.0;
     int q = q0;
     for (; q + 8 <= q1; q += 8) {
@@ -2483,14 +2493,43 @@ struct Ipm {
         aa[e] = val[q + e];
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) xx[e] = v[voff + ii[e]];
+      for (int e = 0; e < 8; ++e) xx[e] = double(v[voff + ii[e]]);
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
         t0 = fma(aa[e], xx[e], t0);
         t1 = fma(aa[e + 1], xx[e + 1], t1);
       }
     }
-    for (; q < q1; ++q) t0 = fma(val[q], v[voff + idx[q]], t0);
+    for (; q < q1; ++q) t0 = fma(val[q], double(v[voff + idx[q]]), t0);
+    return t0 + t1;
+  }
+  // sum_{q0 <= q < q1} val[q] (scale[idx[q]] v[idx[q]]), loaded the same way.
+  __device__ __forceinline__ static double sparse_dot_scaled(const int* idx, const double* val,
+                                                             const double* v,
+                                                             const double* scale, int q0,
+                                                             int q1) {
+    double t0 = 0.0, t1 = 0.0;
+    int q = q0;
+    for (; q + 8 <= q1; q += 8) {
+      int ii[8];
+      double aa[8], xx[8], ss[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        ii[e] = idx[q + e];
+        aa[e] = val[q + e];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        xx[e] = v[ii[e]];
+        ss[e] = scale[ii[e]];
+      }
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        t0 = fma(aa[e], ss[e] * xx[e], t0);
+        t1 = fma(aa[e + 1], ss[e + 1] * xx[e + 1], t1);
+      }
+    }
+    for (; q < q1; ++q) t0 = fma(val[q], scale[idx[q]] * v[idx[q]], t0);
     return t0 + t1;
   }
   // (P_off v)_k for the owner of row k (P symmetric, so row k = column k).
@@ -2507,87 +2546,93 @@ struct Ipm {
   }
 
   // Column j of the Gram matrix G = P_off + diag(Rx) + A^T diag(1/Ry) A,
-  // rows j .. j + bw, into acc[0 .. bw].  The loads of every level are issued
-  // in batches of 8 before they are used (column j's rows and their
-  // scalings, then each row's entries), so that this latency-bound gather
-  // keeps several loads in flight.
+  // rows j .. j + bw, into acc[0 .. bw] (shared memory), by one warp: the
+  // lanes take 32 of the column's rows (index, value, scaling, extent), then
+  // the warp walks those rows, four at a time with their entries' loads
+  // issued together, each lane one or two entries of a row.  The entries of a
+  // row lie in different columns, so the lanes never meet, and every sum runs
+  // over the rows in order.  (A thread per column, its 2700 products of a T =
+  // 50 MPC column one after the other through shared memory, took 5.5 ms per
+  // factorisation of one QP in a 128-thread block.)
   template <typename T>
   __device__ __forceinline__ void band_gram_column(int j, T* acc) const {
     QTQP_BAND_LOCALS;
     const double* reg = vec(kREG);
     const double* wsc = vec(kPW);
-    for (int d = 0; d <= bw; ++d) acc[d] = T(0);
+    const int lane = threadIdx.x & 31;
+    for (int d = lane; d <= bw; d += 32) acc[d] = T(0);
     const int qa = jp[j], qb = jp[j + 1];
-    for (int q0 = qa; q0 < qb; q0 += 8) {
-      int rr[8], r0[8], r1[8];
-      double ww[8], aq[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool ok = q0 + u < qb;
-        rr[u] = ok ? jx[q0 + u] : 0;
-        aq[u] = ok ? at[q0 + u] : 0.0;
+    for (int q0 = qa; q0 < qb; q0 += 32) {
+      const int q = q0 + lane, cnt = min(32, qb - q0);
+      int r0 = 0, r1 = 0;
+      double w = 0.0;
+      T arj = T(0);
+      if (lane < cnt) {
+        const int r = jx[q];
+        w = wsc[n + r];
+        r0 = ip[r];
+        r1 = ip[r + 1];
+        arj = T(at[q] * w);
       }
+      __syncwarp();
+      constexpr int RB = 4;  // rows whose loads are issued together
+      for (int u0 = 0; u0 < cnt; u0 += RB) {
+        int b1[RB], q2[RB], i0[RB], i1[RB];
+        double a0[RB], a1[RB];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool ok = q0 + u < qb;
-        ww[u] = ok ? wsc[n + rr[u]] : 0.0;
-        r0[u] = ok ? ip[rr[u]] : 0;
-        r1[u] = ok ? ip[rr[u] + 1] : 0;
-      }
-#pragma unroll 1
-      for (int u = 0; u < 8 && q0 + u < qb; ++u) {
-        const double w = ww[u];
-        const T arj = T(aq[u] * w);
-        const int q1 = r1[u];
-        int q2 = r0[u];
-        for (; q2 + 8 <= q1; q2 += 8) {
-          int ii[8];
-          double aa[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            ii[e] = ix[q2 + e];
-            aa[e] = av[q2 + e];
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int i = ii[e];
-            if (i >= j && i - j <= bw) acc[i - j] = fma(arj, T(aa[e] * w), acc[i - j]);
-          }
+        for (int v = 0; v < RB; ++v) {
+          const int src = min(u0 + v, 31);
+          q2[v] = __shfl_sync(0xffffffffu, r0, src) + lane;
+          b1[v] = u0 + v < cnt ? __shfl_sync(0xffffffffu, r1, src) : 0;
+          i0[v] = q2[v] < b1[v] ? ix[q2[v]] : -1;
+          a0[v] = q2[v] < b1[v] ? av[q2[v]] : 0.0;
+          i1[v] = q2[v] + 32 < b1[v] ? ix[q2[v] + 32] : -1;
+          a1[v] = q2[v] + 32 < b1[v] ? av[q2[v] + 32] : 0.0;
         }
-        for (; q2 < q1; ++q2) {
-          const int i = ix[q2];
-          if (i >= j && i - j <= bw) acc[i - j] = fma(arj, T(av[q2] * w), acc[i - j]);
+#pragma unroll
+        for (int v = 0; v < RB; ++v) {
+          const int src = min(u0 + v, 31);
+          const double wv = __shfl_sync(0xffffffffu, w, src);
+          const T av_j = __shfl_sync(0xffffffffu, arj, src);
+          const int d0 = i0[v] - j, d1 = i1[v] - j;
+          if (d0 >= 0 && d0 <= bw) acc[d0] = fma(av_j, T(a0[v] * wv), acc[d0]);
+          if (d1 >= 0 && d1 <= bw) acc[d1] = fma(av_j, T(a1[v] * wv), acc[d1]);
+          for (int e = q2[v] + 64; e < b1[v]; e += 32) {
+            const int d = ix[e] - j;
+            if (d >= 0 && d <= bw) acc[d] = fma(av_j, T(av[e] * wv), acc[d]);
+          }
+          __syncwarp();
         }
       }
     }
+    __syncwarp();
     if (has_p) {
-      for (int q = pp[j]; q < pp[j + 1]; ++q) {
+      for (int q = pp[j] + lane; q < pp[j + 1]; q += 32) {
         const int i = px[q];
         if (i > j && i - j <= bw) acc[i - j] = T(pv[q]) + acc[i - j];
       }
+      __syncwarp();
     }
-    acc[0] = T(reg[j]) + acc[0];
+    if (lane == 0) acc[0] = T(reg[j]) + acc[0];
+    __syncwarp();
   }
 
   // The Gram matrix in column band storage (Lb) plus the relative diagonal
-  // jitter of the dense backend.  acc_smem: this thread's column scratch in
-  // shared memory (bw + 1 entries), or null to accumulate in place.
+  // jitter of the dense backend; a warp per column.  acc: the block's
+  // scratch, bw + 1 entries per warp.
   template <typename T>
-  __device__ void band_gram(T* acc_smem) {
-    const int ldl = bw + 1;
+  __device__ void band_gram(T* acc) {
+    const int ldl = bw + 1, lane = threadIdx.x & 31;
     T* L = reinterpret_cast<T*>(Lb);
+    T* wacc = acc + size_t(threadIdx.x >> 5) * ldl;
     double dmax[1] = {0.0};
     double dummy[1] = {0.0};
-    for (int j0 = 0; j0 < n; j0 += NT) {
-      const int j = j0 + tid;
-      if (j < n) {
-        T* col = L + size_t(j) * ldl;
-        T* acc = acc_smem != nullptr ? acc_smem : col;
-        band_gram_column<T>(j, acc);
-        dmax[0] = nanmax(dmax[0], double(acc[0]));
-        if (acc_smem != nullptr)
-          for (int d = 0; d <= bw; ++d) col[d] = acc[d];
-      }
+    for (int j = tid >> 5; j < n; j += NT / 32) {
+      T* col = L + size_t(j) * ldl;
+      band_gram_column<T>(j, wacc);
+      dmax[0] = nanmax(dmax[0], double(wacc[0]));
+      for (int d = lane; d <= bw; d += 32) col[d] = wacc[d];
+      __syncwarp();
     }
     reduce<0, 1>(dummy, dmax);
     const double jit = (sizeof(T) == 8 ? 1e-14 : 2.384185791015625e-07) * dmax[0];
@@ -2596,12 +2641,10 @@ struct Ipm {
   }
 
   // Gram matrix in column band storage, then Cholesky.  With the shared-
-  // memory window (bw <= kBandWinMaxBw): each thread accumulates its Gram
-  // column in shared memory, and the factorisation keeps the active
-  // (bw+2) x (bw+2) part of the band in shared memory (band_chol_window_range).
-  // Otherwise the global-memory variant below runs.  In grid mode the
-  // partitioned factorisation runs (band_grid.cuh).  The diagonal of the
-  // factor keeps 1 / l_kk.
+  // memory window (bw <= kBandWinMaxBw) the blocked factorisation
+  // (band_chol_panel_range), whose diagonal blocks are then inverted for the
+  // solves; otherwise the global-memory variant below runs.  In grid mode the
+  // partitioned factorisation runs (band_grid.cuh).
   template <typename T>
   __device__ int band_factorize() {
     if constexpr (FMT == kFmtSparse) {
@@ -2611,29 +2654,42 @@ struct Ipm {
     } else {
       if (bwin == nullptr) return band_factorize_global<T>();
       QTQP_TIC();
-      band_gram<T>(reinterpret_cast<T*>(bwin) + size_t(tid) * (bw + 1));
+      band_gram<T>(reinterpret_cast<T*>(bwin));
       QTQP_TOC(kPhGram);
       QTQP_RETIC();
-      const int info = bw + kBandPanel <= NT
-                           ? band_chol_panel_range<T, NT>(tid, 0, n, n, nullptr, 0)
-                           : band_chol_window_range<T, NT>(tid, 0, n, n, nullptr, 0);
+      const int info = band_chol_panel_range<T, NT>(tid, 0, n, n, nullptr, 0);
       QTQP_TOC(kPhChol);
+      QTQP_RETIC();
+      if (info == 0) band_invert_diag<T, NT>(0, n);
+      QTQP_TOC(kPhInv);
       return info;
     }
   }
 
-  // Blocked form of band_chol_window_range (same arguments and results):
-  // kBandPanel-column panels.  Each panel is factorised tall-skinny in
-  // registers (thread r holds the panel's entries of row k + r, for the
-  // kBandPanel + bw rows the panel touches; per column the diagonal block's
-  // rows publish their entry, one barrier, then every row scales its entry
-  // by one reciprocal square root and updates the rest of its panel row),
-  // written to the factor, and applied to the active bw x bw window as one
-  // rank-kBandPanel update.  The window is circular with period B = bw +
-  // kBandPanel (lower triangle, shared memory); the kBandPanel rows that
-  // enter it are loaded from the Gram matrix during the panel, and the
-  // window columns left of an entering row's band are zeroed.  Needs
-  // kBandPanel + bw <= BT.
+  // Band Cholesky with the active part of the band in shared memory, over
+  // the principal submatrix of rows / columns [lo, lo + nsub) of which the
+  // first ne columns are eliminated (ne == nsub: the whole factorisation), by
+  // the BT threads of a block (lt: this thread's index), BT >= kBandPanel +
+  // bw.  The diagonal of the factor keeps 1 / l_kk.  tail (when ne < nsub):
+  // the lower triangle of the trailing (nsub-ne)^2 block after the
+  // elimination (the Schur complement of the eliminated columns), row-major
+  // with leading dimension ldt.  Columns before lo are not part of the
+  // submatrix.  Returns 0 or the 1-based global column of the first
+  // non-positive pivot.
+  //
+  // kBandPanel-column panels; the window is circular with period B = bw +
+  // kBandPanel (lower triangle, row-major).  Per panel, two barriers:
+  //  * every thread that holds a row of the panel (kBandPanel + bw rows)
+  //    factors the panel's 8 x 8 diagonal block for itself, in registers, and
+  //    solves its own row with it as it goes, so no barrier lies on the chain
+  //    from column to column (eight barriers and publishes per panel before);
+  //    the finished columns go to global memory and to the panel buffer;
+  //  * the rank-8 update of the window's lower bw x bw part, by 8 x 8 tiles,
+  //    a warp per tile, on the FP64 tensor cores (DMMA; 64 tiles' worth of
+  //    products are 1/6 of the shared-memory reads of a thread per entry).
+  //    The kBandPanel rows that enter the window, loaded from the Gram matrix
+  //    during the panel, are stored, and the columns left of their band
+  //    zeroed.
   template <typename T, int BT>
   __device__ int band_chol_panel_range(int lt, int lo, int nsub, int ne, T* tail, int ldt) {
     constexpr int KP = kBandPanel, PP = KP + 1;
@@ -2641,15 +2697,17 @@ struct Ipm {
     T* L = reinterpret_cast<T*>(Lb) + size_t(lo) * ldl;
     T* W = reinterpret_cast<T*>(bwin);
     T* Pn = W + B * B;
-    T* pub = Pn + (KP + bw) * PP;
-    uint16_t* pairs = reinterpret_cast<uint16_t*>(pub + 2 * KP);
-    const int npairs = bw * (bw + 1) / 2;
-    for (int a = lt; a < bw; a += BT)
-      for (int b = 0; b <= a; ++b) pairs[a * (a + 1) / 2 + b] = uint16_t(a | (b << 8));
+    uint16_t* tiles = reinterpret_cast<uint16_t*>(Pn + B * PP);
+    __shared__ int s_bad;
+    const int nt8 = (bw + 7) >> 3, ntiles = nt8 * (nt8 + 1) / 2;
+    const int lane = lt & 31, warp = lt >> 5, gi = lane >> 2, tg = lane & 3;
+    for (int a = lt; a < nt8; a += BT)
+      for (int b = 0; b <= a; ++b) tiles[a * (a + 1) / 2 + b] = uint16_t(a | (b << 8));
     for (int e = lt; e < B * B; e += BT) {
       const int i = e / B, j = e - i * B;
       W[e] = (j <= i && i - j <= bw && i < nsub) ? L[size_t(j) * ldl + (i - j)] : T(0);
     }
+    if (lt == 0) s_bad = 0;
     group_sync<BT>();
     int bad = 0;
     constexpr int MAXPRE = (KP * 128 + BT - 1) / BT;  // entering entries per thread (bw < 128)
@@ -2671,59 +2729,87 @@ struct Ipm {
         const int r = k + B + e;
         pre[q] = (e < pw && r < nsub) ? L[size_t(r - bw + d) * ldl + (bw - d)] : T(0);
       }
-      T v[KP];
+      if (lt < nr) {
+        // The diagonal block (the same in every thread) and this thread's row.
+        T dg[KP][KP], v[KP];
+        int sc[KP];
 #pragma unroll
-      for (int c = 0; c < KP; ++c)
-        v[c] = (lt < nr && c < pw && c <= lt) ? W[sl(lt) * B + sl(c)] : T(0);
+        for (int c = 0; c < KP; ++c) sc[c] = sl(c);
+        const T* wr = W + sl(lt) * B;
 #pragma unroll
-      for (int c = 0; c < KP; ++c) {
-        if (c < pw) {
-          T* pc = pub + (c & 1) * KP;
-          if (lt >= c && lt < pw) pc[lt] = v[c];
-          group_sync<BT>();
-          const T piv = pc[c];
-          if (!(piv > T(0))) {
-            bad = k + c + 1;
-            break;
-          }
-          const T il = rsqrt(piv);
-          if (lt < nr) {
-            if (lt == c) {
-              v[c] = il;  // the factor keeps 1 / l_cc
-            } else if (lt > c) {
+        for (int a = 0; a < KP; ++a) {
+#pragma unroll
+          for (int c = 0; c <= a; ++c) dg[a][c] = a < pw ? W[sc[a] * B + sc[c]] : T(0);
+          v[a] = (a < pw && a <= lt) ? wr[sc[a]] : T(0);
+        }
+        int f = 0;
+#pragma unroll
+        for (int c = 0; c < KP; ++c) {
+          if (c < pw && f == 0) {
+            const T piv = dg[c][c];
+            if (!(piv > T(0))) {
+              f = k + c + 1;
+            } else {
+              const T il = rsqrt(piv);
               const T lic = v[c] * il;
-              v[c] = lic;
+              v[c] = lt == c ? il : lic;  // the factor keeps 1 / l_cc
 #pragma unroll
-              for (int j = c + 1; j < KP; ++j)
-                if (j < pw) v[j] = fma(-lic, pc[j] * il, v[j]);
+              for (int a = c + 1; a < KP; ++a) dg[a][c] *= il;
+#pragma unroll
+              for (int a = c + 1; a < KP; ++a) {
+                v[a] = fma(-lic, dg[a][c], v[a]);
+#pragma unroll
+                for (int b = c + 1; b <= a; ++b) dg[a][b] = fma(-dg[a][c], dg[b][c], dg[a][b]);
+              }
             }
           }
         }
-      }
-      if (bad) break;
-      if (lt < nr) {
+        if (f != 0) {
+          if (lt == 0) s_bad = f;
+        } else {
 #pragma unroll
-        for (int c = 0; c < KP; ++c)
-          if (c < pw && c <= lt && lt - c <= bw) L[size_t(k + c) * ldl + (lt - c)] = v[c];
-        if (lt >= pw) {
+          for (int c = 0; c < KP; ++c)
+            if (c < pw && c <= lt && lt - c <= bw) L[size_t(k + c) * ldl + (lt - c)] = v[c];
+          if (lt >= pw) {
 #pragma unroll
-          for (int c = 0; c < KP; ++c) Pn[lt * PP + c] = v[c];
+            for (int c = 0; c < KP; ++c) Pn[lt * PP + c] = v[c];
+          }
         }
       }
       group_sync<BT>();
+      bad = s_bad;
+      if (bad) break;
       // Trailing update of the window: rows / columns k + pw .. k + pw + bw - 1.
-      for (int pi = lt; pi < npairs; pi += BT) {
-        const int pr = pairs[pi];
-        const int a = pr & 0xff, b = pr >> 8;
-        const int i = pw + a, j = pw + b;
-        if (k + i < nsub) {
-          const T* ri = Pn + i * PP;
-          const T* rj = Pn + j * PP;
-          T acc = T(0);
+      const int span = min(bw, nsub - k - pw);  // of which these exist
+      for (int t = warp; t < ntiles; t += BT / 32) {
+        const int pr = tiles[t];
+        const int ta = (pr & 0xff) * 8, tb = (pr >> 8) * 8;
+        if (ta >= span) continue;
+        T acc[2] = {T(0), T(0)};
+        const int a = ta + gi, b0 = tb + 2 * tg;
+        if constexpr (sizeof(T) == 8) {
+          const int bj = tb + gi;
+          const T* ra = Pn + (pw + a) * PP + tg;
+          const T* rb = Pn + (pw + bj) * PP + tg;
+          const bool oka = a < span, okb = bj < span;
+          const double a0 = oka ? ra[0] : 0.0, a1 = oka ? ra[4] : 0.0;
+          const double c0 = okb ? rb[0] : 0.0, c1 = okb ? rb[4] : 0.0;
+          dmma_8x8x4(acc, a0, c0);
+          dmma_8x8x4(acc, a1, c1);
+        } else if (a < span) {
+          const T* ra = Pn + (pw + a) * PP;
 #pragma unroll
-          for (int c = 0; c < KP; ++c) acc = fma(ri[c], rj[c], acc);
-          T* w = W + sl(i) * B + sl(j);
-          *w -= acc;
+          for (int e = 0; e < 2; ++e) {
+            if (b0 + e > a) continue;
+            const T* rb = Pn + (pw + b0 + e) * PP;
+#pragma unroll
+            for (int c = 0; c < KP; ++c) acc[e] = fma(ra[c], rb[c], acc[e]);
+          }
+        }
+        if (a < span) {
+          T* wr = W + sl(pw + a) * B;
+          if (b0 <= a) wr[sl(pw + b0)] -= acc[0];
+          if (b0 + 1 <= a) wr[sl(pw + b0 + 1)] -= acc[1];
         }
       }
       // Entering rows: band entries, and zeros left of the band.
@@ -2751,96 +2837,54 @@ struct Ipm {
     return bad == 0 ? 0 : lo + bad;
   }
 
-  // Band Cholesky with the active part of the band in shared memory, over
-  // the principal submatrix of rows / columns [lo, lo + nsub) of which the
-  // first ne columns are eliminated (ne == nsub: the whole factorisation).
-  // Local rows and columns k .. k+bw+1 live in a (bw+2) x (bw+2) window with
-  // circular indices (slot = index mod (bw+2)); step k reads the still-
-  // unscaled column k, writes the finished column k of L to global memory,
-  // updates the window, and stores row k+bw+1 of the Gram matrix (prefetched
-  // into registers during the previous step) into the slots that row k-1
-  // and column k-1 have freed.  One barrier per column.  Columns before lo
-  // are not part of the submatrix.  tail (when ne < nsub): the lower
-  // triangle of the trailing (nsub-ne)^2 block after the elimination (the
-  // Schur complement of the eliminated columns), row-major with leading
-  // dimension ldt.  lt: this thread's index among the BT threads of the
-  // group.  Returns 0 or the 1-based global column of the first
-  // non-positive pivot.
+  // In-place inverse of the diagonal blocks of the factor that the blocked
+  // solves use: band_solve_block(bw) columns each, from column lo on, the
+  // last one shorter.  The inverse of a lower-triangular block is lower
+  // triangular and its last row is at most bw below its first column, so it
+  // takes the block's own place in the band (whose diagonal is that of the
+  // inverse already).  A warp per block, lane c its column c, kept at (c, k)
+  // of the staged block's unused upper triangle: X_rc = -(sum_{c<=k<r} L_rk
+  // X_kc) / l_rr.  As many warps as the shared memory holds blocks.
   template <typename T, int BT>
-  __device__ int band_chol_window_range(int lt, int lo, int nsub, int ne, T* tail, int ldt) {
-    const int bw = this->bw, ldl = bw + 1;
-    T* L = reinterpret_cast<T*>(Lb) + size_t(lo) * ldl;
-    T* W = reinterpret_cast<T*>(bwin);
-    const int B = bw + 2;
-    // Offsets (oi, oj), 1 <= oj <= oi <= bw, of the trailing update relative
-    // to k, the same every step; thread t handles pairs t, t + BT, ...
-    uint32_t* pairs = reinterpret_cast<uint32_t*>(bwin + (size_t(B) * B * sizeof(T) + 7) / 8);
-    const int npairs = bw * (bw + 1) / 2;
-    for (int oi = 1 + lt; oi <= bw; oi += BT)
-      for (int oj = 1; oj <= oi; ++oj) pairs[(oi - 1) * oi / 2 + oj - 1] = uint32_t(oi) | (uint32_t(oj) << 16);
-    // Rows 0 .. min(bw, nsub-1): entries (i, j), j <= i.
-    for (int e = lt; e < B * B; e += BT) {
-      const int i = e / B, j = e - i * B;
-      W[e] = (j <= i && i <= bw && i < nsub) ? L[size_t(j) * ldl + (i - j)] : T(0);
-    }
-    // Prefetch of the row that enters at step k: r = k + bw + 1, entries
-    // (r, j) for j in [r - bw, r]; thread t takes j = r - bw + t.
-    auto fetch = [&](int k) {
-      const int r = k + bw + 1, j = r - bw + lt;
-      return (r < nsub && lt <= bw) ? L[size_t(j) * ldl + (r - j)] : T(0);
-    };
-    T pre = fetch(0);
-    group_sync<BT>();
-    int info = 0;
-    for (int k = 0; k < ne; ++k) {
-      const int ks = k % B;
-      const T d = W[ks * B + ks];
-      if (!(d > T(0))) {
-        info = k + 1;
-        break;
-      }
-      const T il = rsqrt(d), inv_d = il * il;  // no division on this chain
-      const int last = min(nsub - 1, k + bw);
-      auto slot = [&](int i) {  // i % B for i in [k, k + B)
-        const int t = ks + (i - k);
-        return t >= B ? t - B : t;
-      };
-      // Finished column k of L (global); the window keeps it unscaled.
-      for (int i = k + 1 + lt; i <= last; i += BT) L[size_t(k) * ldl + (i - k)] = W[slot(i) * B + ks] * il;
-      if (lt == 0) L[size_t(k) * ldl] = il;
-      // Trailing update: W_ij -= W_ik W_jk / d for k < j <= i <= last.
-      const int span = last - k;
-#pragma unroll 4
-      for (int pi = lt; pi < npairs; pi += BT) {
-        const uint32_t pr = pairs[pi];
-        const int oi = int(pr & 0xffffu), oj = int(pr >> 16);
-        if (oi <= span) {
-          const int is = slot(k + oi), js = slot(k + oj);
-          W[is * B + js] = fma(-W[is * B + ks] * inv_d, W[js * B + ks], W[is * B + js]);
+  __device__ void band_invert_diag(int lo, int ne) {
+    const int bw = this->bw, ldl = bw + 1, KB = band_solve_block(bw), P = KB + 1;
+    if (KB == 1) return;
+    T* L = reinterpret_cast<T*>(Lb);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nw = min(BT / 32, int(bwin_bytes / (size_t(KB) * P * sizeof(T))));
+    const int nblk = (ne + KB - 1) / KB;
+    T* S = reinterpret_cast<T*>(bwin) + size_t(warp) * KB * P;
+    for (int blk = warp; blk < nblk && warp < nw; blk += nw) {
+      const int k0 = lo + blk * KB, pw = min(KB, lo + ne - k0);
+      T* Lk = L + size_t(k0) * ldl;
+#pragma unroll 8
+      for (int c = 0; c < pw; ++c)
+        if (c + lane < pw) S[(c + lane) * P + c] = Lk[size_t(c) * ldl + lane];
+      __syncwarp();
+      const T* U = S + lane * P;
+#pragma unroll 1
+      for (int r = 1; r < pw; ++r) {
+        const T* Sr = S + r * P;
+        T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
+        if (lane < r) {
+          int k = lane;
+          for (; k + 3 < r; k += 4) {
+            a0 = fma(Sr[k], U[k], a0);
+            a1 = fma(Sr[k + 1], U[k + 1], a1);
+            a2 = fma(Sr[k + 2], U[k + 2], a2);
+            a3 = fma(Sr[k + 3], U[k + 3], a3);
+          }
+          for (; k < r; ++k) a0 = fma(Sr[k], U[k], a0);
+          S[lane * P + r] = -((a0 + a1) + (a2 + a3)) * Sr[r];
         }
+        __syncwarp();
       }
-      // Row r = k + bw + 1 enters: row slot (k-1) mod B, column slots of
-      // j in [k+1, r] (never ks; the diagonal lands in column k-1's slot).
-      {
-        const int r = k + bw + 1;
-        if (r < nsub && lt <= bw) {
-          const int rs = ks == 0 ? B - 1 : ks - 1;  // (k - 1) mod B
-          const int j = r - bw + lt;                // in [k + 1, r]
-          W[rs * B + (j - k == B - 1 ? rs : slot(j))] = pre;
-        }
-        pre = fetch(k + 1);
-      }
-      group_sync<BT>();
+#pragma unroll 8
+      for (int c = 0; c < pw; ++c)
+        if (lane > 0 && c + lane < pw) Lk[size_t(c) * ldl + lane] = S[c * P + c + lane];
+      __syncwarp();
     }
     group_sync<BT>();
-    if (tail != nullptr && info == 0) {
-      const int t = nsub - ne;
-      for (int e = lt; e < t * t; e += BT) {
-        const int i = e / t, j = e - i * t;
-        if (j <= i) tail[size_t(i) * ldt + j] = W[((ne + i) % B) * B + (ne + j) % B];
-      }
-    }
-    return info == 0 ? 0 : lo + info;
   }
 
   // Global-memory variant (wide bands): Gram in column band storage, then
@@ -2938,34 +2982,52 @@ struct Ipm {
   }
 
   // Blocked band triangular solves, run by all BT threads of the group (lt:
-  // this thread's index).  Forward: z_k = (v_k - sum_c l_kc z_c) / l_kk for
-  // the columns [lo, lo + ne) into w[k], the rows [lo + ne, R) of v receiving
-  // their updates.  Backward: x_k = (w_k - sum_d l_{k+d,k} x_{k+d}) / l_kk for
-  // k in [lo, hi) into v[k], the rows [hi, R) holding known values of x in v
-  // (the separator that follows a partition).
-  // per block of 8 columns one thread solves the 8 x 8 diagonal block, then
-  // one thread per row applies the block's 8 values to the next bw rows, with
-  // the next block's factor entries copied in (cp.async) meanwhile.  The
-  // active vector entries live in 256 circular slots of shared memory.
-  static constexpr int kSolveBlk = 8;
+  // this thread's index), over the columns [lo, lo + ne) in the blocks whose
+  // diagonal blocks band_invert_diag inverted (X_b).  Forward, per block:
+  // z_b = X_b v_b into w, then the next bw rows of v take their updates (the
+  // rows [lo + ne, R) among them, written back at the end).  Backward, per
+  // block from the last: x_b = X_b^T (w_b - the block's columns below it
+  // times x) into v, the rows [hi, R) holding known values of x in v (the
+  // separator that follows a partition).  Both phases of a block are dot
+  // products shared by several lanes each (two barriers per block); the next
+  // block's factor columns, contiguous in the band, are copied in (cp.async)
+  // meanwhile.  The active vector entries live in 256 circular slots.
+  // (T = 50 MPC QP, half-bandwidth 99: blocks of 8 columns with one thread
+  // solving each diagonal block took about 0.5 ms per direction in a
+  // 128-thread block.)
+  template <typename T, int BT>
+  __device__ __forceinline__ void band_issue_block(T* dst, const T* src, int nel, int lt) {
+    constexpr int V = 16 / int(sizeof(T));
+    if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
+      const int nv = nel / V;
+      for (int e = lt; e < nv; e += BT) cp_async16(dst + e * V, src + e * V);
+      if (lt < nel - nv * V) cp_async_elem(dst + nv * V + lt, src + nv * V + lt, true);
+    } else {
+      for (int e = lt; e < nel; e += BT) cp_async_elem(dst + e, src + e, true);
+    }
+    cp_async_commit();
+  }
+  // Lanes sharing one of `rows` dot products: a power of two up to 32.
+  template <int BT>
+  __device__ __forceinline__ static int band_lanes(int rows) {
+    int s = 1;
+    while (s < 32 && 2 * s * rows <= BT) s *= 2;
+    return s;
+  }
+
   template <typename T, int BT>
   __device__ void band_fwd_blocked(T* v, T* w, int lo, int ne, int R, int lt) {
-    constexpr int KB = kSolveBlk;
-    const int bw = this->bw, ldl = bw + 1, hi = lo + ne;
+    const int bw = this->bw, ldl = bw + 1, hi = lo + ne, KB = band_solve_block(bw);
     const T* L = reinterpret_cast<const T*>(Lb);
     T* win = reinterpret_cast<T*>(bwin);  // 256 slots: row r at r & 255
     T* pan = win + 256;                   // 2 x (KB ldl): factor columns of a block
-    T* zz = pan + 2 * KB * ldl;           // the block's KB values
-    auto issue = [&](int k0, int buf) {
-      T* dst = pan + buf * KB * ldl;
-      const int nel = min(KB, hi - k0) * ldl;
-      for (int e = lt; e < KB * ldl; e += BT)
-        cp_async_elem(dst + e, L + (e < nel ? size_t(k0) * ldl + e : 0), e < nel);
-      cp_async_commit();
-    };
+    T* zz = pan + 2 * KB * ldl;           // the block's values
+    const int S1 = band_lanes<BT>(KB), r1 = lt / S1, s1 = lt % S1;
+    const int S2 = band_lanes<BT>(bw), r2 = lt / S2, s2 = lt % S2;
     int loaded = min(R, lo + bw + KB);
     for (int r = lo + lt; r < loaded; r += BT) win[r & 255] = v[r];
-    if (lo < hi) issue(lo, 0);
+    if (lo < hi)
+      band_issue_block<T, BT>(pan, L + size_t(lo) * ldl, min(KB, hi - lo) * ldl, lt);
     int buf = 0;
     for (int k0 = lo; k0 < hi; k0 += KB, buf ^= 1) {
       const int pw = min(KB, hi - k0);
@@ -2973,36 +3035,50 @@ struct Ipm {
       // previous block: the next block's copies may now fill the other buffer.
       cp_async_wait<0>();
       group_sync<BT>();
-      if (k0 + KB < hi) issue(k0 + KB, buf ^ 1);
+      if (k0 + KB < hi)
+        band_issue_block<T, BT>(pan + (buf ^ 1) * KB * ldl, L + size_t(k0 + KB) * ldl,
+                                min(KB, hi - k0 - KB) * ldl, lt);
+      const int nload = min(R, k0 + 2 * KB + bw);  // rows the next block's window adds
+      const bool ld = loaded + lt < nload;
+      const T nv = ld ? v[loaded + lt] : T(0);
       const T* pc = pan + buf * KB * ldl;  // column k0 + c: pc[c * ldl + d], d = row - column
-      if (lt == 0) {
-        T zl[KB];
-#pragma unroll
-        for (int c = 0; c < KB; ++c) {
-          if (c < pw) {
-            T t = win[(k0 + c) & 255];
-#pragma unroll
-            for (int c2 = 0; c2 < c; ++c2)
-              if (c - c2 <= bw) t = fma(-pc[c2 * ldl + (c - c2)], zl[c2], t);
-            zl[c] = t * pc[c * ldl];
-            zz[c] = zl[c];
-            w[k0 + c] = zl[c];
+      {
+        T a0 = T(0), a1 = T(0);
+        if (r1 < pw) {
+          int c = s1;
+          for (; c + S1 <= r1; c += 2 * S1) {
+            a0 = fma(pc[c * ldl + r1 - c], win[(k0 + c) & 255], a0);
+            a1 = fma(pc[(c + S1) * ldl + r1 - c - S1], win[(k0 + c + S1) & 255], a1);
           }
+          if (c <= r1) a0 = fma(pc[c * ldl + r1 - c], win[(k0 + c) & 255], a0);
+        }
+        T z = a0 + a1;
+        for (int o = 1; o < S1; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if (s1 == 0 && r1 < pw) {
+          zz[r1] = z;
+          w[k0 + r1] = z;
         }
       }
       group_sync<BT>();
-      const int rend = min(R, k0 + pw + bw);
-      for (int r = k0 + pw + lt; r < rend; r += BT) {
-        T t = win[r & 255];
-#pragma unroll
-        for (int c = 0; c < KB; ++c) {
-          const int d = r - k0 - c;
-          if (c < pw && d <= bw) t = fma(-pc[c * ldl + d], zz[c], t);
+      const int rows = min(R, k0 + pw + bw) - (k0 + pw);
+      for (int rb = 0; rb < rows; rb += BT / S2) {
+        const int r = k0 + pw + rb + r2;
+        T a0 = T(0), a1 = T(0);
+        if (rb + r2 < rows) {
+          const T* pr = pc + (r - k0);  // entry of column c at pr[c * bw]
+          const int c0 = max(0, r - k0 - bw);
+          int c = c0 + s2;
+          for (; c + S2 < pw; c += 2 * S2) {
+            a0 = fma(pr[c * bw], zz[c], a0);
+            a1 = fma(pr[(c + S2) * bw], zz[c + S2], a1);
+          }
+          if (c < pw) a0 = fma(pr[c * bw], zz[c], a0);
         }
-        win[r & 255] = t;
+        T t = a0 + a1;
+        for (int o = 1; o < S2; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (s2 == 0 && rb + r2 < rows) win[r & 255] -= t;
       }
-      const int nload = min(R, k0 + 2 * KB + bw);
-      for (int r = loaded + lt; r < nload; r += BT) win[r & 255] = v[r];
+      if (ld) win[(loaded + lt) & 255] = nv;
       loaded = max(loaded, nload);
     }
     cp_async_wait<0>();
@@ -3013,79 +3089,60 @@ struct Ipm {
 
   template <typename T, int BT>
   __device__ void band_bwd_blocked(T* v, T* w, int lo, int hi, int R, int lt) {
-    constexpr int KB = kSolveBlk;
-    const int bw = this->bw, ldl = bw + 1;
+    const int bw = this->bw, ldl = bw + 1, KB = band_solve_block(bw);
     const T* L = reinterpret_cast<const T*>(Lb);
-    T* win = reinterpret_cast<T*>(bwin);
-    T* stg = win + 256;                   // 2 x ((bw + KB) x KB): entries L(kb + q, i)
-    T* xx = stg + 2 * (bw + KB) * KB;     // the block's KB values
-    const int SR = bw + KB;               // staged rows per block: i in [kb - bw, kb + KB)
-    // Stage, for the block of rows [kb, k1], the entries L(kb + q, i) (band
-    // column i, offset kb + q - i) for i in [kb - bw, k1].
-    auto issue = [&](int kb, int k1, int buf) {
-      T* dst = stg + buf * SR * KB;
-      for (int e = lt; e < SR * KB; e += BT) {
-        const int ii = e / KB, q = e - ii * KB, i = kb - bw + ii, d = kb + q - i;
-        const bool ok = i >= lo && i <= k1 && kb + q <= k1 && d >= 0 && d <= bw;
-        cp_async_elem(dst + e, L + (ok ? size_t(i) * ldl + d : 0), ok);
-      }
-      cp_async_commit();
-    };
-    // Window: w for rows [max(lo, hi - bw - KB), hi), the known x for [hi, R).
-    const int wlo = max(lo, hi - bw - KB);
-    for (int r = wlo + lt; r < R; r += BT) win[r & 255] = r >= hi ? v[r] : w[r];
-    int kb = max(lo, hi - KB);
-    if (lo < hi) issue(kb, hi - 1, 0);
-    group_sync<BT>();
-    // Known rows [hi, R): w_i -= sum_r L(r, i) x_r for i in [hi - bw, hi).
-    if (R > hi) {
-      for (int i = max(lo, hi - bw) + lt; i < hi; i += BT) {
-        T t = win[i & 255];
-        const int rmax = min(R - 1, i + bw);
-        for (int r = hi; r <= rmax; ++r) t = fma(-L[size_t(i) * ldl + (r - i)], win[r & 255], t);
-        win[i & 255] = t;
-      }
-    }
-    int loaded = wlo;  // rows [loaded, hi) are in the window
-    int buf = 0;
-    for (int k1 = hi - 1; k1 >= lo; k1 = kb - 1, buf ^= 1) {
-      kb = max(lo, k1 - KB + 1);
-      const int pw = k1 - kb + 1;
-      const int kbn = max(lo, kb - KB);
-      // As in the forward: this block's entries have landed and the other
+    T* win = reinterpret_cast<T*>(bwin);  // 256 slots: x_r at r & 255
+    T* pan = win + 256;
+    T* uu = pan + 2 * KB * ldl;
+    const int S1 = band_lanes<BT>(KB), c1 = lt / S1, s1 = lt % S1;
+    if (hi <= lo) return;
+    for (int r = hi + lt; r < R; r += BT) win[r & 255] = v[r];
+    int k0 = lo + (hi - 1 - lo) / KB * KB, buf = 0;
+    band_issue_block<T, BT>(pan, L + size_t(k0) * ldl, (hi - k0) * ldl, lt);
+    for (; k0 >= lo; k0 -= KB, buf ^= 1) {
+      const int pw = min(KB, hi - k0);
+      const T wv = (s1 == 0 && c1 < pw) ? w[k0 + c1] : T(0);
+      // As in the forward: this block's columns have landed and the other
       // buffer is free once every thread has passed the barrier.
       cp_async_wait<0>();
       group_sync<BT>();
-      if (kb > lo) issue(kbn, kb - 1, buf ^ 1);
-      const T* sg = stg + buf * SR * KB;  // L(kb + q, i) at sg[(i - kb + bw) * KB + q]
-      if (lt == 0) {
-        T xl[KB];
-#pragma unroll
-        for (int c = KB - 1; c >= 0; --c) {
-          if (c < pw) {
-            const int r = kb + c;
-            T t = win[r & 255];
-#pragma unroll
-            for (int c2 = c + 1; c2 < KB; ++c2)
-              if (c2 < pw) t = fma(-sg[(c + bw) * KB + c2], xl[c2], t);
-            xl[c] = t * sg[(c + bw) * KB + c];
-            xx[c] = xl[c];
-            v[r] = xl[c];
+      if (k0 > lo)
+        band_issue_block<T, BT>(pan + (buf ^ 1) * KB * ldl, L + size_t(k0 - KB) * ldl, KB * ldl,
+                                lt);
+      const T* pc = pan + buf * KB * ldl + c1 * ldl;  // column k0 + c1
+      {
+        T a0 = T(0), a1 = T(0);
+        if (c1 < pw) {
+          const int dmax = min(bw, R - 1 - k0 - c1), rb = k0 + c1;
+          int d = pw - c1 + s1;
+          for (; d + S1 <= dmax; d += 2 * S1) {
+            a0 = fma(pc[d], win[(rb + d) & 255], a0);
+            a1 = fma(pc[d + S1], win[(rb + d + S1) & 255], a1);
           }
+          if (d <= dmax) a0 = fma(pc[d], win[(rb + d) & 255], a0);
         }
+        T t = a0 + a1;
+        for (int o = 1; o < S1; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (s1 == 0 && c1 < pw) uu[c1] = wv - t;
       }
       group_sync<BT>();
-      for (int i = max(lo, kb - bw) + lt; i < kb; i += BT) {
-        T t = win[i & 255];
-        const T* si = sg + (i - kb + bw) * KB;
-#pragma unroll
-        for (int q = 0; q < KB; ++q)
-          if (q < pw) t = fma(-si[q], xx[q], t);
-        win[i & 255] = t;
+      {
+        T a0 = T(0), a1 = T(0);
+        if (c1 < pw) {
+          int r = c1 + s1;
+          for (; r + S1 < pw; r += 2 * S1) {
+            a0 = fma(pc[r - c1], uu[r], a0);
+            a1 = fma(pc[r + S1 - c1], uu[r + S1], a1);
+          }
+          if (r < pw) a0 = fma(pc[r - c1], uu[r], a0);
+        }
+        T x = a0 + a1;
+        for (int o = 1; o < S1; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (s1 == 0 && c1 < pw) {
+          v[k0 + c1] = x;
+          win[(k0 + c1) & 255] = x;
+        }
       }
-      const int nload = max(lo, kbn - bw);
-      for (int r = nload + lt; r < loaded; r += BT) win[r & 255] = w[r];
-      loaded = min(loaded, nload);
     }
     cp_async_wait<0>();
     group_sync<BT>();
@@ -3126,12 +3183,7 @@ struct Ipm {
     double* tmp = vec(kTMP);
     float* t32 = this->t32();
     for (int j = tid; j < n; j += NT) {
-      double acc = 0.0;
-      for (int q = jp[j]; q < jp[j + 1]; ++q) {
-        const int i = jx[q];
-        acc = fma(at[q], iry[n + i] * r[n + i], acc);
-      }
-      const double g = r[j] + acc;
+      const double g = r[j] + sparse_dot_scaled(jx, at, r + n, iry + n, jp[j], jp[j + 1]);
       if (fp64) {
         tmp[j] = g;
       } else {
@@ -3150,12 +3202,8 @@ struct Ipm {
         val = fp64 ? tmp[k] : double(t32[k]);
       } else {
         const int i = k - n;
-        double ax = 0.0;
-        if (fp64) {
-          for (int q = ip[i]; q < ip[i + 1]; ++q) ax = fma(av[q], tmp[ix[q]], ax);
-        } else {
-          for (int q = ip[i]; q < ip[i + 1]; ++q) ax = fma(av[q], double(t32[ix[q]]), ax);
-        }
+        const double ax = fp64 ? sparse_dot(ix, av, tmp, 0, ip[i], ip[i + 1])
+                               : sparse_dot(ix, av, t32, 0, ip[i], ip[i + 1]);
         val = iry[k] * (ax - r[k]);
       }
       out[k] = accumulate ? out[k] + val : val;
