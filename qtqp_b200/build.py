@@ -71,7 +71,13 @@ def build(force: bool = False, debug: bool = False, verbose: bool = False,
   with tempfile.TemporaryDirectory(prefix="qtqp_build_") as tmp:
     def compile_one(src):
       obj = os.path.join(tmp, os.path.basename(src) + ".o")
-      proc = subprocess.run([*common, "-c", src, "-o", obj], capture_output=True, text=True)
+      extra = []
+      if phase_timers and os.path.basename(src) == "band_batch.cu":
+        # Relocatable phase functions do not see their kernel's launch bounds
+        # (at most 128 registers per thread).
+        extra = ["-maxrregcount=128"]
+      proc = subprocess.run([*common, *extra, "-c", src, "-o", obj], capture_output=True,
+                            text=True)
       return src, obj, proc
     objs = []
     with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as ex:
