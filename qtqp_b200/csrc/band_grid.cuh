@@ -81,7 +81,7 @@ __host__ __device__ inline int band_grid_max_parts(int n, int bw) {
 __host__ __device__ inline int sep_pitch(int bw) { return bw | 1; }
 
 // Dynamic shared memory of one block (sized for FP64): the largest of the
-// band window, solves and Gram columns (band_win_bytes), the spike window, the
+// band window, solves and Gram rows (band_win_bytes), the spike window, the
 // products' staging, the separator reduction, and the solves' extra scratch.
 __host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
   const size_t e = sizeof(double);

@@ -85,10 +85,11 @@ __host__ __device__ inline InstLayout plan_layout(int n, int m, size_t smem_cap)
 }
 
 // Global workspace of one banded instance: vectors, the band factor (n x
-// (bw+1)) and working copies of the A (CSR and CSC) and P value arrays.
+// (bw+1)), working copies of the A (CSR and CSC) and P value arrays, and the
+// rows of the Gram product's column groups (band_gram_groups).
 struct BandLayout {
   int np;
-  size_t v_bytes, l_bytes, val_bytes, total;
+  size_t v_bytes, l_bytes, val_bytes, row_bytes, total;
 };
 __host__ __device__ inline BandLayout plan_band_layout(int n, int m, int bw, int nnz_a,
                                                        int nnz_p) {
@@ -97,7 +98,8 @@ __host__ __device__ inline BandLayout plan_band_layout(int n, int m, int bw, int
   L.v_bytes = round16(size_t(kNumVec) * L.np * 8);
   L.l_bytes = round16(size_t(n) * (bw + 1) * 8);
   L.val_bytes = round16((2 * size_t(nnz_a) + size_t(nnz_p)) * 8);
-  L.total = L.v_bytes + L.l_bytes + L.val_bytes;
+  L.row_bytes = round16((size_t(nnz_a) + size_t(n) / 8 + 2) * sizeof(int));
+  L.total = L.v_bytes + L.l_bytes + L.val_bytes + L.row_bytes;
   return L;
 }
 
@@ -117,21 +119,30 @@ __host__ __device__ inline int band_solve_block(int bw) {
 __host__ __device__ inline size_t band_solve_elems(int bw) {
   return 256 + 2 * size_t(band_solve_block(bw)) * (size_t(bw) + 1) + 32;
 }
+// The Gram product of the banded format: a warp forms kGramCols columns from
+// four dense rows of their entries in shared memory.  The pitch is 4 (mod 16)
+// doubles, so that a half-warp's fragment loads hit 16 different banks.
+constexpr int kGramCols = 8;
+__host__ __device__ inline int gram_pitch(int bw) {
+  const int w = (bw + 7 + 8) / 8 * 8;  // whole 8-column tiles
+  return w + (4 - w % 16 + 16) % 16;
+}
+__host__ __device__ inline size_t gram_warp_elems(int bw) { return 4 * size_t(gram_pitch(bw)); }
 constexpr int kBandPanel = 8;  // columns per panel of the blocked band Cholesky
 // Shared memory of the blocked band Cholesky (band_chol_panel_range): the
 // circular (bw + kBandPanel)^2 window, the panel rows and the list of the
-// window's lower 8 x 8 tiles.
+// window's lower 16 x 16 tiles.
 __host__ __device__ inline size_t band_panel_bytes(int bw) {
-  const size_t B = size_t(bw) + kBandPanel, nt8 = (size_t(bw) + 7) / 8;
+  const size_t B = size_t(bw) + kBandPanel, nt16 = (size_t(bw) + 15) / 16;
   return (B * B + B * (kBandPanel + 1)) * sizeof(double) +
-         nt8 * (nt8 + 1) / 2 * sizeof(uint16_t);
+         nt16 * (nt16 + 1) / 2 * sizeof(uint16_t);
 }
 // The shared memory a band needs in a block of nt threads: the Cholesky, the
-// solves, one Gram column per warp, one diagonal block to invert.
+// solves, the Gram rows of every warp, one diagonal block to invert.
 __host__ __device__ inline size_t band_win_bytes(int bw, int nt) {
   size_t e = band_panel_bytes(bw);
   const size_t kb = band_solve_block(bw);
-  const size_t cols = size_t(nt / 32) * (size_t(bw) + 1) * sizeof(double);
+  const size_t cols = size_t(nt / 32) * gram_warp_elems(bw) * sizeof(double);
   const size_t solve = band_solve_elems(bw) * sizeof(double);
   const size_t inv = kb * (kb + 1) * sizeof(double);
   if (cols > e) e = cols;
@@ -260,6 +271,8 @@ struct Ipm {
   double* pv;
   double* Lb;
   int bw, nnz_a, nnz_p;
+  int* grow;  // band_gram_groups
+  int* gcnt;
   // Shared-memory window of the banded factorisation and solves (null: the
   // band is too wide for it and the global-memory variants run).
   double* bwin;
@@ -2378,6 +2391,8 @@ struct Ipm {
     av = reinterpret_cast<double*>(gmem + L.v_bytes + L.l_bytes);
     at = av + nnz_a;
     pv = at + nnz_a;
+    grow = reinterpret_cast<int*>(gmem + L.v_bytes + L.l_bytes + L.val_bytes);
+    gcnt = grow + nnz_a;
     A = P = nullptr;
     lda = ldp = ldg = 0;
   }
@@ -2410,7 +2425,13 @@ struct Ipm {
     }
     for (int q = tid; q < nnz_p; q += NT) pv[q] = has_p ? pv0[q] : 0.0;
     for (int k = tid; k < N; k += NT) de[k] = 1.0;
+    if constexpr (FMT == kFmtBand) {
+      if (bwin != nullptr) band_gram_groups();
+    }
     sync();
+    if constexpr (FMT == kFmtBand) {
+      if (bwin != nullptr) band_gram_duplicates();
+    }
     auto scale_of = [](double mx) {
       if (mx == 0.0) mx = 1.0;
       return fmin(fmax(1.0 / sqrt(mx), 1e-3), 1e3);
@@ -2545,95 +2566,199 @@ struct Ipm {
     return sparse_dot(ix, av, v, 0, ip[i], ip[i + 1]);
   }
 
-  // Column j of the Gram matrix G = P_off + diag(Rx) + A^T diag(1/Ry) A,
-  // rows j .. j + bw, into acc[0 .. bw] (shared memory), by one warp: the
-  // lanes take 32 of the column's rows (index, value, scaling, extent), then
-  // the warp walks those rows, four at a time with their entries' loads
-  // issued together, each lane one or two entries of a row.  The entries of a
-  // row lie in different columns, so the lanes never meet, and every sum runs
-  // over the rows in order.  (A thread per column, its 2700 products of a T =
-  // 50 MPC column one after the other through shared memory, took 5.5 ms per
-  // factorisation of one QP in a 128-thread block.)
-  template <typename T>
-  __device__ __forceinline__ void band_gram_column(int j, T* acc) const {
+  // The rows of A that meet each group of kGramCols columns, once per solve:
+  // grow[jp[8 g] ..) holds the rows of group g (gcnt[g] of them), each where
+  // it first meets the group.  A warp per group compacts the group's CSC
+  // entries that are their row's first in the group (the row's preceding
+  // entry, found by a binary search of its CSR columns, lies before it).
+  __device__ void band_gram_groups() {
     QTQP_BAND_LOCALS;
-    const double* reg = vec(kREG);
-    const double* wsc = vec(kPW);
     const int lane = threadIdx.x & 31;
-    for (int d = lane; d <= bw; d += 32) acc[d] = T(0);
-    const int qa = jp[j], qb = jp[j + 1];
-    for (int q0 = qa; q0 < qb; q0 += 32) {
-      const int q = q0 + lane, cnt = min(32, qb - q0);
-      int r0 = 0, r1 = 0;
-      double w = 0.0;
-      T arj = T(0);
-      if (lane < cnt) {
-        const int r = jx[q];
-        w = wsc[n + r];
-        r0 = ip[r];
-        r1 = ip[r + 1];
-        arj = T(at[q] * w);
+    const int ng = (n + kGramCols - 1) / kGramCols;
+    for (int g = tid >> 5; g < ng; g += NT / 32) {
+      const int j0 = g * kGramCols, q0 = jp[j0], q1 = jp[min(n, j0 + kGramCols)];
+      int cnt = 0;
+      for (int qb = q0; qb < q1; qb += 32) {
+        const int q = qb + lane;
+        bool first = false;
+        int r = 0;
+        if (q < q1) {
+          r = jx[q];
+          // Entries of row r before column j0; the entry at q is the first in
+          // the group when it stands right behind them.
+          int lo = ip[r], hi = ip[r + 1];
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (ix[mid] < j0) {
+              lo = mid + 1;
+            } else {
+              hi = mid;
+            }
+          }
+          const int jc = ix[lo];  // the row's first column in the group
+          first = q >= jp[jc] && q < jp[jc + 1] && (q == jp[jc] || jx[q - 1] != r);
+        }
+        const unsigned int m = __ballot_sync(0xffffffffu, first);
+        if (first) grow[q0 + cnt + __popc(m & ((1u << lane) - 1))] = r;
+        cnt += __popc(m);
+      }
+      if (lane == 0) gcnt[g] = cnt;
+    }
+    if (tid == 0) gcnt[ng] = 0;
+  }
+  // Whether a row of A stores an entry twice (sorted, so side by side), in
+  // gcnt[number of groups]; after a barrier that follows band_gram_groups.
+  __device__ void band_gram_duplicates() {
+    QTQP_BAND_LOCALS;
+    for (int q = 1 + tid; q < nnz_a; q += NT) {
+      if (ix[q] != ix[q - 1]) continue;
+      int lo = 0, hi = m;  // the row of entry q: the last i with ip[i] <= q
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (ip[mid] <= q) {
+          lo = mid;
+        } else {
+          hi = mid;
+        }
+      }
+      if (ip[lo] < q) gcnt[(n + kGramCols - 1) / kGramCols] = 1;  // q - 1 is in the same row
+    }
+  }
+
+  // The Gram matrix G = P_off + diag(Rx) + A^T diag(1/Ry) A in column band
+  // storage (Lb) plus the relative diagonal jitter of the dense backend.  A
+  // warp per group of 8 columns: the rows that meet the group are taken four
+  // at a time, their entries at columns j0 .. j0 + bw + 7 scattered (scaled
+  // by 1/sqrt(Ry)) into four dense rows of shared memory, and G[j0 .. j0 + 8,
+  // j0 ..] += the product of their first 8 columns with all of them: FP64
+  // tensor-core steps (DMMA m8n8k4) into (bw + 14) / 8 accumulators, which
+  // stay in registers.  T = 50 MPC QP (2000 rows of 61 entries, half-bandwidth
+  // 99): 5.5 ms per factorisation with a thread per column, 2.7 ms with a warp
+  // per column accumulating in shared memory (a row's every visit by a column
+  // cost some 60 instructions; a group of 8 columns now shares one visit).
+  // buf: the block's scratch, gram_warp_elems(bw) entries per warp.
+  // dup: rows may store an entry twice; their values are added up.
+  template <typename T, int NT8>
+  __device__ __forceinline__ void band_gram_group(int g, T* buf, bool dup, double& dmax) const {
+    QTQP_BAND_LOCALS;
+    const double* wsc = vec(kPW);
+    const double* reg = vec(kREG);
+    const int lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+    const int pitch = gram_pitch(bw), width = min(bw + kGramCols, pitch);
+    const int j0 = g * kGramCols, cnt = gcnt[g];
+    const int* rows = grow + jp[j0];
+    const int nt = (bw + 7 + 8) >> 3;  // 8-column tiles from j0 to j0 + bw + 7
+    T acc[NT8][2];
+#pragma unroll
+    for (int t = 0; t < NT8; ++t) acc[t][0] = acc[t][1] = T(0);
+    const int rr = lane >> 3, sub = lane & 7;  // this lane's row of the four, its share of it
+    int rn = rr < cnt ? rows[rr] : -1;
+    for (int c0 = 0; c0 < cnt; c0 += 4) {
+      const int r = rn;
+      rn = c0 + 4 + rr < cnt ? rows[c0 + 4 + rr] : -1;
+      for (int e = lane; e < 4 * pitch; e += 32) buf[e] = T(0);
+      __syncwarp();
+      if (r >= 0) {
+        const double w = wsc[n + r];
+        const int e1 = ip[r + 1];
+        T* row = buf + rr * pitch;
+        int e = ip[r] + sub;
+        if (dup) {
+          for (; e < e1; e += 8) {
+            const int i = ix[e] - j0;
+            if (i >= 0 && i < width) atomicAdd(row + i, T(av[e] * w));
+          }
+        }
+        for (; e + 24 < e1; e += 32) {  // four loads in flight
+          int ii[4];
+          double aa[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            ii[u] = ix[e + 8 * u] - j0;
+            aa[u] = av[e + 8 * u];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (ii[u] >= 0 && ii[u] < width) row[ii[u]] = T(aa[u] * w);
+        }
+        for (; e < e1; e += 8) {
+          const int i = ix[e] - j0;
+          const double x = av[e];
+          if (i >= 0 && i < width) row[i] = T(x * w);
+        }
       }
       __syncwarp();
-      constexpr int RB = 4;  // rows whose loads are issued together
-      for (int u0 = 0; u0 < cnt; u0 += RB) {
-        int b1[RB], q2[RB], i0[RB], i1[RB];
-        double a0[RB], a1[RB];
+      if constexpr (sizeof(T) == 8) {
+        const T* br = buf + tg * pitch + gi;
+        const double a = br[0];
 #pragma unroll
-        for (int v = 0; v < RB; ++v) {
-          const int src = min(u0 + v, 31);
-          q2[v] = __shfl_sync(0xffffffffu, r0, src) + lane;
-          b1[v] = u0 + v < cnt ? __shfl_sync(0xffffffffu, r1, src) : 0;
-          i0[v] = q2[v] < b1[v] ? ix[q2[v]] : -1;
-          a0[v] = q2[v] < b1[v] ? av[q2[v]] : 0.0;
-          i1[v] = q2[v] + 32 < b1[v] ? ix[q2[v] + 32] : -1;
-          a1[v] = q2[v] + 32 < b1[v] ? av[q2[v] + 32] : 0.0;
-        }
+        for (int t = 0; t < NT8; ++t)
+          if (t < nt) dmma_8x8x4(acc[t], a, br[8 * t]);
+      } else {
 #pragma unroll
-        for (int v = 0; v < RB; ++v) {
-          const int src = min(u0 + v, 31);
-          const double wv = __shfl_sync(0xffffffffu, w, src);
-          const T av_j = __shfl_sync(0xffffffffu, arj, src);
-          const int d0 = i0[v] - j, d1 = i1[v] - j;
-          if (d0 >= 0 && d0 <= bw) acc[d0] = fma(av_j, T(a0[v] * wv), acc[d0]);
-          if (d1 >= 0 && d1 <= bw) acc[d1] = fma(av_j, T(a1[v] * wv), acc[d1]);
-          for (int e = q2[v] + 64; e < b1[v]; e += 32) {
-            const int d = ix[e] - j;
-            if (d >= 0 && d <= bw) acc[d] = fma(av_j, T(av[e] * wv), acc[d]);
+        for (int k = 0; k < 4; ++k) {
+          const T* br = buf + k * pitch;
+          const T a = br[gi];
+#pragma unroll
+          for (int t = 0; t < NT8; ++t) {
+            if (t < nt) {
+              acc[t][0] = fma(a, br[8 * t + 2 * tg], acc[t][0]);
+              acc[t][1] = fma(a, br[8 * t + 2 * tg + 1], acc[t][1]);
+            }
           }
-          __syncwarp();
         }
       }
+      __syncwarp();
+    }
+    // Lane (gi, tg) holds G[j0 + gi][j0 + 8 t + 2 tg + e].
+    const int j = j0 + gi;
+    T* col = reinterpret_cast<T*>(Lb) + size_t(j) * ldl;
+    if (j < n) {
+#pragma unroll
+      for (int t = 0; t < NT8; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int d = 8 * t + 2 * tg + e - gi;
+          if (d >= 0 && d <= bw) col[d] = d == 0 ? T(reg[j]) + acc[t][e] : acc[t][e];
+        }
     }
     __syncwarp();
-    if (has_p) {
-      for (int q = pp[j] + lane; q < pp[j + 1]; q += 32) {
-        const int i = px[q];
-        if (i > j && i - j <= bw) acc[i - j] = T(pv[q]) + acc[i - j];
+    if (j < n && has_p && tg == 0) {
+      const int q1 = pp[j + 1];
+      for (int q = pp[j]; q < q1; q += 4) {
+        int dd[4];
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          dd[u] = q + u < q1 ? px[q + u] - j : 0;
+          x[u] = q + u < q1 ? pv[q + u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (dd[u] > 0 && dd[u] <= bw) col[dd[u]] = T(x[u]) + col[dd[u]];
       }
-      __syncwarp();
     }
-    if (lane == 0) acc[0] = T(reg[j]) + acc[0];
+    if (j < n && tg == 0) dmax = nanmax(dmax, double(col[0]));
     __syncwarp();
   }
 
-  // The Gram matrix in column band storage (Lb) plus the relative diagonal
-  // jitter of the dense backend; a warp per column.  acc: the block's
-  // scratch, bw + 1 entries per warp.
   template <typename T>
-  __device__ void band_gram(T* acc) {
-    const int ldl = bw + 1, lane = threadIdx.x & 31;
+  __device__ void band_gram(T* buf) {
+    const int ldl = bw + 1;
     T* L = reinterpret_cast<T*>(Lb);
-    T* wacc = acc + size_t(threadIdx.x >> 5) * ldl;
+    T* wbuf = buf + size_t(threadIdx.x >> 5) * gram_warp_elems(bw);
     double dmax[1] = {0.0};
     double dummy[1] = {0.0};
-    for (int j = tid >> 5; j < n; j += NT / 32) {
-      T* col = L + size_t(j) * ldl;
-      band_gram_column<T>(j, wacc);
-      dmax[0] = nanmax(dmax[0], double(wacc[0]));
-      for (int d = lane; d <= bw; d += 32) col[d] = wacc[d];
-      __syncwarp();
+    const int ng = (n + kGramCols - 1) / kGramCols;
+    const bool dup = gcnt[ng] != 0;
+    for (int g = tid >> 5; g < ng; g += NT / 32) {
+      if (bw <= 32) {
+        band_gram_group<T, 6>(g, wbuf, dup, dmax[0]);
+      } else {
+        band_gram_group<T, 17>(g, wbuf, dup, dmax[0]);
+      }
     }
+    static_assert((kBandWinMaxBw + 7 + 8) / 8 <= 17 && (32 + 7 + 8) / 8 <= 6, "tiles");
     reduce<0, 1>(dummy, dmax);
     const double jit = (sizeof(T) == 8 ? 1e-14 : 2.384185791015625e-07) * dmax[0];
     for (int j = tid; j < n; j += NT) L[size_t(j) * ldl] = T(double(L[size_t(j) * ldl]) + jit);
@@ -2684,9 +2809,8 @@ struct Ipm {
   //    solves its own row with it as it goes, so no barrier lies on the chain
   //    from column to column (eight barriers and publishes per panel before);
   //    the finished columns go to global memory and to the panel buffer;
-  //  * the rank-8 update of the window's lower bw x bw part, by 8 x 8 tiles,
-  //    a warp per tile, on the FP64 tensor cores (DMMA; 64 tiles' worth of
-  //    products are 1/6 of the shared-memory reads of a thread per entry).
+  //  * the rank-8 update of the window's lower bw x bw part, by 16 x 16 tiles,
+  //    a warp per tile, on the FP64 tensor cores (DMMA).
   //    The kBandPanel rows that enter the window, loaded from the Gram matrix
   //    during the panel, are stored, and the columns left of their band
   //    zeroed.
@@ -2699,9 +2823,9 @@ struct Ipm {
     T* Pn = W + B * B;
     uint16_t* tiles = reinterpret_cast<uint16_t*>(Pn + B * PP);
     __shared__ int s_bad;
-    const int nt8 = (bw + 7) >> 3, ntiles = nt8 * (nt8 + 1) / 2;
+    const int nt16 = (bw + 15) >> 4, ntiles = nt16 * (nt16 + 1) / 2;
     const int lane = lt & 31, warp = lt >> 5, gi = lane >> 2, tg = lane & 3;
-    for (int a = lt; a < nt8; a += BT)
+    for (int a = lt; a < nt16; a += BT)
       for (int b = 0; b <= a; ++b) tiles[a * (a + 1) / 2 + b] = uint16_t(a | (b << 8));
     for (int e = lt; e < B * B; e += BT) {
       const int i = e / B, j = e - i * B;
@@ -2711,10 +2835,16 @@ struct Ipm {
     group_sync<BT>();
     int bad = 0;
     constexpr int MAXPRE = (KP * 128 + BT - 1) / BT;  // entering entries per thread (bw < 128)
-    for (int k = 0; k < ne; k += KP) {
+    int pre_e[MAXPRE], pre_d[MAXPRE];
+#pragma unroll
+    for (int q = 0; q < MAXPRE; ++q) {
+      pre_e[q] = (lt + BT * q) / (bw + 1);
+      pre_d[q] = (lt + BT * q) % (bw + 1);
+    }
+    int sk = 0;  // k mod B
+    for (int k = 0; k < ne; k += KP, sk = sk + KP >= B ? sk + KP - B : sk + KP) {
       const int pw = min(KP, ne - k);
       const int nr = min(pw + bw, nsub - k);
-      const int sk = k % B;
       auto sl = [&](int x) {  // slot of index k + x, 0 <= x < 2 B
         int t = sk + x;
         t = t >= B ? t - B : t;
@@ -2725,8 +2855,7 @@ struct Ipm {
       T pre[MAXPRE];
 #pragma unroll
       for (int q = 0; q < MAXPRE; ++q) {
-        const int f = lt + BT * q, e = f / (bw + 1), d = f - e * (bw + 1);
-        const int r = k + B + e;
+        const int e = pre_e[q], d = pre_d[q], r = k + B + e;
         pre[q] = (e < pw && r < nsub) ? L[size_t(r - bw + d) * ldl + (bw - d)] : T(0);
       }
       if (lt < nr) {
@@ -2783,40 +2912,64 @@ struct Ipm {
       const int span = min(bw, nsub - k - pw);  // of which these exist
       for (int t = warp; t < ntiles; t += BT / 32) {
         const int pr = tiles[t];
-        const int ta = (pr & 0xff) * 8, tb = (pr >> 8) * 8;
+        const int ta = (pr & 0xff) * 16, tb = (pr >> 8) * 16;
         if (ta >= span) continue;
-        T acc[2] = {T(0), T(0)};
-        const int a = ta + gi, b0 = tb + 2 * tg;
+        T acc[2][2][2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = T(0);
         if constexpr (sizeof(T) == 8) {
-          const int bj = tb + gi;
-          const T* ra = Pn + (pw + a) * PP + tg;
-          const T* rb = Pn + (pw + bj) * PP + tg;
-          const bool oka = a < span, okb = bj < span;
-          const double a0 = oka ? ra[0] : 0.0, a1 = oka ? ra[4] : 0.0;
-          const double c0 = okb ? rb[0] : 0.0, c1 = okb ? rb[4] : 0.0;
-          dmma_8x8x4(acc, a0, c0);
-          dmma_8x8x4(acc, a1, c1);
-        } else if (a < span) {
-          const T* ra = Pn + (pw + a) * PP;
+          double fa[2][2], fb[2][2];
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (b0 + e > a) continue;
-            const T* rb = Pn + (pw + b0 + e) * PP;
+          for (int x = 0; x < 2; ++x) {
+            const int a = ta + 8 * x + gi, b = tb + 8 * x + gi;
+            const T* ra = Pn + (pw + min(a, span - 1)) * PP + tg;
+            const T* rb = Pn + (pw + min(b, span - 1)) * PP + tg;
 #pragma unroll
-            for (int c = 0; c < KP; ++c) acc[e] = fma(ra[c], rb[c], acc[e]);
+            for (int h = 0; h < 2; ++h) {
+              fa[x][h] = a < span ? ra[4 * h] : 0.0;
+              fb[x][h] = b < span ? rb[4 * h] : 0.0;
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+              for (int y = 0; y < 2; ++y) dmma_8x8x4(acc[x][y], fa[x][h], fb[y][h]);
+        } else {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const T* ra = Pn + (pw + min(ta + 8 * x + gi, span - 1)) * PP;
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const T* rb = Pn + (pw + min(tb + 8 * y + 2 * tg + e, span - 1)) * PP;
+#pragma unroll
+                for (int c = 0; c < KP; ++c) acc[x][y][e] = fma(ra[c], rb[c], acc[x][y][e]);
+              }
           }
         }
-        if (a < span) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int a = ta + 8 * x + gi;
+          if (a >= span) continue;
           T* wr = W + sl(pw + a) * B;
-          if (b0 <= a) wr[sl(pw + b0)] -= acc[0];
-          if (b0 + 1 <= a) wr[sl(pw + b0 + 1)] -= acc[1];
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int b = tb + 8 * y + 2 * tg + e;
+              if (b <= a) wr[sl(pw + b)] -= acc[x][y][e];
+            }
         }
       }
       // Entering rows: band entries, and zeros left of the band.
 #pragma unroll
       for (int q = 0; q < MAXPRE; ++q) {
-        const int f = lt + BT * q, e = f / (bw + 1), d = f - e * (bw + 1);
-        const int r = k + B + e;
+        const int e = pre_e[q], d = pre_d[q], r = k + B + e;
         if (e < pw && r < nsub) W[sl(B + e) * B + sl(KP + e + d)] = pre[q];
       }
       for (int f = lt; f < pw * (KP - 1); f += BT) {

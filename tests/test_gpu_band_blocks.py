@@ -75,3 +75,31 @@ def test_more_qps_than_sms(bw):
   for sol in sols:
     np.testing.assert_array_equal(sol.x, sols[0].x)
   _check(sols[0], q, ref)
+
+
+def test_entries_stored_twice():
+  """A CSC matrix may store an entry twice (their sum is the entry): here
+  every seventh entry is split in two equal parts, which leaves the products
+  exact."""
+  from qtqp_b200 import band, batch
+  bw, n = 20, 130
+  a, b, c, z, p = _banded(bw, n, 3)
+  a.sort_indices()
+  reps = np.where(np.arange(a.nnz) % 7 == 3, 2, 1)
+  ptr = np.concatenate([[0], np.cumsum(np.add.reduceat(reps, a.indptr[:-1]))])
+  twice = sp.csc_matrix((np.repeat(a.data / reps, reps), np.repeat(a.indices, reps), ptr),
+                        shape=a.shape)
+  assert twice.nnz > a.nnz and abs(twice - a).max() == 0
+  opts = batch.SolveOptions(equilibrate=False)
+  outs = []
+  for mat in (a, twice):
+    hb = band.HostBandBatch([band.BandProblem(mat, b, c, z, p)], opts)
+    for dev in (band.DeviceBandBatch(hb), band.DeviceBandGrid(hb)):
+      dev.upload()
+      dev.launch()
+      res, x, *_ = dev.fetch()
+      assert res["status"][0] == 0
+      outs.append(x.copy())
+  # The same QP: solutions agree to the solver's tolerance on its objective.
+  for x in outs[1:]:
+    assert kkt_checks.objective_rel_err(x, outs[0], c, p) <= OBJ_TOL
