@@ -114,10 +114,11 @@ __host__ __device__ inline int band_solve_block(int bw) {
   while (kb < 32 && 2 * kb <= bw + 1) kb *= 2;
   return kb;
 }
-// Shared-memory elements of the blocked band solves: 256 window slots, two
-// staged blocks of factor columns and the block's values.
+// Shared-memory elements of the blocked band solves: 256 window slots, a ring
+// of staged blocks of factor columns and the block's values.
+constexpr int kBandSolveStages = 4;
 __host__ __device__ inline size_t band_solve_elems(int bw) {
-  return 256 + 2 * size_t(band_solve_block(bw)) * (size_t(bw) + 1) + 32;
+  return 256 + kBandSolveStages * size_t(band_solve_block(bw)) * (size_t(bw) + 1) + 32;
 }
 // The Gram product of the banded format: a warp forms kGramCols columns from
 // four dense rows of their entries in shared memory.  The pitch is 4 (mod 16)
@@ -130,11 +131,11 @@ __host__ __device__ inline int gram_pitch(int bw) {
 __host__ __device__ inline size_t gram_warp_elems(int bw) { return 4 * size_t(gram_pitch(bw)); }
 constexpr int kBandPanel = 8;  // columns per panel of the blocked band Cholesky
 // Shared memory of the blocked band Cholesky (band_chol_panel_range): the
-// circular (bw + kBandPanel)^2 window, the panel rows and the list of the
-// window's lower 16 x 16 tiles.
+// circular (bw + kBandPanel)^2 window, the panel rows, two stages of entering
+// rows and the list of the window's lower 16 x 16 tiles.
 __host__ __device__ inline size_t band_panel_bytes(int bw) {
   const size_t B = size_t(bw) + kBandPanel, nt16 = (size_t(bw) + 15) / 16;
-  return (B * B + B * (kBandPanel + 1)) * sizeof(double) +
+  return (B * B + B * (kBandPanel + 1) + 2 * kBandPanel * (size_t(bw) + 1)) * sizeof(double) +
          nt16 * (nt16 + 1) / 2 * sizeof(uint16_t);
 }
 // The shared memory a band needs in a block of nt threads: the Cholesky, the
@@ -291,8 +292,7 @@ struct Ipm {
   GridCtl* gctl;
   // Large format: padded sizes (multiples of 128 / 32), the factor in FP64
   // (g64) or FP32 (g32), both npad x npad row-major (lower triangle), the
-  // inverses of its 128 x 128 diagonal blocks (linv, in the factor's
-  // precision), the split TF32 operands X = (diag(1/sqrt(Ry)) A)^T
+  // split TF32 operands X = (diag(1/sqrt(Ry)) A)^T
   // (xhi / xlo, npad x mpad), their tensor maps, the CTA's shared-memory
   // arena (tensor-core ring / staging tiles), its TMEM accumulator and the
   // per-thread pipeline counters of the tensor-core ring.
@@ -300,7 +300,6 @@ struct Ipm {
   int* linfo;  // factorisation status shared by the grid
   double* g64;
   float* g32l;
-  double* linv;
   double* sinv;  // sub-block inverses of the current panel step
   double* colpart;  // per-block column sums of large_products (gridDim x npad)
   float* xhi;
@@ -2811,9 +2810,9 @@ struct Ipm {
   //    the finished columns go to global memory and to the panel buffer;
   //  * the rank-8 update of the window's lower bw x bw part, by 16 x 16 tiles,
   //    a warp per tile, on the FP64 tensor cores (DMMA).
-  //    The kBandPanel rows that enter the window, loaded from the Gram matrix
-  //    during the panel, are stored, and the columns left of their band
-  //    zeroed.
+  //    The kBandPanel rows that enter the window, copied from the Gram matrix
+  //    (cp.async) since the panel before, are stored, and the columns left of
+  //    their band zeroed.
   template <typename T, int BT>
   __device__ int band_chol_panel_range(int lt, int lo, int nsub, int ne, T* tail, int ldt) {
     constexpr int KP = kBandPanel, PP = KP + 1;
@@ -2821,7 +2820,8 @@ struct Ipm {
     T* L = reinterpret_cast<T*>(Lb) + size_t(lo) * ldl;
     T* W = reinterpret_cast<T*>(bwin);
     T* Pn = W + B * B;
-    uint16_t* tiles = reinterpret_cast<uint16_t*>(Pn + B * PP);
+    T* En = Pn + B * PP;  // two stages of the rows that enter the window
+    uint16_t* tiles = reinterpret_cast<uint16_t*>(En + 2 * KP * (bw + 1));
     __shared__ int s_bad;
     const int nt16 = (bw + 15) >> 4, ntiles = nt16 * (nt16 + 1) / 2;
     const int lane = lt & 31, warp = lt >> 5, gi = lane >> 2, tg = lane & 3;
@@ -2841,6 +2841,20 @@ struct Ipm {
       pre_e[q] = (lt + BT * q) / (bw + 1);
       pre_d[q] = (lt + BT * q) % (bw + 1);
     }
+    // Rows kk + B .. kk + B + 7 enter after the panel of column kk: their band
+    // entries (row r, column r - bw + d), each stored later by the thread that
+    // copies it.
+    auto issue_rows = [&](int kk) {
+#pragma unroll
+      for (int q = 0; q < MAXPRE; ++q) {
+        const int e = pre_e[q], d = pre_d[q], r = kk + B + e;
+        if (e < KP && kk < ne && r < nsub)
+          cp_async_elem(En + ((kk / KP) & 1) * KP * (bw + 1) + lt + BT * q,
+                        L + size_t(r - bw + d) * ldl + (bw - d), true);
+      }
+      cp_async_commit();
+    };
+    issue_rows(0);
     int sk = 0;  // k mod B
     for (int k = 0; k < ne; k += KP, sk = sk + KP >= B ? sk + KP - B : sk + KP) {
       const int pw = min(KP, ne - k);
@@ -2850,14 +2864,7 @@ struct Ipm {
         t = t >= B ? t - B : t;
         return t >= B ? t - B : t;
       };
-      // Rows k + B .. k + B + pw - 1 enter after this panel: prefetch their
-      // band entries (row r, column r - bw + d).
-      T pre[MAXPRE];
-#pragma unroll
-      for (int q = 0; q < MAXPRE; ++q) {
-        const int e = pre_e[q], d = pre_d[q], r = k + B + e;
-        pre[q] = (e < pw && r < nsub) ? L[size_t(r - bw + d) * ldl + (bw - d)] : T(0);
-      }
+      issue_rows(k + KP);
       if (lt < nr) {
         // The diagonal block (the same in every thread) and this thread's row.
         T dg[KP][KP], v[KP];
@@ -2871,27 +2878,30 @@ struct Ipm {
           for (int c = 0; c <= a; ++c) dg[a][c] = a < pw ? W[sc[a] * B + sc[c]] : T(0);
           v[a] = (a < pw && a <= lt) ? wr[sc[a]] : T(0);
         }
+        // Columns from pw on (the last panel) have a zero diagonal block and
+        // are not used.  A non-positive pivot is only noted: the panel then
+        // runs to its end on whatever follows, and nothing of it is kept.
         int f = 0;
 #pragma unroll
         for (int c = 0; c < KP; ++c) {
-          if (c < pw && f == 0) {
-            const T piv = dg[c][c];
-            if (!(piv > T(0))) {
-              f = k + c + 1;
-            } else {
-              const T il = rsqrt(piv);
-              const T lic = v[c] * il;
-              v[c] = lt == c ? il : lic;  // the factor keeps 1 / l_cc
+          const T piv = dg[c][c];
+          f = f == 0 && c < pw && !(piv > T(0)) ? k + c + 1 : f;
+          const T il = rsqrt(piv);
+          const T lic = v[c] * il;
+          v[c] = lt == c ? il : lic;  // the factor keeps 1 / l_cc
 #pragma unroll
-              for (int a = c + 1; a < KP; ++a) dg[a][c] *= il;
+          for (int a = c + 1; a < KP; ++a) dg[a][c] *= il;
 #pragma unroll
-              for (int a = c + 1; a < KP; ++a) {
-                v[a] = fma(-lic, dg[a][c], v[a]);
+          for (int a = c + 1; a < KP; ++a) {
+            v[a] = fma(-lic, dg[a][c], v[a]);
 #pragma unroll
-                for (int b = c + 1; b <= a; ++b) dg[a][b] = fma(-dg[a][c], dg[b][c], dg[a][b]);
-              }
-            }
+            for (int b = c + 1; b <= a; ++b) dg[a][b] = fma(-dg[a][c], dg[b][c], dg[a][b]);
           }
+        }
+        if (pw < KP) {  // zero columns for the rank-8 update
+#pragma unroll
+          for (int c = 0; c < KP; ++c)
+            if (c >= pw) v[c] = T(0);
         }
         if (f != 0) {
           if (lt == 0) s_bad = f;
@@ -2967,10 +2977,12 @@ struct Ipm {
         }
       }
       // Entering rows: band entries, and zeros left of the band.
+      cp_async_wait<1>();  // this panel's; the next one's may be in flight
 #pragma unroll
       for (int q = 0; q < MAXPRE; ++q) {
         const int e = pre_e[q], d = pre_d[q], r = k + B + e;
-        if (e < pw && r < nsub) W[sl(B + e) * B + sl(KP + e + d)] = pre[q];
+        if (e < pw && r < nsub)
+          W[sl(B + e) * B + sl(KP + e + d)] = En[((k / KP) & 1) * KP * (bw + 1) + lt + BT * q];
       }
       for (int f = lt; f < pw * (KP - 1); f += BT) {
         const int e = f / (KP - 1), t = f - e * (KP - 1);
@@ -2979,6 +2991,7 @@ struct Ipm {
       }
       group_sync<BT>();
     }
+    cp_async_wait<0>();
     if (tail != nullptr && bad == 0) {
       const int t = nsub - ne;
       for (int e = lt; e < t * t; e += BT) {
@@ -3143,8 +3156,9 @@ struct Ipm {
   // times x) into v, the rows [hi, R) holding known values of x in v (the
   // separator that follows a partition).  Both phases of a block are dot
   // products shared by several lanes each (two barriers per block); the next
-  // block's factor columns, contiguous in the band, are copied in (cp.async)
-  // meanwhile.  The active vector entries live in 256 circular slots.
+  // three blocks' factor columns, contiguous in the band, are copied in
+  // (cp.async) meanwhile: 148 QPs' factors of 2.4 MB come from HBM.  The
+  // active vector entries live in 256 circular slots.
   // (T = 50 MPC QP, half-bandwidth 99: blocks of 8 columns with one thread
   // solving each diagonal block took about 0.5 ms per direction in a
   // 128-thread block.)
@@ -3158,7 +3172,6 @@ struct Ipm {
     } else {
       for (int e = lt; e < nel; e += BT) cp_async_elem(dst + e, src + e, true);
     }
-    cp_async_commit();
   }
   // Lanes sharing one of `rows` dot products: a power of two up to 32.
   template <int BT>
@@ -3173,24 +3186,27 @@ struct Ipm {
     const int bw = this->bw, ldl = bw + 1, hi = lo + ne, KB = band_solve_block(bw);
     const T* L = reinterpret_cast<const T*>(Lb);
     T* win = reinterpret_cast<T*>(bwin);  // 256 slots: row r at r & 255
-    T* pan = win + 256;                   // 2 x (KB ldl): factor columns of a block
-    T* zz = pan + 2 * KB * ldl;           // the block's values
+    T* pan = win + 256;                   // the ring: factor columns of a block, KB ldl each
+    T* zz = pan + kBandSolveStages * KB * ldl;  // the block's values
     const int S1 = band_lanes<BT>(KB), r1 = lt / S1, s1 = lt % S1;
     const int S2 = band_lanes<BT>(bw), r2 = lt / S2, s2 = lt % S2;
     int loaded = min(R, lo + bw + KB);
     for (int r = lo + lt; r < loaded; r += BT) win[r & 255] = v[r];
-    if (lo < hi)
-      band_issue_block<T, BT>(pan, L + size_t(lo) * ldl, min(KB, hi - lo) * ldl, lt);
+    auto issue = [&](int k, int st) {
+      if (k < hi)
+        band_issue_block<T, BT>(pan + st * KB * ldl, L + size_t(k) * ldl, min(KB, hi - k) * ldl,
+                                lt);
+      cp_async_commit();
+    };
+    for (int st = 0; st + 1 < kBandSolveStages; ++st) issue(lo + st * KB, st);
     int buf = 0;
-    for (int k0 = lo; k0 < hi; k0 += KB, buf ^= 1) {
+    for (int k0 = lo; k0 < hi; k0 += KB, buf = (buf + 1) % kBandSolveStages) {
       const int pw = min(KB, hi - k0);
       // This block's columns have landed and every thread is done with the
-      // previous block: the next block's copies may now fill the other buffer.
-      cp_async_wait<0>();
+      // previous block, whose buffer the copies of the block three ahead fill.
+      cp_async_wait<kBandSolveStages - 2>();
       group_sync<BT>();
-      if (k0 + KB < hi)
-        band_issue_block<T, BT>(pan + (buf ^ 1) * KB * ldl, L + size_t(k0 + KB) * ldl,
-                                min(KB, hi - k0 - KB) * ldl, lt);
+      issue(k0 + (kBandSolveStages - 1) * KB, (buf + kBandSolveStages - 1) % kBandSolveStages);
       const int nload = min(R, k0 + 2 * KB + bw);  // rows the next block's window adds
       const bool ld = loaded + lt < nload;
       const T nv = ld ? v[loaded + lt] : T(0);
@@ -3246,22 +3262,25 @@ struct Ipm {
     const T* L = reinterpret_cast<const T*>(Lb);
     T* win = reinterpret_cast<T*>(bwin);  // 256 slots: x_r at r & 255
     T* pan = win + 256;
-    T* uu = pan + 2 * KB * ldl;
+    T* uu = pan + kBandSolveStages * KB * ldl;
     const int S1 = band_lanes<BT>(KB), c1 = lt / S1, s1 = lt % S1;
     if (hi <= lo) return;
     for (int r = hi + lt; r < R; r += BT) win[r & 255] = v[r];
     int k0 = lo + (hi - 1 - lo) / KB * KB, buf = 0;
-    band_issue_block<T, BT>(pan, L + size_t(k0) * ldl, (hi - k0) * ldl, lt);
-    for (; k0 >= lo; k0 -= KB, buf ^= 1) {
+    auto issue = [&](int k, int st) {
+      if (k >= lo)
+        band_issue_block<T, BT>(pan + st * KB * ldl, L + size_t(k) * ldl, min(KB, hi - k) * ldl,
+                                lt);
+      cp_async_commit();
+    };
+    for (int st = 0; st + 1 < kBandSolveStages; ++st) issue(k0 - st * KB, st);
+    for (; k0 >= lo; k0 -= KB, buf = (buf + 1) % kBandSolveStages) {
       const int pw = min(KB, hi - k0);
       const T wv = (s1 == 0 && c1 < pw) ? w[k0 + c1] : T(0);
-      // As in the forward: this block's columns have landed and the other
-      // buffer is free once every thread has passed the barrier.
-      cp_async_wait<0>();
+      // As in the forward.
+      cp_async_wait<kBandSolveStages - 2>();
       group_sync<BT>();
-      if (k0 > lo)
-        band_issue_block<T, BT>(pan + (buf ^ 1) * KB * ldl, L + size_t(k0 - KB) * ldl, KB * ldl,
-                                lt);
+      issue(k0 - (kBandSolveStages - 1) * KB, (buf + kBandSolveStages - 1) % kBandSolveStages);
       const T* pc = pan + buf * KB * ldl + c1 * ldl;  // column k0 + c1
       {
         T a0 = T(0), a1 = T(0);
