@@ -76,7 +76,6 @@ __global__ void __launch_bounds__(kGridBT, 1)
   s.mpad = L.mpad;
   s.g64 = reinterpret_cast<double*>(p.ws + L.g64_off);
   s.g32l = reinterpret_cast<float*>(p.ws + L.g32_off);
-  s.linv = reinterpret_cast<double*>(p.ws + L.linv_off);
   s.sinv = reinterpret_cast<double*>(p.ws + L.sinv_off);
   s.xhi = reinterpret_cast<float*>(p.ws + L.xhi_off);
   s.xlo = reinterpret_cast<float*>(p.ws + L.xlo_off);

@@ -40,8 +40,8 @@ __host__ __device__ inline int round_up(int v, int q) { return (v + q - 1) / q *
 // Global workspace of a large solve.
 struct LargeLayout {
   int n, m, npad, mpad, nblk, np;
-  size_t ctl_off, info_off, v_off, a_off, p_off, g64_off, g32_off, linv_off, sinv_off, xhi_off,
-      xlo_off, cp_off, total;
+  size_t ctl_off, info_off, v_off, a_off, p_off, g64_off, g32_off, sinv_off, xhi_off, xlo_off,
+      cp_off, total;
 };
 __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   LargeLayout L;
@@ -67,8 +67,6 @@ __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   off += al(size_t(L.npad) * L.npad * 8);
   L.g32_off = off;
   off += al(size_t(L.npad) * L.npad * 4);
-  L.linv_off = off;
-  off += al(2 * size_t(L.nblk) * kLB * kLB * 8);  // inverses and their transposes
   L.sinv_off = off;
   off += al(4 * 32 * 33 * 8);                      // sub-block inverses of one step
   L.xhi_off = off;
@@ -478,16 +476,14 @@ __device__ void large_finish_gram(S& s, T* g) {
 
 // ---------------------------------------------------------------------------
 // Blocked Cholesky of the lower triangle of g (npad x npad), then the
-// inverses of the diagonal blocks into linv (and, resident in each CTA's
-// shared memory, the inverse of the block the CTA owns in the solves).
+// inverses of the diagonal blocks, each resident in the shared memory of the
+// CTA that owns the block in the solves.
 // Returns 0 or the 1-based index of the first non-positive pivot (uniform
 // over the grid).
 //
 // Step k (panel width 128):
-//   (a) one CTA factors the diagonal block in shared memory, in four 32-wide
-//       steps: one warp factors the 32 x 32 diagonal sub-block in registers
-//       and inverts it, the rows below are solved with that inverse, and the
-//       trailing part of the block is updated;
+//   (a) one CTA factors the diagonal block in shared memory (cta_chol128) and
+//       inverts its four 32 x 32 diagonal sub-blocks;
 //   (b) every warp takes panel rows and solves x L_kk^T = g_i with the four
 //       sub-block inverses (one lane per column, broadcasts by shuffle);
 //   (c) the lower 128 x 128 tiles right of the panel get g_ij -= L_ik L_jk^T
@@ -516,73 +512,266 @@ __device__ __forceinline__ void stage_block(T* dst, const T* g, size_t ld, int r
   }
 }
 
-// One warp factors the 32 x 32 lower block at sm[o][o] (pitch kPitch) and
-// writes its inverse to inv32[r * kSubPitch + c].  Returns 0 or the 1-based
-// failing pivot (the same in every lane).
+// Cholesky of the 128 x 128 block in shared memory (lower, pitch kPitch) by
+// the CTA: every thread owns up to three 4 x 4 tiles of the lower triangle in
+// registers, right-looking in 4-column panels with one barrier per panel.
+// Tiles are numbered down the columns, so that the tiles of one panel belong
+// to one or two warps: while these finish panel k + 1 (each thread factors the
+// 4 x 4 diagonal tile for itself), the other warps apply panel k to theirs.
+// Panel k's tiles are published in pb (two panels, 17 elements per tile); the
+// diagonal tile of panel k + 2, one update short, in dg (two tiles), and its
+// readers apply the missing update themselves, in the owner's order.
+// On return sm holds L, rd the reciprocals of its diagonal.  sflag: two slots.
+// Returns 0 or the 1-based index of the first non-positive pivot.
 //
-// Factor: Crout order, lane r holds row r in registers; step c forms
-// s_r = a_rc - sum_{k<c} l_rk l_ck (row c of L read back from shared memory,
-// the same address in every lane), l_cc = sqrt(s_c), l_rc = s_r / l_cc.
-// Inverse: lane c forms column c top-down, X_rc = -(sum_{c<=k<r} L_rk X_kc)
-// / l_rr.  Every division and square root goes through one reciprocal
-// square root per pivot (1 / l_cc = rsqrt(s_c)), kept for the inverse:
-// these are the long-latency operations of this sequential chain.
+// The chain is 128 reciprocal square roots (75 cycles each) and about as long
+// again in products, loads and barriers: 12 us, against some 85 us for 32-wide
+// blocks factored by one warp in Crout order.
+constexpr int kTileCholTiles = 3;
+constexpr int kTileCholPb = 2 * 32 * 17;
 template <typename T>
-__device__ __noinline__ int warp_chol32(T* sm, int o, T* inv32, int lane) {
-  T* Lr = sm + (o + lane) * kPitch + o;  // this lane's row
-  T idg[32];                              // 1 / l_cc (the same in every lane)
-  int bad = 0;
-  {
-    T a[32];
+__device__ __noinline__ int cta_chol128(T* sm, T* pb, T* dg, T* rd, volatile int* sflag) {
+  constexpr int TPT = kTileCholTiles, NB = kLB / 4;
+  static_assert(TPT * kGridBT >= NB * (NB + 1) / 2, "tiles");
+  bool mine[TPT];
+  int bi[TPT], bj[TPT];
+  T acc[TPT][4][4];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) a[j] = (j <= lane) ? Lr[j] : T(0);
+  for (int q = 0; q < TPT; ++q) {
+    const int t = threadIdx.x + q * kGridBT;
+    mine[q] = t < NB * (NB + 1) / 2;
+    // Column c starts at c NB - c (c - 1) / 2.
+    int c = int((2 * NB + 1 - sqrtf(float((2 * NB + 1) * (2 * NB + 1) - 8 * t))) * 0.5f);
+    c = min(max(c, 0), NB - 1);
+    while (c > 0 && c * NB - c * (c - 1) / 2 > t) --c;
+    while (c + 1 < NB && (c + 1) * NB - (c + 1) * c / 2 <= t) ++c;
+    bj[q] = c;
+    bi[q] = c + t - (c * NB - c * (c - 1) / 2);
+    if (!mine[q]) bi[q] = bj[q] = 0;
 #pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      const T* Lc = sm + (o + c) * kPitch + o;
-      T s0 = a[c], s1 = T(0);
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int k = 0; k < c; ++k) {
-        if (k & 1) {
-          s1 = fma(-a[k], Lc[k], s1);
-        } else {
-          s0 = fma(-a[k], Lc[k], s0);
+      for (int b = 0; b < 4; ++b)
+        acc[q][a][b] = mine[q] ? sm[(bi[q] * 4 + a) * kPitch + bj[q] * 4 + b] : T(0);
+  }
+  if (threadIdx.x < 2) sflag[threadIdx.x] = 0;
+  auto put_diag = [&](int t) {
+#pragma unroll
+    for (int q = 0; q < TPT; ++q) {
+      if (!mine[q] || bi[q] != t || bj[q] != t) continue;
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b <= a; ++b) dg[(t & 1) * 16 + a * 4 + b] = acc[q][a][b];
+    }
+  };
+  // acc -= L_{i,k} L_{j,k}^T with panel k.
+  auto update = [&](int q, int k) {
+    const T* pi = pb + (k & 1) * (NB * 17) + bi[q] * 17;
+    const T* pj = pb + (k & 1) * (NB * 17) + bj[q] * 17;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      T li[4], lj[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        li[a] = pi[a * 4 + c];
+        lj[a] = pj[a * 4 + c];
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[q][a][b] = fma(-li[a], lj[b], acc[q][a][b]);
+    }
+  };
+  // The tiles of column t (updated by panels < t) become L, published.
+  auto do_panel = [&](int t) {
+#pragma unroll
+    for (int q = 0; q < TPT; ++q) {
+      if (!mine[q] || bj[q] != t) continue;
+      T d[4][4], lc[4][4], il[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b <= a; ++b) d[a][b] = dg[(t & 1) * 16 + a * 4 + b];
+      if (t > 0) {
+        const T* pr = pb + ((t - 1) & 1) * (NB * 17) + t * 17;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          T l[4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) l[a] = pr[a * 4 + c];
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b) d[a][b] = fma(-l[a], l[b], d[a][b]);
         }
       }
-      const T sr = s0 + s1;
-      const T piv = __shfl_sync(0xffffffffu, sr, c);
-      if (!(piv > T(0)) && bad == 0) bad = c + 1;
-      const T il = rsqrt(piv);
-      idg[c] = il;
-      if (lane == c) {
-        a[c] = piv * il;
-      } else if (lane > c) {
-        a[c] = sr * il;
+      int bad = 0;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const T piv = d[c][c];
+        if (bad == 0 && !(piv > T(0))) bad = 4 * t + c + 1;
+        il[c] = rsqrt(piv);
+        lc[c][c] = piv * il[c];
+#pragma unroll
+        for (int a = c + 1; a < 4; ++a) lc[a][c] = d[a][c] * il[c];
+#pragma unroll
+        for (int a = c + 1; a < 4; ++a)
+#pragma unroll
+          for (int b = c + 1; b <= a; ++b) d[a][b] = fma(-lc[a][c], lc[b][c], d[a][b]);
       }
-      if (lane >= c) Lr[c] = a[c];
-      __syncwarp();
+      if (bi[q] == t) {
+        if (bad) sflag[t & 1] = bad;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          rd[4 * t + a] = il[a];
+#pragma unroll
+          for (int b = 0; b < 4; ++b) acc[q][a][b] = b <= a ? lc[a][b] : T(0);
+        }
+      } else {
+        T* dst = pb + (t & 1) * (NB * 17) + bi[q] * 17;
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            T x = acc[q][a][c];
+#pragma unroll
+            for (int e = 0; e < c; ++e) x = fma(-acc[q][a][e], lc[c][e], x);
+            acc[q][a][c] = x * il[c];
+            dst[a * 4 + c] = acc[q][a][c];
+          }
+      }
     }
+  };
+  put_diag(0);
+  put_diag(1);
+  __syncthreads();
+  do_panel(0);
+  __syncthreads();
+  int bad = sflag[0];
+#pragma unroll 1
+  for (int k = 0; bad == 0 && k + 1 < NB; ++k) {
+#pragma unroll
+    for (int q = 0; q < TPT; ++q)
+      if (mine[q] && bj[q] == k + 1) update(q, k);
+    do_panel(k + 1);
+#pragma unroll
+    for (int q = 0; q < TPT; ++q)
+      if (mine[q] && bj[q] > k + 1) update(q, k);
+    if (k + 2 < NB) put_diag(k + 2);
+    __syncthreads();
+    // Panel k + 2 notes its failure in the other slot, so every thread reads
+    // the same value here.
+    bad = sflag[(k + 1) & 1];
   }
-  if (bad) return bad;
-  T x[32];
+#pragma unroll
+  for (int q = 0; q < TPT; ++q)
+    if (mine[q])
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (bi[q] != bj[q] || b <= a) sm[(bi[q] * 4 + a) * kPitch + bj[q] * 4 + b] = acc[q][a][b];
+  __syncthreads();
+  return bad;
+}
+
+// Inverses of the four 32 x 32 diagonal sub-blocks of the factored block sm
+// (rd: the reciprocals of its diagonal) into inv[q] (pitch kSubPitch, zero
+// above the diagonal), a warp each: lane c forms column c top-down, X_rc =
+// -(sum_{k<r} L_rk X_kc) / l_rr (X_kc = 0 for k < c).  No barrier inside.
+template <typename T>
+__device__ __noinline__ void cta_sub_inverses(const T* sm, const T* rd, T* inv) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= 4) return;
+  const int o = 32 * warp;
+  T* X = inv + warp * 32 * kSubPitch;
   const T* L = sm + o * kPitch + o;
-#pragma unroll
+#pragma unroll 1
   for (int r = 0; r < 32; ++r) {
-    T a0 = T(0), a1 = T(0);
-#pragma unroll
-    for (int k = 0; k < r; ++k) {
-      if (k >= lane) {
-        if (k & 1) {
-          a1 = fma(L[r * kPitch + k], x[k], a1);
-        } else {
-          a0 = fma(L[r * kPitch + k], x[k], a0);
-        }
-      }
+    T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
+    const T* Lr = L + r * kPitch;
+    int k = 0;
+#pragma unroll 2
+    for (; k + 3 < r; k += 4) {
+      a0 = fma(Lr[k], X[k * kSubPitch + lane], a0);
+      a1 = fma(Lr[k + 1], X[(k + 1) * kSubPitch + lane], a1);
+      a2 = fma(Lr[k + 2], X[(k + 2) * kSubPitch + lane], a2);
+      a3 = fma(Lr[k + 3], X[(k + 3) * kSubPitch + lane], a3);
     }
-    x[r] = r < lane ? T(0) : (r == lane ? idg[r] : -(a0 + a1) * idg[r]);
+    for (; k < r; ++k) a0 = fma(Lr[k], X[k * kSubPitch + lane], a0);
+    const T il = rd[o + r];
+    X[r * kSubPitch + lane] = r < lane ? T(0) : (r == lane ? il : -((a0 + a1) + (a2 + a3)) * il);
+    __syncwarp();
+  }
+}
+
+// C = s A B for 32-row, 32-column blocks in shared memory (leading dimensions
+// pa, pb, pc; inner length K, a multiple of 4), the CTA's eight warps two 8 x
+// 8 tiles each (FP64: DMMA), then a barrier.
+template <typename T>
+__device__ __forceinline__ void cta_gemm32(T* C, int pc, const T* A, int pa, const T* B, int pb,
+                                           int K, T scale) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+  const int r0 = (warp >> 1) * 8, c0 = (warp & 1) * 16;
+  T acc[2][2] = {{T(0), T(0)}, {T(0), T(0)}};
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4) {
+      const double a = A[(r0 + gi) * pa + k + tg];
+      const double b0 = B[(k + tg) * pb + c0 + gi], b1 = B[(k + tg) * pb + c0 + 8 + gi];
+      dmma_8x8x4(acc[0], a, b0);
+      dmma_8x8x4(acc[1], a, b1);
+    }
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      const T a = A[(r0 + gi) * pa + k];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          acc[h][e] = fma(a, B[k * pb + c0 + 8 * h + 2 * tg + e], acc[h][e]);
+    }
   }
 #pragma unroll
-  for (int r = 0; r < 32; ++r) inv32[r * kSubPitch + lane] = x[r];
-  return 0;
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) C[(r0 + gi) * pc + c0 + 8 * h + 2 * tg + e] = scale * acc[h][e];
+  __syncthreads();
+}
+
+// In place, the inverse of the factored 128 x 128 block sm (lower, pitch
+// kPitch) from the inverses of its 32 x 32 diagonal blocks: block column by
+// block column, X_ij = -X_ii sum_{j<=k<i} L_ik X_kj (block column j of L is
+// not needed by the later ones).  tmp: 32 x kSubPitch.
+template <typename T>
+__device__ __noinline__ void cta_inverse128(T* sm, const T* inv, T* tmp) {
+  for (int j = 0; j < 4; ++j) {
+    for (int i = j + 1; i < 4; ++i) {
+      // X_jj for k = j, then the rows j + 1 .. i - 1 of this block column.
+      cta_gemm32<T>(tmp, kSubPitch, sm + 32 * i * kPitch + 32 * j, kPitch,
+                    inv + j * 32 * kSubPitch, kSubPitch, 32, T(1));
+      if (i > j + 1) {
+        // The rest of the sum into the block's own place, then both added.
+        cta_gemm32<T>(sm + 32 * i * kPitch + 32 * j, kPitch,
+                      sm + 32 * i * kPitch + 32 * (j + 1), kPitch,
+                      sm + 32 * (j + 1) * kPitch + 32 * j, kPitch, 32 * (i - j - 1), T(1));
+        for (int e = threadIdx.x; e < 1024; e += kGridBT)
+          tmp[(e >> 5) * kSubPitch + (e & 31)] +=
+              sm[(32 * i + (e >> 5)) * kPitch + 32 * j + (e & 31)];
+        __syncthreads();
+      }
+      cta_gemm32<T>(sm + 32 * i * kPitch + 32 * j, kPitch, inv + i * 32 * kSubPitch, kSubPitch,
+                    tmp, kSubPitch, 32, T(-1));
+    }
+    // X_jj: rows of L_jj are not needed any more (the columns to its right
+    // do not touch block column j).
+    for (int e = threadIdx.x; e < 1024; e += kGridBT)
+      sm[(32 * j + (e >> 5)) * kPitch + 32 * j + (e & 31)] =
+          inv[j * 32 * kSubPitch + (e >> 5) * kSubPitch + (e & 31)];
+    __syncthreads();
+  }
 }
 
 template <typename T, class S>
@@ -591,78 +780,35 @@ __device__ int large_cholesky(S& s, T* g) {
   int* info = s.linfo;
   T* sm = reinterpret_cast<T*>(s.arena);   // staged 128 x 128 block (pitch kPitch)
   T* sinv = sm + kLB * kPitch;              // 4 sub-block inverses (pitch kSubPitch)
-  volatile int* sflag = reinterpret_cast<volatile int*>(sinv + 4 * 32 * kSubPitch);
+  T* pbuf = sinv + 4 * 32 * kSubPitch;      // published panels of cta_chol128
+  T* dbuf = pbuf + kTileCholPb;
+  T* rdiag = dbuf + 32;                     // reciprocal diagonal
+  T* tmp32 = rdiag + kLB;                   // 32 x kSubPitch
+  volatile int* sflag = reinterpret_cast<volatile int*>(tmp32 + 32 * kSubPitch);
+  static_assert((size_t(kLB) * kPitch + 5 * 32 * kSubPitch + kTileCholPb + 32 + kLB) *
+                        sizeof(double) + 16 <= kArenaBytes, "the factorisation's shared memory");
   T* ginv = reinterpret_cast<T*>(s.sinv);   // the same inverses in global memory
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gwarp = blockIdx.x * (kGridBT / 32) + warp, nwarps = gridDim.x * (kGridBT / 32);
   if (s.tid == 0) *info = 0;
   s.sync();
   QTQP_TIC();
-  // (a) Factor the diagonal block starting at column k0 (the calling CTA):
-  // in shared memory, 32 columns at a time, then back to g with the four
+  // (a) Factor the diagonal block starting at column k0 (the calling CTA) in
+  // shared memory, then back to g with the reciprocal diagonal and the four
   // 32 x 32 sub-block inverses (also to global memory, for the panel step).
   auto factor_diag = [&](int k0) {
-    QTQP_TIC();
     stage_block(sm, g, npad, k0, k0, true);
     __syncthreads();
-    QTQP_TOC(kPhNormalize);
-    int bad = 0;
-    for (int q = 0; q < 4 && !bad; ++q) {
-      const int o = 32 * q;
-      QTQP_RETIC();
-      if (warp == 0) {
-        const int b = warp_chol32(sm, o, sinv + q * 32 * kSubPitch, lane);
-        if (lane == 0) *sflag = b ? o + b : 0;
-      }
-      __syncthreads();
-      QTQP_TOC(kPhStep);
-      QTQP_RETIC();
-      bad = *sflag;
-      if (bad) break;
-      // Rows below the sub-block: x = row inv(L_qq)^T (thread per row).
-      const T* iq = sinv + q * 32 * kSubPitch;
-      const int rows = kLB - o - 32;
-      if (int(threadIdx.x) < rows) {
-        T* row = sm + (o + 32 + threadIdx.x) * kPitch + o;
-        T v[32];
-#pragma unroll
-        for (int l = 0; l < 32; ++l) v[l] = row[l];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          T acc = T(0);
-#pragma unroll
-          for (int l = 0; l <= j; ++l) acc = fma(v[l], iq[j * kSubPitch + l], acc);
-          row[j] = acc;
-        }
-      }
-      __syncthreads();
-      // Trailing lower part of the block: a_ij -= sum_l a_il a_jl.
-      const int t0 = o + 32, tn = kLB - t0, cnt = tn * (tn + 1) / 2;
-      for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-        int i = int((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
-        while (i * (i + 1) / 2 > e) --i;
-        while ((i + 1) * (i + 2) / 2 <= e) ++i;
-        const int j = e - i * (i + 1) / 2;
-        const T* ri = sm + (t0 + i) * kPitch + o;
-        const T* rj = sm + (t0 + j) * kPitch + o;
-        T acc0 = T(0), acc1 = T(0);
-#pragma unroll
-        for (int l = 0; l < 32; l += 2) {
-          acc0 = fma(ri[l], rj[l], acc0);
-          acc1 = fma(ri[l + 1], rj[l + 1], acc1);
-        }
-        sm[(t0 + i) * kPitch + t0 + j] -= acc0 + acc1;
-      }
-      __syncthreads();
-      QTQP_TOC(kPhOther);
-    }
+    const int bad = cta_chol128<T>(sm, pbuf, dbuf, rdiag, sflag);
     if (bad) {
       if (threadIdx.x == 0) atomicCAS(info, 0, k0 + bad);
     } else {
+      cta_sub_inverses<T>(sm, rdiag, sinv);
       for (int e = threadIdx.x; e < kLB * kLB; e += blockDim.x) {
         const int r = e >> 7, c = e & 127;
         if (c <= r) g[size_t(k0 + r) * npad + k0 + c] = sm[r * kPitch + c];
       }
+      __syncthreads();
       for (int e = threadIdx.x; e < 4 * 32 * kSubPitch; e += blockDim.x) ginv[e] = sinv[e];
     }
     __syncthreads();
@@ -838,48 +984,17 @@ __device__ int large_cholesky(S& s, T* g) {
   const int rc = *reinterpret_cast<volatile int*>(info);
   if (rc != 0) return rc;
   QTQP_RETIC();
-  // Inverses of the diagonal blocks: column c of inv(L_bb) by thread c.
-  T* lv = reinterpret_cast<T*>(s.linv);
-  for (int b = blockIdx.x; b < nblk; b += gridDim.x) {
-    const int b0 = b * kLB;
+  // Each CTA inverts the diagonal block it owns in the solves and keeps it
+  // resident in shared memory until the next factorisation.
+  if (int(blockIdx.x) < nblk) {
+    const int b0 = int(blockIdx.x) * kLB;
     stage_block(sm, g, npad, b0, b0, true);
     __syncthreads();
-    T* inv = lv + size_t(b) * kLB * kLB;                 // inv(L_bb), row-major
-    T* invt = lv + size_t(nblk + b) * kLB * kLB;         // its transpose
-    T* rdiag = sm + kLB * kPitch;  // 1 / L_rr
     if (threadIdx.x < kLB) rdiag[threadIdx.x] = T(1) / sm[threadIdx.x * kPitch + threadIdx.x];
     __syncthreads();
-    if (threadIdx.x < kLB) {
-      const int c = threadIdx.x;
-      // Column c of inv(L_bb) = row c of its transpose (contiguous for this
-      // thread): x_c = 1 / L_cc; x_r = -(sum_{c <= l < r} L_rl x_l) / L_rr.
-      T* xc = invt + size_t(c) * kLB;
-      for (int r = 0; r < c; ++r) xc[r] = T(0);
-      xc[c] = rdiag[c];
-      for (int r = c + 1; r < kLB; ++r) {
-        T acc0 = T(0), acc1 = T(0);
-        int l = c;
-        for (; l + 1 < r; l += 2) {
-          acc0 = fma(sm[r * kPitch + l], xc[l], acc0);
-          acc1 = fma(sm[r * kPitch + l + 1], xc[l + 1], acc1);
-        }
-        if (l < r) acc0 = fma(sm[r * kPitch + l], xc[l], acc0);
-        xc[r] = -(acc0 + acc1) * rdiag[r];
-      }
-    }
+    cta_sub_inverses<T>(sm, rdiag, sinv);
     __syncthreads();
-    for (int e = threadIdx.x; e < kLB * kLB; e += blockDim.x) {
-      const int r = e >> 7, c = e & 127;
-      inv[e] = invt[size_t(c) * kLB + r];
-    }
-    __syncthreads();
-  }
-  s.sync();
-  // Each CTA keeps the inverse of the block it owns in the solves resident
-  // in shared memory until the next factorisation.
-  if (int(blockIdx.x) < nblk) {
-    stage_block(sm, lv + size_t(blockIdx.x) * kLB * kLB, kLB, 0, 0, false);
-    __syncthreads();
+    cta_inverse128<T>(sm, sinv, tmp32);
   }
   QTQP_TOC(kPhLgInv);
   return 0;
