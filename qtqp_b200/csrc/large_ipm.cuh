@@ -338,7 +338,7 @@ __device__ void large_gram_tc(S& s) {
     tc::fence_before_sync();
     __syncthreads();  // TMEM free for the next tile's MMAs
   }
-  if (threadIdx.x == 0 && *failed) atomicExch(&s.gctl->err, 1);
+  if (threadIdx.x == 0 && *failed) grid_fail(s.gctl);
 }
 
 // G_lower = A^T diag(1/Ry) A in FP64 on the FP64 tensor cores (DMMA,
