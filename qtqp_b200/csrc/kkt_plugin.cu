@@ -1,9 +1,13 @@
 // Dense KKT backend behind the direct.LinearSolver plugin interface
 // (src/qtqp/direct.py:49-109), algorithm of src/qtqp/solvers_dense.py:99-142.
-// Each call is one single-block launch on the caller's stream; the workspace
-// holds A, P_off, the factor and the vectors (layout of dense_ipm.cuh with
-// every region in global memory) behind a small header.
-#include "dense_ipm.cuh"
+// Each call is one launch on the caller's stream: of a single block, or of the
+// whole GPU from kKktGridN variables on (kkt_grid.cuh; the FP64 factor only).
+// The workspace holds A, P_off, the factor and the vectors (layout of
+// dense_ipm.cuh with every region in global memory) behind a small header, and
+// the whole-GPU form's regions after them.
+#include <algorithm>
+
+#include "kkt_grid.cuh"
 
 namespace qtqp {
 
@@ -14,6 +18,8 @@ __host__ __device__ inline size_t plugin_bytes(int n, int m) {
   const InstLayout L = plan_layout(n, m, 0);
   return kPluginHeader + L.global_bytes;
 }
+// Where the whole-GPU form's regions start.
+inline size_t grid_part(int n, int m) { return (plugin_bytes(n, m) + 255) & ~size_t(255); }
 
 __device__ inline void plugin_bind(DenseIpm<kPluginThreads>& s, int n, int m, char* ws,
                                    double* red) {
@@ -29,14 +35,17 @@ __global__ void __launch_bounds__(kPluginThreads)
     plugin_set_kernel(int n, int m, const double* a, const double* p_off, char* ws) {
   DenseIpm<kPluginThreads> s;
   plugin_bind(s, n, m, ws, nullptr);
-  for (int idx = threadIdx.x; idx < m * n; idx += kPluginThreads) {
+  const int t0 = blockIdx.x * kPluginThreads + threadIdx.x, step = gridDim.x * kPluginThreads;
+  for (int idx = t0; idx < m * n; idx += step) {
     const int i = idx / n, j = idx - i * n;
     s.A[i * s.lda + j] = a[idx];
   }
-  for (int idx = threadIdx.x; idx < n * n; idx += kPluginThreads) {
+  for (int idx = t0; idx < n * n; idx += step) {
     const int i = idx / n, j = idx - i * n;
     s.P[i * s.ldp + j] = (i == j) ? 0.0 : p_off[idx];
   }
+  // The factor's precision: none yet.
+  if (t0 == 0) *reinterpret_cast<int*>(ws) = 0;
 }
 
 __global__ void __launch_bounds__(kPluginThreads)
@@ -117,7 +126,7 @@ using namespace qtqp;
 
 extern "C" size_t qtqp_kkt_dense_workspace_bytes(int32_t n, int32_t m) {
   if (n < 1 || m < 1) return 0;
-  return plugin_bytes(n, m);
+  return kkt_grid_form(n) ? grid_part(n, m) + kkt_grid_bytes(n, m) : plugin_bytes(n, m);
 }
 
 extern "C" int qtqp_kkt_dense_set(int32_t n, int32_t m, const double* d_a,
@@ -125,9 +134,14 @@ extern "C" int qtqp_kkt_dense_set(int32_t n, int32_t m, const double* d_a,
   int rc = plugin_args(n, m, d_ws);
   if (rc) return rc;
   if (d_a == nullptr || d_p_off == nullptr) return fail(QTQP_ERR_BAD_ARG, "dense KKT: null A/P");
-  plugin_set_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      n, m, d_a, d_p_off, static_cast<char*>(d_ws));
-  return cuda_check(cudaGetLastError(), "plugin_set_kernel launch");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  char* ws = static_cast<char*>(d_ws);
+  const int blocks = int(std::min<int64_t>((int64_t(m) * n + kPluginThreads - 1) / kPluginThreads,
+                                           4 * 148));
+  plugin_set_kernel<<<blocks, kPluginThreads, 0, st>>>(n, m, d_a, d_p_off, ws);
+  rc = cuda_check(cudaGetLastError(), "plugin_set_kernel launch");
+  if (rc || !kkt_grid_form(n)) return rc;
+  return kkt_grid_reset(ws + grid_part(n, m), st);
 }
 
 extern "C" int qtqp_kkt_dense_factorize(int32_t n, int32_t m, const double* d_diag,
@@ -139,8 +153,13 @@ extern "C" int qtqp_kkt_dense_factorize(int32_t n, int32_t m, const double* d_di
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: null diag/info");
   if (precision != QTQP_PREC_FP64 && precision != QTQP_PREC_MIXED)
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: unknown precision");
+  char* ws = static_cast<char*>(d_ws);
+  // (An FP32 factor keeps the single block's plain FP32 arithmetic.)
+  if (kkt_grid_form(n) && precision == QTQP_PREC_FP64)
+    return kkt_grid_factorize(n, m, d_diag, ws, kPluginHeader, ws + grid_part(n, m), d_info,
+                              static_cast<cudaStream_t>(stream));
   plugin_factorize_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      n, m, d_diag, precision, static_cast<char*>(d_ws), d_info);
+      n, m, d_diag, precision, ws, d_info);
   return cuda_check(cudaGetLastError(), "plugin_factorize_kernel launch");
 }
 
@@ -150,8 +169,12 @@ extern "C" int qtqp_kkt_dense_solve(int32_t n, int32_t m, const double* d_rhs, d
   if (rc) return rc;
   if (d_rhs == nullptr || d_out == nullptr || d_rhs == d_out)
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: rhs/out must be distinct device vectors");
-  plugin_solve_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      n, m, d_rhs, d_out, static_cast<char*>(d_ws));
+  char* ws = static_cast<char*>(d_ws);
+  if (kkt_grid_form(n))
+    return kkt_grid_solve(n, m, d_rhs, d_out, ws, kPluginHeader, ws + grid_part(n, m),
+                          static_cast<cudaStream_t>(stream));
+  plugin_solve_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(n, m, d_rhs,
+                                                                                  d_out, ws);
   return cuda_check(cudaGetLastError(), "plugin_solve_kernel launch");
 }
 
@@ -161,8 +184,12 @@ extern "C" int qtqp_kkt_dense_matvec(int32_t n, int32_t m, const double* d_x, do
   if (rc) return rc;
   if (d_x == nullptr || d_out == nullptr || d_x == d_out)
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: x/out must be distinct device vectors");
-  plugin_matvec_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      n, m, d_x, d_out, static_cast<char*>(d_ws));
+  char* ws = static_cast<char*>(d_ws);
+  if (kkt_grid_form(n))
+    return kkt_grid_matvec(n, m, d_x, d_out, ws, kPluginHeader, ws + grid_part(n, m),
+                           static_cast<cudaStream_t>(stream));
+  plugin_matvec_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(n, m, d_x,
+                                                                                   d_out, ws);
   return cuda_check(cudaGetLastError(), "plugin_matvec_kernel launch");
 }
 

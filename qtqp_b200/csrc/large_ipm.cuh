@@ -350,7 +350,7 @@ __device__ void large_gram_tc(S& s) {
 // m, n are zero-filled.
 template <class S>
 __device__ __noinline__ void large_gram_dmma(S& s) {
-  const int n = s.n, m = s.m, npad = s.npad;
+  const int n = s.n, m = s.m, npad = s.npad, lda = s.lda;
   const double* A = s.A;
   const double* iry = s.vec(kPI) + n;  // 1 / Ry
   constexpr int KS = 16;               // rows per slice
@@ -371,9 +371,9 @@ __device__ __noinline__ void large_gram_dmma(S& s) {
     for (int q = 0; q < 8; ++q) {
       const int e = threadIdx.x + q * kGridBT, r = e >> 7, c = e & 127, i = r0 + r;
       const bool ok = i < m;
-      cp_async8(sa + r * LP + c, A + (ok && i0 + c < n ? size_t(i) * n + i0 + c : 0),
+      cp_async8(sa + r * LP + c, A + (ok && i0 + c < n ? size_t(i) * lda + i0 + c : 0),
                 ok && i0 + c < n);
-      cp_async8(sb + r * LP + c, A + (ok && j0 + c < n ? size_t(i) * n + j0 + c : 0),
+      cp_async8(sb + r * LP + c, A + (ok && j0 + c < n ? size_t(i) * lda + j0 + c : 0),
                 ok && j0 + c < n);
     }
     if (threadIdx.x < KS) {
@@ -462,7 +462,7 @@ __device__ void large_finish_gram(S& s, T* g) {
       g[e] = (i == j) ? T(1) : T(0);
       continue;
     }
-    double base = P[size_t(i) * n + j];
+    double base = P[size_t(i) * s.ldp + j];
     if (i == j) base += reg[i];
     const T v = T(base) + g[e];
     g[e] = v;
@@ -1224,6 +1224,12 @@ __device__ void large_chol_solve(S& s, T* v, T* w) {
     if (threadIdx.x == 0) flag_publish(gc, j, gen_bwd);
   }
   s.sync();
+  // The KKT backend (no options) has no result record to report a wait that
+  // gave up: its solution becomes NaN.
+  if (s.o == nullptr && __syncthreads_or(*reinterpret_cast<volatile int*>(&gc->err) != 0)) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) v[k] = T(NAN);
+    __syncthreads();
+  }
   QTQP_TOC(kPhLgBwd);
 }
 
