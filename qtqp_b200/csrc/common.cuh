@@ -23,6 +23,18 @@ __device__ __forceinline__ double nanmax(double a, double b) {
   return (a != a || b != b) ? __longlong_as_double(0x7ff8000000000000ll) : fmax(a, b);
 }
 
+// A double as a signed integer of the same order, and back: the block
+// reductions take their maxima in integers (a compare and a select; the NaN
+// test and FP64 maximum of nanmax cost three times as much).  A NaN without
+// its sign bit, which is what fabs and nanmax give, is above every number.
+__device__ __forceinline__ long long max_key(double v) {
+  const long long i = __double_as_longlong(v);
+  return i ^ ((i >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double from_max_key(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+
 // The IPM's heavy phases are compiled as separate device functions: each then
 // gets its own register allocation, which keeps the long solve loop's live
 // state from spilling into the phases' inner loops.
@@ -48,17 +60,17 @@ __device__ __forceinline__ void block_reduce(double (&sums)[NS > 0 ? NS : 1],
   // site, and fully unrolled they made up much of the per-iteration code
   // that competes for the instruction cache.  The order of the operations
   // is the same either way.
+  long long keys[NM > 0 ? NM : 1];
+#pragma unroll
+  for (int k = 0; k < NM; ++k) keys[k] = max_key(maxs[k]);
 #pragma unroll 1
   for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
     for (int k = 0; k < NS; ++k) sums[k] += __shfl_xor_sync(0xffffffffu, sums[k], off);
 #pragma unroll
-    for (int k = 0; k < NM; ++k)
-      maxs[k] = nanmax(maxs[k], __shfl_xor_sync(0xffffffffu, maxs[k], off));
+    for (int k = 0; k < NM; ++k) keys[k] = max(keys[k], __shfl_xor_sync(0xffffffffu, keys[k], off));
   }
-  if constexpr (NW == 1) {
-    return;
-  } else {
+  if constexpr (NW > 1) {
     double* buf = red + phase * (NW * kRedMax);
     phase ^= 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -66,23 +78,26 @@ __device__ __forceinline__ void block_reduce(double (&sums)[NS > 0 ? NS : 1],
 #pragma unroll
       for (int k = 0; k < NS; ++k) buf[warp * kRedMax + k] = sums[k];
 #pragma unroll
-      for (int k = 0; k < NM; ++k) buf[warp * kRedMax + NS + k] = maxs[k];
+      for (int k = 0; k < NM; ++k) buf[warp * kRedMax + NS + k] = __longlong_as_double(keys[k]);
     }
     __syncthreads();
+    // Lane l starts from warp l % NW's values; log2(NW) shuffles combine them.
+    const double* mine = buf + (lane & (NW - 1)) * kRedMax;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) sums[k] = 0.0;
+    for (int k = 0; k < NS; ++k) sums[k] = mine[k];
 #pragma unroll
-    for (int k = 0; k < NM; ++k) maxs[k] = buf[NS + k];
+    for (int k = 0; k < NM; ++k) keys[k] = __double_as_longlong(mine[NS + k]);
 #pragma unroll 1
-    for (int w = 0; w < NW; ++w) {
+    for (int off = NW / 2; off > 0; off >>= 1) {
 #pragma unroll
-      for (int k = 0; k < NS; ++k) sums[k] += buf[w * kRedMax + k];
-      if (w > 0) {
+      for (int k = 0; k < NS; ++k) sums[k] += __shfl_xor_sync(0xffffffffu, sums[k], off);
 #pragma unroll
-        for (int k = 0; k < NM; ++k) maxs[k] = nanmax(maxs[k], buf[w * kRedMax + NS + k]);
-      }
+      for (int k = 0; k < NM; ++k)
+        keys[k] = max(keys[k], __shfl_xor_sync(0xffffffffu, keys[k], off));
     }
   }
+#pragma unroll
+  for (int k = 0; k < NM; ++k) maxs[k] = from_max_key(keys[k]);
 }
 
 // A barrier for the whole group (one thread block).

@@ -52,7 +52,7 @@ __host__ __device__ inline size_t round16(size_t b) { return (b + 15) & ~size_t(
 // Panel buffer (PB): the tile Cholesky's two panels of (n+3)/4 tiles of
 // 4 x 4, each tile padded to 17 elements so that lanes reading different
 // tiles hit different banks; outside the factorisation, the staged column
-// sums of fused_products (up to 8 warps x n) and a vector of n.
+// sums of dense_products (up to 8 warps x n).
 __host__ __device__ inline size_t panel_buf_elems(int n) {
   return size_t(34) * ((n + 3) >> 2) + size_t(2) * n;
 }
@@ -341,14 +341,17 @@ struct Ipm {
   }
   __device__ __forceinline__ float* g32() const { return reinterpret_cast<float*>(G); }
 
-  // Lanes cooperating on one dot product when K outputs share the block.
-  __device__ __forceinline__ int lanes_for(int K) const {
-    int s = 1;
-    while (s < 32 && K * s * 2 <= NT) s <<= 1;
-    return s;
+  // log2 of the lanes cooperating on one dot product when K outputs share the
+  // block: the largest power of two S <= 32 with K S <= NT (1 when K > NT).
+  __device__ __forceinline__ int lanes_log2(int K) const {
+    if constexpr ((NT & (NT - 1)) == 0) {  // no division: a call costs 350 cycles less
+      return max(0, min(5, 31 - __clz(NT) - (K > 1 ? 32 - __clz(K - 1) : 0)));
+    } else {
+      return K >= NT ? 0 : min(5, 31 - __clz(NT / K));
+    }
   }
 
-  // out_k = sum_{i < len} body(k, i) for k < K, S = lanes_for(K) lanes per
+  // out_k = sum_{i < len} body(k, i) for k < K, S = 2^lanes_log2(K) lanes per
   // output.  The S lanes of an output are strided across the warp (lane =
   // s * (32/S) + g) so that neighbouring lanes work on neighbouring outputs;
   // their partial sums are combined with xor shuffles, and lane s == 0 calls
@@ -356,11 +359,12 @@ struct Ipm {
   template <int NACC, bool MAXOP = false, int FORCE_S = 0, typename AccT = double,
             typename Body, typename Epi>
   __device__ __forceinline__ void rowdot(int K, int len, Body body, Epi epi) const {
-    const int S = FORCE_S > 0 ? FORCE_S : lanes_for(K);
-    const int per_warp = 32 / S;
+    static_assert(FORCE_S == 0 || FORCE_S == 32, "a warp per output or the automatic split");
+    const int ls = FORCE_S > 0 ? 5 : lanes_log2(K);
+    const int S = 1 << ls, per_warp = 32 >> ls;
     const int tid = this->tid;
     const int lane = tid & 31, warp = tid >> 5;
-    const int s = lane / per_warp, g = lane - s * per_warp;
+    const int s = lane >> (5 - ls), g = lane & (per_warp - 1);
     const int per_pass = (NT / 32) * per_warp;
     for (int k0 = 0; k0 < K; k0 += per_pass) {
       const int k = k0 + warp * per_warp + g;
@@ -639,7 +643,7 @@ struct Ipm {
         for (int b = 0; b < 4; ++b) acc[q][a][b] = T(0);
     }
     if constexpr (sizeof(T) == 8) {
-      // FP64 Gram on the FP64 tensor cores: each warp forms 8 x 8 lower
+      // FP64 Gram on the FP64 tensor cores: each warp forms 16 x 16 lower
       // blocks of A^T diag(1/Ry) A with mma.sync m8n8k4 (DMMA) over 4-row
       // slices of A, writes them to g, and each thread then reads its tiles.
       gram_dmma(g);
@@ -711,57 +715,69 @@ struct Ipm {
     return info;
   }
 
-  // Lower 8 x 8 blocks of the FP64 Gram A^T diag(1/Ry) A into g (entries
+  // Lower 16 x 16 blocks of the FP64 Gram A^T diag(1/Ry) A into g (entries
   // i >= j, i, j < n), one warp per block, on the FP64 tensor cores: for each
   // 4-row slice of A, lane l holds a = A[r + l%4][I + l/4] / Ry and
-  // b = A[r + l%4][J + l/4] (dmma_8x8x4's fragment layout), rows past m and
-  // columns past n are zero.  Ends with a barrier.
+  // b = A[r + l%4][J + l/4] (dmma_8x8x4's fragment layout) of the block's two
+  // row and column halves, rows past m and columns past n are zero.  Ends with
+  // a barrier.
   __device__ __forceinline__ void gram_dmma(double* g) {
     QTQP_LOCALS;
     const double* iry = vec(kPI) + n;  // 1 / Ry
     const int lane = tid & 31, warp = tid >> 5;
     const int lr = lane & 3, lc = lane >> 2;
-    const int n8 = (n + 7) >> 3;
-    const int nblk = n8 * (n8 + 1) / 2;
+    const int n16 = (n + 15) >> 4;
+    const int nblk = n16 * (n16 + 1) / 2;
+#pragma unroll 1
     for (int t = warp; t < nblk; t += NT / 32) {
-      int bi8 = int((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
-      while (bi8 * (bi8 + 1) / 2 > t) --bi8;
-      while ((bi8 + 1) * (bi8 + 2) / 2 <= t) ++bi8;
-      const int bj8 = t - bi8 * (bi8 + 1) / 2;
-      const int ci = bi8 * 8 + lc, cj = bj8 * 8 + lc;
-      const bool ci_ok = ci < n, cj_ok = cj < n;
-      double d[2] = {0.0, 0.0};
-      int r = 0;
-      // Four slices per step with their loads issued first (A may come from
-      // L2 when it does not fit on chip); the products accumulate in the
-      // same order as one slice at a time.
-      for (; r + 16 <= m; r += 16) {
-        double a[4], b[4];
+      int bi = 0;
+      while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+      const int bj = t - bi * (bi + 1) / 2;
+      int ci[2], cj[2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+      for (int h = 0; h < 2; ++h) {
+        ci[h] = bi * 16 + 8 * h + lc;
+        cj[h] = bj * 16 + 8 * h + lc;
+      }
+      double d[2][2][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) d[h][q][0] = d[h][q][1] = 0.0;
+      // Two slices per step, their loads issued first (A may come from L2
+      // when it does not fit on chip); the products accumulate in row order.
+#pragma unroll 1
+      for (int r = 0; r < m; r += 8) {
+        double a[2][2], b[2][2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
           const int rr = r + 4 * u + lr;
+          const bool in = rr < m;
           const double* row = A + rr * lda;
-          a[u] = ci_ok ? row[ci] * iry[rr] : 0.0;
-          b[u] = cj_ok ? row[cj] : 0.0;
+          const double w = in ? iry[rr] : 0.0;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            a[u][h] = in && ci[h] < n ? row[ci[h]] * w : 0.0;
+            b[u][h] = in && cj[h] < n ? row[cj[h]] : 0.0;
+          }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) dmma_8x8x4(d, a[u], b[u]);
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) dmma_8x8x4(d[h][q], a[u][h], b[u][q]);
       }
-      for (; r < m; r += 4) {
-        const int rr = r + lr;
-        double a = 0.0, b = 0.0;
-        if (rr < m) {
-          const double* row = A + rr * lda;
-          if (ci_ok) a = row[ci] * iry[rr];
-          if (cj_ok) b = row[cj];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int i = ci[h], j = bj * 16 + 8 * q + 2 * lr;
+          if (i < n) {
+            if (j <= i) g[i * ldg + j] = d[h][q][0];
+            if (j + 1 <= i) g[i * ldg + j + 1] = d[h][q][1];
+          }
         }
-        dmma_8x8x4(d, a, b);
-      }
-      const int i = bi8 * 8 + lc, j = bj8 * 8 + 2 * lr;
-      if (i < n) {
-        if (j <= i) g[i * ldg + j] = d[0];
-        if (j + 1 <= i) g[i * ldg + j + 1] = d[1];
-      }
     }
     sync();
   }
@@ -880,21 +896,24 @@ struct Ipm {
       T ld[4][4];
       const int f = diag_factor(t, ld);
       if (f != 0) {
-        *s_info = f;
+        s_info[t & 1] = f;
         return;
       }
 #pragma unroll
       for (int q = 0; q < TPT; ++q)
         if (mine[q] && bj[q] == t) finish_panel(q, t, ld);
     };
-    __shared__ int s_info;
-    if (tid == 0) s_info = 0;
+    // A failure is noted in the slot of the panel's parity, which the next
+    // panel does not write, so every thread reads the same value after the
+    // barrier.
+    __shared__ int s_info[2];
+    if (tid < 2) s_info[tid] = 0;
     put_diag(0);
     put_diag(1);
     sync();
-    do_panel(0, &s_info);
+    do_panel(0, s_info);
     sync();
-    int info = s_info;
+    int info = s_info[0];
     for (int kb = 0; info == 0 && kb + 1 < nb; ++kb) {
 #pragma unroll
       for (int q = 0; q < TPT; ++q) {
@@ -916,10 +935,10 @@ struct Ipm {
             for (int b = 0; b < 4; ++b) acc[q][a][b] = fma(-li[a], lj[b], acc[q][a][b]);
         }
       }
-      do_panel(kb + 1, &s_info);
+      do_panel(kb + 1, s_info);
       if (kb + 2 < nb) put_diag(kb + 2);
       sync();
-      info = s_info;
+      info = s_info[(kb + 1) & 1];
     }
     if (info == 0) {
 #pragma unroll
@@ -1047,76 +1066,63 @@ struct Ipm {
     return 0;
   }
 
-  // In-place inverse of each 32x32 lower-triangular diagonal block of L,
-  // top-down: X_cc = 1 / L_cc, X_rc = -(sum_{c<=k<r} L_rk X_kc) / L_rr for
-  // r > c.  Both Cholesky variants already store 1 / L_jj on the diagonal,
-  // which is also the inverse's diagonal.  Column c of X keeps X_kc (k > c)
-  // in the block's unused upper triangle at (c, k), so with the diagonal
-  // U_ck = X_kc for every k >= c; L_rk is the same entry for every column (a
-  // broadcast).  A block gets a team of P warps (P = 1, 2 or 4, as many as
-  // the block's warps allow) and each column P neighbouring lanes of one
-  // warp, which split the row's dot product (strided over k, combined by
-  // xor shuffles), so the columns of a warp need no barrier but __syncwarp.
-  // The loops stay rolled: the batch kernel runs several QPs per SM at
-  // different phases of the IPM, and their code competes for the
-  // instruction cache.  After a barrier the columns are copied from the
-  // upper triangles into the lower ones.
+  // In-place inverse of each 32x32 lower-triangular diagonal block of L (the
+  // last one smaller), whose diagonal holds 1 / L_jj already, by doubling:
+  // with the s x s diagonal blocks inverted, the block below each pair's first
+  // becomes X21 = -X22 (L21 X11), s = 1, 2, 4, 8, 16.  The transpose of T = L21
+  // X11 is formed in the unused upper triangle, L21's mirror image.  Two barriers per level,
+  // dots of at most s products: 3k cycles for n = 24 (column by column, 31
+  // dependent steps with shuffles, 17k).
   template <typename T>
   QTQP_PHASE void invert_diag_blocks(T* g) {
     QTQP_LOCALS;
     QTQP_TIC();
-    const int warp = tid >> 5, lane = tid & 31;
-    constexpr int NW = NT / 32;
     const int nblk = (n + 31) >> 5;
-    int lanes = 1;  // P, the lanes per column
-    while (lanes < 4 && 2 * lanes * nblk <= NW) lanes <<= 1;
-    const int teams = NW / lanes, team = warp / lanes;
-    const int c = (warp % lanes) * (32 / lanes) + lane / lanes, sub = lane % lanes;
-    for (int blk = team; blk < nblk; blk += teams) {
-      const int kb = blk * 32, bs = min(32, n - kb);
-      T* L = g + kb * ldg + kb;
-      T* U = L + c * ldg;  // row c: U[k] = X_kc for k >= c
 #pragma unroll 1
-      for (int r = 1; r < bs; ++r) {
-        const T* Lr = L + r * ldg;
-        T acc = T(0);
-        // Four entries per lane and step, loads issued ahead of the FMAs.
+    for (int ls = 0; ls < 5; ++ls) {
+      const int s = 1 << ls;
 #pragma unroll 1
-        for (int k0 = c + sub; k0 < r; k0 += 4 * lanes) {
-          T lv[4], uv[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u * lanes;
-            lv[u] = k < r ? Lr[k] : T(0);
-            uv[u] = k < r ? U[k] : T(0);
+      for (int half = 0; half < 2; ++half) {
+#pragma unroll 1
+        for (int e = tid; e < nblk << (4 + ls); e += NT) {
+          // Element (i, j) of pair p of 32-block b.
+          const int j = e & (s - 1), i = (e >> ls) & (s - 1);
+          const int p = (e >> (2 * ls)) & ((16 >> ls) - 1), b = e >> (4 + ls);
+          const int r0 = b * 32 + p * 2 * s;  // the pair's first row
+          if (r0 + s + i >= n) continue;
+          T* row = g + (r0 + s + i) * ldg + r0;   // row i of [L21 X22]
+          T* up = g + (r0 + j) * ldg + r0 + s;    // T_kj at up[k]
+          T a0 = T(0), a1 = T(0);
+          if (half == 0) {  // T_ij = sum_{k >= j} L21_ik X11_kj
+            const T* x = g + r0 * ldg + r0 + j;
+            int k = j;
+            for (; k + 1 < s; k += 2) {
+              a0 = fma(row[k], x[k * ldg], a0);
+              a1 = fma(row[k + 1], x[(k + 1) * ldg], a1);
+            }
+            if (k < s) a0 = fma(row[k], x[k * ldg], a0);
+            up[i] = a0 + a1;
+          } else {  // X21_ij = -sum_{k <= i} X22_ik T_kj
+            int k = 0;
+            for (; k < i; k += 2) {
+              a0 = fma(row[s + k], up[k], a0);
+              a1 = fma(row[s + k + 1], up[k + 1], a1);
+            }
+            if (k == i) a0 = fma(row[s + k], up[k], a0);
+            row[j] = -(a0 + a1);
           }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) acc = fma(lv[u], uv[u], acc);
         }
-        for (int o = 1; o < lanes; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (sub == 0 && c < r) U[r] = -acc * Lr[r];
-        __syncwarp();
+        sync();
       }
     }
-    // Every column reads row r of L up to r - 1, including the columns of
-    // the team's other warps, so the copy waits for all of them.
-    sync();
-    for (int blk = team; blk < nblk; blk += teams) {
-      const int kb = blk * 32, bs = min(32, n - kb);
-      T* L = g + kb * ldg + kb;
-      const T* U = L + c * ldg;
-#pragma unroll 1
-      for (int r = c + 1 + sub; r < bs; r += lanes) L[r * ldg + c] = U[r];
-    }
-    sync();
     QTQP_TOC(kPhInv);
   }
 
   // Solves L L^T v = v in place with the block-inverted factor: forward
   // z_b = X_bb (v_b - sum_{c<b} L_bc z_c), backward x_b = X_bb^T (z_b -
   // sum_{c>b} L_cb^T x_c), two barriers per 32-block; w is n scratch entries.
-  // Each phase is a set of row dots (rowdot: several lanes per row, partial
-  // sums combined by shuffles), so no thread walks a 32-long chain alone.
+  // Each phase is a set of dots with several lanes each (block_mv), so no
+  // thread walks a 32-long chain alone.
   template <typename T>
   QTQP_PHASE void chol_solve(const T* g, T* v, T* w) {
     if constexpr (FMT == kFmtLarge) {
@@ -1125,44 +1131,55 @@ struct Ipm {
     }
     QTQP_LOCALS;
     const int nblk = (n + 31) >> 5;
+#pragma unroll 1
     for (int blk = 0; blk < nblk; ++blk) {
-      const int kb = blk * 32, bs = min(32, n - kb);
+      const int kb = blk * 32, bs = min(32, n - kb), rest = n - kb - bs;
       const T* gb = g + kb * ldg + kb;
-      rowdot<1, false, 0, T>(bs, bs,
-                [&](int r, int k, T* acc) {
-                  if (k <= r) acc[0] = fma(gb[r * ldg + k], v[kb + k], acc[0]);
-                },
-                [&](int r, T* acc) { w[kb + r] = acc[0]; });
-      sync();
-      if (kb + bs < n) {
-        const T* gl = g + (kb + bs) * ldg + kb;
-        rowdot<1, false, 0, T>(n - kb - bs, bs,
-                  [&](int i, int k, T* acc) {
-                    acc[0] = fma(gl[i * ldg + k], w[kb + k], acc[0]);
-                  },
-                  [&](int i, T* acc) { v[kb + bs + i] -= acc[0]; });
-        sync();
-      }
+      block_mv<T>(gb, ldg, 1, bs, bs, 1, v + kb, w + kb, false);
+      if (rest > 0) block_mv<T>(gb + bs * ldg, ldg, 1, rest, bs, 0, w + kb, v + kb + bs, true);
     }
+#pragma unroll 1
     for (int blk = nblk - 1; blk >= 0; --blk) {
       const int kb = blk * 32, bs = min(32, n - kb);
       const T* gb = g + kb * ldg + kb;
-      rowdot<1, false, 0, T>(bs, bs,
-                [&](int r, int k, T* acc) {
-                  if (k >= r) acc[0] = fma(gb[k * ldg + r], w[kb + k], acc[0]);
-                },
-                [&](int r, T* acc) { v[kb + r] = acc[0]; });
-      sync();
-      if (kb > 0) {
-        const T* gc = g + kb * ldg;
-        rowdot<1, false, 0, T>(kb, bs,
-                  [&](int i, int k, T* acc) {
-                    acc[0] = fma(gc[k * ldg + i], v[kb + k], acc[0]);
-                  },
-                  [&](int i, T* acc) { w[i] -= acc[0]; });
-        sync();
-      }
+      block_mv<T>(gb, 1, ldg, bs, bs, 2, w + kb, v + kb, false);
+      if (kb > 0) block_mv<T>(g + kb * ldg, 1, ldg, kb, bs, 0, v + kb, w, true);
     }
+  }
+
+  // out_k = sum_i M[k sk + i si] v_i (sub: out_k -= it) for k < K over i < len
+  // (tri 0), i <= k (tri 1) or i >= k (tri 2), several lanes per output as in
+  // rowdot, then a barrier.  One short copy for every step of a triangular
+  // solve, for the instruction cache.
+  template <typename T>
+  QTQP_PHASE void block_mv(const T* M, int sk, int si, int K, int len, int tri, const T* v, T* out,
+                           bool sub) {
+    const int ls = lanes_log2(K), S = 1 << ls, per_warp = 32 >> ls;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sl = lane >> (5 - ls), gl = lane & (per_warp - 1);
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += (NT / 32) * per_warp) {
+      const int k = k0 + warp * per_warp + gl;
+      const T* Mk = M + k * sk;
+      const int i1 = tri == 1 ? min(len, k + 1) : len;
+      T a0 = T(0), a1 = T(0);
+      if (k < K) {
+        int i = sl;
+        if (tri == 2) i += (k - sl + S - 1) >> ls << ls;  // the first i >= k of this lane
+        if (tri == 2 && i < sl) i = sl;
+#pragma unroll 1
+        for (; i + S < i1; i += 2 * S) {
+          a0 = fma(Mk[i * si], v[i], a0);
+          a1 = fma(Mk[(i + S) * si], v[i + S], a1);
+        }
+        if (i < i1) a0 = fma(Mk[i * si], v[i], a0);
+      }
+      a0 += a1;
+#pragma unroll 1
+      for (int off = 16; off >= per_warp; off >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+      if (k < K && sl == 0) out[k] = sub ? out[k] - a0 : a0;
+    }
+    sync();
   }
 
   // --------------------------------------------------------------------------
@@ -1198,6 +1215,10 @@ struct Ipm {
       if constexpr (FMT == kFmtLarge) {
         large_products(*this, nullptr, r + n, iry + n, nullptr, [](int, double) {},
                        [&](int k, double cs) { put_g(k, r[k] + cs); });
+      } else if (fused_ok()) {
+        dense_products(nullptr, r + n, iry + n, nullptr, nullptr);
+        sync();
+        for (int k = tid; k < n; k += NT) put_g(k, r[k] + fused_colsum(k));
       } else {
         rowdot<1>(n, m,
                   [&](int k, int i, double* acc) {
@@ -1220,9 +1241,20 @@ struct Ipm {
     for (int k = tid; k < n; k += NT) {
       const double val = fp64 ? tmp[k] : double(t32[k]);
       out[k] = accumulate ? out[k] + val : val;
+      if (fused_ok() && !fp64) tmp[k] = val;
     }
     // y = (A x - r_y) / Ry
-    {
+    if (fused_ok()) {
+      QTQP_TIC();
+      if (!fp64) sync();  // the converted x
+      dense_products(tmp, nullptr, nullptr, nullptr, tmp + n);
+      sync();
+      for (int k = own(n); k < N; k += NT) {
+        const double val = iry[k] * (tmp[k] - r[k]);
+        out[k] = accumulate ? out[k] + val : val;
+      }
+      QTQP_TOC(kPhSolveRows);
+    } else {
       QTQP_TIC();
       rowdot<1, false, kRowS>(m, n,
                 [&](int k, int j, double* acc) {
@@ -1238,72 +1270,102 @@ struct Ipm {
     QTQP_TOC(kPhSolve);
   }
 
-  // One pass over A (and P) for the products a dense block needs together,
-  // for n <= 64: the column sums c_k = sum_{i<m} A_ik wy_i + sum_{i<n} P_ik
-  // wp_i (k < n; the P part only when has_p and wp is given), staged per warp
-  // in the panel buffer PB
-  // (PB[w * n + k]; the caller sums the warps' rows after a barrier), and
-  // the row products (A vx)_i, passed to row_epi(i, value) by one lane each.
-  // Each warp takes 16 rows of A at a time, lane l columns l and l + 32; the
-  // 16 row sums are reduced across the warp in 16 shuffles (each step sends
-  // half of the values to the partner lane and keeps the other half).
+  // The products of a dense block for n <= 64, each from one coalesced pass
+  // over A (and P): with wy, the column sums c_k = sum_{i<m} A_ik wy_i (ws_i)
+  // + sum_{i<n} P_ik wp_i (k < n; wy, ws, wp may be null), staged per warp in
+  // the panel buffer PB (PB[w * n + k]; fused_colsum adds the warps' rows after
+  // a barrier); with vx, the row products (A vx)_i into rows_out[i].  A warp
+  // takes kProdRows rows at a time, lane l columns l and l + 32, their loads
+  // issued first; the row sums are reduced across the warp, the first steps
+  // sending half of the values to the partner lane and keeping the other half.
+  // Ends without a barrier.
+  //
+  // What bounds these small solves is instruction fetch: code that an
+  // iteration runs once through costs about 0.4 cycles per byte whatever it
+  // does (one n = 24 QP alone on an SM spent 5.7k cycles per residual), loops
+  // whose body stays in the nearest instruction cache next to nothing.  So one
+  // short loop, in one copy, serves the residual, both products of a KKT
+  // solve, the tau equations and the termination test.
   static constexpr bool kFused = FMT == kFmtDense && NT <= 1024;
+  static constexpr int kProdRows = 4;
   __device__ __forceinline__ bool fused_ok() const { return kFused && n <= 64; }
-  template <typename RowEpi>
-  __device__ void fused_products(const double* vx, const double* wy, const double* wp,
-                                 RowEpi row_epi) const {
+  QTQP_PHASE void dense_products(const double* vx, const double* wy, const double* ws,
+                                 const double* wp, double* rows_out) const {
     QTQP_LOCALS;
-    constexpr int NW = NT / 32;
+    constexpr int NW = NT / 32, RB = kProdRows;
     const int lane = tid & 31, warp = tid >> 5;
     const int c0 = lane, c1 = lane + 32;
     const bool ok0 = c0 < n, ok1 = c1 < n;
-    const double x0 = ok0 ? vx[c0] : 0.0, x1 = ok1 ? vx[c1] : 0.0;
     double cs0 = 0.0, cs1 = 0.0;
-    const int rsel = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 +
-                     ((lane >> 1) & 1);  // the row of the 16 this lane ends with
-    for (int base = warp * 16; base < m; base += NW * 16) {
-      double t[16];
+    if (vx != nullptr || wy != nullptr) {
+      const double x0 = ok0 && vx != nullptr ? vx[c0] : 0.0;
+      const double x1 = ok1 && vx != nullptr ? vx[c1] : 0.0;
+      const int rsel = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);  // the row a lane ends with
+#pragma unroll 1
+      for (int base = warp * RB; base < m; base += NW * RB) {
+        double t[RB], a1[RB];
 #pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        const int i = base + r;
-        double a0 = 0.0, a1 = 0.0, w = 0.0;
-        if (i < m) {
-          const double* row = A + i * lda;
-          a0 = ok0 ? row[c0] : 0.0;
-          a1 = ok1 ? row[c1] : 0.0;
-          w = wy[i];
+        for (int r = 0; r < RB; ++r) {
+          const double* row = A + (base + r) * lda;
+          const bool in = base + r < m;
+          t[r] = in && ok0 ? row[c0] : 0.0;
+          a1[r] = in && ok1 ? row[c1] : 0.0;
         }
-        cs0 = fma(a0, w, cs0);
-        cs1 = fma(a1, w, cs1);
-        t[r] = fma(a0, x0, a1 * x1);
-      }
+        if (wy != nullptr) {
 #pragma unroll
-      for (int half = 8, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-        const bool hi = (lane & bit) != 0;
+          for (int r = 0; r < RB; ++r) {
+            const int i = min(base + r, m - 1);  // rows from m on hold zeros
+            const double w = ws != nullptr ? ws[i] * wy[i] : wy[i];
+            cs0 = fma(t[r], w, cs0);
+            cs1 = fma(a1[r], w, cs1);
+          }
+        }
+        if (vx != nullptr) {
 #pragma unroll
-        for (int j = 0; j < half; ++j) {
-          const double send = hi ? t[j] : t[j + half];
-          const double keep = hi ? t[j + half] : t[j];
-          t[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+          for (int r = 0; r < RB; ++r) t[r] = fma(t[r], x0, a1[r] * x1);
+#pragma unroll
+          for (int half = RB / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+            const bool hi = (lane & bit) != 0;
+#pragma unroll
+            for (int j = 0; j < half; ++j) {
+              const double send = hi ? t[j] : t[j + half];
+              const double keep = hi ? t[j + half] : t[j];
+              t[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            }
+          }
+#pragma unroll
+          for (int bit = 4; bit >= 1; bit >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
+          if ((lane & 7) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
         }
       }
-      t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
-      const int i = base + rsel;
-      if ((lane & 1) == 0 && i < m) row_epi(i, t[0]);
     }
-    if (has_p && wp != nullptr) {
-      for (int i = warp; i < n; i += NW) {
-        const double* row = P + i * ldp;
-        const double w = wp[i];
-        if (ok0) cs0 = fma(row[c0], w, cs0);
-        if (ok1) cs1 = fma(row[c1], w, cs1);
+    static_assert(RB == 4, "rsel and the full steps");
+    if (wp != nullptr) {
+#pragma unroll 1
+      for (int i0 = warp; i0 < n; i0 += 4 * NW) {
+        double p0[4], p1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * NW;
+          const double* row = P + i * ldp;
+          p0[u] = i < n && ok0 ? row[c0] : 0.0;
+          p1[u] = i < n && ok1 ? row[c1] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double w = wp[min(i0 + u * NW, n - 1)];
+          cs0 = fma(p0[u], w, cs0);
+          cs1 = fma(p1[u], w, cs1);
+        }
       }
     }
-    double* stage = PB + warp * n;
-    if (ok0) stage[c0] = cs0;
-    if (ok1) stage[c1] = cs1;
+    if (wy != nullptr || wp != nullptr) {
+      double* stage = PB + warp * n;
+      if (ok0) stage[c0] = cs0;
+      if (ok1) stage[c1] = cs1;
+    }
   }
-  // Column sum k of fused_products (after a barrier).
+  // Column sum k of dense_products (after a barrier).
   __device__ __forceinline__ double fused_colsum(int k) const {
     constexpr int NW = NT / 32;
     double t = 0.0;
@@ -1325,17 +1387,10 @@ struct Ipm {
     if (fused_ok()) {
       const double* reg = vec(kREG);
       const double* corr = vec(kCORR);
-      fused_products(v, v + n, v, [&](int i, double ax) {
-        const int kk = n + i;
-        const double kv = ax - (-reg[kk]) * v[kk];
-        const double rk = krhs[kk] - kv + corr[kk] * v[kk];
-        res[kk] = rk;
-        mres = nanmax(mres, fabs(rk));
-        vnan = fmax(vnan, (v[kk] != v[kk]) ? 1.0 : 0.0);
-      });
+      dense_products(v, v + n, nullptr, has_p ? v : nullptr, res + n);
       sync();
-      for (int k = tid; k < n; k += NT) {
-        const double kv = fused_colsum(k) + reg[k] * v[k];
+      for (int k = tid; k < N; k += NT) {
+        const double kv = k < n ? fused_colsum(k) + reg[k] * v[k] : res[k] - (-reg[k]) * v[k];
         const double rk = krhs[k] - kv + corr[k] * v[k];
         res[k] = rk;
         mres = nanmax(mres, fabs(rk));
@@ -1569,6 +1624,10 @@ struct Ipm {
       };
       if constexpr (kSparseA) {
         for (int k = tid; k < n; k += NT) epi(k, band_poff_row(kr, k));
+      } else if (fused_ok()) {
+        dense_products(nullptr, nullptr, nullptr, kr, nullptr);
+        sync();
+        for (int k = tid; k < n; k += NT) epi(k, fused_colsum(k));
       } else {
         const double* Pp = P;
         const int lp = ldp;
@@ -1698,17 +1757,20 @@ struct Ipm {
       for (int k = tid; k < n; k += NT) epi_x(k, band_at_col(xy, k), band_poff_row(xy, k));
       for (int k = tid; k < m; k += NT) epi_y(k, band_a_row(xy, k));
     } else if (fused_ok()) {
-      // A^T y and A x in one pass over A; P x as row dots.  P x goes to the
-      // panel buffer behind the warps' staged column sums.
-      double* pxs = PB + (NT / 32) * n;
+      // P x, then A^T y and A x in one pass over A (the residual's vector is
+      // free here).
+      double* pxs = vec(kRES);
+      double* axs = vec(kRES) + n;
       if (hp) {
-        rowdot<1>(n, n,
-                  [&](int k, int i, double* acc) { acc[0] = fma(Pp[i * lp + k], xy[i], acc[0]); },
-                  [&](int k, double* acc) { pxs[k] = acc[0]; });
+        dense_products(nullptr, nullptr, nullptr, xy, nullptr);
+        sync();
+        for (int k = tid; k < n; k += NT) pxs[k] = fused_colsum(k);
+        sync();
       }
-      fused_products(xy, xy + nn, nullptr, [&](int i, double ax) { epi_y(i, ax); });
+      dense_products(xy, xy + nn, nullptr, nullptr, axs);
       sync();
       for (int k = tid; k < n; k += NT) epi_x(k, fused_colsum(k), hp ? pxs[k] : 0.0);
+      for (int k = own(n) - n; k < m; k += NT) epi_y(k, axs[k]);
     } else {
       rowdot<2>(n, m + plen,
                 [&](int k, int i, double* acc) {
@@ -2155,6 +2217,14 @@ struct Ipm {
           };
           if constexpr (kSparseA) {
             for (int k = tid; k < n; k += NT) epi(k, band_poff_row(kq, k), band_poff_row(xy, k));
+          } else if (fused_ok()) {
+            dense_products(nullptr, nullptr, nullptr, kq, nullptr);
+            sync();
+            for (int k = tid; k < n; k += NT) pkq[k] = fused_colsum(k);
+            sync();
+            dense_products(nullptr, nullptr, nullptr, xy, nullptr);
+            sync();
+            for (int k = tid; k < n; k += NT) epi(k, pkq[k], fused_colsum(k));
           } else {
             const double* Pp = P;
             const int lp = ldp;
