@@ -318,13 +318,13 @@ assert BAND_DTYPE.itemsize == ctypes.sizeof(BandInstance)
 class SparseDesc(ctypes.Structure):
   """qtqp_sparse_desc: sizes and pool offsets of a supernodal symbolic plan."""
   _fields_ = ([(f, ctypes.c_int32) for f in ("n", "nsuper", "blocks", "top_levels", "max_rows",
-                                              "max_width", "tree_levels", "reserved")] +
+                                              "max_width", "tree_levels", "dense_cols")] +
               [(f, ctypes.c_int64) for f in ("nvals", "ngram", "nrows", "nupd", "nranges",
                                               "ntop", "nnz_l", "top_row_slabs")] +
               [("flops", ctypes.c_double)] +
               [(f, ctypes.c_int64) for f in ("o_first", "o_colsn", "o_rows", "o_upd_ptr",
                                               "o_upd_src", "o_upd_off", "o_upd_cnt",
                                               "o_cta_ptr", "o_cta_range", "o_top_ptr",
-                                              "o_top_list", "o_top_slab", "o_gcol", "o_grow",
-                                              "o_rowptr",
+                                              "o_top_list", "o_top_slab", "o_top_upd", "o_gcol",
+                                              "o_grow", "o_rowptr",
                                               "o_valptr", "o_gpos", "n32", "n64")])

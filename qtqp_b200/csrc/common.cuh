@@ -130,6 +130,7 @@ constexpr int kGridBT = 256;  // threads per block of a grid-mode solve
 // the host symbolic stage and the device phases use them.
 constexpr int kSnMaxWidth = 64;
 constexpr int kSnSlabRows = 64;
+constexpr int kSnDenseMax = 4096;  // most columns of the dense part above the subtrees
 constexpr uint32_t kGridWaitLimit = 1u << 25;
 
 struct GridCtl {

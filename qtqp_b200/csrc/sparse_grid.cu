@@ -28,15 +28,17 @@ struct SparseGridParams {
 __host__ __device__ inline size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
 struct SparseLayout {
-  size_t band_off, vals_off, z_off, parts_off, upd_off, ctl_off, info_off, total;
+  size_t band_off, vals_off, z_off, parts_off, upd_off, dense_off, dinv_off, ctl_off, info_off,
+      total;
 };
 // Workspace: the banded backend's vectors and working values, the factor
 // (nvals), the forward products (one per stored row), the backward partial
 // sums (kSnMaxW per top-level row slab), the partial updates of split row
-// slabs, the grid's barrier state and the factorisation status.
+// slabs, the dense part (padded to 128 columns) and the inverses of its panel
+// step, the grid's barrier state and the factorisation status.
 __host__ __device__ inline SparseLayout plan_sparse_layout(int n, int m, int nnz_a, int nnz_p,
                                                            int64_t nvals, int64_t nrows,
-                                                           int64_t nslabs) {
+                                                           int64_t nslabs, int dense_cols) {
   SparseLayout L;
   const BandLayout B = plan_band_layout(n, m, 0, nnz_a, nnz_p);
   L.band_off = 0;
@@ -44,7 +46,10 @@ __host__ __device__ inline SparseLayout plan_sparse_layout(int n, int m, int nnz
   L.z_off = round256(L.vals_off + size_t(nvals) * 8);
   L.parts_off = round256(L.z_off + size_t(nrows) * 8);
   L.upd_off = round256(L.parts_off + size_t(nslabs) * kSnMaxW * 8);
-  L.ctl_off = round256(L.upd_off + size_t(kSparseGridBlocks) * kSnSlab * kSnMaxW * 8);
+  const size_t npad = round_up(dense_cols, kLB);
+  L.dense_off = round256(L.upd_off + size_t(kSnUbuf) * kSnSlab * kSnMaxW * 8);
+  L.dinv_off = round256(L.dense_off + npad * npad * 8);
+  L.ctl_off = round256(L.dinv_off + size_t(4) * 32 * kSubPitch * 8);
   L.info_off = round256(L.ctl_off + sizeof(GridCtl));
   L.total = L.info_off + 256;
   return L;
@@ -54,10 +59,11 @@ __global__ void __launch_bounds__(kGridBT, 1) sparse_grid_kernel(const SparseGri
   __shared__ double red[2 * (kGridBT / 32) * kRedMax];
   __shared__ qtqp_options sopt;
   __shared__ SnFactor sf;
-  extern __shared__ double snmem[];
+  extern __shared__ __align__(16) unsigned char arena[];
   const qtqp_band_instance& d = p.d;
   const SparseLayout L =
-      plan_sparse_layout(d.n, d.m, d.nnz_a, d.nnz_p, p.f.nvals, p.f.nrows, p.f.nslabs);
+      plan_sparse_layout(d.n, d.m, d.nnz_a, d.nnz_p, p.f.nvals, p.f.nrows, p.f.nslabs,
+                         p.f.dense_cols);
   if (threadIdx.x == 0) {
     sopt = p.opt;
     sf = p.f;
@@ -65,6 +71,13 @@ __global__ void __launch_bounds__(kGridBT, 1) sparse_grid_kernel(const SparseGri
     sf.zbuf = reinterpret_cast<double*>(p.ws + L.z_off);
     sf.pbuf = reinterpret_cast<double*>(p.ws + L.parts_off);
     sf.ubuf = reinterpret_cast<double*>(p.ws + L.upd_off);
+    sf.dense = reinterpret_cast<double*>(p.ws + L.dense_off);
+    sf.dinv = reinterpret_cast<double*>(p.ws + L.dinv_off);
+    // The dense part: supernodes [dense_sn, nsuper), levels [dense_level, top_levels).
+    sf.dense_sn = sf.dense_cols > 0 ? sf.colsn[sf.n - sf.dense_cols] : sf.nsuper;
+    int lv = 0;
+    while (lv < sf.top_levels && sf.top_list[sf.top_ptr[lv]] < sf.dense_sn) ++lv;
+    sf.dense_level = lv;
   }
   __syncthreads();
   Ipm<kSparseGridNT, kFmtSparse> s;
@@ -87,7 +100,11 @@ __global__ void __launch_bounds__(kGridBT, 1) sparse_grid_kernel(const SparseGri
   s.gctl = reinterpret_cast<GridCtl*>(p.ws + L.ctl_off);
   s.linfo = reinterpret_cast<int*>(p.ws + L.info_off);
   s.sn = &sf;
-  s.bwin = snmem;
+  // The dense part's shared memory (a resident inverse between the solves) from
+  // the front of the arena, the supernodes' scratch at its end.
+  s.arena = arena;
+  s.tri_gen = 0;
+  s.bwin = reinterpret_cast<double*>(arena + kArenaBytes - kSparseSmem);
   s.bwin_bytes = kSparseSmem;
   s.red = red;
   s.phase = 0;
@@ -112,7 +129,8 @@ static int check_sparse(const qtqp_band_instance* h, const qtqp_sparse_desc* sd,
   if (d.n < 1 || d.m < 1 || d.z < 0 || d.z >= d.m || d.nnz_a < 0 || d.nnz_p < 0)
     return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": needs n >= 1, m >= 1, 0 <= z < m");
   if (sd->n != d.n || sd->blocks != kSparseGridBlocks || sd->max_width > kSnMaxW ||
-      sd->nsuper < 1 || sd->nvals < d.n)
+      sd->nsuper < 1 || sd->nvals < d.n || sd->dense_cols < 0 || sd->dense_cols > d.n ||
+      sd->dense_cols > kSnDenseMax)
     return fail(QTQP_ERR_BAD_ARG, std::string(who) + ": the plan does not match the instance "
                                                      "(n, " + std::to_string(kSparseGridBlocks) +
                                       " blocks, supernodes at most " + std::to_string(kSnMaxW) +
@@ -131,7 +149,7 @@ extern "C" size_t qtqp_sparse_grid_workspace_bytes(const qtqp_band_instance* h_i
   if (check_sparse(h_inst, h_desc, "qtqp_sparse_grid_workspace_bytes") != QTQP_OK) return 0;
   const qtqp_band_instance& d = *h_inst;
   return plan_sparse_layout(d.n, d.m, d.nnz_a, d.nnz_p, h_desc->nvals, h_desc->nrows,
-                            top_slabs(*h_desc))
+                            top_slabs(*h_desc), h_desc->dense_cols)
       .total;
 }
 
@@ -158,7 +176,7 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   const qtqp_band_instance& d = *h_inst;
   const qtqp_sparse_desc& sd = *h_desc;
   const SparseLayout L = plan_sparse_layout(d.n, d.m, d.nnz_a, d.nnz_p, sd.nvals, sd.nrows,
-                                            top_slabs(sd));
+                                            top_slabs(sd), sd.dense_cols);
   if (workspace_bytes < L.total)
     return fail(QTQP_ERR_BAD_ARG, "qtqp_sparse_grid_solve: workspace smaller than "
                                   "qtqp_sparse_grid_workspace_bytes(inst, plan)");
@@ -172,7 +190,7 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   if (rc) return rc;
   rc = cuda_check(cudaFuncSetAttribute(sparse_grid_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(kSparseSmem)),
+                                       int(kArenaBytes)),
                   "cudaFuncSetAttribute(sparse_grid_kernel)");
   if (rc) return rc;
   int dev = 0, sms = 0, per_sm = 0, coop = 0;
@@ -180,7 +198,7 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sparse_grid_kernel,
-                                                                kGridBT, kSparseSmem),
+                                                                kGridBT, kArenaBytes),
                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
   if (rc) return rc;
   if (!coop || per_sm * sms < kSparseGridBlocks)
@@ -193,6 +211,8 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   f.n = sd.n;
   f.nsuper = sd.nsuper;
   f.top_levels = sd.top_levels;
+  f.dense_cols = sd.dense_cols;
+  f.dense_sn = f.dense_level = 0;  // set on the device, as the pointers below
   f.nvals = sd.nvals;
   f.ngram = sd.ngram;
   f.nrows = sd.nrows;
@@ -209,12 +229,13 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   f.top_ptr = d_sn32 + sd.o_top_ptr;
   f.top_list = d_sn32 + sd.o_top_list;
   f.top_slab = d_sn32 + sd.o_top_slab;
+  f.top_upd = d_sn32 + sd.o_top_upd;
   f.gcol = d_sn32 + sd.o_gcol;
   f.grow = d_sn32 + sd.o_grow;
   f.rowptr = d_sn64 + sd.o_rowptr;
   f.valptr = d_sn64 + sd.o_valptr;
   f.gpos = d_sn64 + sd.o_gpos;
-  f.vals = nullptr;  // set on the device (inside the workspace)
+  f.vals = f.zbuf = f.pbuf = f.ubuf = f.dense = f.dinv = nullptr;  // inside the workspace
   p.ipool = d_ipool;
   p.vpool = d_vpool;
   p.b_pool = d_b_pool;
@@ -229,6 +250,6 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
   void* args[] = {&p};
   return cuda_check(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(sparse_grid_kernel),
                                                 dim3(kSparseGridBlocks), dim3(kGridBT), args,
-                                                kSparseSmem, st),
+                                                kArenaBytes, st),
                     "sparse_grid_kernel cooperative launch");
 }

@@ -33,9 +33,21 @@
 // blocks, rows below), each solve direction in two (diagonal solves and the
 // slabs' products / partial sums), with a grid barrier after each step.  The
 // backward solve runs the schedule in reverse.
+//
+// The last levels, single supernodes one after the other, are bound by those
+// barriers and by each step's chain of dependent loads (110-180 us per level
+// in the factorisation, 30-40 us in each solve, next to no arithmetic).  From
+// the level that the symbolic stage chose (dense_level) on they are therefore
+// one dense matrix: one update step over all its row slabs, then the large
+// path's blocked Cholesky and its flag-synchronised solves (large_ipm.cuh),
+// whose chain is one 128-column block long instead of one supernode.  Measured
+// per solve of the QP: 60 x 60 network flow (1240 of 14160 columns dense, 6
+// levels instead of 21) 45.6 -> 27.3 ms, n = 2000 random sparse rows (562
+// columns, 1 level instead of 16) 45.0 -> 13.9 ms.
 #pragma once
 
 #include "dense_ipm.cuh"
+#include "large_ipm.cuh"
 
 namespace qtqp {
 
@@ -47,16 +59,22 @@ constexpr int kSnStageK = 32;           // descendant columns staged per pass
 constexpr int kSnCg = 8;                // target columns per thread in an update pass
 constexpr int kSnSlab = kSnSlabRows;    // rows of a top-level supernode per work item
 constexpr int kSnMaxSplit = 32;         // blocks sharing one slab's update list, at most
+constexpr int kSnUbuf = 4 * kSparseGridBlocks;  // partial update blocks (kSnSlab x kSnMaxW)
 // Dynamic shared memory of a block: the diagonal block, its reciprocal
 // diagonal, the staged descendant rows, and the partial sums of the solves.
 constexpr size_t kSparseSmemElems =
     size_t(kSnMaxW) * kSnLd + kSnMaxW + size_t(kSnMaxW) * (kSnStageK + 1) + kGridBT + kSnMaxW;
 constexpr size_t kSparseSmem = kSparseSmemElems * sizeof(double);
+static_assert((size_t(kLB) * kPitch + kLB) * sizeof(double) + kSparseSmem <= kArenaBytes,
+              "the supernodes' scratch would overwrite the dense part's resident inverse");
 
 // Device view of the symbolic plan (qtqp_sparse_desc offsets into the pools)
 // and the factor's value storage.
 struct SnFactor {
   int n, nsuper, top_levels;
+  int dense_cols;   // the last columns, one dense matrix (0: none)
+  int dense_sn;     // their first supernode (nsuper: none)
+  int dense_level;  // their first top level
   int64_t nvals, ngram, nrows, nslabs;
   const int32_t* first;
   const int32_t* colsn;
@@ -70,6 +88,7 @@ struct SnFactor {
   const int32_t* top_ptr;
   const int32_t* top_list;
   const int32_t* top_slab;  // prefix counts of row slabs over top_list (ntop + 1)
+  const int32_t* top_upd;   // prefix counts of update list entries over the levels
   const int32_t* gcol;
   const int32_t* grow;
   const int64_t* rowptr;
@@ -78,8 +97,44 @@ struct SnFactor {
   double* vals;
   double* zbuf;  // forward products per stored row (nrows)
   double* pbuf;  // backward partial sums per top-level row slab (kSnMaxW each)
-  double* ubuf;  // partial updates of split row slabs (kSparseGridBlocks x kSnSlab x kSnMaxW)
+  double* ubuf;  // partial updates of split row slabs (kSnUbuf x kSnSlab x kSnMaxW)
+  double* dense;  // the dense part, row-major, padded to a multiple of kLB
+  double* dinv;   // its panel step's inverses
 };
+
+// The dense part as the large path's Cholesky and solves see it.
+struct SnDense {
+  int n, npad, tid;
+  int* linfo;
+  unsigned char* arena;
+  double* sinv;
+  double* g64;
+  float* g32l;
+  GridCtl* gctl;
+  uint32_t& tri_gen;
+  const qtqp_options* o;
+  __device__ __forceinline__ void sync() const { grid_sync(gctl); }
+};
+template <class S>
+__device__ __forceinline__ SnDense sn_dense(S& s) {
+  const SnFactor& F = *s.sn;
+  return {F.dense_cols, round_up(F.dense_cols, kLB), s.tid, s.linfo + 16, s.arena, F.dinv, F.dense,
+          reinterpret_cast<float*>(F.dense), s.gctl, s.tri_gen, s.o};
+}
+
+// The end of supernode sn's update list before the descendants in the dense part.
+__device__ __forceinline__ int sn_upd_end(const SnFactor& F, int sn) {
+  int lo = F.upd_ptr[sn], hi = F.upd_ptr[sn + 1];
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (F.upd_src[mid] < F.dense_sn) {
+      lo = mid + 1;
+    } else {
+      hi = mid;
+    }
+  }
+  return lo;
+}
 
 // Position of `key` in the sorted rows[0 .. len) (present by construction).
 __device__ __forceinline__ int sn_find(const int32_t* rows, int len, int key) {
@@ -151,7 +206,7 @@ __device__ double sn_gram_entry(const S& s, int i, int j) {
 // the sums from the block, else they go to out (kSnSlab x kSnMaxW, row r - r0
 // at out[(r - r0) * kSnMaxW + col]) for sn_add_partials.
 template <typename T>
-__device__ void sn_update_slab(const SnFactor& F, T* L, int sn, int r0, int r1, int u0, int u1,
+__device__ __noinline__ void sn_update_slab(const SnFactor& F, T* L, int sn, int r0, int r1, int u0, int u1,
                                double* out) {
   const int t = threadIdx.x;
   const int f = F.first[sn], w = F.first[sn + 1] - f;
@@ -600,6 +655,88 @@ __device__ void sn_bwd_diag(const SnFactor& F, const T* L, double* smem, const d
   __syncthreads();
 }
 
+// The dense part: the updates of all its rows by the supernodes before it (one
+// step over the whole grid, as above the subtrees), the result as one dense
+// matrix, and its Cholesky by the large path.
+template <typename T, class S>
+__device__ __noinline__ int sn_dense_factorize(S& s) {
+  const SnFactor& F = *s.sn;
+  T* L = reinterpret_cast<T*>(F.vals);
+  T* g = reinterpret_cast<T*>(F.dense);
+  SnDense D = sn_dense(s);
+  const int G = int(gridDim.x), b = blockIdx.x;
+  const int c0 = F.n - F.dense_cols;
+  const int q0 = F.top_ptr[F.dense_level], q1 = F.top_ptr[F.top_levels];
+  const int items = F.top_slab[q1] - F.top_slab[q0];
+  const int ulen = F.top_upd[F.top_levels] - F.top_upd[F.dense_level];
+  const int split = max(1, min(min(kSnMaxSplit, kSnUbuf / items), ulen / (8 * (q1 - q0))));
+  QTQP_TIC();
+  for (int it = b; it < items * split; it += G) {
+    const int slab = it / split, part = it % split;
+    int sn, r0, r1;
+    sn_slab_item(F, q0, q1, F.top_slab[q0] + slab, sn, r0, r1);
+    const int ua = F.upd_ptr[sn], len = sn_upd_end(F, sn) - ua;
+    sn_update_slab<T>(F, L, sn, r0, r1, ua + len * part / split, ua + len * (part + 1) / split,
+                      split > 1 ? F.ubuf + size_t(it) * kSnSlab * kSnMaxW : nullptr);
+  }
+  for (int r = b; r < D.npad; r += G)
+    for (int c = threadIdx.x; c <= r; c += blockDim.x)
+      g[size_t(r) * D.npad + c] = T(r == c && r >= D.n ? 1 : 0);
+  s.sync();
+  QTQP_TOC(kPhSnTopUpd);
+  for (int it = b; it < items; it += G) {
+    int sn, r0, r1;
+    sn_slab_item(F, q0, q1, F.top_slab[q0] + it, sn, r0, r1);
+    const int f = F.first[sn], w = F.first[sn + 1] - f;
+    const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]), rows = r1 - r0;
+    const int32_t* R = F.rows + F.rowptr[sn];
+    const T* Ls = L + F.valptr[sn];
+    const double* part = F.ubuf + size_t(it) * split * kSnSlab * kSnMaxW;
+    for (int e = threadIdx.x; e < rows * w; e += blockDim.x) {
+      const int rl = e % rows, col = e / rows, r = R[r0 + rl];
+      if (f + col > r) continue;  // the block's upper triangle
+      double v = double(Ls[size_t(r0 + rl) + size_t(col) * nr]);
+      if (split > 1) {
+        double sum = 0.0;
+        for (int c = 0; c < split; ++c)
+          sum += part[size_t(c) * kSnSlab * kSnMaxW + rl * kSnMaxW + col];
+        v -= sum;
+      }
+      g[size_t(r - c0) * D.npad + (f + col - c0)] = T(v);
+    }
+  }
+  return large_cholesky<T>(D, g);  // begins with a grid barrier
+}
+
+// Forward and backward solve of the dense part, v[c0 ..) in place: the products
+// of the supernodes before it are gathered by the whole grid, then the block
+// that owns a 128-row block subtracts its columns' (no barrier in between).
+template <typename T, class S>
+__device__ __noinline__ void sn_dense_solve(S& s, T* v, T* w) {
+  const SnFactor& F = *s.sn;
+  SnDense D = sn_dense(s);
+  const int G = int(gridDim.x), b = blockIdx.x;
+  const int c0 = F.n - F.dense_cols, nq = F.nsuper - F.dense_sn;
+  const int split = max(1, min(kSnMaxSplit, G / nq));
+  for (int it = b; it < nq * split; it += G) {
+    const int sn = F.dense_sn + it / split, part = it % split;
+    const int ua = F.upd_ptr[sn], len = sn_upd_end(F, sn) - ua;
+    sn_fwd_gather(F, F.zbuf, s.bwin, sn, ua + len * part / split, ua + len * (part + 1) / split,
+                  F.ubuf + size_t(it) * kSnMaxW);
+  }
+  s.sync();
+  const int k = b * kLB + int(threadIdx.x);
+  if (int(threadIdx.x) < kLB && k < D.n) {
+    const int sn = F.colsn[c0 + k];
+    const double* p = F.ubuf + size_t(sn - F.dense_sn) * split * kSnMaxW + (c0 + k - F.first[sn]);
+    double sum = 0.0;
+    for (int c = 0; c < split; ++c) sum += p[c * kSnMaxW];
+    v[c0 + k] = T(double(v[c0 + k]) - sum);
+  }
+  __syncthreads();
+  large_chol_solve<T>(D, v + c0, w + c0);
+}
+
 template <typename T, class S>
 __device__ int sparse_factorize(S& s) {
   const SnFactor& F = *s.sn;
@@ -645,11 +782,10 @@ __device__ int sparse_factorize(S& s) {
   // by the diagonal step (slab 0 of each supernode) and the row step (the
   // other slabs), so the split costs no extra barrier.
   const int G = int(gridDim.x);
-  for (int l = 0; l < F.top_levels; ++l) {
+  for (int l = 0; l < F.dense_level; ++l) {
     const int q0 = F.top_ptr[l], q1 = F.top_ptr[l + 1];
     const int items = F.top_slab[q1] - F.top_slab[q0];
-    int ulen = 0;  // update list entries of the level (the same in every block)
-    for (int q = q0; q < q1; ++q) ulen += F.upd_ptr[F.top_list[q] + 1] - F.upd_ptr[F.top_list[q]];
+    const int ulen = F.top_upd[l + 1] - F.top_upd[l];  // update list entries of the level
     // At least 8 list entries per part on average: short lists stay whole.
     const int split = 2 * items > G ? 1
                                     : max(1, min(min(kSnMaxSplit, G / items), ulen / (8 * (q1 - q0))));
@@ -691,12 +827,18 @@ __device__ int sparse_factorize(S& s) {
     QTQP_TOC(kPhSnTopPanel);
   }
   QTQP_TOC(kPhSnTop);
-  return *reinterpret_cast<volatile int*>(s.linfo);
+  int info = *reinterpret_cast<volatile int*>(s.linfo);
+  if (F.dense_cols > 0) {
+    QTQP_RETIC();
+    const int dinfo = sn_dense_factorize<T>(s);
+    if (info == 0 && dinfo != 0) info = F.n - F.dense_cols + dinfo;
+    QTQP_TOC(kPhChol);
+  }
+  return info;
 }
 
 template <typename T, class S>
 __device__ void sparse_solve(S& s, T* v, T* w) {
-  (void)w;
   const SnFactor& F = *s.sn;
   const T* L = reinterpret_cast<const T*>(F.vals);
   double* smem = s.bwin;
@@ -715,12 +857,11 @@ __device__ void sparse_solve(S& s, T* v, T* w) {
   QTQP_TOC(kPhSnFwdSub);
   QTQP_RETIC();
   const int G = int(gridDim.x);
-  for (int l = 0; l < F.top_levels; ++l) {
+  for (int l = 0; l < F.dense_level; ++l) {
     const int q0 = F.top_ptr[l], q1 = F.top_ptr[l + 1];
     // Long update lists are gathered by several blocks first (one more
     // barrier), each on a contiguous part, then summed in order.
-    int ulen = 0;
-    for (int q = q0; q < q1; ++q) ulen += F.upd_ptr[F.top_list[q] + 1] - F.upd_ptr[F.top_list[q]];
+    const int ulen = F.top_upd[l + 1] - F.top_upd[l];
     const int nq = q1 - q0;
     const int split = ulen < 8 * kGridBT / 32 * nq || 2 * nq > G ? 1 : min(kSnMaxSplit, G / nq);
     if (split > 1) {
@@ -748,11 +889,12 @@ __device__ void sparse_solve(S& s, T* v, T* w) {
       s.sync();
     }
   }
+  if (F.dense_cols > 0) sn_dense_solve<T>(s, v, w);
   QTQP_TOC(kPhSnFwdTop);
   QTQP_RETIC();
   // Backward: the top levels in reverse (every row slab's partial sums, then
   // the diagonal solves), then the subtrees in reverse.
-  for (int l = F.top_levels - 1; l >= 0; --l) {
+  for (int l = F.dense_level - 1; l >= 0; --l) {
     const int q0 = F.top_ptr[l], q1 = F.top_ptr[l + 1];
     const int items = F.top_slab[q1] - F.top_slab[q0];
     for (int it = b; it < items; it += gridDim.x) {

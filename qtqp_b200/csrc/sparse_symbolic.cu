@@ -32,6 +32,9 @@
 //     level;
 //  7. the map of G's lower entries (in the final ordering) to positions in
 //     the supernodes' column-major value blocks.
+// When the top levels from some level on are worth more as one dense matrix
+// (dense_level), their columns are moved to the end of the ordering (an
+// equivalent one: they are closed under ancestors) and stages 4-7 run again.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -250,10 +253,11 @@ struct Plan {
   std::vector<int32_t> first, rows, colsn;
   std::vector<int64_t> rowptr, valptr;
   std::vector<int32_t> upd_ptr, upd_src, upd_off, upd_cnt;
-  std::vector<int32_t> cta_ptr, cta_range, top_ptr, top_list, top_slab;
+  std::vector<int32_t> cta_ptr, cta_range, top_ptr, top_list, top_slab, top_upd;
   std::vector<int32_t> gcol, grow;
   std::vector<int64_t> gpos;
   int max_rows = 0, max_width = 0, tree_levels = 0;
+  int dense_cols = 0;  // the last columns, factorised as one dense matrix
   int64_t nnz_l = 0;
   double flops = 0.0;
 };
@@ -383,6 +387,30 @@ static std::vector<int> postorder(const std::vector<int>& parent) {
   return post;
 }
 
+// The top level from which on the supernodes are cheaper as one dense matrix
+// over their columns (the number of levels: none).  Measured on a B200, per
+// interior-point iteration (one factorisation, about 4.5 solves): a top level
+// costs some 250 us of grid barriers and dependent steps, whatever its size; a
+// 128-column block of the dense part some 180 us (its diagonal chain and its
+// step in the solves), the dense part 150 us once, and its trailing updates run
+// at 20 TFLOP/s.
+static int dense_level(const Plan& P, const std::vector<int>& first, int levels) {
+  int best = levels, cols = 0;
+  double best_us = 250.0 * levels;
+  for (int l = levels - 1; l >= 0; --l) {
+    for (int q = P.top_ptr[l]; q < P.top_ptr[l + 1]; ++q)
+      cols += first[P.top_list[q] + 1] - first[P.top_list[q]];
+    if (cols > kSnDenseMax) break;
+    const double us = 250.0 * l + 150.0 + 180.0 * ((cols + 127) / 128) +
+                      2.0 / 3.0 * cols * double(cols) * cols / 2e7;
+    if (us < best_us) {
+      best_us = us;
+      best = l;
+    }
+  }
+  return best;
+}
+
 static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const int32_t* pp,
                       const int32_t* pi, int ordering, int blocks, Plan& P) {
   Adj adj;
@@ -403,8 +431,8 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   std::vector<int> perm(n);
   for (int k = 0; k < n; ++k) perm[k] = order[post[k]];
   for (int k = 0; k < n; ++k) pinv[perm[k]] = k;
-  const Adj g = relabel(adj, perm, pinv);
-  const std::vector<int> parent = etree(g);
+  Adj g = relabel(adj, perm, pinv);
+  std::vector<int> parent = etree(g);
   // Column counts of L (row subtrees).
   std::vector<int> cc(n, 0), mark(n, -1), nchild(n, 0);
   for (int k = 0; k < n; ++k) {
@@ -479,6 +507,12 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   }
   fin_first.push_back(n);
   const int S = int(fin_first.size()) - 1;
+  // The level from which the top levels form the dense part, and which
+  // supernodes are above the subtrees (decided in the first pass).
+  int dense_from = -1;
+  std::vector<char> top(S, 0);
+  for (int pass = 0; pass < 2; ++pass) {
+  P = Plan();
   P.n = n;
   P.nsuper = S;
   P.blocks = blocks;
@@ -604,12 +638,11 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   for (int s = 0; s < S; ++s)
     if (sparent[s] < 0) total += sub[s];
   const double chunk = total / (4.0 * blocks);
-  std::vector<char> top(S, 0);
   std::vector<int> roots;
   for (int s = S - 1; s >= 0; --s) {
     const bool above = sparent[s] < 0 || top[sparent[s]];
     if (!above) continue;
-    if (sub[s] > chunk && !kids[s].empty()) {
+    if (pass == 0 ? sub[s] > chunk && !kids[s].empty() : top[s] != 0) {
       top[s] = 1;
     } else {
       roots.push_back(s);
@@ -652,12 +685,42 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
     for (int s = 0; s < S; ++s)
       if (top[s]) P.top_list[fl[tlev[s]]++] = s;
   }
+  if (pass == 0) {
+    dense_from = dense_level(P, fin_first, ntl);
+    if (dense_from == ntl) break;
+    // The dense part's supernodes last, everything else in its order.
+    std::vector<int> seq, widths;
+    std::vector<char> ntop;
+    for (int part = 0; part < 2; ++part)
+      for (int s = 0; s < S; ++s)
+        if ((top[s] && tlev[s] >= dense_from) == (part == 1)) {
+          for (int j = fin_first[s]; j < fin_first[s + 1]; ++j) seq.push_back(perm[j]);
+          widths.push_back(fin_first[s + 1] - fin_first[s]);
+          ntop.push_back(top[s]);
+        }
+    perm = seq;
+    top = ntop;
+    fin_first.assign(1, 0);
+    for (int w : widths) fin_first.push_back(fin_first.back() + w);
+    for (int k = 0; k < n; ++k) pinv[perm[k]] = k;
+    g = relabel(adj, perm, pinv);
+    parent = etree(g);
+    continue;
+  }
+  P.dense_cols = n - fin_first[P.top_list[P.top_ptr[dense_from]]];
+  }
   // Row slabs of the top supernodes (work items of the grid), prefix counts.
   P.top_slab.assign(P.top_list.size() + 1, 0);
   for (size_t q = 0; q < P.top_list.size(); ++q) {
     const int s = P.top_list[q];
     const int nr = int(P.rowptr[s + 1] - P.rowptr[s]);
     P.top_slab[q + 1] = P.top_slab[q] + (nr + kSnSlabRows - 1) / kSnSlabRows;
+  }
+  P.top_upd.assign(P.top_ptr.size(), 0);
+  for (size_t l = 0; l + 1 < P.top_ptr.size(); ++l) {
+    P.top_upd[l + 1] = P.top_upd[l];
+    for (int q = P.top_ptr[l]; q < P.top_ptr[l + 1]; ++q)
+      P.top_upd[l + 1] += P.upd_ptr[P.top_list[q] + 1] - P.upd_ptr[P.top_list[q]];
   }
   // G's lower entries (diagonal first in each column) and their positions.
   for (int j = 0; j < n; ++j) {
@@ -722,6 +785,7 @@ extern "C" int qtqp_sparse_analyze(int32_t n, int32_t m, const int32_t* h_a_colp
   d.max_rows = P->max_rows;
   d.max_width = P->max_width;
   d.tree_levels = P->tree_levels;
+  d.dense_cols = P->dense_cols;
   d.nvals = P->valptr.back();
   d.ngram = int64_t(P->gcol.size());
   d.nrows = int64_t(P->rows.size());
@@ -748,6 +812,7 @@ extern "C" int qtqp_sparse_analyze(int32_t n, int32_t m, const int32_t* h_a_colp
   put(d.o_top_ptr, P->top_ptr.size());
   put(d.o_top_list, P->top_list.size());
   put(d.o_top_slab, P->top_slab.size());
+  put(d.o_top_upd, P->top_upd.size());
   put(d.o_gcol, P->gcol.size());
   put(d.o_grow, P->grow.size());
   d.n32 = o;
@@ -794,6 +859,7 @@ extern "C" int qtqp_sparse_export(const void* h_plan, const qtqp_sparse_desc* h_
   cp(d.o_top_ptr, P.top_ptr);
   cp(d.o_top_list, P.top_list);
   cp(d.o_top_slab, P.top_slab);
+  cp(d.o_top_upd, P.top_upd);
   cp(d.o_gcol, P.gcol);
   cp(d.o_grow, P.grow);
   cp64(d.o_rowptr, P.rowptr);
