@@ -317,6 +317,13 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
                "l"(src)
                : "memory");
 }
+// The same with the first `bytes` (0, 8 or 16) read and the rest zero-filled.
+__device__ __forceinline__ void cp_async16z(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(bytes)
+               : "memory");
+}
 // Element copy of T (double or float), zero-filled when !valid.
 template <typename T>
 __device__ __forceinline__ void cp_async_elem(T* dst, const T* src, bool valid) {

@@ -301,6 +301,7 @@ struct Ipm {
   double* g64;
   float* g32l;
   double* sinv;  // sub-block inverses of the current panel step
+  double* gpart;    // parts of split Gram tiles (GramSplit)
   double* colpart;  // per-block column sums of large_products (gridDim x npad)
   float* xhi;
   float* xlo;

@@ -9,9 +9,9 @@ namespace qtqp {
 
 struct KktGridLayout {
   int npad, nblk;
-  size_t gen_off, info_off, g_off, inv_off, sinv_off, cp_off, total;
+  size_t gen_off, info_off, g_off, inv_off, sinv_off, cp_off, gpart_off, total;
 };
-static __host__ __device__ inline KktGridLayout plan_kkt_grid(int n) {
+static __host__ __device__ inline KktGridLayout plan_kkt_grid(int n, int m) {
   KktGridLayout L;
   L.npad = round_up(n, kLB);
   L.nblk = L.npad / kLB;
@@ -28,13 +28,14 @@ static __host__ __device__ inline KktGridLayout plan_kkt_grid(int n) {
   off += al(size_t(4) * 32 * kSubPitch * 8);
   L.cp_off = off;
   off += al(size_t(kLargeBlocks) * L.npad * 8);
+  L.gpart_off = off;
+  off += al(GramSplit(L.npad, m).slot_bytes());
   L.total = off;
   return L;
 }
 
 size_t kkt_grid_bytes(int n, int m) {
-  (void)m;
-  return plan_kkt_grid(n).total;
+  return plan_kkt_grid(n, m).total;
 }
 
 using KktGridIpm = Ipm<kLargeNT, kFmtLarge>;
@@ -42,7 +43,7 @@ using KktGridIpm = Ipm<kLargeNT, kFmtLarge>;
 __device__ inline void kkt_grid_bind(KktGridIpm& s, int n, int m, char* ws, char* gws,
                                      unsigned char* arena, double* red) {
   const InstLayout I = plan_layout(n, m, 0);
-  const KktGridLayout L = plan_kkt_grid(n);
+  const KktGridLayout L = plan_kkt_grid(n, m);
   s.tid = blockIdx.x * blockDim.x + threadIdx.x;
   s.n = n;
   s.m = m;
@@ -64,6 +65,7 @@ __device__ inline void kkt_grid_bind(KktGridIpm& s, int n, int m, char* ws, char
   s.G = s.g64;
   s.g32l = nullptr;
   s.sinv = reinterpret_cast<double*>(gws + L.sinv_off);
+  s.gpart = reinterpret_cast<double*>(gws + L.gpart_off);
   s.colpart = reinterpret_cast<double*>(gws + L.cp_off);
   s.arena = arena;
   s.tri_gen = *reinterpret_cast<const uint32_t*>(gws + L.gen_off);
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
   extern __shared__ __align__(16) unsigned char arena[];
   KktGridIpm s;
   kkt_grid_bind(s, n, m, ws + header, gws, arena, red);
-  const KktGridLayout L = plan_kkt_grid(n);
+  const KktGridLayout L = plan_kkt_grid(n, m);
   s.kkt_diag_given(diag);
   s.sync();
   const int rc = s.template factorize<double>();
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
   }
   KktGridIpm s;
   kkt_grid_bind(s, n, m, ws + header, gws, arena, red);
-  const KktGridLayout L = plan_kkt_grid(n);
+  const KktGridLayout L = plan_kkt_grid(n, m);
   if (int(blockIdx.x) < L.nblk)
     stage_block(reinterpret_cast<double*>(arena),
                 reinterpret_cast<const double*>(gws + L.inv_off) + size_t(blockIdx.x) * kLB * kLB,

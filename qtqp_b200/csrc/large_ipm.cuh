@@ -37,11 +37,36 @@ constexpr size_t kLargeSmem = 1024 + kArenaBytes + 256;    // + alignment + barr
 
 __host__ __device__ inline int round_up(int v, int q) { return (v + q - 1) / q * q; }
 
+// The split of the FP64 Gram matrix over the CTAs: the lower 128 x 128 tiles,
+// row by row, times their slices of kGramKS rows of A are one sequence of
+// units, of which CTA c < ctas takes [unit0(c), unit0(c + 1)).  Whole tiles go
+// straight to G; a part of a tile goes to the CTA's slot 2 c (its first tile) or
+// 2 c + 1 (its last), and large_finish_gram adds a tile's parts in order.
+// Whole tiles only would leave the last wave nearly empty (n = 4096: 528 tiles
+// = 3.6 waves of 148) or most CTAs idle (n = 1000: 36 tiles).
+constexpr int kGramKS = 32;
+constexpr int kGramMinUnits = 4;  // slices per CTA at least, else fewer CTAs
+struct GramSplit {
+  int slices, ctas;
+  long long units;
+  __host__ __device__ GramSplit(int npad, int m) {
+    const int nt = npad / kLB;
+    const long long tiles = (long long)nt * (nt + 1) / 2;
+    slices = m > kGramKS ? (m + kGramKS - 1) / kGramKS : 1;
+    units = tiles * slices;
+    const long long want = units / kGramMinUnits > tiles ? units / kGramMinUnits : tiles;
+    ctas = want < kLargeBlocks ? int(want) : kLargeBlocks;
+  }
+  __host__ __device__ size_t slot_bytes() const { return size_t(2) * ctas * kLB * kLB * 8; }
+  __device__ long long unit0(int c) const { return c * units / ctas; }
+  __device__ int owner(long long u) const { return int(((u + 1) * ctas - 1) / units); }
+};
+
 // Global workspace of a large solve.
 struct LargeLayout {
   int n, m, npad, mpad, nblk, np;
   size_t ctl_off, info_off, v_off, a_off, p_off, g64_off, g32_off, sinv_off, xhi_off, xlo_off,
-      cp_off, total;
+      cp_off, gpart_off, total;
 };
 __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   LargeLayout L;
@@ -75,6 +100,8 @@ __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   off += al(size_t(L.npad) * L.mpad * 4);
   L.cp_off = off;  // per-block column sums of large_products
   off += al(size_t(kLargeBlocks) * L.npad * 8);
+  L.gpart_off = off;  // parts of split Gram tiles
+  off += al(GramSplit(L.npad, m).slot_bytes());
   L.total = off;
   return L;
 }
@@ -341,40 +368,61 @@ __device__ void large_gram_tc(S& s) {
   if (threadIdx.x == 0 && *failed) grid_fail(s.gctl);
 }
 
+// Row and column of lower tile t (row by row).
+__device__ __forceinline__ void lower_tile(int t, int& ti, int& tj) {
+  ti = int((sqrtf(8.0f * float(t) + 1.0f) - 1.0f) * 0.5f);
+  while (ti * (ti + 1) / 2 > t) --ti;
+  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+  tj = t - ti * (ti + 1) / 2;
+}
+
 // G_lower = A^T diag(1/Ry) A in FP64 on the FP64 tensor cores (DMMA,
-// mma.sync m8n8k4): one CTA per 128 x 128 lower tile; K-slices of 16 rows of
-// A (both column panels) and their weights staged by cp.async in a ring of
-// four buffers (three slices in flight), with a row pitch of 132 so that each half-warp's fragment loads
-// hit 16 different banks; warp w computes the 64 x 32 block (w / 4, w % 4)
-// of the tile with 8 x 4 accumulators of 8 x 8.  Rows and columns beyond
-// m, n are zero-filled.
-template <class S>
+// mma.sync m8n8k4): slices of 32 rows of A (both column panels) and their
+// weights staged by cp.async into two buffers, with a row pitch of 132 so that
+// each half-warp's fragment loads hit 16 different banks; warp w computes the
+// 64 x 32 block (w / 4, w % 4) of the tile with 8 x 4 accumulators of 8 x 8.
+// Rows and columns beyond m, n are zero-filled.  Rows of A that start on 16
+// bytes (even lda) are copied 16 bytes at a time.
+// Bound by the FP64 tensor cores (36.7 TFLOP/s alone).  n = 4096, m = 8192, rate
+// within a tile: 26.5 TFLOP/s with 8-byte copies, slices of 16 rows, two barriers
+// each and the weights on the longer fragment; 29.1 with 16-byte copies, 30.6
+// with one barrier and the weights on the shorter one, 31.2 with slices of 32
+// rows.  (Row copies by the TMA unit: 31.0, so the copies no longer matter.)
+template <int VEC, class S>
 __device__ __noinline__ void large_gram_dmma(S& s) {
   const int n = s.n, m = s.m, npad = s.npad, lda = s.lda;
   const double* A = s.A;
   const double* iry = s.vec(kPI) + n;  // 1 / Ry
-  constexpr int KS = 16;               // rows per slice
+  constexpr int KS = kGramKS;
   constexpr int LP = kLB + 4;          // staged row pitch
   constexpr int SL = 2 * KS * LP + KS; // doubles per buffer
-  constexpr int NS = 4;                // slices in flight (ring of NS buffers)
-  static_assert(NS * SL * sizeof(double) <= kArenaBytes, "Gram ring exceeds the arena");
+  static_assert(2 * SL * sizeof(double) <= kArenaBytes, "Gram buffers exceed the arena");
   double* smem = reinterpret_cast<double*>(s.arena);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gi = lane >> 2, tg = lane & 3;
   const int wr = warp >> 2, wc = warp & 3;
-  const int nt = npad / kLB, tiles = nt * (nt + 1) / 2;
+  const GramSplit P(npad, m);
+  if (int(blockIdx.x) >= P.ctas) return;
   auto issue = [&](int r0, int i0, int j0, int buf) {
     double* sa = smem + buf * SL;
     double* sb = sa + KS * LP;
     double* sw = sb + KS * LP;
+    constexpr int kPer = kLB / VEC;  // copies per row and panel
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = threadIdx.x + q * kGridBT, r = e >> 7, c = e & 127, i = r0 + r;
+    for (int q = 0; q < KS * kPer / kGridBT; ++q) {
+      const int e = threadIdx.x + q * kGridBT, r = e / kPer, c = e % kPer * VEC, i = r0 + r;
       const bool ok = i < m;
-      cp_async8(sa + r * LP + c, A + (ok && i0 + c < n ? size_t(i) * lda + i0 + c : 0),
-                ok && i0 + c < n);
-      cp_async8(sb + r * LP + c, A + (ok && j0 + c < n ? size_t(i) * lda + j0 + c : 0),
-                ok && j0 + c < n);
+      if constexpr (VEC == 2) {
+        const int ba = ok ? max(0, min(16, 8 * (n - i0 - c))) : 0;
+        const int bb = ok ? max(0, min(16, 8 * (n - j0 - c))) : 0;
+        cp_async16z(sa + r * LP + c, A + (ba ? size_t(i) * lda + i0 + c : 0), ba);
+        cp_async16z(sb + r * LP + c, A + (bb ? size_t(i) * lda + j0 + c : 0), bb);
+      } else {
+        cp_async8(sa + r * LP + c, A + (ok && i0 + c < n ? size_t(i) * lda + i0 + c : 0),
+                  ok && i0 + c < n);
+        cp_async8(sb + r * LP + c, A + (ok && j0 + c < n ? size_t(i) * lda + j0 + c : 0),
+                  ok && j0 + c < n);
+      }
     }
     if (threadIdx.x < KS) {
       const int i = r0 + threadIdx.x;
@@ -382,38 +430,26 @@ __device__ __noinline__ void large_gram_dmma(S& s) {
     }
     cp_async_commit();
   };
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-    int ti = 0;
-    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-    const int tj = t - ti * (ti + 1) / 2;
+  const long long u0 = P.unit0(blockIdx.x), u1 = P.unit0(blockIdx.x + 1);
+  for (long long u = u0; u < u1;) {
+    const int t = int(u / P.slices), qa = int(u - (long long)t * P.slices);
+    const int qb = int(min((long long)P.slices, qa + (u1 - u)));
+    int ti, tj;
+    lower_tile(t, ti, tj);
     const int i0 = ti * kLB, j0 = tj * kLB;
     double acc[8][4][2];
 #pragma unroll
     for (int a = 0; a < 8; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    const int nsl = (m + KS - 1) / KS;
-    // Slices 0 .. NS-2 in flight (empty groups past the end keep the count).
-#pragma unroll
-    for (int q = 0; q < NS - 1; ++q) {
-      if (q < nsl) {
-        issue(q * KS, i0, j0, q);
-      } else {
-        cp_async_commit();
-      }
-    }
-    for (int q = 0; q < nsl; ++q) {
-      // Slice q + NS - 1 goes into the buffer read at step q - 1 (released by
-      // that step's closing barrier); then slice q has landed.
-      const int nx = q + NS - 1;
-      if (nx < nsl) {
-        issue(nx * KS, i0, j0, nx % NS);
-      } else {
-        cp_async_commit();
-      }
-      cp_async_wait<NS - 1>();
+    issue(qa * KS, i0, j0, 0);
+    int buf = 0;
+    for (int q = qa; q < qb; ++q) {
+      // Slice q has landed, and every warp is done with slice q - 1, whose
+      // buffer takes slice q + 1.
+      cp_async_wait<0>();
       __syncthreads();
-      const int buf = q % NS;
+      if (q + 1 < qb) issue((q + 1) * KS, i0, j0, buf ^ 1);
       const double* sa = smem + buf * SL + wr * 64 + gi;
       const double* sb = smem + buf * SL + KS * LP + wc * 32 + gi;
       const double* sw = smem + buf * SL + 2 * KS * LP;
@@ -423,30 +459,34 @@ __device__ __noinline__ void large_gram_dmma(S& s) {
         const double w = sw[r];
         double a[8], b[4];
 #pragma unroll
-        for (int mi = 0; mi < 8; ++mi) a[mi] = sa[r * LP + mi * 8] * w;
+        for (int mi = 0; mi < 8; ++mi) a[mi] = sa[r * LP + mi * 8];
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) b[ni] = sb[r * LP + ni * 8];
+        for (int ni = 0; ni < 4; ++ni) b[ni] = sb[r * LP + ni * 8] * w;
 #pragma unroll
         for (int mi = 0; mi < 8; ++mi)
 #pragma unroll
           for (int ni = 0; ni < 4; ++ni) dmma_8x8x4(acc[mi][ni], a[mi], b[ni]);
       }
-      __syncthreads();  // everyone is done with `buf` before it is refilled
+      buf ^= 1;
     }
+    __syncthreads();
+    const bool whole = qb - qa == P.slices;
+    double* out = whole ? s.g64 + size_t(i0) * npad + j0
+                        : s.gpart + (size_t(2) * blockIdx.x + (u == u0 ? 0 : 1)) * kLB * kLB;
+    const size_t ldo = whole ? npad : kLB;
 #pragma unroll
     for (int mi = 0; mi < 8; ++mi)
 #pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const int i = i0 + wr * 64 + mi * 8 + gi, j = j0 + wc * 32 + ni * 8 + 2 * tg;
-        s.g64[size_t(i) * npad + j] = acc[mi][ni][0];
-        s.g64[size_t(i) * npad + j + 1] = acc[mi][ni][1];
-      }
+      for (int ni = 0; ni < 4; ++ni)
+        *reinterpret_cast<double2*>(out + (wr * 64 + mi * 8 + gi) * ldo + wc * 32 + ni * 8 + 2 * tg) =
+            make_double2(acc[mi][ni][0], acc[mi][ni][1]);
+    u += qb - qa;
   }
 }
 
-// G += P_off + diag(Rx) on the lower triangle, identity padding, then the
-// relative diagonal jitter (1e-14 in FP64 as solvers_dense.py:112; 2^-22 at
-// FP32 resolution).
+// G += P_off + diag(Rx) on the lower triangle (FP64: of the sums of the tiles'
+// parts, see GramSplit), identity padding, then the relative diagonal jitter
+// (1e-14 in FP64 as solvers_dense.py:112; 2^-22 at FP32 resolution).
 template <typename T, class S>
 __device__ void large_finish_gram(S& s, T* g) {
   const int n = s.n, npad = s.npad, tid = s.tid;
@@ -454,19 +494,52 @@ __device__ void large_finish_gram(S& s, T* g) {
   const double* reg = s.vec(kREG);
   double dmax[1] = {0.0};
   double dummy[1] = {0.0};
-  const size_t total = size_t(npad) * npad;
-  for (size_t e = tid; e < total; e += kLargeNT) {
-    const int i = int(e / npad), j = int(e % npad);
-    if (j > i) continue;
-    if (i >= n || j >= n) {
-      g[e] = (i == j) ? T(1) : T(0);
-      continue;
+  const GramSplit sp(npad, s.m);
+  const int nt = npad / kLB, tiles = nt * (nt + 1) / 2;
+  constexpr int kRows = 16;  // rows of a work item, two per warp
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int it = blockIdx.x; it < tiles * (kLB / kRows); it += gridDim.x) {
+    const int t = it / (kLB / kRows);
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    const int row0 = it % (kLB / kRows) * kRows + 2 * warp;
+    // This lane's entries q: row row0 + q / 4, column lane + 32 (q % 4) of the tile.
+    T* gt = g + (size_t(ti) * kLB + row0) * npad + tj * kLB + lane;
+    T sum[8];
+    int c0 = 0, c1 = 0;
+    if constexpr (sizeof(T) == 8) {
+      c0 = sp.owner((long long)t * sp.slices);
+      c1 = sp.owner((long long)(t + 1) * sp.slices - 1);
     }
-    double base = P[size_t(i) * s.ldp + j];
-    if (i == j) base += reg[i];
-    const T v = T(base) + g[e];
-    g[e] = v;
-    if (i == j) dmax[0] = nanmax(dmax[0], double(v));
+    if (c0 == c1) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sum[q] = gt[size_t(q >> 2) * npad + 32 * (q & 3)];
+    } else if constexpr (sizeof(T) == 8) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sum[q] = 0.0;
+      for (int k = c0; k <= c1; ++k) {
+        const bool first = sp.unit0(k) >= (long long)t * sp.slices;
+        const double* part =
+            s.gpart + ((size_t(2) * k + (first ? 0 : 1)) * kLB + row0) * kLB + lane;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum[q] += part[(q >> 2) * kLB + 32 * (q & 3)];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = ti * kLB + row0 + (q >> 2), j = tj * kLB + lane + 32 * (q & 3);
+      if (j > i) continue;
+      T* ge = gt + size_t(q >> 2) * npad + 32 * (q & 3);
+      if (i >= n || j >= n) {
+        *ge = (i == j) ? T(1) : T(0);
+        continue;
+      }
+      double base = P[size_t(i) * s.ldp + j];
+      if (i == j) base += reg[i];
+      const T v = T(base) + sum[q];
+      *ge = v;
+      if (i == j) dmax[0] = nanmax(dmax[0], double(v));
+    }
   }
   s.template reduce<0, 1>(dummy, dmax);
   const double jit = (sizeof(T) == 8 ? 1e-14 : 2.384185791015625e-07) * dmax[0];
@@ -1014,7 +1087,11 @@ __device__ int large_factorize(S& s) {
     QTQP_RETIC();
     info = large_cholesky<float>(s, s.g32l);
   } else {
-    large_gram_dmma(s);
+    if (s.lda % 2 == 0) {
+      large_gram_dmma<2>(s);
+    } else {
+      large_gram_dmma<1>(s);
+    }
     s.sync();
     large_finish_gram<double>(s, s.g64);
     QTQP_TOC(kPhGram);
