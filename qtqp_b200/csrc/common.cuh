@@ -135,9 +135,8 @@ constexpr uint32_t kGridWaitLimit = 1u << 25;
 
 struct GridCtl {
   unsigned long long arrive;  // grid_sync's counter; kGridErrBit: a wait gave up
-  int err;                    // 1: a barrier or flag wait gave up
+  int err;                    // 1: a barrier or slot wait gave up
   int pad;
-  unsigned int flag[kGridMaxBlocks];        // per-block publication flags (flags_ready)
   double part[2][kGridMaxBlocks][kRedMax];  // per-block partials (double-buffered)
 };
 
@@ -171,53 +170,59 @@ __device__ __forceinline__ void grid_sync(GridCtl* g, uint32_t limit = kGridWait
   __syncthreads();
 }
 
-// Point-to-point hand-off between the blocks of a cooperative grid.  Block c
-// publishes a result by writing it, fencing, and storing a generation number
-// to flag[c] with release semantics (flag_publish); a consumer's warp polls
-// the flags with acquire loads (flags_ready).  Generations only grow within a
-// launch and the flags start at zero with the rest of GridCtl, so a flag is
-// never reset.  A wait that exceeds `limit` polls sets the sticky err flag;
-// every later wait then returns at once, as grid_sync does.
-__device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
+// Point-to-point hand-off between the blocks of a cooperative grid: a 16-byte
+// slot per value, the value with the tag of the step that wrote it, stored and
+// loaded as one 128-bit access.  So the value itself is what a consumer polls;
+// no fence, flag or barrier lies between the two blocks.  Tags only grow and the
+// slots start at zero, so a slot is never reset.
+struct alignas(16) GridSlot {
+  unsigned long long bits, tag;
+};
+__device__ __forceinline__ void slot_store(GridSlot* p, double v, unsigned long long tag) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"(tag)
+      : "memory");
 }
-__device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ GridSlot slot_load(const GridSlot* p) {
+  GridSlot r;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(r.bits), "=l"(r.tag)
+      : "l"(p)
+      : "memory");
+  return r;
 }
 
-// Called by one whole warp.  Looks at flag[c], flag[c + dir], ... (up to 32
-// of them, stopping before index `end`, dir = +1 or -1) and returns how many
-// consecutive ones, starting at c, have reached `gen`; waits (bounded) until
-// that is at least one.  Returns 0 only when the wait gave up or an earlier
-// wait had (err set).  Every lane returns the same value.
-__device__ __forceinline__ int flags_ready(GridCtl* g, int c, int dir, int end, unsigned int gen,
+// Called by one whole warp: the values of slots p[0], p[stride], ... (K per
+// lane), once all of the warp's carry `tag` (bounded wait).  A wait that exceeds
+// `limit` polls sets the sticky err flag, after which every later wait returns
+// soon, with whatever is there (the solve runs to its end and reports it).
+template <int K>
+__device__ __forceinline__ void slots_wait(GridCtl* g, const GridSlot* p, int stride,
+                                           unsigned long long tag, double (&out)[K],
                                            uint32_t limit = kGridWaitLimit) {
-  const int lane = threadIdx.x & 31;
-  const int i = c + dir * lane;
-  const bool in = dir > 0 ? i < end : i > end;
   for (uint32_t it = 0;; ++it) {
-    const bool ok = in && ld_acquire_gpu(&g->flag[i]) >= gen;
-    const unsigned int mask = __ballot_sync(0xffffffffu, ok);
-    if (mask & 1u) return mask == 0xffffffffu ? 32 : __ffs(~mask) - 1;
+    bool ok = true;
+    GridSlot r[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) r[k] = slot_load(p + k * stride);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      ok = ok && r[k].tag == tag;
+      out[k] = __longlong_as_double(r[k].bits);
+    }
+    if (__all_sync(0xffffffffu, ok)) return;
+    const int lane = threadIdx.x & 31;
     if ((it & 15) == 15) {  // each look at the error is another L2 round trip
       int err = lane == 0 ? *reinterpret_cast<volatile int*>(&g->err) : 0;
-      err = __shfl_sync(0xffffffffu, err, 0);
-      if (err) return 0;
+      if (__shfl_sync(0xffffffffu, err, 0)) return;
     }
     if (it >= limit) {
       if (lane == 0) grid_fail(g);
-      return 0;
+      return;
     }
-    if (it >= 256) __nanosleep(64);  // each poll is an L2 round trip; back off later
   }
-}
-
-// Called by thread 0 after a __syncthreads that follows the block's writes
-// (each writing thread fenced its own stores with __threadfence()).
-__device__ __forceinline__ void flag_publish(GridCtl* g, int c, unsigned int gen) {
-  st_release_gpu(&g->flag[c], gen);
 }
 
 // NS sums and NM maxima over every thread of the grid; all threads receive

@@ -213,7 +213,7 @@ enum MatFormat : int {
 template <typename T, class S>
 __device__ int large_factorize(S& s);
 template <typename T, class S>
-__device__ void large_chol_solve(S& s, T* v, T* w);
+__device__ __noinline__ void large_chol_solve(S& s, T* v, T* w);
 template <class S, class RowEpi, class ColEpi>
 __device__ void large_products(S& s, const double* vx, const double* vy, const double* vs,
                                const double* vp, RowEpi row_epi, ColEpi col_epi);
@@ -310,7 +310,8 @@ struct Ipm {
   unsigned char* arena;
   uint32_t tmem;
   uint32_t tc_load, tc_mma, tc_tiles;
-  uint32_t tri_gen;  // flag generations used by the whole-GPU triangular solves
+  uint32_t tri_gen;   // whole-GPU triangular solves so far (their slots' tags)
+  GridSlot* tri_slot; // and the slots, one per row
 
   __device__ __forceinline__ void sync() const {
     if constexpr (NT > 1024) {

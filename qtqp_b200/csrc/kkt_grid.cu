@@ -9,14 +9,16 @@ namespace qtqp {
 
 struct KktGridLayout {
   int npad, nblk;
-  size_t gen_off, info_off, g_off, inv_off, sinv_off, cp_off, gpart_off, total;
+  size_t tri_off, gen_off, info_off, g_off, inv_off, sinv_off, cp_off, gpart_off, total;
 };
 static __host__ __device__ inline KktGridLayout plan_kkt_grid(int n, int m) {
   KktGridLayout L;
   L.npad = round_up(n, kLB);
   L.nblk = L.npad / kLB;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  size_t off = al(sizeof(GridCtl));  // the barrier and the flags come first
+  size_t off = al(sizeof(GridCtl));  // the barrier and the slots come first
+  L.tri_off = off;
+  off += al(size_t(L.npad) * sizeof(GridSlot));
   L.gen_off = off;
   L.info_off = off + 16;
   off += 256;
@@ -69,6 +71,7 @@ __device__ inline void kkt_grid_bind(KktGridIpm& s, int n, int m, char* ws, char
   s.colpart = reinterpret_cast<double*>(gws + L.cp_off);
   s.arena = arena;
   s.tri_gen = *reinterpret_cast<const uint32_t*>(gws + L.gen_off);
+  s.tri_slot = reinterpret_cast<GridSlot*>(gws + L.tri_off);
   s.red = red;
   s.phase = 0;
   s.o = nullptr;
@@ -147,8 +150,8 @@ static int coop_launch(const void* kern, void** args, cudaStream_t stream, const
                     what);
 }
 
-int kkt_grid_reset(void* gws, cudaStream_t stream) {
-  return cuda_check(cudaMemsetAsync(gws, 0, ((sizeof(GridCtl) + 255) & ~size_t(255)) + 256, stream),
+int kkt_grid_reset(int n, int m, void* gws, cudaStream_t stream) {
+  return cuda_check(cudaMemsetAsync(gws, 0, plan_kkt_grid(n, m).g_off, stream),
                     "cudaMemsetAsync");
 }
 

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
   s.tmem = tmem_slot;
   s.tc_load = s.tc_mma = s.tc_tiles = 0;
   s.tri_gen = 0;
+  s.tri_slot = reinterpret_cast<GridSlot*>(p.ws + L.tri_off);
   s.red = red;
   s.phase = 0;
   s.o = &sopt;
@@ -148,7 +149,7 @@ extern "C" int qtqp_dense_large_solve(int32_t n, int32_t m, int32_t z, int32_t f
     return fail(QTQP_ERR_BAD_ARG, "qtqp_dense_large_solve: workspace must be 1024-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(d_workspace);
-  int rc = cuda_check(cudaMemsetAsync(ws + L.ctl_off, 0, sizeof(GridCtl), st), "cudaMemsetAsync");
+  int rc = cuda_check(cudaMemsetAsync(ws + L.ctl_off, 0, L.info_off - L.ctl_off, st), "cudaMemsetAsync");
   if (rc) return rc;
   CUtensorMap mh, ml;
   rc = make_map_f32(&mh, reinterpret_cast<const float*>(ws + L.xhi_off), L.npad, L.mpad, L.mpad);

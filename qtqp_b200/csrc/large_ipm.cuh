@@ -65,7 +65,7 @@ struct GramSplit {
 // Global workspace of a large solve.
 struct LargeLayout {
   int n, m, npad, mpad, nblk, np;
-  size_t ctl_off, info_off, v_off, a_off, p_off, g64_off, g32_off, sinv_off, xhi_off, xlo_off,
+  size_t ctl_off, tri_off, info_off, v_off, a_off, p_off, g64_off, g32_off, sinv_off, xhi_off, xlo_off,
       cp_off, gpart_off, total;
 };
 __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
@@ -80,6 +80,8 @@ __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   size_t off = 0;
   L.ctl_off = off;
   off += al(sizeof(GridCtl));
+  L.tri_off = off;  // slots of the triangular solves; zeroed with the control block
+  off += al(size_t(L.npad) * sizeof(GridSlot));
   L.info_off = off;
   off += al(16);
   L.v_off = off;
@@ -1104,21 +1106,26 @@ __device__ int large_factorize(S& s) {
 
 // ---------------------------------------------------------------------------
 // L L^T v = v in place (v, w: n entries of T; w is scratch), block by block
-// with flags instead of grid barriers.  CTA j (j < nb) owns block row j and
+// with slots instead of grid barriers.  CTA j (j < nb) owns block row j and
 // keeps inv(L_jj) resident in shared memory since the factorisation.
-//   Forward:  z_j = inv(L_jj) (v_j - sum_{c<j} L_jc z_c) into w.  CTA j adds
-//             L_jc z_c as soon as flag c shows z_c published, in the order
-//             c = 0, 1, ..., so only the last product L_{j,j-1} z_{j-1} and
-//             the diagonal step lie on the chain from one block to the next.
-//   Backward: x_j = inv(L_jj)^T (z_j - sum_{c>j} L_cj^T x_c) into v, the
-//             same way from c = nb-1 down.
+//   Forward:  z_j = inv(L_jj) (v_j - sum_{c<j} L_jc z_c), into w and the
+//             block's slots.  CTA j adds L_jc z_c as soon as the slots hold
+//             z_c, in the order c = 0, 1, ..., so only the last product
+//             L_{j,j-1} z_{j-1} and the diagonal step lie on the chain from one
+//             block to the next; L_{j,j-1} waits in registers.
+//   Backward: x_j = inv(L_jj)^T (z_j - sum_{c>j} L_cj^T x_c) into v and the
+//             slots, the same way from c = nb-1 down, with L_{j+1,j} in registers.
 // Every sum runs in a fixed order (c ascending or descending, then the
 // lanes' and warps' partials in a fixed tree), so results do not depend on
-// timing.  Flag generations: 2t - 1 (forward) and 2t (backward) for the t-th
-// solve of the launch.  One grid barrier at the end.
+// timing.  Tags: 2t - 1 (forward) and 2t (backward) for the t-th solve; a block
+// overwrites its z with its x only after every later block has published its
+// own x, and so has read that z.  One grid barrier at the end.
+// The chain of 2 nb steps bounds it: 3.0 us per step at n = 4096 and 2.4 us at
+// n = 1000 in FP32; 6.0 and 5.0 us when a block published by fences and a flag
+// that one warp polled for the CTA, and the chain's block came from L2 (128 KB).
 // ---------------------------------------------------------------------------
 template <typename T, class S>
-__device__ void large_chol_solve(S& s, T* v, T* w) {
+__device__ __noinline__ void large_chol_solve(S& s, T* v, T* w) {
   const int n = s.n, npad = s.npad;
   const int nb = (n + kLB - 1) / kLB;
   const T* g = sizeof(T) == 4 ? reinterpret_cast<const T*>(s.g32l)
@@ -1126,72 +1133,63 @@ __device__ void large_chol_solve(S& s, T* v, T* w) {
   constexpr int WPB = kGridBT / 32;
   static_assert(WPB * 16 == kLB, "one warp per 16 rows of a block");
   // Shared memory: inv(L_bb) (pitch kPitch), then the block's right-hand side
-  // (kLB), the warps' column partials of the backward step (WPB x kLB), and
-  // the hand-off of the polling warp's result.
+  // (kLB) and the warps' column partials of the backward step (WPB x kLB).
   const T* rinv = reinterpret_cast<const T*>(s.arena);
   T* red = reinterpret_cast<T*>(s.arena) + kLB * kPitch;
   T* cpart = red + kLB;
-  volatile int* sready = reinterpret_cast<volatile int*>(cpart + WPB * kLB);
   static_assert((size_t(kLB) * kPitch + kLB) * sizeof(double) <= kPrSmemOff,
                 "large_products would overwrite the resident inverse");
-  static_assert((size_t(kLB) * kPitch + kLB + WPB * kLB) * sizeof(double) + sizeof(int) <=
-                    kArenaBytes, "the solve's shared memory exceeds the arena");
+  static_assert((size_t(kLB) * kPitch + kLB + WPB * kLB) * sizeof(double) <= kArenaBytes,
+                "the solve's shared memory exceeds the arena");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = blockIdx.x;
-  auto bsz = [&](int b) { return min(kLB, n - b * kLB); };
   s.tri_gen += 1;
-  const unsigned int gen_fwd = 2 * s.tri_gen - 1, gen_bwd = 2 * s.tri_gen;
+  const unsigned long long tag_fwd = 2ull * s.tri_gen - 1, tag_bwd = 2ull * s.tri_gen;
   GridCtl* gc = s.gctl;
-  // The polling warp's count of consecutive published blocks from c (dir +1
-  // or -1, stopping before `end`), passed to the whole CTA; `none` when the
-  // wait gave up (the solve then runs to its end on whatever is there, and the
-  // sticky error reports it).
-  auto ready_until = [&](int c, int dir, int end) {
-    if (warp == 0) {
-      const int k = flags_ready(gc, c, dir, end, dir > 0 ? gen_fwd : gen_bwd);
-      if (lane == 0) *sready = k > 0 ? c + dir * k : end;
-    }
-    __syncthreads();
-    const int r = *sready;
-    __syncthreads();
-    return r;
-  };
-  // Brings the 128 x 128 block of g at (row block rb, column block cb) into
-  // L2 ahead of the step that has it on the chain between blocks (L_{j,j-1}
-  // forward, L_{j+1,j} backward), one 128-byte line per request.
-  auto prefetch_block = [&](int rb, int cb) {
-    constexpr int kLines = kLB * int(sizeof(T)) / 128;  // lines per block row
-    const int rows = bsz(rb);
-    for (int e = threadIdx.x; e < rows * kLines; e += blockDim.x) {
-      const T* p = g + size_t(rb * kLB + e / kLines) * npad + cb * kLB +
-                   (e % kLines) * (128 / int(sizeof(T)));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-    }
-  };
+  GridSlot* slots = s.tri_slot;
   QTQP_TIC();
   if (j < nb) {
-    const int b0 = j * kLB, bs = bsz(j);
+    const int b0 = j * kLB, bs = min(kLB, n - b0);
     const int r0 = 16 * warp;  // this warp's 16 rows of the block
-    if (j > 1) prefetch_block(j, j - 1);
+    const T* lrow = g + size_t(b0 + r0) * npad + lane;
+    // Rows beyond n are padding inside g (npad rows): read, never used.
+    // (The first block reads its own: a conditional load puts the array into
+    // local memory.)
+    T near[16][4];
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        near[r][q] = lrow[size_t(r) * npad + max(j - 1, 0) * kLB + 32 * q];
     // Forward: lane partials of rows r0 + r over columns lane + 32 q.
     T acc[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) acc[r] = T(0);
-    for (int c = 0; c < j;) {
-      const int hi = ready_until(c, 1, j);
-      for (; c < hi; ++c) {
-        T z[4];
+    double z[4];
+    for (int c = 0; c < j - 1; ++c) {
+      const T* lr = lrow + c * kLB;
+      T far[4][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) z[q] = __ldcg(w + c * kLB + lane + 32 * q);
-        const T* lr = g + size_t(b0 + r0) * npad + c * kLB + lane;
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          if (r0 + r < bs) {
+        for (int q = 0; q < 4; ++q) far[r][q] = lr[size_t(r) * npad + 32 * q];
+      slots_wait<4>(gc, slots + c * kLB + lane, 32, tag_fwd, z);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[r] = fma(lr[size_t(r) * npad + 32 * q], z[q], acc[r]);
-          }
+      for (int r = 0; r < 16; ++r) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[r] = fma(far[r & 3][q], T(z[q]), acc[r]);
+        if (r < 12) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) far[r & 3][q] = lr[size_t(r + 4) * npad + 32 * q];
         }
       }
+    }
+    if (j > 0) {
+      slots_wait<4>(gc, slots + (j - 1) * kLB + lane, 32, tag_fwd, z);
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[r] = fma(near[r][q], T(z[q]), acc[r]);
     }
     // Sum the 16 rows over the warp: each exchange step sends half of the
     // values to the partner lane and keeps the other half, so lane l ends with
@@ -1230,38 +1228,58 @@ __device__ void large_chol_solve(S& s, T* v, T* w) {
       }
       T zr = (a0 + a1) + (a2 + a3);
       zr += __shfl_xor_sync(0xffffffffu, zr, 16);
-      if (h == 0 && r < bs) {
-        w[b0 + r] = zr;
-        __threadfence();
+      if (h == 0) {
+        if (r >= bs) zr = T(0);
+        slot_store(slots + b0 + r, double(zr), tag_fwd);
+        if (r < bs) w[b0 + r] = zr;
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) flag_publish(gc, j, gen_fwd);
   }
   QTQP_TOC(kPhLgFwd);
   QTQP_RETIC();
   if (j < nb) {
-    const int b0 = j * kLB, bs = bsz(j);
+    const int b0 = j * kLB, bs = min(kLB, n - b0);
     const int r0 = 16 * warp;
-    if (j + 1 < nb) prefetch_block(j + 1, j);
+    const T* lcol = g + size_t(r0) * npad + b0 + lane;
+    T near[16][4];
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        near[r][q] = lcol[size_t(min(j + 1, nb - 1) * kLB + r) * npad + 32 * q];
     // Backward: lane partials of columns lane + 32 q of block j over this
-    // warp's 16 rows of every later block.
+    // warp's 16 rows of every later block (lane l holds x of row l % 16).
+    // The last block's rows beyond n have x = 0 in their slots.
     T acc[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[q] = T(0);
-    for (int c = nb - 1; c > j;) {
-      const int lo = ready_until(c, -1, j);
-      for (; c > lo; --c) {
-        const int cb0 = c * kLB, cbs = bsz(c);
+    double x[1];
+    for (int c = nb - 1; c > j + 1; --c) {
+      const T* lc = lcol + size_t(c) * kLB * npad;
+      T far[4][4];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          if (r0 + r < cbs) {
-            const T xi = __ldcg(v + cb0 + r0 + r);
-            const T* lr = g + size_t(cb0 + r0 + r) * npad + b0 + lane;
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] = fma(lr[32 * q], xi, acc[q]);
-          }
+        for (int q = 0; q < 4; ++q) far[r][q] = lc[size_t(r) * npad + 32 * q];
+      slots_wait<1>(gc, slots + c * kLB + r0 + (lane & 15), 0, tag_bwd, x);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const T xi = __shfl_sync(0xffffffffu, T(x[0]), r);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fma(far[r & 3][q], xi, acc[q]);
+        if (r < 12) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) far[r & 3][q] = lc[size_t(r + 4) * npad + 32 * q];
         }
+      }
+    }
+    if (j + 1 < nb) {
+      slots_wait<1>(gc, slots + (j + 1) * kLB + r0 + (lane & 15), 0, tag_bwd, x);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const T xi = __shfl_sync(0xffffffffu, T(x[0]), r);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fma(near[r][q], xi, acc[q]);
       }
     }
 #pragma unroll
@@ -1292,13 +1310,12 @@ __device__ void large_chol_solve(S& s, T* v, T* w) {
       }
       T xr = (a0 + a1) + (a2 + a3);
       xr += __shfl_xor_sync(0xffffffffu, xr, 16);
-      if (h == 0 && r < bs) {
-        v[b0 + r] = xr;
-        __threadfence();
+      if (h == 0) {
+        if (r >= bs) xr = T(0);
+        slot_store(slots + b0 + r, double(xr), tag_bwd);
+        if (r < bs) v[b0 + r] = xr;
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) flag_publish(gc, j, gen_bwd);
   }
   s.sync();
   // The KKT backend (no options) has no result record to report a wait that

@@ -9,10 +9,10 @@
 //   mode 0: a cooperative grid where one host-chosen block never reaches the
 //           barrier the others wait at;
 //   mode 1: a wait on an mbarrier that nothing arrives on;
-//   mode 2: the per-block flags of the whole-GPU triangular solves
-//           (flags_ready / flag_publish): a cooperative grid where block b
-//           waits for block b - 1's flag and then publishes its own, and a
-//           host-chosen block never publishes.
+//   mode 2: the value slots of the whole-GPU triangular solves
+//           (slots_wait / slot_store): a cooperative grid where block b
+//           waits for block b - 1's slot and then writes its own, and a
+//           host-chosen block never writes.
 // Nothing faults: the waits simply stop and the kernels return.
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -42,9 +42,13 @@ __global__ void __launch_bounds__(kSelftestThreads)
     flag_wait_selftest_kernel(GridCtl* g, int skip_block, uint32_t limit) {
   const int b = blockIdx.x;
   if (b == skip_block) return;  // never publishes
-  if (b > 0 && threadIdx.x < 32) flags_ready(g, b - 1, 1, b, 1u, limit);
+  GridSlot* slots = reinterpret_cast<GridSlot*>(g->part);
+  if (b > 0 && threadIdx.x < 32) {
+    double v[1];
+    slots_wait<1>(g, slots + b - 1, 0, 1u, v, limit);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) flag_publish(g, b, 1u);
+  if (threadIdx.x == 0) slot_store(slots + b, 0.0, 1u);
 }
 
 __global__ void grid_status_kernel(const GridCtl* g, int* status) {

@@ -28,14 +28,14 @@ struct SparseGridParams {
 __host__ __device__ inline size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
 struct SparseLayout {
-  size_t band_off, vals_off, z_off, parts_off, upd_off, dense_off, dinv_off, ctl_off, info_off,
+  size_t band_off, vals_off, z_off, parts_off, upd_off, dense_off, dinv_off, ctl_off, tri_off, info_off,
       total;
 };
 // Workspace: the banded backend's vectors and working values, the factor
 // (nvals), the forward products (one per stored row), the backward partial
 // sums (kSnMaxW per top-level row slab), the partial updates of split row
 // slabs, the dense part (padded to 128 columns) and the inverses of its panel
-// step, the grid's barrier state and the factorisation status.
+// step, the grid's barrier state, the solves' slots and the factorisation status.
 __host__ __device__ inline SparseLayout plan_sparse_layout(int n, int m, int nnz_a, int nnz_p,
                                                            int64_t nvals, int64_t nrows,
                                                            int64_t nslabs, int dense_cols) {
@@ -50,7 +50,8 @@ __host__ __device__ inline SparseLayout plan_sparse_layout(int n, int m, int nnz
   L.dense_off = round256(L.upd_off + size_t(kSnUbuf) * kSnSlab * kSnMaxW * 8);
   L.dinv_off = round256(L.dense_off + npad * npad * 8);
   L.ctl_off = round256(L.dinv_off + size_t(4) * 32 * kSubPitch * 8);
-  L.info_off = round256(L.ctl_off + sizeof(GridCtl));
+  L.tri_off = round256(L.ctl_off + sizeof(GridCtl));
+  L.info_off = L.tri_off + npad * sizeof(GridSlot);
   L.total = L.info_off + 256;
   return L;
 }
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(kGridBT, 1) sparse_grid_kernel(const SparseGri
   // the front of the arena, the supernodes' scratch at its end.
   s.arena = arena;
   s.tri_gen = 0;
+  s.tri_slot = reinterpret_cast<GridSlot*>(p.ws + L.tri_off);
   s.bwin = reinterpret_cast<double*>(arena + kArenaBytes - kSparseSmem);
   s.bwin_bytes = kSparseSmem;
   s.red = red;
@@ -186,7 +188,7 @@ extern "C" int qtqp_sparse_grid_solve(const qtqp_band_instance* h_inst,
                                   "16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(d_workspace);
-  rc = cuda_check(cudaMemsetAsync(ws + L.ctl_off, 0, sizeof(GridCtl), st), "cudaMemsetAsync");
+  rc = cuda_check(cudaMemsetAsync(ws + L.ctl_off, 0, L.info_off - L.ctl_off, st), "cudaMemsetAsync");
   if (rc) return rc;
   rc = cuda_check(cudaFuncSetAttribute(sparse_grid_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -112,6 +112,7 @@ struct SnDense {
   float* g32l;
   GridCtl* gctl;
   uint32_t& tri_gen;
+  GridSlot* tri_slot;
   const qtqp_options* o;
   __device__ __forceinline__ void sync() const { grid_sync(gctl); }
 };
@@ -119,7 +120,7 @@ template <class S>
 __device__ __forceinline__ SnDense sn_dense(S& s) {
   const SnFactor& F = *s.sn;
   return {F.dense_cols, round_up(F.dense_cols, kLB), s.tid, s.linfo + 16, s.arena, F.dinv, F.dense,
-          reinterpret_cast<float*>(F.dense), s.gctl, s.tri_gen, s.o};
+          reinterpret_cast<float*>(F.dense), s.gctl, s.tri_gen, s.tri_slot, s.o};
 }
 
 // The end of supernode sn's update list before the descendants in the dense part.
