@@ -37,6 +37,13 @@ constexpr size_t kLargeSmem = 1024 + kArenaBytes + 256;    // + alignment + barr
 
 __host__ __device__ inline int round_up(int v, int q) { return (v + q - 1) / q * q; }
 
+constexpr int kPitch = kLB + 1;   // shared-memory pitch of a staged 128 x 128 block
+constexpr int kSubPitch = 36;     // pitch of a staged 32 x 32 block
+// Pitch of a 128 x 128 block whose rows feed the FP64 tensor cores: 4 (mod 16),
+// so that a half-warp's fragment (4 rows x 4 columns) hits 16 banks, as does
+// kSubPitch.
+constexpr int kMmaPitch = kLB + 4;
+
 // The split of the FP64 Gram matrix over the CTAs: the lower 128 x 128 tiles,
 // row by row, times their slices of kGramKS rows of A are one sequence of
 // units, of which CTA c < ctas takes [unit0(c), unit0(c + 1)).  Whole tiles go
@@ -95,7 +102,7 @@ __host__ __device__ inline LargeLayout plan_large_layout(int n, int m) {
   L.g32_off = off;
   off += al(size_t(L.npad) * L.npad * 4);
   L.sinv_off = off;
-  off += al(4 * 32 * 33 * 8);                      // sub-block inverses of one step
+  off += al(4 * 32 * kSubPitch * 8);               // sub-block inverses of one step
   L.xhi_off = off;
   off += al(size_t(L.npad) * L.mpad * 4);
   L.xlo_off = off;
@@ -564,9 +571,6 @@ __device__ void large_finish_gram(S& s, T* g) {
 //   (c) the lower 128 x 128 tiles right of the panel get g_ij -= L_ik L_jk^T
 //       with 8 x 8 outputs per thread and cp.async double-buffered slices.
 // ---------------------------------------------------------------------------
-constexpr int kPitch = kLB + 1;   // shared-memory pitch of a staged 128 x 128 block
-constexpr int kSubPitch = 33;     // pitch of a staged 32 x 32 block
-
 // 128 x 128 block of g at (r0, c0) into dst[r * kPitch + c], eight loads in
 // flight per thread; the strict upper part is zero when lower_only.
 template <typename T>
@@ -587,227 +591,383 @@ __device__ __forceinline__ void stage_block(T* dst, const T* g, size_t ld, int r
   }
 }
 
-// Cholesky of the 128 x 128 block in shared memory (lower, pitch kPitch) by
-// the CTA: every thread owns up to three 4 x 4 tiles of the lower triangle in
-// registers, right-looking in 4-column panels with one barrier per panel.
-// Tiles are numbered down the columns, so that the tiles of one panel belong
-// to one or two warps: while these finish panel k + 1 (each thread factors the
-// 4 x 4 diagonal tile for itself), the other warps apply panel k to theirs.
-// Panel k's tiles are published in pb (two panels, 17 elements per tile); the
-// diagonal tile of panel k + 2, one update short, in dg (two tiles), and its
-// readers apply the missing update themselves, in the owner's order.
-// On return sm holds L, rd the reciprocals of its diagonal.  sflag: two slots.
-// Returns 0 or the 1-based index of the first non-positive pivot.
-//
-// The chain is 128 reciprocal square roots (75 cycles each) and about as long
-// again in products, loads and barriers: 12 us, against some 85 us for 32-wide
-// blocks factored by one warp in Crout order.
-constexpr int kTileCholTiles = 3;
-constexpr int kTileCholPb = 2 * 32 * 17;
+// Two or four consecutive values of T from global memory as doubles.
+__device__ __forceinline__ void load_pair(double (&v)[2], const double* p) {
+  const double2 t = *reinterpret_cast<const double2*>(p);
+  v[0] = t.x;
+  v[1] = t.y;
+}
+__device__ __forceinline__ void load_pair(double (&v)[2], const float* p) {
+  const float2 t = *reinterpret_cast<const float2*>(p);
+  v[0] = t.x;
+  v[1] = t.y;
+}
+__device__ __forceinline__ void store_pair(double* p, const double (&v)[2]) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
+__device__ __forceinline__ void store_pair(float* p, const double (&v)[2]) {
+  *reinterpret_cast<float2*>(p) = make_float2(float(v[0]), float(v[1]));
+}
+
+// The 128 x 128 block of g (leading dimension ld) at (r0, c0) as doubles into
+// dst (pitch kMmaPitch).
 template <typename T>
-__device__ __noinline__ int cta_chol128(T* sm, T* pb, T* dg, T* rd, volatile int* sflag) {
-  constexpr int TPT = kTileCholTiles, NB = kLB / 4;
-  static_assert(TPT * kGridBT >= NB * (NB + 1) / 2, "tiles");
-  bool mine[TPT];
-  int bi[TPT], bj[TPT];
-  T acc[TPT][4][4];
+__device__ __forceinline__ void stage_mma(double* dst, const T* g, size_t ld, int r0, int c0) {
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 8
+    for (int q = 0; q < kLB * kLB / 2 / kGridBT; ++q) {
+      const int e = threadIdx.x + q * kGridBT, r = e >> 6, c = 2 * (e & 63);
+      cp_async16(dst + r * kMmaPitch + c, g + size_t(r0 + r) * ld + c0 + c);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  } else {
+#pragma unroll 1
+    for (int base = 0; base < kLB * kLB / 2; base += 8 * kGridBT) {
+      double v[8][2];
 #pragma unroll
-  for (int q = 0; q < TPT; ++q) {
-    const int t = threadIdx.x + q * kGridBT;
-    mine[q] = t < NB * (NB + 1) / 2;
-    // Column c starts at c NB - c (c - 1) / 2.
-    int c = int((2 * NB + 1 - sqrtf(float((2 * NB + 1) * (2 * NB + 1) - 8 * t))) * 0.5f);
-    c = min(max(c, 0), NB - 1);
-    while (c > 0 && c * NB - c * (c - 1) / 2 > t) --c;
-    while (c + 1 < NB && (c + 1) * NB - (c + 1) * c / 2 <= t) ++c;
-    bj[q] = c;
-    bi[q] = c + t - (c * NB - c * (c - 1) / 2);
-    if (!mine[q]) bi[q] = bj[q] = 0;
+      for (int q = 0; q < 8; ++q) {
+        const int e = base + threadIdx.x + q * kGridBT;
+        load_pair(v[q], g + size_t(r0 + (e >> 6)) * ld + c0 + 2 * (e & 63));
+      }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        acc[q][a][b] = mine[q] ? sm[(bi[q] * 4 + a) * kPitch + bj[q] * 4 + b] : T(0);
+      for (int q = 0; q < 8; ++q) {
+        const int e = base + threadIdx.x + q * kGridBT;
+        store_pair(dst + (e >> 6) * kMmaPitch + 2 * (e & 63), v[q]);
+      }
+    }
   }
-  if (threadIdx.x < 2) sflag[threadIdx.x] = 0;
-  auto put_diag = [&](int t) {
+  __syncthreads();
+}
+
+// sm = (the diagonal block of g at row b0) - L L^T, lower part, with L the 128
+// rows b0 .. of the panel at column k0 (pitch kMmaPitch; the strict upper part
+// of sm is undefined).  The block's 20 lower 16 x 32 units go to the eight
+// warps, five per pair that shares a tensor core, with L staged whole.
+// Bound by the SM's FP64 tensor cores: 29000 cycles, against 70000 for a square
+// tile through the trailing update's loop, written back and staged again (and
+// that on the chain of the factorisation).
+template <typename T>
+__device__ __noinline__ void cta_diag_update(double* sm, const T* g, size_t ld, int b0, int k0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+  stage_mma(sm, g, ld, b0, k0);
+  // Unit u: 16 rows at 16 ui, 32 columns at 32 uj (2 uj <= ui + 1).
+  int ui[3], uj[3];
 #pragma unroll
-    for (int q = 0; q < TPT; ++q) {
-      if (!mine[q] || bi[q] != t || bj[q] != t) continue;
+  for (int q = 0; q < 3; ++q) {
+    const int u = warp + 8 * q;
+    // Units of the row pair p (rows 32 p ..): 2 (p + 1), starting at p (p + 1).
+    int p = 0;
+    while (p < 3 && (p + 1) * (p + 2) <= u) ++p;
+    const int e = u - p * (p + 1);
+    ui[q] = 2 * p + (e > p ? 1 : 0);
+    uj[q] = e > p ? e - p - 1 : e;
+  }
+  double acc[3][2][4][2];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+  for (int q = 0; q < 3; ++q)
 #pragma unroll
-        for (int b = 0; b <= a; ++b) dg[(t & 1) * 16 + a * 4 + b] = acc[q][a][b];
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[q][a][b][0] = acc[q][a][b][1] = 0.0;
+  const bool third = warp < 4;
+#pragma unroll 2
+  for (int k = 0; k < kLB; k += 4) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (q == 2 && !third) continue;
+      const double* ra = sm + (16 * ui[q] + gi) * kMmaPitch + k + tg;
+      const double* rb = sm + (32 * uj[q] + gi) * kMmaPitch + k + tg;
+      double a[2], b[4];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) a[x] = ra[x * 8 * kMmaPitch];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) b[x] = rb[x * 8 * kMmaPitch];
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) dmma_8x8x4(acc[q][x][y], a[x], b[y]);
     }
-  };
-  // acc -= L_{i,k} L_{j,k}^T with panel k.
-  auto update = [&](int q, int k) {
-    const T* pi = pb + (k & 1) * (NB * 17) + bi[q] * 17;
-    const T* pj = pb + (k & 1) * (NB * 17) + bj[q] * 17;
+  }
+  __syncthreads();
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      T li[4], lj[4];
+  for (int q = 0; q < 3; ++q) {
+    if (q == 2 && !third) continue;
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        li[a] = pi[a * 4 + c];
-        lj[a] = pj[a * 4 + c];
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int r = 16 * ui[q] + 8 * x + gi, c = 32 * uj[q] + 8 * y + 2 * tg;
+        double v[2];
+        load_pair(v, g + size_t(b0 + r) * ld + b0 + c);
+        v[0] -= acc[q][x][y][0];
+        v[1] -= acc[q][x][y][1];
+        store_pair(sm + r * kMmaPitch + c, v);
       }
+  }
+  __syncthreads();
+}
+
+// Cholesky of the 128 x 128 block in shared memory (lower, pitch kMmaPitch) by
+// the CTA, and the inverses of its four 32 x 32 diagonal sub-blocks into inv
+// (pitch kSubPitch, zero above the diagonal).  Per sub-block b:
+//   * warp 0 factors it, lane l with row l in registers: per column one chain of
+//     pivot shuffle, reciprocal square root, scaling and the update of the next
+//     pivot, the other updates beside it;
+//   * warp 1 inverts it, lane c with column c of the inverse in registers, eight
+//     columns of L behind warp 0 (named barrier 1);
+//   * warps 2 - 7 meanwhile apply the previous sub-block's products to the rest
+//     of the block, all but the sub-block in work;
+//   * then all warps multiply the rows below by the inverse's transpose and
+//     update the next sub-block (FP64 tensor cores).
+// rd: 32 doubles, sflag: one slot.  Returns 0 or the 1-based index of the first
+// non-positive pivot.
+// The chain over the columns bounds it: 43700 cycles in all.  Register tiles of
+// 4 x 4 over the whole block with a barrier per four columns took 75000 cycles,
+// and the inverses, a column per lane from shared memory, another 18000.
+template <int K0>
+__device__ __forceinline__ void chol32_columns(double (&a)[32], int lane, double* rd, int& bad) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+  for (int k = K0; k < K0 + 8; ++k) {
+    const double d = __shfl_sync(0xffffffffu, a[k], k);
+    if (bad == 0 && !(d > 0.0)) bad = k + 1;
+    const double r = rsqrt(d);
+    const double l = lane >= k ? a[k] * r : 0.0;
+    a[k] = l;
+    if (lane == k) rd[k] = r;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[q][a][b] = fma(-li[a], lj[b], acc[q][a][b]);
-    }
-  };
-  // The tiles of column t (updated by panels < t) become L, published.
-  auto do_panel = [&](int t) {
+    for (int j = k + 1; j < 32; ++j) a[j] = fma(-l, __shfl_sync(0xffffffffu, l, j), a[j]);
+  }
+}
+template <int K0>
+__device__ __forceinline__ void inv32_columns(double (&w)[32], const double* L, const double* rd) {
 #pragma unroll
-    for (int q = 0; q < TPT; ++q) {
-      if (!mine[q] || bj[q] != t) continue;
-      T d[4][4], lc[4][4], il[4];
+  for (int k = K0; k < K0 + 8; ++k) {
+    const double x = w[k] * rd[k];
+    w[k] = x;
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b <= a; ++b) d[a][b] = dg[(t & 1) * 16 + a * 4 + b];
-      if (t > 0) {
-        const T* pr = pb + ((t - 1) & 1) * (NB * 17) + t * 17;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          T l[4];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) l[a] = pr[a * 4 + c];
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b <= a; ++b) d[a][b] = fma(-l[a], l[b], d[a][b]);
-        }
-      }
+    for (int i = k + 1; i < 32; ++i) w[i] = fma(-L[i * kMmaPitch + k], x, w[i]);
+  }
+}
+__device__ __forceinline__ void pair_barrier() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
+__device__ __noinline__ static int cta_chol128(double* sm, double* inv, double* rd, volatile int* sflag) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+  if (threadIdx.x == 0) *sflag = 0;
+#pragma unroll 1
+  for (int b = 0; b < 4; ++b) {
+    const int o = 32 * b;
+    double* D = sm + o * kMmaPitch + o;
+    if (warp == 0) {
+      double a[32];
       int bad = 0;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const T piv = d[c][c];
-        if (bad == 0 && !(piv > T(0))) bad = 4 * t + c + 1;
-        il[c] = rsqrt(piv);
-        lc[c][c] = piv * il[c];
+      for (int c = 0; c < 32; ++c) a[c] = D[lane * kMmaPitch + c];
+      auto put = [&](int c0) {
 #pragma unroll
-        for (int a = c + 1; a < 4; ++a) lc[a][c] = d[a][c] * il[c];
+        for (int c = 0; c < 32; ++c)
+          if (c >= c0 && c < c0 + 8 && c <= lane) D[lane * kMmaPitch + c] = a[c];
+      };
+      chol32_columns<0>(a, lane, rd, bad);
+      put(0);
+      pair_barrier();
+      chol32_columns<8>(a, lane, rd, bad);
+      put(8);
+      pair_barrier();
+      chol32_columns<16>(a, lane, rd, bad);
+      put(16);
+      pair_barrier();
+      chol32_columns<24>(a, lane, rd, bad);
+      put(24);
+      pair_barrier();
+      if (bad != 0 && lane == 0) *sflag = o + bad;
+    } else if (warp == 1) {
+      double w[32];
 #pragma unroll
-        for (int a = c + 1; a < 4; ++a)
+      for (int i = 0; i < 32; ++i) w[i] = i == lane ? 1.0 : 0.0;
+      pair_barrier();
+      inv32_columns<0>(w, D, rd);
+      pair_barrier();
+      inv32_columns<8>(w, D, rd);
+      pair_barrier();
+      inv32_columns<16>(w, D, rd);
+      pair_barrier();
+      inv32_columns<24>(w, D, rd);
+      double* X = inv + b * 32 * kSubPitch + lane;
 #pragma unroll
-          for (int b = c + 1; b <= a; ++b) d[a][b] = fma(-lc[a][c], lc[b][c], d[a][b]);
-      }
-      if (bi[q] == t) {
-        if (bad) sflag[t & 1] = bad;
+      for (int i = 0; i < 32; ++i) X[i * kSubPitch] = w[i];
+    } else if (b > 0) {
+      // The products of sub-block column b - 1 for the lower 16 x 16 units of
+      // rows and columns >= o, without the sub-block at o itself (units 0 - 2).
+      const int units = (8 - 2 * b) * (9 - 2 * b) / 2;
+      for (int u = 3 + warp - 2; u < units; u += 6) {
+        int p = 0;
+        while ((p + 1) * (p + 2) / 2 <= u) ++p;
+        const int r0 = o + 16 * p, c0 = o + 16 * (u - p * (p + 1) / 2);
+        const double* ra = sm + (r0 + gi) * kMmaPitch + o - 32 + tg;
+        const double* rb = sm + (c0 + gi) * kMmaPitch + o - 32 + tg;
+        double acc[2][2][2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          rd[4 * t + a] = il[a];
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) acc[q][a][b] = b <= a ? lc[a][b] : T(0);
-        }
-      } else {
-        T* dst = pb + (t & 1) * (NB * 17) + bi[q] * 17;
+          for (int y = 0; y < 2; ++y)
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+            for (int e = 0; e < 2; ++e)
+              acc[x][y][e] = sm[(r0 + 8 * x + gi) * kMmaPitch + c0 + 8 * y + 2 * tg + e];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            T x = acc[q][a][c];
+        for (int k = 0; k < 32; k += 4) {
+          double av[2], bv[2];
 #pragma unroll
-            for (int e = 0; e < c; ++e) x = fma(-acc[q][a][e], lc[c][e], x);
-            acc[q][a][c] = x * il[c];
-            dst[a * 4 + c] = acc[q][a][c];
+          for (int x = 0; x < 2; ++x) {
+            av[x] = -ra[x * 8 * kMmaPitch + k];
+            bv[x] = rb[x * 8 * kMmaPitch + k];
           }
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) dmma_8x8x4(acc[x][y], av[x], bv[y]);
+        }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+            store_pair(sm + (r0 + 8 * x + gi) * kMmaPitch + c0 + 8 * y + 2 * tg, acc[x][y]);
       }
     }
-  };
-  put_diag(0);
-  put_diag(1);
-  __syncthreads();
-  do_panel(0);
-  __syncthreads();
-  int bad = sflag[0];
-#pragma unroll 1
-  for (int k = 0; bad == 0 && k + 1 < NB; ++k) {
-#pragma unroll
-    for (int q = 0; q < TPT; ++q)
-      if (mine[q] && bj[q] == k + 1) update(q, k);
-    do_panel(k + 1);
-#pragma unroll
-    for (int q = 0; q < TPT; ++q)
-      if (mine[q] && bj[q] > k + 1) update(q, k);
-    if (k + 2 < NB) put_diag(k + 2);
     __syncthreads();
-    // Panel k + 2 notes its failure in the other slot, so every thread reads
-    // the same value here.
-    bad = sflag[(k + 1) & 1];
+    const int bad = *sflag;
+    if (bad != 0 || b == 3) return bad;
+    // The rows below: L_ib = A_ib inv(L_bb)^T, eight rows at a time per warp
+    // (in place: a warp reads its rows' fragments before it writes them).
+    const double* X = inv + b * 32 * kSubPitch;
+    for (int r = o + 32 + 8 * warp; r < kLB; r += 64) {
+      double* row = sm + (r + gi) * kMmaPitch + o;
+      double av[8], acc[4][2];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) av[k] = row[4 * k + tg];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) acc[y][0] = acc[y][1] = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)  // inv(L_bb) is zero right of its diagonal
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+          if (4 * k < 8 * y + 8)
+            dmma_8x8x4(acc[y], av[k], X[(8 * y + gi) * kSubPitch + 4 * k + tg]);
+      __syncwarp();
+#pragma unroll
+      for (int y = 0; y < 4; ++y) store_pair(row + 8 * y + 2 * tg, acc[y]);
+    }
+    __syncthreads();
+    // The next sub-block's update: its ten lower 8 x 8 tiles.
+    for (int t = warp; t < 10; t += 8) {
+      int p = 0;
+      while ((p + 1) * (p + 2) / 2 <= t) ++p;
+      const int r0 = o + 32 + 8 * p, c0 = o + 32 + 8 * (t - p * (p + 1) / 2);
+      double* out = sm + (r0 + gi) * kMmaPitch + c0 + 2 * tg;
+      double acc[2][2] = {{out[0], out[1]}, {0.0, 0.0}};
+#pragma unroll
+      for (int k = 0; k < 32; k += 4)
+        dmma_8x8x4(acc[(k >> 2) & 1], -sm[(r0 + gi) * kMmaPitch + o + k + tg],
+                   sm[(c0 + gi) * kMmaPitch + o + k + tg]);
+      acc[0][0] += acc[1][0];
+      acc[0][1] += acc[1][1];
+      store_pair(out, acc[0]);
+    }
+    __syncthreads();
   }
+  return 0;
+}
+
+// Eight rows of the panel at column k0 of g (leading dimension ld) from row r
+// on, the calling warp: x L_kk^T = g_row for each row, 32 columns at a time
+// (x_q = (g_q - sum_{p<q} x_p L_qp^T) inv(L_qq)^T) on the FP64 tensor cores.
+// lkk: L_kk (pitch kMmaPitch), inv: the inverses of its diagonal sub-blocks.
+template <typename T>
+__device__ __forceinline__ void warp_panel_rows(T* g, size_t ld, int r, int k0, const double* lkk,
+                                                const double* inv) {
+  const int lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+  T* row = g + size_t(r + gi) * ld + k0 + 2 * tg;
+  double v[4][4][2];  // the 8 x 128 values in accumulator layout
 #pragma unroll
-  for (int q = 0; q < TPT; ++q)
-    if (mine[q])
+  for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+    for (int y = 0; y < 4; ++y) load_pair(v[q][y], row + 32 * q + 8 * y);
+  // Accumulator layout (row gi, columns 8 y + 2 tg + e) to the fragment of step
+  // k (row gi, column 4 k + tg).
+  auto fragment = [&](const double (&c)[4][2], int k) {
+    const int src = 4 * gi + 2 * (k & 1) + (tg >> 1);
+    const double e0 = __shfl_sync(0xffffffffu, c[k >> 1][0], src);
+    const double e1 = __shfl_sync(0xffffffffu, c[k >> 1][1], src);
+    return (tg & 1) ? e1 : e0;
+  };
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (bi[q] != bj[q] || b <= a) sm[(bi[q] * 4 + a) * kPitch + bj[q] * 4 + b] = acc[q][a][b];
-  __syncthreads();
-  return bad;
+  for (int q = 0; q < 4; ++q) {
+    double x[4][2];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) x[y][0] = x[y][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const double f = fragment(v[q], k);
+#pragma unroll
+      for (int y = 0; y < 4; ++y)
+        if (4 * k < 8 * y + 8)
+          dmma_8x8x4(x[y], f, inv[q * 32 * kSubPitch + (8 * y + gi) * kSubPitch + 4 * k + tg]);
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y) store_pair(row + 32 * q + 8 * y, x[y]);
+    if (q < 3) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double f = -fragment(x, k);
+#pragma unroll
+        for (int q2 = q + 1; q2 < 4; ++q2)
+#pragma unroll
+          for (int y = 0; y < 4; ++y)
+            dmma_8x8x4(v[q2][y], f, lkk[(32 * q2 + 8 * y + gi) * kMmaPitch + 32 * q + 4 * k + tg]);
+      }
+    }
+  }
 }
 
 // Inverses of the four 32 x 32 diagonal sub-blocks of the factored block sm
-// (rd: the reciprocals of its diagonal) into inv[q] (pitch kSubPitch, zero
-// above the diagonal), a warp each: lane c forms column c top-down, X_rc =
-// -(sum_{k<r} L_rk X_kc) / l_rr (X_kc = 0 for k < c).  No barrier inside.
-template <typename T>
-__device__ __noinline__ void cta_sub_inverses(const T* sm, const T* rd, T* inv) {
+// (pitch kPitch) into inv[q] (pitch kSubPitch, zero above the diagonal), a warp
+// each, lane c with column c in registers; then a barrier.
+__device__ __noinline__ static void cta_sub_inverses(const double* sm, double* inv) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= 4) return;
-  const int o = 32 * warp;
-  T* X = inv + warp * 32 * kSubPitch;
-  const T* L = sm + o * kPitch + o;
-#pragma unroll 1
-  for (int r = 0; r < 32; ++r) {
-    T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
-    const T* Lr = L + r * kPitch;
-    int k = 0;
-#pragma unroll 2
-    for (; k + 3 < r; k += 4) {
-      a0 = fma(Lr[k], X[k * kSubPitch + lane], a0);
-      a1 = fma(Lr[k + 1], X[(k + 1) * kSubPitch + lane], a1);
-      a2 = fma(Lr[k + 2], X[(k + 2) * kSubPitch + lane], a2);
-      a3 = fma(Lr[k + 3], X[(k + 3) * kSubPitch + lane], a3);
+  if (warp < 4) {
+    const double* L = sm + 32 * warp * (kPitch + 1);
+    const double rl = 1.0 / L[lane * kPitch + lane];
+    double w[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) w[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const double x = w[k] * __shfl_sync(0xffffffffu, rl, k);
+      w[k] = x;
+#pragma unroll
+      for (int i = k + 1; i < 32; ++i) w[i] = fma(-L[i * kPitch + k], x, w[i]);
     }
-    for (; k < r; ++k) a0 = fma(Lr[k], X[k * kSubPitch + lane], a0);
-    const T il = rd[o + r];
-    X[r * kSubPitch + lane] = r < lane ? T(0) : (r == lane ? il : -((a0 + a1) + (a2 + a3)) * il);
-    __syncwarp();
+    double* X = inv + warp * 32 * kSubPitch + lane;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) X[i * kSubPitch] = w[i];
   }
+  __syncthreads();
 }
 
 // C = s A B for 32-row, 32-column blocks in shared memory (leading dimensions
-// pa, pb, pc; inner length K, a multiple of 4), the CTA's eight warps two 8 x
-// 8 tiles each (FP64: DMMA), then a barrier.
-template <typename T>
-__device__ __forceinline__ void cta_gemm32(T* C, int pc, const T* A, int pa, const T* B, int pb,
-                                           int K, T scale) {
+// pa, pb, pc; inner length K, a multiple of 4) on the FP64 tensor cores, the
+// CTA's eight warps two 8 x 8 tiles each, then a barrier.
+__device__ __forceinline__ void cta_gemm32(double* C, int pc, const double* A, int pa,
+                                           const double* B, int pb, int K, double scale) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
   const int r0 = (warp >> 1) * 8, c0 = (warp & 1) * 16;
-  T acc[2][2] = {{T(0), T(0)}, {T(0), T(0)}};
-  if constexpr (sizeof(T) == 8) {
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll 4
-    for (int k = 0; k < K; k += 4) {
-      const double a = A[(r0 + gi) * pa + k + tg];
-      const double b0 = B[(k + tg) * pb + c0 + gi], b1 = B[(k + tg) * pb + c0 + 8 + gi];
-      dmma_8x8x4(acc[0], a, b0);
-      dmma_8x8x4(acc[1], a, b1);
-    }
-  } else {
-#pragma unroll 4
-    for (int k = 0; k < K; ++k) {
-      const T a = A[(r0 + gi) * pa + k];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          acc[h][e] = fma(a, B[k * pb + c0 + 8 * h + 2 * tg + e], acc[h][e]);
-    }
+  for (int k = 0; k < K; k += 4) {
+    const double a = A[(r0 + gi) * pa + k + tg];
+    const double b0 = B[(k + tg) * pb + c0 + gi], b1 = B[(k + tg) * pb + c0 + 8 + gi];
+    dmma_8x8x4(acc[0], a, b0);
+    dmma_8x8x4(acc[1], a, b1);
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h)
@@ -820,25 +980,24 @@ __device__ __forceinline__ void cta_gemm32(T* C, int pc, const T* A, int pa, con
 // kPitch) from the inverses of its 32 x 32 diagonal blocks: block column by
 // block column, X_ij = -X_ii sum_{j<=k<i} L_ik X_kj (block column j of L is
 // not needed by the later ones).  tmp: 32 x kSubPitch.
-template <typename T>
-__device__ __noinline__ void cta_inverse128(T* sm, const T* inv, T* tmp) {
+__device__ __noinline__ static void cta_inverse128(double* sm, const double* inv, double* tmp) {
   for (int j = 0; j < 4; ++j) {
     for (int i = j + 1; i < 4; ++i) {
       // X_jj for k = j, then the rows j + 1 .. i - 1 of this block column.
-      cta_gemm32<T>(tmp, kSubPitch, sm + 32 * i * kPitch + 32 * j, kPitch,
-                    inv + j * 32 * kSubPitch, kSubPitch, 32, T(1));
+      cta_gemm32(tmp, kSubPitch, sm + 32 * i * kPitch + 32 * j, kPitch,
+                    inv + j * 32 * kSubPitch, kSubPitch, 32, 1.0);
       if (i > j + 1) {
         // The rest of the sum into the block's own place, then both added.
-        cta_gemm32<T>(sm + 32 * i * kPitch + 32 * j, kPitch,
+        cta_gemm32(sm + 32 * i * kPitch + 32 * j, kPitch,
                       sm + 32 * i * kPitch + 32 * (j + 1), kPitch,
-                      sm + 32 * (j + 1) * kPitch + 32 * j, kPitch, 32 * (i - j - 1), T(1));
+                      sm + 32 * (j + 1) * kPitch + 32 * j, kPitch, 32 * (i - j - 1), 1.0);
         for (int e = threadIdx.x; e < 1024; e += kGridBT)
           tmp[(e >> 5) * kSubPitch + (e & 31)] +=
               sm[(32 * i + (e >> 5)) * kPitch + 32 * j + (e & 31)];
         __syncthreads();
       }
-      cta_gemm32<T>(sm + 32 * i * kPitch + 32 * j, kPitch, inv + i * 32 * kSubPitch, kSubPitch,
-                    tmp, kSubPitch, 32, T(-1));
+      cta_gemm32(sm + 32 * i * kPitch + 32 * j, kPitch, inv + i * 32 * kSubPitch, kSubPitch,
+                    tmp, kSubPitch, 32, -1.0);
     }
     // X_jj: rows of L_jj are not needed any more (the columns to its right
     // do not touch block column j).
@@ -853,38 +1012,33 @@ template <typename T, class S>
 __device__ int large_cholesky(S& s, T* g) {
   const int npad = s.npad, nblk = npad / kLB;
   int* info = s.linfo;
-  T* sm = reinterpret_cast<T*>(s.arena);   // staged 128 x 128 block (pitch kPitch)
-  T* sinv = sm + kLB * kPitch;              // 4 sub-block inverses (pitch kSubPitch)
-  T* pbuf = sinv + 4 * 32 * kSubPitch;      // published panels of cta_chol128
-  T* dbuf = pbuf + kTileCholPb;
-  T* rdiag = dbuf + 32;                     // reciprocal diagonal
-  T* tmp32 = rdiag + kLB;                   // 32 x kSubPitch
+  T* sm = reinterpret_cast<T*>(s.arena);      // the trailing update's slices
+  // The diagonal block and the panel rows are computed in FP64 whatever T is.
+  double* blk = reinterpret_cast<double*>(s.arena);  // 128 x 128 block
+  double* sinv = blk + kLB * kMmaPitch;              // 4 sub-block inverses
+  double* rdiag = sinv + 4 * 32 * kSubPitch;
+  double* tmp32 = rdiag + 32;                        // 32 x kSubPitch
   volatile int* sflag = reinterpret_cast<volatile int*>(tmp32 + 32 * kSubPitch);
-  static_assert((size_t(kLB) * kPitch + 5 * 32 * kSubPitch + kTileCholPb + 32 + kLB) *
-                        sizeof(double) + 16 <= kArenaBytes, "the factorisation's shared memory");
-  T* ginv = reinterpret_cast<T*>(s.sinv);   // the same inverses in global memory
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gwarp = blockIdx.x * (kGridBT / 32) + warp, nwarps = gridDim.x * (kGridBT / 32);
+  static_assert((size_t(kLB) * kMmaPitch + 5 * 32 * kSubPitch + 32) * sizeof(double) + 16 <=
+                    kArenaBytes, "the factorisation's shared memory");
+  double* ginv = s.sinv;  // the same inverses in global memory
+  const int warp = threadIdx.x >> 5;
   if (s.tid == 0) *info = 0;
   s.sync();
   QTQP_TIC();
-  // (a) Factor the diagonal block starting at column k0 (the calling CTA) in
-  // shared memory, then back to g with the reciprocal diagonal and the four
-  // 32 x 32 sub-block inverses (also to global memory, for the panel step).
+  // (a) Factor the diagonal block at column k0, in blk (the calling CTA), then
+  // to g, and the four 32 x 32 sub-block inverses to global memory for the
+  // panel step.
   auto factor_diag = [&](int k0) {
-    stage_block(sm, g, npad, k0, k0, true);
-    __syncthreads();
-    const int bad = cta_chol128<T>(sm, pbuf, dbuf, rdiag, sflag);
+    const int bad = cta_chol128(blk, sinv, rdiag, sflag);
     if (bad) {
       if (threadIdx.x == 0) atomicCAS(info, 0, k0 + bad);
     } else {
-      cta_sub_inverses<T>(sm, rdiag, sinv);
-      for (int e = threadIdx.x; e < kLB * kLB; e += blockDim.x) {
+      for (int e = threadIdx.x; e < 4 * 32 * kSubPitch; e += kGridBT) ginv[e] = sinv[e];
+      for (int e = threadIdx.x; e < kLB * kLB; e += kGridBT) {
         const int r = e >> 7, c = e & 127;
-        if (c <= r) g[size_t(k0 + r) * npad + k0 + c] = sm[r * kPitch + c];
+        if (c <= r) g[size_t(k0 + r) * npad + k0 + c] = T(blk[r * kMmaPitch + c]);
       }
-      __syncthreads();
-      for (int e = threadIdx.x; e < 4 * 32 * kSubPitch; e += blockDim.x) ginv[e] = sinv[e];
     }
     __syncthreads();
   };
@@ -893,41 +1047,23 @@ __device__ int large_cholesky(S& s, T* g) {
     QTQP_RETIC();
     // (a) diagonal block: only for the first one; every later one is
     // factored during the previous step's trailing update (lookahead).
-    if (k == 0 && blockIdx.x == 0) factor_diag(k0);
+    if (k == 0 && blockIdx.x == 0) {
+      stage_mma(blk, g, npad, 0, 0);
+      factor_diag(0);
+    }
     if (k == 0) s.sync();
     QTQP_TOC(kPhLgDiag);
     QTQP_RETIC();
     if (*reinterpret_cast<volatile int*>(info) != 0) break;
     const int rest = npad - k0 - kLB;
     if (rest == 0) break;
-    // (b) panel rows.
-    if (k0 + kLB + int(blockIdx.x) * (kGridBT / 32) < npad) {  // this CTA has rows
-      stage_block(sm, g, npad, k0, k0, true);
-      for (int e = threadIdx.x; e < 4 * 32 * kSubPitch; e += blockDim.x) sinv[e] = ginv[e];
+    // (b) panel rows, eight per warp, spread over the CTAs before the warps.
+    if (int(blockIdx.x) * 8 < rest) {
+      stage_mma(blk, g, npad, k0, k0);
+      for (int e = threadIdx.x; e < 4 * 32 * kSubPitch; e += kGridBT) sinv[e] = ginv[e];
       __syncthreads();
-      for (int row = k0 + kLB + gwarp; row < npad; row += nwarps) {
-        T* gr = g + size_t(row) * npad + k0;
-        T v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = gr[32 * q + lane];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const T* iq = sinv + q * 32 * kSubPitch;
-          T x = T(0);
-#pragma unroll
-          for (int l = 0; l < 32; ++l)
-            x = fma(__shfl_sync(0xffffffffu, v[q], l), iq[lane * kSubPitch + l], x);
-          v[q] = x;
-#pragma unroll
-          for (int q2 = q + 1; q2 < 4; ++q2) {
-            const T* lr = sm + (32 * q2 + lane) * kPitch + 32 * q;
-#pragma unroll
-            for (int l = 0; l < 32; ++l) v[q2] = fma(-__shfl_sync(0xffffffffu, x, l), lr[l], v[q2]);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gr[32 * q + lane] = v[q];
-      }
+      for (int t = blockIdx.x + warp * gridDim.x; 8 * t < rest; t += gridDim.x * (kGridBT / 32))
+        warp_panel_rows<T>(g, npad, k0 + kLB + 8 * t, k0, blk, sinv);
     }
     s.sync();
     QTQP_TOC(kPhLgPanel);
@@ -957,16 +1093,18 @@ __device__ int large_cholesky(S& s, T* g) {
         }
         cp_async_commit();
       };
-      // Lookahead: the CTA that owns the next diagonal block updates tile 0
-      // (that block) first and factors it at once; the other tiles go round
-      // robin over the other CTAs.
+      // Lookahead: the CTA that owns the next diagonal block (tile 0) updates it
+      // and factors it at once; the other tiles go round robin over the others.
       const int G = int(gridDim.x), owner = (k + 1) % G, me = int(blockIdx.x);
-      const int first_t = me == owner ? 0 : 1 + (me - owner - 1 + G) % G;
-      const int step_t = me == owner ? tiles : G - 1;
-      for (int t = first_t; t < tiles; t += (t == 0 ? tiles : step_t)) {
-        int ti = 0;
-        while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-        const int tj = t - ti * (ti + 1) / 2;
+      const int first_t = me == owner ? tiles : 1 + (me - owner - 1 + G) % G;
+      const int step_t = G - 1;
+      if (me == owner) {
+        cta_diag_update<T>(blk, g, npad, base, k0);
+        factor_diag(base);
+      }
+      for (int t = first_t; t < tiles; t += step_t) {
+        int ti, tj;
+        lower_tile(t, ti, tj);
         const int i0 = base + ti * kLB, j0 = base + tj * kLB;
         T acc[8][8];
 #pragma unroll
@@ -1047,10 +1185,6 @@ __device__ int large_cholesky(S& s, T* g) {
             }
           }
         }
-        if (t == 0) {  // the next diagonal block is final: factor it now
-          __syncthreads();
-          factor_diag(base);
-        }
       }
     }
     s.sync();
@@ -1063,13 +1197,31 @@ __device__ int large_cholesky(S& s, T* g) {
   // resident in shared memory until the next factorisation.
   if (int(blockIdx.x) < nblk) {
     const int b0 = int(blockIdx.x) * kLB;
-    stage_block(sm, g, npad, b0, b0, true);
+    // L (pitch kPitch) and its four diagonal sub-blocks' inverses.
+    for (int e = threadIdx.x; e < kLB * kLB; e += kGridBT) {
+      const int r = e >> 7, c = e & 127;
+      blk[r * kPitch + c] = c <= r ? double(g[size_t(b0 + r) * npad + b0 + c]) : 0.0;
+    }
     __syncthreads();
-    if (threadIdx.x < kLB) rdiag[threadIdx.x] = T(1) / sm[threadIdx.x * kPitch + threadIdx.x];
-    __syncthreads();
-    cta_sub_inverses<T>(sm, rdiag, sinv);
-    __syncthreads();
-    cta_inverse128<T>(sm, sinv, tmp32);
+    cta_sub_inverses(blk, sinv);
+    cta_inverse128(blk, sinv, tmp32);
+    if constexpr (sizeof(T) == 4) {  // to T in place, 16 rows at a time
+      for (int r0 = 0; r0 < kLB; r0 += 16) {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int e = threadIdx.x + q * kGridBT;
+          v[q] = T(blk[(r0 + (e >> 7)) * kPitch + (e & 127)]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int e = threadIdx.x + q * kGridBT;
+          sm[(r0 + (e >> 7)) * kPitch + (e & 127)] = v[q];
+        }
+        __syncthreads();
+      }
+    }
   }
   QTQP_TOC(kPhLgInv);
   return 0;
