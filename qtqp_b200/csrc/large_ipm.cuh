@@ -708,49 +708,134 @@ __device__ __noinline__ void cta_diag_update(double* sm, const T* g, size_t ld, 
   __syncthreads();
 }
 
+// C -= A B^T for one 8 x 8 tile and inner length 8, all in shared memory with
+// pitch kMmaPitch, the calling warp; valid: whether to store (uniform).
+__device__ __forceinline__ void warp_tile8(double* C, const double* A, const double* B, bool valid) {
+  const int lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+  double* out = C + gi * kMmaPitch + 2 * tg;
+  double acc[2];
+  load_pair(acc, out);
+#pragma unroll
+  for (int h = 0; h < 8; h += 4)
+    dmma_8x8x4(acc, -A[gi * kMmaPitch + h + tg], B[gi * kMmaPitch + h + tg]);
+  if (valid) store_pair(out, acc);
+}
+
+// Panel p (columns 8 p ..) of the 32 x 32 block D: lane l has row l.  Returns
+// the updated index of the first bad pivot (0: none).
+__device__ __forceinline__ int warp_chol_panel(double* D, double* rd, int p, int bad) {
+  const int lane = threadIdx.x & 31, c0 = 8 * p;
+  double* row = D + lane * kMmaPitch + c0;
+  double a[8];
+#pragma unroll
+  for (int c = 0; c < 8; c += 2) {
+    double v[2];
+    load_pair(v, row + c);
+    a[c] = lane >= c0 ? v[0] : 0.0;
+    a[c + 1] = lane >= c0 ? v[1] : 0.0;
+  }
+  double d = __shfl_sync(0xffffffffu, a[0], c0);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double r = rsqrt(d);
+    if (bad == 0 && !(d > 0.0)) bad = c0 + k + 1;
+    const double l = lane >= c0 + k ? a[k] * r : 0.0;
+    a[k] = l;
+    if (lane == c0 + k) rd[lane] = r;
+    // The next pivot's lane needs only its own l.
+    if (k < 7) d = __shfl_sync(0xffffffffu, fma(-l, l, a[(k + 1) & 7]), c0 + k + 1);
+#pragma unroll
+    for (int j = k + 1; j < 8; ++j) a[j] = fma(-l, __shfl_sync(0xffffffffu, l, c0 + j), a[j]);
+  }
+  if (lane >= c0) {  // zero above the diagonal
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double v[2] = {a[c], a[c + 1]};
+      store_pair(row + c, v);
+    }
+  }
+  return bad;
+}
+
+// Rows 8 p .. 8 p + 7 of X = inv(L) (pitch kSubPitch) of the 32 x 32 block L
+// (pitch kMmaPitch), the calling warp: X_pp by substitution, X_pc = -X_pp t_c
+// with t_c = sum_{c<=q<p} L_pq X_qc from warp_inv_sums.
+__device__ __forceinline__ void warp_inv_rows(const double* L, const double* rd, double* X, int p,
+                                              const double (&t)[3][2]) {
+  const int lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3, c0 = 8 * p;
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    if (c < p) store_pair(X + (c0 + gi) * kSubPitch + 8 * c + 2 * tg, t[c]);
+  double w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = i == (lane & 7) ? 1.0 : 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    w[k] *= rd[c0 + k];
+#pragma unroll
+    for (int i = k + 1; i < 8; ++i) w[i] = fma(-L[(c0 + i) * kMmaPitch + c0 + k], w[k], w[i]);
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) X[(c0 + i) * kSubPitch + c0 + lane] = w[i];
+  }
+  __syncwarp();
+  if (p == 0) return;
+  double av[2], bv[3][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    av[h] = -X[(c0 + gi) * kSubPitch + c0 + 4 * h + tg];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) bv[c][h] = X[(c0 + 4 * h + tg) * kSubPitch + 8 * c + gi];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    double x[2] = {0.0, 0.0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) dmma_8x8x4(x, av[h], bv[c][h]);
+    if (c < p) store_pair(X + (c0 + gi) * kSubPitch + 8 * c + 2 * tg, x);
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void warp_inv_sums(const double* L, const double* X, int p,
+                                              double (&t)[3][2]) {
+  const int lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) t[c][0] = t[c][1] = 0.0;
+#pragma unroll 1
+  for (int q = 0; q < p; ++q)
+#pragma unroll
+    for (int h = 0; h < 8; h += 4) {
+      const double a = L[(8 * p + gi) * kMmaPitch + 8 * q + h + tg];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)  // X is zero above its diagonal: q < c adds nothing
+        dmma_8x8x4(t[c], a, X[(8 * q + h + tg) * kSubPitch + 8 * c + gi]);
+    }
+}
+__device__ __forceinline__ void pair_barrier() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
 // Cholesky of the 128 x 128 block in shared memory (lower, pitch kMmaPitch) by
 // the CTA, and the inverses of its four 32 x 32 diagonal sub-blocks into inv
 // (pitch kSubPitch, zero above the diagonal).  Per sub-block b:
-//   * warp 0 factors it, lane l with row l in registers: per column one chain of
-//     pivot shuffle, reciprocal square root, scaling and the update of the next
-//     pivot, the other updates beside it;
-//   * warp 1 inverts it, lane c with column c of the inverse in registers, eight
-//     columns of L behind warp 0 (named barrier 1);
+//   * warp 0 factors it in panels of eight columns, lane l with row l's eight
+//     values in registers: per column one chain of pivot shuffle, reciprocal
+//     square root, scaling and the update of the next pivot, the other updates
+//     beside it; then the next panel's update (FP64 tensor cores);
+//   * warp 1 follows a panel behind (named barrier 1): the update of the columns
+//     after the next panel, and the panel's rows of the inverse;
 //   * warps 2 - 7 meanwhile apply the previous sub-block's products to the rest
 //     of the block, all but the sub-block in work;
 //   * then all warps multiply the rows below by the inverse's transpose and
 //     update the next sub-block (FP64 tensor cores).
 // rd: 32 doubles, sflag: one slot.  Returns 0 or the 1-based index of the first
 // non-positive pivot.
-// The chain over the columns bounds it: 43700 cycles in all.  Register tiles of
-// 4 x 4 over the whole block with a barrier per four columns took 75000 cycles,
-// and the inverses, a column per lane from shared memory, another 18000.
-template <int K0>
-__device__ __forceinline__ void chol32_columns(double (&a)[32], int lane, double* rd, int& bad) {
-#pragma unroll
-  for (int k = K0; k < K0 + 8; ++k) {
-    const double d = __shfl_sync(0xffffffffu, a[k], k);
-    if (bad == 0 && !(d > 0.0)) bad = k + 1;
-    const double r = rsqrt(d);
-    const double l = lane >= k ? a[k] * r : 0.0;
-    a[k] = l;
-    if (lane == k) rd[k] = r;
-#pragma unroll
-    for (int j = k + 1; j < 32; ++j) a[j] = fma(-l, __shfl_sync(0xffffffffu, l, j), a[j]);
-  }
-}
-template <int K0>
-__device__ __forceinline__ void inv32_columns(double (&w)[32], const double* L, const double* rd) {
-#pragma unroll
-  for (int k = K0; k < K0 + 8; ++k) {
-    const double x = w[k] * rd[k];
-    w[k] = x;
-#pragma unroll
-    for (int i = k + 1; i < 32; ++i) w[i] = fma(-L[i * kMmaPitch + k], x, w[i]);
-  }
-}
-__device__ __forceinline__ void pair_barrier() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
-
+// The chain over the columns bounds it: 42000 cycles in all with the code in the
+// instruction cache.  Register tiles of 4 x 4 over the whole block with a barrier
+// per four columns took 75000 cycles, and the inverses, a column per lane from
+// shared memory, another 18000.  A block is factored once per step by another SM
+// each time, so the code is short on purpose: with the 32 columns unrolled (43700
+// cycles when cached) a step of the factorisation took 65 us, so it takes 50 us.
 __device__ __noinline__ static int cta_chol128(double* sm, double* inv, double* rd, volatile int* sflag) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gi = lane >> 2, tg = lane & 3;
   if (threadIdx.x == 0) *sflag = 0;
@@ -759,43 +844,46 @@ __device__ __noinline__ static int cta_chol128(double* sm, double* inv, double* 
     const int o = 32 * b;
     double* D = sm + o * kMmaPitch + o;
     if (warp == 0) {
-      double a[32];
       int bad = 0;
+#pragma unroll 1
+      for (int p = 0; p < 4; ++p) {
+        bad = warp_chol_panel(D, rd, p, bad);
+        pair_barrier();
+        if (p == 3) break;
+        // Column tile p + 1.
+        const double* P = D + 8 * p;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) a[c] = D[lane * kMmaPitch + c];
-      auto put = [&](int c0) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (c >= c0 && c < c0 + 8 && c <= lane) D[lane * kMmaPitch + c] = a[c];
-      };
-      chol32_columns<0>(a, lane, rd, bad);
-      put(0);
-      pair_barrier();
-      chol32_columns<8>(a, lane, rd, bad);
-      put(8);
-      pair_barrier();
-      chol32_columns<16>(a, lane, rd, bad);
-      put(16);
-      pair_barrier();
-      chol32_columns<24>(a, lane, rd, bad);
-      put(24);
-      pair_barrier();
+        for (int x = 1; x < 4; ++x) {
+          const int i = min(p + x, 3), j = min(p + 1, 3);
+          warp_tile8(D + 8 * i * kMmaPitch + 8 * j, P + 8 * i * kMmaPitch, P + 8 * j * kMmaPitch,
+                     p + x < 4);
+        }
+        __syncwarp();
+      }
       if (bad != 0 && lane == 0) *sflag = o + bad;
     } else if (warp == 1) {
-      double w[32];
+      double* X = inv + b * 32 * kSubPitch;
+      const double zero[2] = {0.0, 0.0};
+      for (int e = lane; e < 32 * 16; e += 32) store_pair(X + (e >> 4) * kSubPitch + 2 * (e & 15), zero);
+      __syncwarp();
+      double sums[3][2];
+#pragma unroll 1
+      for (int p = 0; p < 4; ++p) {
+        warp_inv_sums(D, X, p, sums);
+        pair_barrier();
+        // The column tiles after p + 1.
+        const double* P = D + 8 * p;
+        if (p < 2) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) w[i] = i == lane ? 1.0 : 0.0;
-      pair_barrier();
-      inv32_columns<0>(w, D, rd);
-      pair_barrier();
-      inv32_columns<8>(w, D, rd);
-      pair_barrier();
-      inv32_columns<16>(w, D, rd);
-      pair_barrier();
-      inv32_columns<24>(w, D, rd);
-      double* X = inv + b * 32 * kSubPitch + lane;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) X[i * kSubPitch] = w[i];
+          for (int q = 0; q < 3; ++q) {
+            const int x = q == 0 ? 2 : 3, y = q == 2 ? 3 : 2;
+            const int i = min(p + x, 3), j = min(p + y, 3);
+            warp_tile8(D + 8 * i * kMmaPitch + 8 * j, P + 8 * i * kMmaPitch,
+                       P + 8 * j * kMmaPitch, p + x < 4);
+          }
+        }
+        warp_inv_rows(D, rd, X, p, sums);
+      }
     } else if (b > 0) {
       // The products of sub-block column b - 1 for the lower 16 x 16 units of
       // rows and columns >= o, without the sub-block at o itself (units 0 - 2).
@@ -839,7 +927,13 @@ __device__ __noinline__ static int cta_chol128(double* sm, double* inv, double* 
     if (bad != 0 || b == 3) return bad;
     // The rows below: L_ib = A_ib inv(L_bb)^T, eight rows at a time per warp
     // (in place: a warp reads its rows' fragments before it writes them).
-    const double* X = inv + b * 32 * kSubPitch;
+    const double* X = inv + b * 32 * kSubPitch + gi * kSubPitch + tg;
+    double xf[4][8];  // its fragments: zero right of the diagonal
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+      for (int k = 0; k < 2 * y + 2; ++k) xf[y][k] = X[8 * y * kSubPitch + 4 * k];
+#pragma unroll 1
     for (int r = o + 32 + 8 * warp; r < kLB; r += 64) {
       double* row = sm + (r + gi) * kMmaPitch + o;
       double av[8], acc[4][2];
@@ -848,30 +942,43 @@ __device__ __noinline__ static int cta_chol128(double* sm, double* inv, double* 
 #pragma unroll
       for (int y = 0; y < 4; ++y) acc[y][0] = acc[y][1] = 0.0;
 #pragma unroll
-      for (int k = 0; k < 8; ++k)  // inv(L_bb) is zero right of its diagonal
+      for (int k = 0; k < 8; ++k)
 #pragma unroll
         for (int y = 0; y < 4; ++y)
-          if (4 * k < 8 * y + 8)
-            dmma_8x8x4(acc[y], av[k], X[(8 * y + gi) * kSubPitch + 4 * k + tg]);
+          if (k < 2 * y + 2) dmma_8x8x4(acc[y], av[k], xf[y][k]);
       __syncwarp();
 #pragma unroll
       for (int y = 0; y < 4; ++y) store_pair(row + 8 * y + 2 * tg, acc[y]);
     }
     __syncthreads();
     // The next sub-block's update: its ten lower 8 x 8 tiles.
-    for (int t = warp; t < 10; t += 8) {
-      int p = 0;
-      while ((p + 1) * (p + 2) / 2 <= t) ++p;
-      const int r0 = o + 32 + 8 * p, c0 = o + 32 + 8 * (t - p * (p + 1) / 2);
-      double* out = sm + (r0 + gi) * kMmaPitch + c0 + 2 * tg;
-      double acc[2][2] = {{out[0], out[1]}, {0.0, 0.0}};
+    {
+      double f[2][2][8], acc[2][2][2];
+      double* out[2];
 #pragma unroll
-      for (int k = 0; k < 32; k += 4)
-        dmma_8x8x4(acc[(k >> 2) & 1], -sm[(r0 + gi) * kMmaPitch + o + k + tg],
-                   sm[(c0 + gi) * kMmaPitch + o + k + tg]);
-      acc[0][0] += acc[1][0];
-      acc[0][1] += acc[1][1];
-      store_pair(out, acc[0]);
+      for (int q = 0; q < 2; ++q) {  // tiles warp and, for two warps, warp + 8
+        const int t = min(warp + 8 * q, 9);
+        const int p = t < 1 ? 0 : t < 3 ? 1 : t < 6 ? 2 : 3;
+        const int r0 = o + 32 + 8 * p, c0 = o + 32 + 8 * (t - p * (p + 1) / 2);
+        out[q] = sm + (r0 + gi) * kMmaPitch + c0 + 2 * tg;
+        load_pair(acc[q][0], out[q]);
+        acc[q][1][0] = acc[q][1][1] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          f[q][0][k] = -sm[(r0 + gi) * kMmaPitch + o + 4 * k + tg];
+          f[q][1][k] = sm[(c0 + gi) * kMmaPitch + o + 4 * k + tg];
+        }
+        if (warp > 1) break;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dmma_8x8x4(acc[q][k & 1], f[q][0][k], f[q][1][k]);
+        acc[q][0][0] += acc[q][1][0];
+        acc[q][0][1] += acc[q][1][1];
+        store_pair(out[q], acc[q][0]);
+        if (warp > 1) break;
+      }
     }
     __syncthreads();
   }
