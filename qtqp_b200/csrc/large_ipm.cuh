@@ -564,12 +564,16 @@ __device__ void large_finish_gram(S& s, T* g) {
 // over the grid).
 //
 // Step k (panel width 128):
-//   (a) one CTA factors the diagonal block in shared memory (cta_chol128) and
-//       inverts its four 32 x 32 diagonal sub-blocks;
-//   (b) every warp takes panel rows and solves x L_kk^T = g_i with the four
-//       sub-block inverses (one lane per column, broadcasts by shuffle);
+//   (a) one CTA factors the diagonal block in shared memory and inverts its four
+//       32 x 32 diagonal sub-blocks (cta_chol128); from the second step on it
+//       does so during the trailing update of the step before, on the block it
+//       has updated itself (cta_diag_update);
+//   (b) every warp takes eight panel rows and solves x L_kk^T = g_i with the
+//       sub-block inverses (warp_panel_rows);
 //   (c) the lower 128 x 128 tiles right of the panel get g_ij -= L_ik L_jk^T
-//       with 8 x 8 outputs per thread and cp.async double-buffered slices.
+//       (trailing_tiles).
+// (a) and (b) run on the FP64 tensor cores whatever T is, so the FP32 factor's
+// diagonal blocks and panels are rounded once.
 // ---------------------------------------------------------------------------
 // 128 x 128 block of g at (r0, c0) into dst[r * kPitch + c], eight loads in
 // flight per thread; the strict upper part is zero when lower_only.
@@ -1115,6 +1119,162 @@ __device__ __noinline__ static void cta_inverse128(double* sm, const double* inv
   }
 }
 
+// Trailing update g_ij -= L_ik L_jk^T of the lower 128 x 128 tiles t0, t0 +
+// step, ... < tiles of the block at (base, base), with the panel at column k0.
+// FP64: on the FP64 tensor cores, warp w on the 64 x 32 block (w / 4, w % 4) of
+// the tile; slices of 32 panel columns staged row by row (pitch kSubPitch, 16-byte
+// copies), two buffers and one barrier per slice; the next tile's first slice
+// is in flight during this one's last.  The upper parts of the diagonal tiles
+// are written too; nothing reads them.
+// n = 4096: the trailing steps with their lookahead take 24.8 ms in 13
+// factorisations, 31.2 with transposed 8-byte copies, slices of 16 columns and
+// two barriers each.
+__device__ __noinline__ static void trailing_tiles(double* sm, double* g, int npad, int base,
+                                                   int k0, int t0, int tiles, int step) {
+  constexpr int KS = 32, SL = 2 * kLB * kSubPitch;
+  static_assert(2 * SL * sizeof(double) <= kArenaBytes, "trailing buffers exceed the arena");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gi = lane >> 2, tg = lane & 3;
+  const int wr = warp >> 2, wc = warp & 3;
+  if (t0 >= tiles) return;
+  auto issue = [&](int t, int s, int buf) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    double* pa = sm + buf * SL;
+    double* pb = pa + kLB * kSubPitch;
+    const double* ga = g + size_t(base + ti * kLB) * npad + k0 + s * KS;
+    const double* gb = g + size_t(base + tj * kLB) * npad + k0 + s * KS;
+#pragma unroll
+    for (int q = 0; q < kLB * KS / 2 / kGridBT; ++q) {
+      const int e = threadIdx.x + q * kGridBT, r = e >> 4, c = 2 * (e & 15);
+      cp_async16(pa + r * kSubPitch + c, ga + size_t(r) * npad + c);
+      cp_async16(pb + r * kSubPitch + c, gb + size_t(r) * npad + c);
+    }
+    cp_async_commit();
+  };
+  issue(t0, 0, 0);
+  int buf = 0;
+  for (int t = t0; t < tiles; t += step) {
+    double acc[8][4][2];
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll 1
+    for (int s = 0; s < kLB / KS; ++s) {
+      cp_async_wait<0>();
+      __syncthreads();
+      if (s + 1 < kLB / KS) {
+        issue(t, s + 1, buf ^ 1);
+      } else if (t + step < tiles) {
+        issue(t + step, 0, buf ^ 1);
+      }
+      const double* pa = sm + buf * SL + (wr * 64 + gi) * kSubPitch + tg;
+      const double* pb = sm + buf * SL + (kLB + wc * 32 + gi) * kSubPitch + tg;
+#pragma unroll
+      for (int k = 0; k < KS; k += 4) {
+        double a[8], b[4];
+#pragma unroll
+        for (int mi = 0; mi < 8; ++mi) a[mi] = pa[mi * 8 * kSubPitch + k];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) b[ni] = pb[ni * 8 * kSubPitch + k];
+#pragma unroll
+        for (int mi = 0; mi < 8; ++mi)
+#pragma unroll
+          for (int ni = 0; ni < 4; ++ni) dmma_8x8x4(acc[mi][ni], a[mi], b[ni]);
+      }
+      buf ^= 1;
+    }
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    double* out = g + size_t(base + ti * kLB + wr * 64 + gi) * npad + base + tj * kLB + wc * 32 +
+                  2 * tg;
+#pragma unroll
+    for (int m0 = 0; m0 < 8; m0 += 2) {
+      double v[2][4][2];
+#pragma unroll
+      for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+          load_pair(v[mi][ni], out + size_t(8 * (m0 + mi)) * npad + 8 * ni);
+#pragma unroll
+      for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          v[mi][ni][0] -= acc[m0 + mi][ni][0];
+          v[mi][ni][1] -= acc[m0 + mi][ni][1];
+          store_pair(out + size_t(8 * (m0 + mi)) * npad + 8 * ni, v[mi][ni]);
+        }
+    }
+  }
+}
+
+// FP32: 8 x 8 outputs per thread, slices of 16 panel columns, transposed.
+__device__ __noinline__ static void trailing_tiles(float* sm, float* g, int npad, int base, int k0,
+                                                   int t0, int tiles, int step) {
+  constexpr int KS = 16;
+  constexpr int SP = kLB + 1;      // slice pitch
+  constexpr int SL = 2 * KS * SP;  // elements per buffer
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  auto issue = [&](int kk0, int i0, int j0, int buf) {
+    float* pa = sm + buf * SL;
+    float* pb = pa + KS * SP;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = threadIdx.x + q * kGridBT, r = e >> 4, kk = e & 15;
+      cp_async4(pa + kk * SP + r, g + size_t(i0 + r) * npad + k0 + kk0 + kk);
+      cp_async4(pb + kk * SP + r, g + size_t(j0 + r) * npad + k0 + kk0 + kk);
+    }
+    cp_async_commit();
+  };
+  for (int t = t0; t < tiles; t += step) {
+    int ti, tj;
+    lower_tile(t, ti, tj);
+    const int i0 = base + ti * kLB, j0 = base + tj * kLB;
+    float acc[8][8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) acc[a][b] = 0.0f;
+    issue(0, i0, j0, 0);
+    int buf = 0;
+    for (int kk0 = 0; kk0 < kLB; kk0 += KS) {
+      if (kk0 + KS < kLB) {
+        issue(kk0 + KS, i0, j0, buf ^ 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncthreads();
+      const float* pa = sm + buf * SL;
+      const float* pb = pa + KS * SP;
+#pragma unroll 2
+      for (int kk = 0; kk < KS; ++kk) {
+        float av[8], bv[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+          av[a] = pa[kk * SP + ty + 16 * a];
+          bv[a] = pb[kk * SP + tx + 16 * a];
+        }
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+      }
+      __syncthreads();
+      buf ^= 1;
+    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int i = i0 + ty + 16 * a;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const int j = j0 + tx + 16 * b;
+        if (j <= i) g[size_t(i) * npad + j] -= acc[a][b];
+      }
+    }
+  }
+}
+
 template <typename T, class S>
 __device__ int large_cholesky(S& s, T* g) {
   const int npad = s.npad, nblk = npad / kLB;
@@ -1175,123 +1335,17 @@ __device__ int large_cholesky(S& s, T* g) {
     s.sync();
     QTQP_TOC(kPhLgPanel);
     QTQP_RETIC();
-    // (c) trailing update (FP64: on the FP64 tensor cores, DMMA m8n8k4, warp w
-    // on the 64 x 32 block (w / 4, w % 4) of the tile; FP32: 8 x 8 SIMT tiles).
+    // (c) trailing update.  Lookahead: the CTA that owns the next diagonal block
+    // (tile 0) updates it and factors it at once; the other tiles go round robin
+    // over the others.
     {
-      constexpr int KS = 16;
-      constexpr int SP = sizeof(T) == 8 ? kLB + 4 : kLB + 1;  // slice pitch
-      constexpr int SL = 2 * KS * SP;                 // elements per buffer
-      const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-      const int nt = rest / kLB, tiles = nt * (nt + 1) / 2;
-      const int base = k0 + kLB;
-      auto issue = [&](int kk0, int i0, int j0, int buf) {
-        T* pa = sm + buf * SL;
-        T* pb = pa + KS * SP;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int e = threadIdx.x + q * kGridBT, r = e >> 4, kk = e & 15;
-          if constexpr (sizeof(T) == 8) {
-            cp_async8(pa + kk * SP + r, g + size_t(i0 + r) * npad + k0 + kk0 + kk, true);
-            cp_async8(pb + kk * SP + r, g + size_t(j0 + r) * npad + k0 + kk0 + kk, true);
-          } else {
-            cp_async4(pa + kk * SP + r, g + size_t(i0 + r) * npad + k0 + kk0 + kk);
-            cp_async4(pb + kk * SP + r, g + size_t(j0 + r) * npad + k0 + kk0 + kk);
-          }
-        }
-        cp_async_commit();
-      };
-      // Lookahead: the CTA that owns the next diagonal block (tile 0) updates it
-      // and factors it at once; the other tiles go round robin over the others.
+      const int nt = rest / kLB, tiles = nt * (nt + 1) / 2, base = k0 + kLB;
       const int G = int(gridDim.x), owner = (k + 1) % G, me = int(blockIdx.x);
-      const int first_t = me == owner ? tiles : 1 + (me - owner - 1 + G) % G;
-      const int step_t = G - 1;
       if (me == owner) {
         cta_diag_update<T>(blk, g, npad, base, k0);
         factor_diag(base);
-      }
-      for (int t = first_t; t < tiles; t += step_t) {
-        int ti, tj;
-        lower_tile(t, ti, tj);
-        const int i0 = base + ti * kLB, j0 = base + tj * kLB;
-        T acc[8][8];
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-          for (int b = 0; b < 8; ++b) acc[a][b] = T(0);
-        issue(0, i0, j0, 0);
-        int buf = 0;
-        for (int kk0 = 0; kk0 < kLB; kk0 += KS) {
-          if (kk0 + KS < kLB) {
-            issue(kk0 + KS, i0, j0, buf ^ 1);
-            cp_async_wait<1>();
-          } else {
-            cp_async_wait<0>();
-          }
-          __syncthreads();
-          const T* pa = sm + buf * SL;
-          const T* pb = pa + KS * SP;
-          if constexpr (sizeof(T) == 8) {
-            // acc[mi][ni / 2][...]: the 8 x 4 DMMA accumulators of this warp.
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            const int gi = lane >> 2, tg = lane & 3, wr = warp >> 2, wc = warp & 3;
-#pragma unroll
-            for (int k4 = 0; k4 < KS; k4 += 4) {
-              const double* ra = reinterpret_cast<const double*>(pa) + (k4 + tg) * SP + wr * 64 + gi;
-              const double* rb = reinterpret_cast<const double*>(pb) + (k4 + tg) * SP + wc * 32 + gi;
-              double a[8], b[4];
-#pragma unroll
-              for (int mi = 0; mi < 8; ++mi) a[mi] = ra[mi * 8];
-#pragma unroll
-              for (int ni = 0; ni < 4; ++ni) b[ni] = rb[ni * 8];
-#pragma unroll
-              for (int mi = 0; mi < 8; ++mi)
-#pragma unroll
-                for (int ni = 0; ni < 4; ++ni)
-                  dmma_8x8x4(reinterpret_cast<double(&)[2]>(acc[mi][2 * ni]), a[mi], b[ni]);
-            }
-          } else {
-#pragma unroll 2
-            for (int kk = 0; kk < KS; ++kk) {
-              T av[8], bv[8];
-#pragma unroll
-              for (int a = 0; a < 8; ++a) {
-                av[a] = pa[kk * SP + ty + 16 * a];
-                bv[a] = pb[kk * SP + tx + 16 * a];
-              }
-#pragma unroll
-              for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 8; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
-            }
-          }
-          __syncthreads();
-          buf ^= 1;
-        }
-        if constexpr (sizeof(T) == 8) {
-          const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-          const int gi = lane >> 2, tg = lane & 3, wr = warp >> 2, wc = warp & 3;
-#pragma unroll
-          for (int mi = 0; mi < 8; ++mi) {
-            const int i = i0 + wr * 64 + mi * 8 + gi;
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int j = j0 + wc * 32 + ni * 8 + 2 * tg + e;
-                if (j <= i) g[size_t(i) * npad + j] -= acc[mi][2 * ni + e];
-              }
-          }
-        } else {
-#pragma unroll
-          for (int a = 0; a < 8; ++a) {
-            const int i = i0 + ty + 16 * a;
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-              const int j = j0 + tx + 16 * b;
-              if (j <= i) g[size_t(i) * npad + j] -= acc[a][b];
-            }
-          }
-        }
+      } else {
+        trailing_tiles(sm, g, npad, base, k0, 1 + (me - owner - 1 + G) % G, tiles, G - 1);
       }
     }
     s.sync();
