@@ -56,7 +56,6 @@ constexpr int kSparseGridNT = kSparseGridBlocks * kGridBT;
 constexpr int kSnMaxW = kSnMaxWidth;    // widest supernode (the symbolic stage's cap)
 constexpr int kSnLd = kSnMaxW + 1;      // leading dimension of the diagonal block in smem
 constexpr int kSnStageK = 32;           // descendant columns staged per pass
-constexpr int kSnCg = 8;                // target columns per thread in an update pass
 constexpr int kSnSlab = kSnSlabRows;    // rows of a top-level supernode per work item
 constexpr int kSnMaxSplit = 32;         // blocks sharing one slab's update list, at most
 constexpr int kSnUbuf = 4 * kSparseGridBlocks;  // partial update blocks (kSnSlab x kSnMaxW)
@@ -193,106 +192,195 @@ __device__ double sn_gram_entry(const S& s, int i, int j) {
   return acc;
 }
 
+// Shared memory of an update step, from the front of the arena (the resident
+// inverse of the dense part is dead during a factorisation): two staged
+// descendants (its rows in the slab and its rows in the columns, [k][row]),
+// the slab's sums, the slab's row keys, positions, and the list's entries.
+constexpr int kSnUpdPitch = 68;   // 4 (mod 16): a half-warp's fragment hits 16 banks
+constexpr int kSnUpdChunk = 256;  // list entries whose sizes are loaded at once
+struct SnUpdSmem {
+  double a[2][kSnMaxW * kSnUpdPitch];
+  double b[2][kSnMaxW * kSnUpdPitch];
+  double acc[kSnSlab * (kSnMaxW + 1)];
+  long long val[kSnUpdChunk], row[kSnUpdChunk];  // L_d[off], R_d[off]
+  int len[kSnUpdChunk], ld[kSnUpdChunk];         // rows from off on, all rows
+  int cnt_w[kSnUpdChunk];                        // rows in the columns << 8 | width
+  int key[kSnSlab];
+  int rpos[2][kSnSlab], cpos[2][kSnMaxW];
+  int ab[3][2];
+};
+static_assert(sizeof(SnUpdSmem) <= kArenaBytes, "update step's shared memory");
+static_assert(kSnMaxW <= 64 && kSnSlab == 64, "one descendant per staged pair of tiles");
+
 // Updates of rows [r0, r1) (at most kSnSlab of them) of supernode sn's block
-// from all its descendants (the calling block): L_s[r, j] -= the sum, over
-// the descendants d holding both row R_s[r] and column f + j, of
-// L_d[row, :] . L_d[col, :].  Each thread owns up to two (target row, kSnCg
-// target columns) items and keeps their sums in registers while the block
-// walks the update list in order: per descendant, the rows of R_d inside the
-// slab (a range found by two binary searches, the same in every thread), then
-// each item's row and columns in it.  No two threads write the same entry,
-// every sum runs in a fixed order, and no barrier separates the descendants.
+// from its descendants (the calling block): L_s[r, j] -= the sum, over the
+// descendants d holding both row R_s[r] and column f + j, of L_d[row, :] .
+// L_d[col, :].  Per descendant: its rows inside the slab (a range of R_d's
+// sorted keys, found by counting; the keys were loaded during the descendant
+// before), their positions in the slab, and its two row sets copied to shared
+// memory by cp.async while the descendant before is multiplied on the FP64 tensor
+// cores and added to the slab's sums.  One writer per sum and entry and a
+// barrier between the descendants: every sum runs in list order.
 //
 // [u0, u1) is the part of the update list to apply; out == nullptr subtracts
 // the sums from the block, else they go to out (kSnSlab x kSnMaxW, row r - r0
 // at out[(r - r0) * kSnMaxW + col]) for sn_add_partials.
+//
+// Bound by latency.  Each thread finding its row and columns of every descendant
+// by binary searches in global memory and forming its dot products from there
+// took 8 us per descendant: 3.5 ms of a 60 x 60 network flow's solve and 2.05 ms
+// of the n = 2000 sparse rows', now 2.0 and 1.5 ms.
 template <typename T>
-__device__ __noinline__ void sn_update_slab(const SnFactor& F, T* L, int sn, int r0, int r1, int u0, int u1,
-                               double* out) {
-  const int t = threadIdx.x;
+__device__ __noinline__ void sn_update_slab(const SnFactor& F, T* L, unsigned char* arena, int sn,
+                                            int r0, int r1, int u0, int u1, double* out) {
+  SnUpdSmem& sm = *reinterpret_cast<SnUpdSmem*>(arena);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, gi = lane >> 2, tg = lane & 3;
   const int f = F.first[sn], w = F.first[sn + 1] - f;
   const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]);
   const int32_t* R = F.rows + F.rowptr[sn];
   T* Ls = L + F.valptr[sn];
-  const int ngrp = (w + kSnCg - 1) / kSnCg;
   const int rows = r1 - r0;
+  if (u0 >= u1 && out == nullptr) return;
+  __syncthreads();  // the arena may still be in use
+  if (t < rows) sm.key[t] = R[r0 + t];
+  for (int e = t; e < kSnSlab * (kSnMaxW + 1); e += kGridBT) sm.acc[e] = 0.0;
   const int lo_key = R[r0], hi_key = R[r1 - 1];
-  constexpr int kItems = kSnSlab * ((kSnMaxW + kSnCg - 1) / kSnCg) / kGridBT;
-  static_assert(kItems * kGridBT >= kSnSlab * ((kSnMaxW + kSnCg - 1) / kSnCg), "items");
-  int key[kItems], ck0[kItems], ck1[kItems];
-  double acc[kItems][kSnCg];
-#pragma unroll
-  for (int it = 0; it < kItems; ++it) {
-    const int item = t + it * kGridBT;
-    key[it] = -1;
-    if (item < rows * ngrp) {
-      const int r = r0 + item % rows, cg = item / rows;
-      ck0[it] = f + cg * kSnCg;
-      ck1[it] = min(ck0[it] + kSnCg, f + w);
-      if (R[r] >= ck0[it]) key[it] = R[r];  // else entirely in the upper triangle
+  for (int ub = u0; ub < u1; ub += kSnUpdChunk) {
+    const int n = min(kSnUpdChunk, u1 - ub);
+    __syncthreads();
+    if (t < 6) sm.ab[t >> 1][t & 1] = 0;
+    if (t < n) {
+      const int d = F.upd_src[ub + t], off = F.upd_off[ub + t], cnt = F.upd_cnt[ub + t];
+      const int nrd = int(F.rowptr[d + 1] - F.rowptr[d]);
+      sm.val[t] = F.valptr[d] + off;
+      sm.row[t] = F.rowptr[d] + off;
+      sm.len[t] = nrd - off;
+      sm.ld[t] = nrd;
+      sm.cnt_w[t] = cnt << 8 | (F.first[d + 1] - F.first[d]);
     }
-#pragma unroll
-    for (int q = 0; q < kSnCg; ++q) acc[it][q] = 0.0;
-  }
-  for (int u = u0; u < u1; ++u) {
-    const int off = F.upd_off[u], cnt = F.upd_cnt[u];
-    const int d = F.upd_src[u];
-    const int nrd = int(F.rowptr[d + 1] - F.rowptr[d]);
-    const int32_t* Rd = F.rows + F.rowptr[d] + off;
-    const int a = sn_find(Rd, nrd - off, lo_key);
-    const int b = sn_find(Rd, nrd - off, hi_key + 1);
-    if (a >= b) continue;  // none of d's rows in this slab
-    const int wd = F.first[d + 1] - F.first[d];
-    const T* Ld = L + F.valptr[d] + off;
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-      if (key[it] < 0) continue;
-      const int i = a + sn_find(Rd + a, b - a, key[it]);
-      if (i >= b || Rd[i] != key[it]) continue;
-      int c = sn_find(Rd, cnt, ck0[it]);
-      const int c1 = sn_find(Rd, cnt, ck1[it]);
-      const T* Li = Ld + i;
-#pragma unroll
-      for (int q = 0; q < kSnCg; ++q) {
-        if (c < c1 && Rd[c] == ck0[it] + q) {
-          const T* Lc = Ld + c;
-          double sum = 0.0;
-          for (int k = 0; k < wd; ++k)
-            sum = fma(double(Li[size_t(k) * nrd]), double(Lc[size_t(k) * nrd]), sum);
-          acc[it][q] += sum;
-          ++c;
+    __syncthreads();
+    constexpr int kNone = 0x7fffffff;
+    int k0 = kNone, k1 = kNone;  // keys t and t + kGridBT of the entry to prepare next
+    auto load_keys = [&](int i) {
+      if (i >= n) return;
+      const int32_t* Rd = F.rows + sm.row[i];
+      const int len = sm.len[i];
+      k0 = t < len ? Rd[t] : kNone;
+      k1 = t + kGridBT < len ? Rd[t + kGridBT] : kNone;
+    };
+    // Finds entry i's rows in the slab, their positions, and starts its copies;
+    // returns their number.
+    auto prepare = [&](int i) {
+      int* ab = sm.ab[i % 3];
+      const int32_t* Rd = F.rows + sm.row[i];
+      const int len = sm.len[i], cnt = sm.cnt_w[i] >> 8, wd = sm.cnt_w[i] & 255;
+      auto count = [&](int key, int base) {  // keys below the slab, and up to its end
+        const unsigned lo = __ballot_sync(0xffffffffu, key < lo_key);
+        const unsigned hi = __ballot_sync(0xffffffffu, key <= hi_key);
+        if (lane == 0 && lo) atomicMax(&ab[0], base + 32 * warp + __popc(lo));
+        if (lane == 0 && hi) atomicMax(&ab[1], base + 32 * warp + __popc(hi));
+      };
+      count(k0, 0);
+      if (len > kGridBT) count(k1, kGridBT);
+      for (int base = 2 * kGridBT; base < len; base += kGridBT)
+        count(base + t < len ? Rd[base + t] : kNone, base);
+      __syncthreads();
+      const int a = ab[0], nrow = ab[1] - ab[0], s = i & 1;
+      if (t == 0) sm.ab[(i + 1) % 3][0] = sm.ab[(i + 1) % 3][1] = 0;
+      if (nrow > 0) {
+        auto place = [&](int key, int idx) {
+          if (idx >= a && idx < a + nrow) {
+            int lo = 0, hi = rows;
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              if (sm.key[mid] < key) {
+                lo = mid + 1;
+              } else {
+                hi = mid;
+              }
+            }
+            sm.rpos[s][idx - a] = lo;
+          }
+        };
+        place(k0, t);
+        if (len > kGridBT) place(k1, t + kGridBT);
+        for (int base = 2 * kGridBT; base < a + nrow; base += kGridBT)
+          if (base + t < len) place(Rd[base + t], base + t);
+        if (t < cnt) sm.cpos[s][t] = k0 - f;
+        const T* Ld = L + sm.val[i];
+        const size_t ld = sm.ld[i];
+        T* A = reinterpret_cast<T*>(sm.a[s]);
+        T* B = reinterpret_cast<T*>(sm.b[s]);
+        const int x = t & 63, wd4 = (wd + 3) & ~3;
+        for (int k = t >> 6; k < wd4; k += kGridBT / 64) {
+          if (x < nrow) cp_async_elem(A + k * kSnUpdPitch + x, Ld + (k < wd ? a + x + k * ld : 0), k < wd);
+          if (x < cnt) cp_async_elem(B + k * kSnUpdPitch + x, Ld + (k < wd ? x + k * ld : 0), k < wd);
         }
       }
-    }
-  }
+      cp_async_commit();
+      return nrow;
+    };
+    load_keys(0);
+    int cur = prepare(0);
+    load_keys(1);
+    for (int i = 0; i < n; ++i) {
+      int next = 0;
+      if (i + 1 < n) {
+        next = prepare(i + 1);
+        load_keys(i + 2);
+      } else {
+        cp_async_commit();
+      }
+      cp_async_wait<1>();
+      __syncthreads();
+      if (cur > 0) {
+        const int s = i & 1, cnt = sm.cnt_w[i] >> 8, wd = sm.cnt_w[i] & 255;
+        const int nrt = (cur + 7) >> 3, nct = (cnt + 7) >> 3;
+        const T* A = reinterpret_cast<const T*>(sm.a[s]) + tg * kSnUpdPitch + gi;
+        const T* B = reinterpret_cast<const T*>(sm.b[s]) + tg * kSnUpdPitch + gi;
+        for (int q = warp; q < nrt * nct; q += kGridBT / 32) {
+          const int ct = q / nrt, rt = q - ct * nrt;
+          double d[2] = {0.0, 0.0};
+#pragma unroll 4
+          for (int k = 0; k < wd; k += 4)
+            dmma_8x8x4(d, double(A[k * kSnUpdPitch + 8 * rt]), double(B[k * kSnUpdPitch + 8 * ct]));
+          const int r = 8 * rt + gi;
+          if (r < cur) {
+            double* row = sm.acc + sm.rpos[s][r] * (kSnMaxW + 1);
 #pragma unroll
-  for (int it = 0; it < kItems; ++it) {
-    if (key[it] < 0) continue;
-    const int item = t + it * kGridBT;
-    const int r = r0 + item % rows, cg = item / rows;
-#pragma unroll
-    for (int q = 0; q < kSnCg; ++q) {
-      if (ck0[it] + q < ck1[it] && ck0[it] + q <= key[it]) {
-        const int col = cg * kSnCg + q;
-        if (out != nullptr) {
-          out[(r - r0) * kSnMaxW + col] = acc[it][q];
-        } else {
-          T* dst = Ls + size_t(r) + size_t(col) * nr;
-          *dst = T(double(*dst) - acc[it][q]);
+            for (int e = 0; e < 2; ++e) {
+              const int c = 8 * ct + 2 * tg + e;
+              if (c < cnt) row[sm.cpos[s][c]] += d[e];
+            }
+          }
         }
       }
+      cur = next;
     }
   }
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int col = warp; col < w; col += kGridBT / 32)
+    for (int r = lane; r < rows; r += 32) {
+      if (f + col > sm.key[r]) continue;  // the block's upper triangle
+      const double sum = sm.acc[r * (kSnMaxW + 1) + col];
+      if (out != nullptr) {
+        out[r * kSnMaxW + col] = sum;
+      } else {
+        T* dst = Ls + size_t(r0 + r) + size_t(col) * nr;
+        *dst = T(double(*dst) - sum);
+      }
+    }
   __syncthreads();
 }
 
 // All rows [r0, r1) of supernode sn, slab by slab, from its whole update list.
 template <typename T>
-__device__ void sn_update_rows(const SnFactor& F, T* L, double* smem, int sn, int r0, int r1) {
-  (void)smem;
+__device__ void sn_update_rows(const SnFactor& F, T* L, unsigned char* arena, int sn, int r0,
+                               int r1) {
   for (int lo = r0; lo < r1; lo += kSnSlab)
-    sn_update_slab<T>(F, L, sn, lo, min(r1, lo + kSnSlab), F.upd_ptr[sn], F.upd_ptr[sn + 1],
-                      nullptr);
+    sn_update_slab<T>(F, L, arena, sn, lo, min(r1, lo + kSnSlab), F.upd_ptr[sn],
+                      F.upd_ptr[sn + 1], nullptr);
 }
 
 // Subtracts from rows [r0, r1) of supernode sn the partial sums that `parts`
@@ -431,9 +519,10 @@ __device__ void sn_panel_rows(const SnFactor& F, T* L, double* smem, int sn, int
 
 // Left-looking factorisation of supernode `sn` by the calling block alone.
 template <typename T>
-__device__ void sn_factor_one(const SnFactor& F, T* L, double* smem, int* info, int sn) {
+__device__ void sn_factor_one(const SnFactor& F, T* L, unsigned char* arena, double* smem,
+                              int* info, int sn) {
   const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]);
-  sn_update_rows<T>(F, L, smem, sn, 0, nr);
+  sn_update_rows<T>(F, L, arena, sn, 0, nr);
   sn_diag<T>(F, L, smem, info, sn);
   sn_panel_rows<T>(F, L, smem, sn, 0, nr, false);
 }
@@ -677,7 +766,7 @@ __device__ __noinline__ int sn_dense_factorize(S& s) {
     int sn, r0, r1;
     sn_slab_item(F, q0, q1, F.top_slab[q0] + slab, sn, r0, r1);
     const int ua = F.upd_ptr[sn], len = sn_upd_end(F, sn) - ua;
-    sn_update_slab<T>(F, L, sn, r0, r1, ua + len * part / split, ua + len * (part + 1) / split,
+    sn_update_slab<T>(F, L, s.arena, sn, r0, r1, ua + len * part / split, ua + len * (part + 1) / split,
                       split > 1 ? F.ubuf + size_t(it) * kSnSlab * kSnMaxW : nullptr);
   }
   for (int r = b; r < D.npad; r += G)
@@ -772,7 +861,7 @@ __device__ int sparse_factorize(S& s) {
   const int b = blockIdx.x;
   for (int q = F.cta_ptr[b]; q < F.cta_ptr[b + 1]; ++q)
     for (int sn = F.cta_range[2 * q]; sn <= F.cta_range[2 * q + 1]; ++sn)
-      sn_factor_one<T>(F, L, smem, s.linfo, sn);
+      sn_factor_one<T>(F, L, s.arena, smem, s.linfo, sn);
   s.sync();
   QTQP_TOC(kPhSnSub);
   QTQP_RETIC();
@@ -796,7 +885,7 @@ __device__ int sparse_factorize(S& s) {
       int sn, r0, r1;
       sn_slab_item(F, q0, q1, F.top_slab[q0] + slab, sn, r0, r1);
       const int ua = F.upd_ptr[sn], len = F.upd_ptr[sn + 1] - ua;
-      sn_update_slab<T>(F, L, sn, r0, r1, ua + len * part / split, ua + len * (part + 1) / split,
+      sn_update_slab<T>(F, L, s.arena, sn, r0, r1, ua + len * part / split, ua + len * (part + 1) / split,
                         split > 1 ? F.ubuf + size_t(it) * kSnSlab * kSnMaxW : nullptr);
     }
     s.sync();
