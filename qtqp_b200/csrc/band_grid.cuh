@@ -79,21 +79,35 @@ __host__ __device__ inline int band_grid_max_parts(int n, int bw) {
 // (column-major, S(i, j) = buf[j * pitch + i]): odd, so that both rows and
 // columns are read without bank conflicts.
 __host__ __device__ inline int sep_pitch(int bw) { return bw | 1; }
+// The same for the products of FP64 blocks on the tensor cores: 4 (mod 16), where
+// two blocks of it fit, so that a half-warp's fragment hits 16 banks (up to 4
+// lanes share one with the odd pitch).
+__host__ __device__ inline int sep_pitch64(int bw) {
+  const int p = (bw + 11) / 16 * 16 + 4;
+  return size_t(bw) * p <= 13500 ? p : sep_pitch(bw);
+}
+template <typename T>
+__host__ __device__ inline int sep_pitch_of(int bw) {
+  return sizeof(T) == 8 ? sep_pitch64(bw) : sep_pitch(bw);
+}
 
 // Dynamic shared memory of one block (sized for FP64): the largest of the
 // band window, solves and Gram rows (band_win_bytes), the spike window, the
-// products' staging, the separator reduction, and the solves' extra scratch.
+// products' staging, the separator reduction, and the solves' scratch (the
+// interiors' and the reduction's).
 __host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
   const size_t e = sizeof(double);
   size_t need = band_win_bytes(bw, kGridBT);
   const size_t spike = (size_t(bw) + 1) * bw * e + 256 * e;
   const size_t prod = size_t(bw) * bw * e + 32 * 4 * ((size_t(bw) + 3) / 4) * e;
-  const size_t chain = (2 * (size_t(bw) * sep_pitch(bw) + 4) + 3 * 128 + 256 + 2 * 16) * e;
+  const size_t chain = (2 * (size_t(bw) * sep_pitch64(bw) + 4) + 3 * 128 + 256 + 2 * 16) * e;
   const size_t solve = (band_solve_elems(bw) + 512) * e;
+  const size_t reduce = (3 * 128 + 2 * 8 * 128) * e;
   if (spike > need) need = spike;
   if (prod > need) need = prod;
   if (chain > need) need = chain;
   if (solve > need) need = solve;
+  if (reduce > need) need = reduce;
   return (need + 15) & ~size_t(15);
 }
 
@@ -287,10 +301,9 @@ __device__ __noinline__ void bandp_products(S& s, const BandParts& bp, int k) {
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ void stage_async(T* buf, int ldm, const T* src, int bw, bool trans) {
-  for (int e = threadIdx.x; e < bw * bw; e += kGridBT) {
-    const int r = e / bw, c = e - r * bw;
-    cp_async_elem(trans ? buf + r * ldm + c : buf + c * ldm + r, src + e, true);
-  }
+  for (int r = threadIdx.x >> 5; r < bw; r += kGridBT / 32)
+    for (int c = threadIdx.x & 31; c < bw; c += 32)
+      cp_async_elem(trans ? buf + r * ldm + c : buf + c * ldm + r, src + size_t(r) * bw + c, true);
 }
 __device__ __forceinline__ void stage_wait() {
   cp_async_commit();
@@ -299,10 +312,8 @@ __device__ __forceinline__ void stage_wait() {
 }
 template <typename T>
 __device__ void unstage(T* dst, const T* buf, int ldm, int bw) {
-  for (int e = threadIdx.x; e < bw * bw; e += kGridBT) {
-    const int r = e / bw, c = e - r * bw;
-    dst[e] = buf[c * ldm + r];
-  }
+  for (int r = threadIdx.x >> 5; r < bw; r += kGridBT / 32)
+    for (int c = threadIdx.x & 31; c < bw; c += 32) dst[size_t(r) * bw + c] = buf[c * ldm + r];
 }
 
 // The FP64 form of smem_gemm_nt on the FP64 tensor cores: each warp takes
@@ -512,21 +523,17 @@ __device__ __forceinline__ int sep_start(const BandParts& bp, int k) {
 // and a copy of Cr_j (its slot is rewritten at this level by j + 2^l).
 template <typename T, class S>
 __device__ __noinline__ int bandp_cr_eliminate(S& s, const BandParts& bp, int l, int j) {
-  const int bw = s.bw, ldm = sep_pitch(bw), N = bp.P - 1, h = 1 << l, k = j - 1;
+  const int bw = s.bw, ldm = sep_pitch_of<T>(bw), N = bp.P - 1, h = 1 << l, k = j - 1;
   CrSmem<T> sm(s.bwin, bw, ldm);
   QTQP_TIC();
   stage_async(sm.Mt, ldm, sep_block<T>(s, k, kSbD), bw, false);
   if (l == 0) stage_async(sm.Mb, ldm, sep_block<T>(s, k, kSbQ), bw, false);
   stage_wait();
-  for (int e = threadIdx.x; e < bw * bw; e += kGridBT) {
-    const int c = e / bw, i = e - c * bw;
-    if (l == 0 && i >= c) sm.Mt[c * ldm + i] -= sm.Mb[c * ldm + i];
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < bw * bw; e += kGridBT) {
-    const int c = e / bw, i = e - c * bw;
-    sm.Mb[c * ldm + i] = i == c ? T(1) : T(0);
-  }
+  for (int c = threadIdx.x >> 5; c < bw; c += kGridBT / 32)
+    for (int i = threadIdx.x & 31; i < bw; i += 32) {
+      if (l == 0 && i >= c) sm.Mt[c * ldm + i] -= sm.Mb[c * ldm + i];
+      sm.Mb[c * ldm + i] = i == c ? T(1) : T(0);
+    }
   __syncthreads();
   QTQP_TOC(kPhBpCrStage);
   QTQP_RETIC();
@@ -564,24 +571,30 @@ __device__ __noinline__ int bandp_cr_eliminate(S& s, const BandParts& bp, int l,
 // Reduction level l, surviving separator j' = 2^(l+1) (b + 1) (block b):
 // D_j' -= Cr Yr of the left neighbour jl = j' - 2^l (and Q at level 0),
 // its new left coupling -Cr Yl of jl, and D_j' -= Cl^T Yl of the right
-// neighbour jr = j' + 2^l.  D (lower, row-major) is updated in place.
+// neighbour jr = j' + 2^l.  D (lower, row-major) is updated in place.  diag,
+// couple: which of the two, D or the coupling, this block does.
 template <typename T, class S>
-__device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, int jp) {
-  const int bw = s.bw, ldm = sep_pitch(bw), N = bp.P - 1, h = 1 << l, k = jp - 1;
+__device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, int jp, bool diag,
+                                              bool couple) {
+  const int bw = s.bw, ldm = sep_pitch_of<T>(bw), N = bp.P - 1, h = 1 << l, k = jp - 1;
   CrSmem<T> sm(s.bwin, bw, ldm);
   QTQP_TIC();
   const int kl = jp - h - 1;
   T* D = sep_block<T>(s, k, kSbD);
   const T* Q = sep_block<T>(s, k, kSbQ);
+  couple = couple && jp - 2 * h >= 1;
+  if (!diag && !couple) return;
   stage_async(sm.Mt, ldm, sep_block<T>(s, kl, kSbR), bw, false);
-  stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXr), bw, true);
-  stage_wait();
-  smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, true, [&](int i, int jj, T acc) {
-    const size_t e = size_t(i) * bw + jj;
-    D[e] -= l == 0 ? acc + Q[e] : acc;
-  });
-  __syncthreads();
-  if (jp - 2 * h >= 1) {
+  if (diag) {
+    stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXr), bw, true);
+    stage_wait();
+    smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, true, [&](int i, int jj, T acc) {
+      const size_t e = size_t(i) * bw + jj;
+      D[e] -= l == 0 ? acc + Q[e] : acc;
+    });
+    __syncthreads();
+  }
+  if (couple) {
     stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXl), bw, true);
     stage_wait();
     T* Cn = sep_block<T>(s, k, kSbC);
@@ -589,7 +602,7 @@ __device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, i
                     [&](int i, int jj, T acc) { Cn[size_t(i) * bw + jj] = -acc; });
     __syncthreads();
   }
-  if (jp + h <= N) {
+  if (diag && jp + h <= N) {
     const int kr = jp + h - 1;
     stage_async(sm.Mt, ldm, l == 0 ? sep_block<T>(s, k, kSbE) : sep_block<T>(s, kr, kSbC), bw,
                 true);
@@ -652,34 +665,93 @@ __device__ int bandp_factorize(S& s) {
       if (bad != 0 && threadIdx.x == 0) atomicMax(const_cast<int*>(info), bad);
     }
     s.sync();
-    const int jp = 2 * h * (k + 1);
-    if (jp <= N && *info == 0) bandp_cr_gather<T>(s, bp, l, jp);
+    // One block per survivor for its D, and one more for its coupling while the
+    // grid has them (D takes two half products, the coupling one whole; bw = 99:
+    // the reduction of a factorisation 1.60 -> 1.53 ms).
+    const int ns = N / (2 * h);
+    const bool two = 2 * ns <= int(gridDim.x);
+    const int jp = 2 * h * ((two && k >= ns ? k - ns : k) + 1);
+    if (jp <= N && k < (two ? 2 * ns : ns) && *info == 0)
+      bandp_cr_gather<T>(s, bp, l, jp, !two || k < ns, !two || k >= ns);
     s.sync();
   }
   QTQP_TOC(kPhBpChain);
   return *info;
 }
 
-// Row / column matrix-vector products with a staged block, two halves of
-// the block over the inner index, combined through red (256 slots):
-// rows: y[i] = sum_c S(i, c) x[c]; cols: y[c] = sum_i S(i, c) x[i].
-// Thread i (< bw) receives y[i].
-template <typename T>
-__device__ __forceinline__ T smem_matvec(const T* S, int ldm, int bw, const T* x, bool cols,
-                                         T* red) {
-  const int i = threadIdx.x & 127, half = threadIdx.x >> 7;
-  T acc = T(0);
-  if (i < bw) {
-    if (cols) {
-      for (int c = half; c < bw; c += 2) acc = fma(S[i * ldm + c], x[c], acc);
+// Matrix-vector products with a row-major bw x bw block S in global memory and
+// x in shared memory (bw <= 128): rows y[i] = sum_c S(i, c) x[c], or (COLS)
+// y[c] = sum_i S(i, c) x[i].  Warp w takes the rows w, w + 8, ..., lane l the
+// columns l + 32 q, with the whole block in flight before the barrier that makes
+// x visible.  Thread i (< bw) receives y[i].  red: 8 x 128 slots.
+// Bound by the L2's latency and one SM's share of its bandwidth (a 99 x 99 block
+// is 78 KB).  Staged in shared memory first by 8-byte copies, the reduction of a
+// solve took 160 us (bw = 99, 127 separators), now 113 us.
+template <bool COLS, typename T>
+__device__ __forceinline__ T block_matvec(const T* S, int bw, const T* x, T* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kNW = kGridBT / 32;
+  T v[16][4], acc[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const int i = warp + kNW * r;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      v[r][q] = i < bw && lane + 32 * q < bw ? S[size_t(i) * bw + lane + 32 * q] : T(0);
+  }
+  __syncthreads();
+  T xq[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) xq[q] = !COLS && lane + 32 * q < bw ? x[lane + 32 * q] : T(0);
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    if constexpr (COLS) {
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int i = warp + kNW * (8 * b + r);
+        const T xi = i < bw ? x[i] : T(0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = fma(v[8 * b + r][q], xi, acc[q]);
+      }
     } else {
-      for (int c = half; c < bw; c += 2) acc = fma(S[c * ldm + i], x[c], acc);
+      // Row sums over the lanes: each step sends half of the rows' partials to
+      // the partner and keeps the other half.
+      T sum[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        sum[r] = fma(v[8 * b + r][3], xq[3],
+                     fma(v[8 * b + r][2], xq[2],
+                         fma(v[8 * b + r][1], xq[1], v[8 * b + r][0] * xq[0])));
+#pragma unroll
+      for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int r = 0; r < half; ++r) {
+          const T send = up ? sum[r] : sum[r + half];
+          const T keep = up ? sum[r + half] : sum[r];
+          sum[r] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+      }
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
+      const int r = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+      const int i = warp + kNW * (8 * b + r);
+      if ((lane & 3) == 0 && i < bw) red[i] = sum[0];
     }
   }
-  red[threadIdx.x] = acc;
+  if constexpr (COLS) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) red[warp * 128 + lane + 32 * q] = acc[q];
+  }
   __syncthreads();
-  const T y = threadIdx.x < 128 ? red[threadIdx.x] + red[threadIdx.x + 128] : T(0);
-  __syncthreads();
+  T y = T(0);
+  if (int(threadIdx.x) < bw) {
+    y = red[threadIdx.x];
+    if constexpr (COLS) {
+#pragma unroll
+      for (int u = 1; u < kNW; ++u) y += red[u * 128 + threadIdx.x];
+    }
+  }
   return y;
 }
 
@@ -688,8 +760,8 @@ __device__ __forceinline__ T smem_matvec(const T* S, int ldm, int bw, const T* x
 // entries.  Every thread of the grid calls it.
 // ---------------------------------------------------------------------------
 template <typename T, class S>
-__device__ void bandp_solve(S& s, T* v, T* w) {
-  const int bw = s.bw, ldm = sep_pitch(bw);
+__device__ __noinline__ void bandp_solve(S& s, T* v, T* w) {
+  const int bw = s.bw;
   const BandParts bp(s.n, bw, s.nparts);
   const int P = bp.P, N = P - 1, k = blockIdx.x, lt = threadIdx.x, lane = lt & 31,
             warp = lt >> 5;
@@ -716,11 +788,10 @@ __device__ void bandp_solve(S& s, T* v, T* w) {
   s.sync();
   QTQP_TOC(kPhBpFwd);
   QTQP_RETIC();
-  CrSmem<T> sm(s.bwin, bw, ldm);
-  T* t = sm.vec;
-  T* xa = sm.vec + 128;
-  T* xb = sm.vec + 256;
-  T* red = sm.red;
+  T* t = reinterpret_cast<T*>(s.bwin);
+  T* xa = t + 128;
+  T* xb = t + 256;
+  T* red = t + 384;  // 2 x 8 x 128
   // t_j at level 0 is v[S] - W_L^T y; later levels keep it in kSvT.
   auto load_t = [&](int l, int kk) {
     if (lt < bw)
@@ -733,9 +804,7 @@ __device__ void bandp_solve(S& s, T* v, T* w) {
   // separator eliminated at level l + 1 is a survivor of level l, so its
   // block forms z right after updating t (one grid barrier per level).
   auto form_z = [&](int kk) {  // t (shared) -> z_kk
-    stage_async(sm.Mt, ldm, sep_block<T>(s, kk, kSbI), bw, false);
-    stage_wait();
-    const T z = smem_matvec(sm.Mt, ldm, bw, t, false, red);
+    const T z = block_matvec<false>(sep_block<T>(s, kk, kSbI), bw, t, red);
     if (lt < bw) sep_vec<T>(s, kk, kSvZ)[lt] = z;
   };
   if (N >= 1 && 2 * k + 1 <= N) {
@@ -750,21 +819,16 @@ __device__ void bandp_solve(S& s, T* v, T* w) {
       load_t(l, jp - 1);
       const int kl = jp - h - 1, kr = jp + h - 1;
       if (lt < bw) xa[lt] = sep_vec<T>(s, kl, kSvZ)[lt];
-      stage_async(sm.Mt, ldm, sep_block<T>(s, kl, kSbR), bw, false);
-      stage_wait();
-      T acc = smem_matvec(sm.Mt, ldm, bw, xa, false, red);
-      if (jp + h <= N) {
-        if (lt < bw) xb[lt] = sep_vec<T>(s, kr, kSvZ)[lt];
-        stage_async(sm.Mt, ldm, l == 0 ? sep_block<T>(s, jp - 1, kSbE) : sep_block<T>(s, kr, kSbC),
-                    bw, false);
-        stage_wait();
-        acc += smem_matvec(sm.Mt, ldm, bw, xb, true, red);
-      }
+      if (lt < bw && jp + h <= N) xb[lt] = sep_vec<T>(s, kr, kSvZ)[lt];
+      T acc = block_matvec<false>(sep_block<T>(s, kl, kSbR), bw, xa, red);
+      if (jp + h <= N)
+        acc += block_matvec<true>(l == 0 ? sep_block<T>(s, jp - 1, kSbE) : sep_block<T>(s, kr, kSbC),
+                                  bw, xb, red + 1024);
       const T tv = lt < bw ? t[lt] - acc : T(0);
       if ((jp & (4 * h - 1)) == 2 * h) {  // eliminated at level l + 1
         __syncthreads();                    // every thread has read t
         if (lt < bw) t[lt] = tv;
-        form_z(jp - 1);                     // stage_wait orders t before the product
+        form_z(jp - 1);                     // begins with a barrier after its loads
       } else if (lt < bw) {
         sep_vec<T>(s, jp - 1, kSvT)[lt] = tv;
       }
@@ -779,15 +843,11 @@ __device__ void bandp_solve(S& s, T* v, T* w) {
       T r = lt < bw ? sep_vec<T>(s, kk, kSvZ)[lt] : T(0);
       if (j - h >= 1) {
         if (lt < bw) xa[lt] = v[sep_start(bp, j - h - 1) + lt];
-        stage_async(sm.Mt, ldm, sep_block<T>(s, kk, kSbXl), bw, false);
-        stage_wait();
-        r -= smem_matvec(sm.Mt, ldm, bw, xa, false, red);
+        r -= block_matvec<false>(sep_block<T>(s, kk, kSbXl), bw, xa, red);
       }
       if (j + h <= N) {
         if (lt < bw) xb[lt] = v[sep_start(bp, j + h - 1) + lt];
-        stage_async(sm.Mt, ldm, sep_block<T>(s, kk, kSbXr), bw, false);
-        stage_wait();
-        r -= smem_matvec(sm.Mt, ldm, bw, xb, false, red);
+        r -= block_matvec<false>(sep_block<T>(s, kk, kSbXr), bw, xb, red + 1024);
       }
       if (lt < bw) v[sep_start(bp, kk) + lt] = r;
     }

@@ -221,7 +221,7 @@ __device__ void large_products(S& s, const double* vx, const double* vy, const d
 template <typename T, class S>
 __device__ int bandp_factorize(S& s);
 template <typename T, class S>
-__device__ void bandp_solve(S& s, T* v, T* w);
+__device__ __noinline__ void bandp_solve(S& s, T* v, T* w);
 // Supernodal factorisation / solve of grid mode (sparse_grid.cuh).
 struct SnFactor;
 template <typename T, class S>
