@@ -212,6 +212,8 @@ enum MatFormat : int {
 // Large-format phases (large_ipm.cuh), called from the Ipm dispatch points.
 template <typename T, class S>
 __device__ int large_factorize(S& s);
+template <class S>
+__device__ __noinline__ void large_equilibrate(S& s);
 template <typename T, class S>
 __device__ __noinline__ void large_chol_solve(S& s, T* v, T* w);
 template <class S, class RowEpi, class ColEpi>
@@ -471,7 +473,9 @@ struct Ipm {
     }
     for (int k = tid; k < N; k += NT) de[k] = 1.0;
     sync();
-    if (equilibrate) {
+    if constexpr (FMT == kFmtLarge) {
+      if (equilibrate) large_equilibrate(*this);
+    } else if (equilibrate) {
       const double* Ap = A;
       const double* Pp = P;
       const int la = lda, lp = ldp, mm = m, nn = n;
