@@ -100,7 +100,7 @@ __host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
   size_t need = band_win_bytes(bw, kGridBT);
   const size_t spike = (size_t(bw) + 1) * bw * e + 256 * e;
   const size_t prod = size_t(bw) * bw * e + 32 * 4 * ((size_t(bw) + 3) / 4) * e;
-  const size_t chain = (2 * (size_t(bw) * sep_pitch64(bw) + 4) + 3 * 128 + 256 + 2 * 16) * e;
+  const size_t chain = (2 * (size_t(bw) * sep_pitch64(bw) + 4) + 2 * 16) * e;
   const size_t solve = (band_solve_elems(bw) + 512) * e;
   const size_t reduce = (3 * 128 + 2 * 8 * 128) * e;
   if (spike > need) need = spike;
@@ -294,7 +294,7 @@ __device__ __noinline__ void bandp_products(S& s, const BandParts& bp, int k) {
 
 // ---------------------------------------------------------------------------
 // Staged separator blocks.  A row-major bw x bw block is staged in shared
-// memory column-major with an odd pitch ldm: S(i, j) = buf[j * ldm + i]
+// memory column-major with pitch ldm (sep_pitch_of): S(i, j) = buf[j * ldm + i]
 // (trans: S(i, j) = src[j][i]), by asynchronous copies that are all in
 // flight at once (one commit group); stage_wait ends the group for the
 // whole block.
@@ -512,22 +512,17 @@ __device__ __noinline__ int smem_chol_stacked(T* Mt, T* Mb, int nb, int bw, int 
   return 0;
 }
 
-// Shared-memory layout of the reduction phases: two staged blocks, three
-// vectors of 128, a 256-slot reduction scratch and the Cholesky panel's
-// publish slots.
+// Shared-memory layout of the factorisation's reduction phases: two staged
+// blocks and the Cholesky panel's publish slots.
 template <typename T>
 struct CrSmem {
   T* Mt;
   T* Mb;
-  T* vec;
-  T* red;
   T* pub;
   __device__ CrSmem(double* base, int bw, int ldm) {
     Mt = reinterpret_cast<T*>(base);
     Mb = Mt + bw * ldm + 4;
-    vec = Mb + bw * ldm + 4;
-    red = vec + 3 * 128;
-    pub = red + 256;
+    pub = Mb + bw * ldm + 4;
   }
 };
 

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
   if (int(blockIdx.x) < L.nblk)
     stage_block(reinterpret_cast<double*>(arena),
                 reinterpret_cast<const double*>(gws + L.inv_off) + size_t(blockIdx.x) * kLB * kLB,
-                kLB, 0, 0, false);
+                kLB, 0, 0);
   __syncthreads();
   s.kkt_solve(rhs, out, false, true);
   // Every block has passed the solve's barriers, so it has read the old value.

@@ -673,16 +673,15 @@ __device__ void large_finish_gram(S& s, T* g) {
 // diagonal blocks and panels are rounded once.
 // ---------------------------------------------------------------------------
 // 128 x 128 block of g at (r0, c0) into dst[r * kPitch + c], eight loads in
-// flight per thread; the strict upper part is zero when lower_only.
+// flight per thread.
 template <typename T>
-__device__ __forceinline__ void stage_block(T* dst, const T* g, size_t ld, int r0, int c0,
-                                            bool lower_only) {
+__device__ __forceinline__ void stage_block(T* dst, const T* g, size_t ld, int r0, int c0) {
   for (int base = threadIdx.x; base < kLB * kLB; base += 8 * kGridBT) {
     T v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int e = base + q * kGridBT, r = e >> 7, c = e & 127;
-      v[q] = (!lower_only || c <= r) ? g[size_t(r0 + r) * ld + c0 + c] : T(0);
+      v[q] = g[size_t(r0 + r) * ld + c0 + c];
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -692,7 +691,7 @@ __device__ __forceinline__ void stage_block(T* dst, const T* g, size_t ld, int r
   }
 }
 
-// Two or four consecutive values of T from global memory as doubles.
+// Two consecutive values of T as doubles, and back.
 __device__ __forceinline__ void load_pair(double (&v)[2], const double* p) {
   const double2 t = *reinterpret_cast<const double2*>(p);
   v[0] = t.x;

@@ -55,14 +55,13 @@ constexpr int kSparseGridBlocks = 128;
 constexpr int kSparseGridNT = kSparseGridBlocks * kGridBT;
 constexpr int kSnMaxW = kSnMaxWidth;    // widest supernode (the symbolic stage's cap)
 constexpr int kSnLd = kSnMaxW + 1;      // leading dimension of the diagonal block in smem
-constexpr int kSnStageK = 32;           // descendant columns staged per pass
 constexpr int kSnSlab = kSnSlabRows;    // rows of a top-level supernode per work item
 constexpr int kSnMaxSplit = 32;         // blocks sharing one slab's update list, at most
 constexpr int kSnUbuf = 4 * kSparseGridBlocks;  // partial update blocks (kSnSlab x kSnMaxW)
-// Dynamic shared memory of a block: the diagonal block, its reciprocal
-// diagonal, the staged descendant rows, and the partial sums of the solves.
+// A block's scratch in shared memory: the diagonal block, its reciprocal
+// diagonal, one row of partial sums, and the partial sums of the solves.
 constexpr size_t kSparseSmemElems =
-    size_t(kSnMaxW) * kSnLd + kSnMaxW + size_t(kSnMaxW) * (kSnStageK + 1) + kGridBT + kSnMaxW;
+    size_t(kSnMaxW) * kSnLd + kSnMaxW + kSnMaxW + kGridBT + kSnMaxW;
 constexpr size_t kSparseSmem = kSparseSmemElems * sizeof(double);
 static_assert((size_t(kLB) * kPitch + kLB) * sizeof(double) + kSparseSmem <= kArenaBytes,
               "the supernodes' scratch would overwrite the dense part's resident inverse");
@@ -579,7 +578,7 @@ __device__ __forceinline__ void sn_fwd_gather(const SnFactor& F, const double* z
   const int w = F.first[sn + 1] - F.first[sn];
   const int W32 = w <= 32 ? 32 : 64;
   const int G = blockDim.x / W32;
-  double* part = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW * (kSnStageK + 1);
+  double* part = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW;
   sn_fwd_gather_block(F, z, sn, ua, ub, part);
   if (t < w) {
     double sum = 0.0;
@@ -606,7 +605,7 @@ __device__ void sn_fwd_diag(const SnFactor& F, const T* L, double* smem, const d
   const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]);
   const T* Ls = L + F.valptr[sn];
   double* D = smem;  // the diagonal block (factor, 1 / l_jj on the diagonal)
-  double* part = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW * (kSnStageK + 1);
+  double* part = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW;
   double* yb = part + kGridBT;
   for (int idx = t; idx < w * w; idx += blockDim.x) {
     const int c = idx / w, r = idx % w;
@@ -665,7 +664,7 @@ __device__ void sn_fwd_rows(const SnFactor& F, const T* L, double* smem, double*
   const int f = F.first[sn], w = F.first[sn + 1] - f;
   const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]);
   const T* Ls = L + F.valptr[sn];
-  double* yb = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW * (kSnStageK + 1) + kGridBT;
+  double* yb = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW + kGridBT;
   if (!from_smem) {
     for (int k = t; k < w; k += blockDim.x) yb[k] = double(v[f + k]);
     __syncthreads();
@@ -711,7 +710,7 @@ __device__ void sn_bwd_diag(const SnFactor& F, const T* L, double* smem, const d
   const int nr = int(F.rowptr[sn + 1] - F.rowptr[sn]);
   const T* Ls = L + F.valptr[sn];
   double* D = smem;
-  double* yb = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW * (kSnStageK + 1) + kGridBT;
+  double* yb = smem + kSnMaxW * kSnLd + kSnMaxW + kSnMaxW + kGridBT;
   for (int idx = t; idx < w * w; idx += blockDim.x) {
     const int c = idx / w, r = idx % w;
     if (r >= c) D[r * kSnLd + c] = double(Ls[size_t(r) + size_t(c) * nr]);
@@ -1000,7 +999,7 @@ __device__ void sparse_solve(S& s, T* v, T* w) {
   }
   QTQP_TOC(kPhSnBwdTop);
   QTQP_RETIC();
-  double* own = smem + kSnMaxW * kSnLd + kSnMaxW;  // one partial row (the staging area)
+  double* own = smem + kSnMaxW * kSnLd + kSnMaxW;  // one partial row
   for (int q = F.cta_ptr[b + 1] - 1; q >= F.cta_ptr[b]; --q)
     for (int sn = F.cta_range[2 * q + 1]; sn >= F.cta_range[2 * q]; --sn) {
       sn_bwd_rows<T>(F, L, v, sn, 0, int(F.rowptr[sn + 1] - F.rowptr[sn]), own);
