@@ -483,7 +483,7 @@ int qtqp_mlp_decode(const float* d_pred, const double* d_scale,
  * qtqp_iter_stats[max_iter] or NULL.  The workspace (>=
  * qtqp_dense_large_workspace_bytes(n, m), 1024-byte aligned) is private.
  * n <= 128 * qtqp_dense_large_blocks(), m * n < 2^31.  A grid barrier or
- * flag wait that waits too long ends the solve with status FAILED and error
+ * slot wait that waits too long ends the solve with status FAILED and error
  * QTQP_ERR_TIMEOUT. */
 size_t qtqp_dense_large_workspace_bytes(int32_t n, int32_t m);
 int32_t qtqp_dense_large_blocks(void);
@@ -552,7 +552,7 @@ int qtqp_dense_equilibrate(int32_t n, int32_t m, const double* d_a,
 /* ---- self-test of the bounded device waits ------------------------------ *
  * No reference counterpart.  Every spin-wait of the kernels gives up after a
  * poll limit and reports an error instead of hanging (the grid barrier and
- * the per-block flags of the whole-GPU solves: QTQP_ERR_TIMEOUT from the
+ * the value slots of the whole-GPU solves: QTQP_ERR_TIMEOUT from the
  * solve; the tensor-core pipelines' mbarrier waits).  This makes one run out on purpose with a short
  * limit (limit polls, at most 2^24) and writes the outcome to *d_status
  * (QTQP_OK or QTQP_ERR_TIMEOUT):
@@ -562,8 +562,8 @@ int qtqp_dense_equilibrate(int32_t n, int32_t m, const double* d_a,
  *           d_workspace: qtqp_wait_selftest_workspace_bytes() bytes;
  *   mode 1: one block waits on an mbarrier that nothing arrives on;
  *   mode 2: a cooperative grid of `blocks` blocks (2..64) where block b
- *           waits for block b - 1's flag, then sets its own, and block
- *           skip_block never sets its flag (-1: a control run); the same
+ *           waits for block b - 1's slot, then writes its own, and block
+ *           skip_block never writes its slot (-1: a control run); the same
  *           workspace as mode 0.
  * Nothing faults: the waits stop and the kernels return. */
 size_t qtqp_wait_selftest_workspace_bytes(void);

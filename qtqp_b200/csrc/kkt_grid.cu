@@ -1,5 +1,5 @@
 // See kkt_grid.cuh.  The factor, the inverses of its diagonal blocks and the
-// flags' generation live in the workspace between the calls; a solve's CTAs
+// slots' generation live in the workspace between the calls; a solve's CTAs
 // bring the inverse of their block back into shared memory first.
 #include "kkt_grid.cuh"
 

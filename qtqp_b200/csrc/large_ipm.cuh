@@ -9,13 +9,12 @@
 //             FP32 accumulation in TMEM).  FP64 factor: lower 128 x 128 tiles
 //             on the FP64 tensor cores (DMMA, mma.sync m8n8k4).
 //   Cholesky  right-looking with 128-wide panels: the diagonal block by one
-//             CTA in shared memory, the panel by row-wise substitution (one
-//             warp per row), the trailing update in 128 x 128 tiles (DMMA in
-//             FP64, 8 x 8 register tiles in FP32); then the inverse of every
-//             diagonal block.
+//             CTA in shared memory, the panel eight rows per warp (both DMMA),
+//             the trailing update in 128 x 128 tiles (DMMA in FP64, 8 x 8
+//             register tiles in FP32); then the inverse of every diagonal block.
 //   Solves    block forward / backward substitution with the inverted
-//             diagonal blocks; CTA j owns block row j and waits on per-block
-//             flags for the blocks it needs, one grid barrier per solve.
+//             diagonal blocks; CTA j owns block row j and polls the value
+//             slots of the blocks it needs, one grid barrier per solve.
 //
 // Padding: the factor is npad x npad (npad = n rounded up to 128) with an
 // identity on the padded diagonal; X is npad x mpad with zero padding.

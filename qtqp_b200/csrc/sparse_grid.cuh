@@ -39,7 +39,7 @@
 // in the factorisation, 30-40 us in each solve, next to no arithmetic).  From
 // the level that the symbolic stage chose (dense_level) on they are therefore
 // one dense matrix: one update step over all its row slabs, then the large
-// path's blocked Cholesky and its flag-synchronised solves (large_ipm.cuh),
+// path's blocked Cholesky and its slot-synchronised solves (large_ipm.cuh),
 // whose chain is one 128-column block long instead of one supernode.  Measured
 // per solve of the QP: 60 x 60 network flow (1240 of 14160 columns dense, 6
 // levels instead of 21) 45.6 -> 27.3 ms, n = 2000 random sparse rows (562
