@@ -473,8 +473,8 @@ int qtqp_mlp_decode(const float* d_pred, const double* d_scale,
  * KKT backend (src/qtqp/solvers_dense.py:25-145) for a single large QP: the
  * same device IPM as the batch, run by one cooperative launch of
  * qtqp_dense_large_blocks() blocks, one per SM of a B200 (grid barriers and
- * reductions; the triangular solves hand blocks over through per-block
- * flags), with a blocked Gram + Cholesky factor
+ * reductions; the triangular solves hand blocks over through value
+ * slots), with a blocked Gram + Cholesky factor
  * (Gram on tcgen05 tensor cores, TF32 hi + lo split, when opt->precision is
  * QTQP_PREC_MIXED; FP64 otherwise) and blocked triangular solves.
  * flags: QTQP_LARGE_HAS_P (P is given) | QTQP_LARGE_COLMAJOR (A and P are
