@@ -9,11 +9,12 @@
 namespace qtqp {
 
 // Threads per block: 512 while every QP gets an SM of its own, 256 (two
-// blocks per SM) for more QPs than SMs.  One set of 148 T = 50 MPC QPs takes
-// 545 ms with 512 threads and 906 ms with 256 (another set 162 ms, against
-// 497 ms with 128 threads, a thread per Gram column and 8-column solve
-// blocks): the sparse products and the window updates are latency-bound and
-// spread over the threads.
+// blocks per SM where their shared memory fits) for more QPs than SMs: the sparse
+// products and the window updates are latency-bound and spread over the threads.
+// MPC QPs of half-bandwidth 29 (n = 540): 148 take 7.7 ms with 512 threads, 149
+// 10.3 and 296 11.5 ms with 256 (with 128 threads and a thread per Gram column
+// 16.6, 17.4 and 20.6).  At half-bandwidth 99 (n = 720) two blocks do not fit: 148
+// take 16.8 ms, 149 38.5 and 296 44.1 (55, 62 and 69).
 constexpr int kBandThreadsWide = 512;
 constexpr int kBandThreads = 256;
 constexpr size_t kBandHeader = 256;

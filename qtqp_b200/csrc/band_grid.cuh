@@ -102,7 +102,7 @@ __host__ __device__ inline size_t band_grid_smem_bytes(int bw) {
   const size_t prod = size_t(bw) * bw * e + 32 * 4 * ((size_t(bw) + 3) / 4) * e;
   const size_t chain = (2 * (size_t(bw) * sep_pitch64(bw) + 4) + 2 * 16) * e;
   const size_t solve = (band_solve_elems(bw) + 512) * e;
-  const size_t reduce = (3 * 128 + 2 * 8 * 128) * e;
+  const size_t reduce = (3 * 128 + 2 * kGridBT) * e;
   if (spike > need) need = spike;
   if (prod > need) need = prod;
   if (chain > need) need = chain;
@@ -310,10 +310,11 @@ __device__ __forceinline__ void stage_wait() {
   cp_async_wait<0>();
   __syncthreads();
 }
+// The staged block's transpose, row-major.
 template <typename T>
-__device__ void unstage(T* dst, const T* buf, int ldm, int bw) {
-  for (int r = threadIdx.x >> 5; r < bw; r += kGridBT / 32)
-    for (int c = threadIdx.x & 31; c < bw; c += 32) dst[size_t(r) * bw + c] = buf[c * ldm + r];
+__device__ void unstage_trans(T* dst, const T* buf, int ldm, int bw) {
+  for (int c = threadIdx.x >> 5; c < bw; c += kGridBT / 32)
+    for (int r = threadIdx.x & 31; r < bw; r += 32) dst[size_t(c) * bw + r] = buf[c * ldm + r];
 }
 
 // The FP64 form of smem_gemm_nt on the FP64 tensor cores: each warp takes
@@ -534,7 +535,8 @@ __device__ __forceinline__ int sep_start(const BandParts& bp, int k) {
 // Reduction level l, eliminated separator j = 2^l (2 b + 1) (1-based;
 // block b): the Cholesky of the stacked [D_j; I] gives L_j^{-T}, then Di_j =
 // L_j^{-T} L_j^{-1}, Yl_j = Di_j Cl_j, Yr_j = Di_j Cr_j^T (tiled products),
-// and a copy of Cr_j (its slot is rewritten at this level by j + 2^l).
+// and a copy of Cr_j (its slot is rewritten at this level by j + 2^l).  The
+// last three are stored transposed, as the solves read them (block_colsum).
 template <typename T, class S>
 __device__ __noinline__ int bandp_cr_eliminate(S& s, const BandParts& bp, int l, int j) {
   const int bw = s.bw, ldm = sep_pitch_of<T>(bw), N = bp.P - 1, h = 1 << l, k = j - 1;
@@ -562,7 +564,7 @@ __device__ __noinline__ int bandp_cr_eliminate(S& s, const BandParts& bp, int l,
     sm.Mt[i * ldm + jj] = acc;
   });
   __syncthreads();
-  unstage(Ig, sm.Mt, ldm, bw);
+  unstage_trans(Ig, sm.Mt, ldm, bw);  // symmetric
   for (int side = 0; side < 2; ++side) {
     const bool has = side == 0 ? j - h >= 1 : j + h <= N;
     if (!has) continue;
@@ -572,10 +574,10 @@ __device__ __noinline__ int bandp_cr_eliminate(S& s, const BandParts& bp, int l,
     __syncthreads();
     stage_async(sm.Mb, ldm, src, bw, side == 0);
     stage_wait();
-    if (side == 1) unstage(sep_block<T>(s, k, kSbR), sm.Mb, ldm, bw);
+    if (side == 1) unstage_trans(sep_block<T>(s, k, kSbR), sm.Mb, ldm, bw);
     T* Y = sep_block<T>(s, k, side == 0 ? kSbXl : kSbXr);
     smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, false,
-                    [&](int i, int jj, T acc) { Y[size_t(i) * bw + jj] = acc; });
+                    [&](int i, int jj, T acc) { Y[size_t(jj) * bw + i] = acc; });
   }
   __syncthreads();
   QTQP_TOC(kPhBpCrGemm);
@@ -598,9 +600,9 @@ __device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, i
   const T* Q = sep_block<T>(s, k, kSbQ);
   couple = couple && jp - 2 * h >= 1;
   if (!diag && !couple) return;
-  stage_async(sm.Mt, ldm, sep_block<T>(s, kl, kSbR), bw, false);
+  stage_async(sm.Mt, ldm, sep_block<T>(s, kl, kSbR), bw, true);
   if (diag) {
-    stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXr), bw, true);
+    stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXr), bw, false);
     stage_wait();
     smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, true, [&](int i, int jj, T acc) {
       const size_t e = size_t(i) * bw + jj;
@@ -609,7 +611,7 @@ __device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, i
     __syncthreads();
   }
   if (couple) {
-    stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXl), bw, true);
+    stage_async(sm.Mb, ldm, sep_block<T>(s, kl, kSbXl), bw, false);
     stage_wait();
     T* Cn = sep_block<T>(s, k, kSbC);
     smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, false,
@@ -620,7 +622,7 @@ __device__ __noinline__ void bandp_cr_gather(S& s, const BandParts& bp, int l, i
     const int kr = jp + h - 1;
     stage_async(sm.Mt, ldm, l == 0 ? sep_block<T>(s, k, kSbE) : sep_block<T>(s, kr, kSbC), bw,
                 true);
-    stage_async(sm.Mb, ldm, sep_block<T>(s, kr, kSbXl), bw, true);
+    stage_async(sm.Mb, ldm, sep_block<T>(s, kr, kSbXl), bw, false);
     stage_wait();
     smem_gemm_nt<T>(sm.Mt, sm.Mb, ldm, bw, 0, bw, 0, bw, true,
                     [&](int i, int jj, T acc) { D[size_t(i) * bw + jj] -= acc; });
@@ -660,9 +662,6 @@ __device__ int bandp_factorize(S& s) {
       bandp_spike<T>(s, bp, k);
       bandp_products<T>(s, bp, k);
     }
-    // The spike has used the factor's diagonal blocks; the solves use their
-    // inverses.
-    if (bad == 0) s.template band_invert_diag<T, kGridBT>(lo, li);
   }
   s.sync();
   QTQP_TOC(kPhBpInterior);
@@ -693,80 +692,46 @@ __device__ int bandp_factorize(S& s) {
   return *info;
 }
 
-// Matrix-vector products with a row-major bw x bw block S in global memory and
-// x in shared memory (bw <= 128): rows y[i] = sum_c S(i, c) x[c], or (COLS)
-// y[c] = sum_i S(i, c) x[i].  Warp w takes the rows w, w + 8, ..., lane l the
-// columns l + 32 q, with the whole block in flight before the barrier that makes
-// x visible.  Thread i (< bw) receives y[i].  red: 8 x 128 slots.
+// y[c] = sum_i S(i, c) x[i] for a row-major bw x bw block S in global memory and x
+// in shared memory (128 entries, zero from bw on).  Threads c and c + 128 add up
+// the even and the odd i in ascending order, 32 rows of each in flight, the first
+// of them before the barrier that makes x visible.  Thread c (< bw) receives y[c].
+// red: kGridBT slots.
 // Bound by the L2's latency and one SM's share of its bandwidth (a 99 x 99 block
 // is 78 KB).  Staged in shared memory first by 8-byte copies, the reduction of a
-// solve took 160 us (bw = 99, 127 separators), now 113 us.
-template <bool COLS, typename T>
-__device__ __forceinline__ T block_matvec(const T* S, int bw, const T* x, T* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kNW = kGridBT / 32;
-  T v[16][4], acc[4] = {T(0), T(0), T(0), T(0)};
+// solve took 160 us (bw = 99, 127 separators).
+template <typename T>
+__device__ __noinline__ T block_colsum(const T* S, int bw, const T* x, T* red) {
+  const int c = threadIdx.x & 127, half = threadIdx.x >> 7;
+  constexpr int kC = 16;
+  const int chunks = (bw + 2 * kC - 1) / (2 * kC);
+  T v[kC], u[kC];
+  auto load = [&](T (&d)[kC], int k) {
+    const int i0 = 2 * kC * k + half;
+    const T* p = S + size_t(i0) * bw + c;
 #pragma unroll
-  for (int r = 0; r < 16; ++r) {
-    const int i = warp + kNW * r;
+    for (int q = 0; q < kC; ++q)
+      d[q] = c < bw && i0 + 2 * q < bw ? p[size_t(2 * q) * bw] : T(0);
+  };
+  T acc = T(0);
+  auto add = [&](const T (&d)[kC], int k) {
+    const T* xp = x + 2 * kC * k + half;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      v[r][q] = i < bw && lane + 32 * q < bw ? S[size_t(i) * bw + lane + 32 * q] : T(0);
-  }
+    for (int q = 0; q < kC; ++q) acc = fma(d[q], xp[2 * q], acc);
+  };
+  load(v, 0);
+  load(u, 1);
   __syncthreads();
-  T xq[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) xq[q] = !COLS && lane + 32 * q < bw ? x[lane + 32 * q] : T(0);
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    if constexpr (COLS) {
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const int i = warp + kNW * (8 * b + r);
-        const T xi = i < bw ? x[i] : T(0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q] = fma(v[8 * b + r][q], xi, acc[q]);
-      }
-    } else {
-      // Row sums over the lanes: each step sends half of the rows' partials to
-      // the partner and keeps the other half.
-      T sum[8];
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-        sum[r] = fma(v[8 * b + r][3], xq[3],
-                     fma(v[8 * b + r][2], xq[2],
-                         fma(v[8 * b + r][1], xq[1], v[8 * b + r][0] * xq[0])));
-#pragma unroll
-      for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-        const bool up = (lane & bit) != 0;
-#pragma unroll
-        for (int r = 0; r < half; ++r) {
-          const T send = up ? sum[r] : sum[r + half];
-          const T keep = up ? sum[r + half] : sum[r];
-          sum[r] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-        }
-      }
-      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
-      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 1);
-      const int r = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-      const int i = warp + kNW * (8 * b + r);
-      if ((lane & 3) == 0 && i < bw) red[i] = sum[0];
-    }
+#pragma unroll 1
+  for (int k = 0; k < chunks; k += 2) {
+    add(v, k);
+    load(v, k + 2);
+    if (k + 1 < chunks) add(u, k + 1);
+    load(u, k + 3);
   }
-  if constexpr (COLS) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) red[warp * 128 + lane + 32 * q] = acc[q];
-  }
+  red[threadIdx.x] = acc;
   __syncthreads();
-  T y = T(0);
-  if (int(threadIdx.x) < bw) {
-    y = red[threadIdx.x];
-    if constexpr (COLS) {
-#pragma unroll
-      for (int u = 1; u < kNW; ++u) y += red[u * 128 + threadIdx.x];
-    }
-  }
-  return y;
+  return threadIdx.x < 128 ? red[threadIdx.x] + red[threadIdx.x + 128] : T(0);
 }
 
 // ---------------------------------------------------------------------------
@@ -805,12 +770,13 @@ __device__ __noinline__ void bandp_solve(S& s, T* v, T* w) {
   T* t = reinterpret_cast<T*>(s.bwin);
   T* xa = t + 128;
   T* xb = t + 256;
-  T* red = t + 384;  // 2 x 8 x 128
+  T* red = t + 384;  // 2 x kGridBT
   // t_j at level 0 is v[S] - W_L^T y; later levels keep it in kSvT.
   auto load_t = [&](int l, int kk) {
-    if (lt < bw)
-      t[lt] = l == 0 ? v[sep_start(bp, kk) + lt] - sep_vec<T>(s, kk, kSvCL)[lt]
-                     : sep_vec<T>(s, kk, kSvT)[lt];
+    if (lt < 128)
+      t[lt] = lt >= bw ? T(0)
+              : l == 0 ? v[sep_start(bp, kk) + lt] - sep_vec<T>(s, kk, kSvCL)[lt]
+                       : sep_vec<T>(s, kk, kSvT)[lt];
   };
   int levels = 0;
   while ((1 << levels) <= N) ++levels;
@@ -818,7 +784,7 @@ __device__ __noinline__ void bandp_solve(S& s, T* v, T* w) {
   // separator eliminated at level l + 1 is a survivor of level l, so its
   // block forms z right after updating t (one grid barrier per level).
   auto form_z = [&](int kk) {  // t (shared) -> z_kk
-    const T z = block_matvec<false>(sep_block<T>(s, kk, kSbI), bw, t, red);
+    const T z = block_colsum(sep_block<T>(s, kk, kSbI), bw, t, red);
     if (lt < bw) sep_vec<T>(s, kk, kSvZ)[lt] = z;
   };
   if (N >= 1 && 2 * k + 1 <= N) {
@@ -832,12 +798,12 @@ __device__ __noinline__ void bandp_solve(S& s, T* v, T* w) {
     if (jp <= N) {  // t_j' -= Cr z (left neighbour) + Cl^T z (right neighbour)
       load_t(l, jp - 1);
       const int kl = jp - h - 1, kr = jp + h - 1;
-      if (lt < bw) xa[lt] = sep_vec<T>(s, kl, kSvZ)[lt];
-      if (lt < bw && jp + h <= N) xb[lt] = sep_vec<T>(s, kr, kSvZ)[lt];
-      T acc = block_matvec<false>(sep_block<T>(s, kl, kSbR), bw, xa, red);
+      if (lt < 128) xa[lt] = lt < bw ? sep_vec<T>(s, kl, kSvZ)[lt] : T(0);
+      if (lt < 128 && jp + h <= N) xb[lt] = lt < bw ? sep_vec<T>(s, kr, kSvZ)[lt] : T(0);
+      T acc = block_colsum(sep_block<T>(s, kl, kSbR), bw, xa, red);
       if (jp + h <= N)
-        acc += block_matvec<true>(l == 0 ? sep_block<T>(s, jp - 1, kSbE) : sep_block<T>(s, kr, kSbC),
-                                  bw, xb, red + 1024);
+        acc += block_colsum(l == 0 ? sep_block<T>(s, jp - 1, kSbE) : sep_block<T>(s, kr, kSbC), bw,
+                            xb, red + kGridBT);
       const T tv = lt < bw ? t[lt] - acc : T(0);
       if ((jp & (4 * h - 1)) == 2 * h) {  // eliminated at level l + 1
         __syncthreads();                    // every thread has read t
@@ -856,12 +822,12 @@ __device__ __noinline__ void bandp_solve(S& s, T* v, T* w) {
       const int kk = j - 1;
       T r = lt < bw ? sep_vec<T>(s, kk, kSvZ)[lt] : T(0);
       if (j - h >= 1) {
-        if (lt < bw) xa[lt] = v[sep_start(bp, j - h - 1) + lt];
-        r -= block_matvec<false>(sep_block<T>(s, kk, kSbXl), bw, xa, red);
+        if (lt < 128) xa[lt] = lt < bw ? v[sep_start(bp, j - h - 1) + lt] : T(0);
+        r -= block_colsum(sep_block<T>(s, kk, kSbXl), bw, xa, red);
       }
       if (j + h <= N) {
-        if (lt < bw) xb[lt] = v[sep_start(bp, j + h - 1) + lt];
-        r -= block_matvec<false>(sep_block<T>(s, kk, kSbXr), bw, xb, red + 1024);
+        if (lt < 128) xb[lt] = lt < bw ? v[sep_start(bp, j + h - 1) + lt] : T(0);
+        r -= block_colsum(sep_block<T>(s, kk, kSbXr), bw, xb, red + kGridBT);
       }
       if (lt < bw) v[sep_start(bp, kk) + lt] = r;
     }

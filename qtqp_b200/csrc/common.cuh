@@ -49,7 +49,10 @@ constexpr int kRedMax = 16;
 // reductions need a single __syncthreads each (a thread can only reach the
 // reduction after next once every thread has finished reading this one,
 // because the next reduction's barrier separates them).
-template <int NT, int NS, int NM>
+// ST < NT: only the first ST threads carry sums (the others' are zero or stale
+// and are not read); their warps' sums are added one after the other, so the
+// result depends on ST alone and not on the block's size.
+template <int NT, int NS, int NM, int ST = NT>
 __device__ __forceinline__ void block_reduce(double (&sums)[NS > 0 ? NS : 1],
                                              double (&maxs)[NM > 0 ? NM : 1],
                                              double* red, int& phase) {
@@ -83,14 +86,24 @@ __device__ __forceinline__ void block_reduce(double (&sums)[NS > 0 ? NS : 1],
     __syncthreads();
     // Lane l starts from warp l % NW's values; log2(NW) shuffles combine them.
     const double* mine = buf + (lane & (NW - 1)) * kRedMax;
+    if constexpr (ST < NT) {
 #pragma unroll
-    for (int k = 0; k < NS; ++k) sums[k] = mine[k];
+      for (int k = 0; k < NS; ++k) {
+        sums[k] = 0.0;
+        for (int w = 0; w < ST / 32; ++w) sums[k] += buf[w * kRedMax + k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NS; ++k) sums[k] = mine[k];
+    }
 #pragma unroll
     for (int k = 0; k < NM; ++k) keys[k] = __double_as_longlong(mine[NS + k]);
 #pragma unroll 1
     for (int off = NW / 2; off > 0; off >>= 1) {
+      if constexpr (ST == NT) {
 #pragma unroll
-      for (int k = 0; k < NS; ++k) sums[k] += __shfl_xor_sync(0xffffffffu, sums[k], off);
+        for (int k = 0; k < NS; ++k) sums[k] += __shfl_xor_sync(0xffffffffu, sums[k], off);
+      }
 #pragma unroll
       for (int k = 0; k < NM; ++k)
         keys[k] = max(keys[k], __shfl_xor_sync(0xffffffffu, keys[k], off));

@@ -17,6 +17,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace qtqp {
@@ -104,21 +106,24 @@ __host__ __device__ inline BandLayout plan_band_layout(int n, int m, int bw, int
 }
 
 // Shared-memory window of the banded factorisation / solves: bands up to
-// kBandWinMaxBw use it (a panel has one row per thread of a 256-thread block;
-// 190 window slots of the solves are live at once, of 256).
+// kBandWinMaxBw use it (a panel has one row per thread of a 256-thread block,
+// a step of the solves one per thread of its first 128).
 constexpr int kBandWinMaxBw = 126;
-// Columns per block of the blocked band solves: the largest power of two up
-// to 32 whose inverted lower-triangular diagonal block fits inside the band.
-__host__ __device__ inline int band_solve_block(int bw) {
-  int kb = 1;
-  while (kb < 32 && 2 * kb <= bw + 1) kb *= 2;
-  return kb;
+// The blocked band solves: kBandSolveBlk columns per step; the rows that a step
+// updates are spread over band_solve_owners(bw) threads (>= bw, a power of two).
+constexpr int kBandSolveBlk = 8;
+__host__ __device__ inline int band_solve_owners(int bw) {
+  return bw <= 32 ? 32 : bw <= 64 ? 64 : 128;
 }
-// Shared-memory elements of the blocked band solves: 256 window slots, a ring
-// of staged blocks of factor columns and the block's values.
-constexpr int kBandSolveStages = 4;
+// Their shared-memory elements: a ring of staged steps (the rows' factor entries,
+// pitch kBandSolveBlk + 1, and the 8 x 8 diagonal block), a step's right-hand
+// side and results, each twice, and the known values behind the last column.
+constexpr int kBandSolveStages = 8;
+__host__ __device__ inline size_t band_solve_stage(int bw) {
+  return size_t(kBandSolveBlk + 1) * band_solve_owners(bw) + kBandSolveBlk * kBandSolveBlk;
+}
 __host__ __device__ inline size_t band_solve_elems(int bw) {
-  return 256 + kBandSolveStages * size_t(band_solve_block(bw)) * (size_t(bw) + 1) + 32;
+  return kBandSolveStages * band_solve_stage(bw) + 4 * kBandSolveBlk + 128;
 }
 // The Gram product of the banded format: a warp forms kGramCols columns from
 // four dense rows of their entries in shared memory.  The pitch is 4 (mod 16)
@@ -139,16 +144,13 @@ __host__ __device__ inline size_t band_panel_bytes(int bw) {
          nt16 * (nt16 + 1) / 2 * sizeof(uint16_t);
 }
 // The shared memory a band needs in a block of nt threads: the Cholesky, the
-// solves, the Gram rows of every warp, one diagonal block to invert.
+// solves, the Gram rows of every warp.
 __host__ __device__ inline size_t band_win_bytes(int bw, int nt) {
   size_t e = band_panel_bytes(bw);
-  const size_t kb = band_solve_block(bw);
   const size_t cols = size_t(nt / 32) * gram_warp_elems(bw) * sizeof(double);
   const size_t solve = band_solve_elems(bw) * sizeof(double);
-  const size_t inv = kb * (kb + 1) * sizeof(double);
   if (cols > e) e = cols;
   if (solve > e) e = solve;
-  if (inv > e) e = inv;
   return (e + 15) & ~size_t(15);
 }
 
@@ -328,7 +330,19 @@ struct Ipm {
     if constexpr (NT > 1024) {
       grid_reduce<kGridBT, NS, NM>(sums, maxs, red, gctl, phase);
     } else {
-      block_reduce<NT, NS, NM>(sums, maxs, red, phase);
+      block_reduce<NT, NS, NM, kSumT>(sums, maxs, red, phase);
+    }
+  }
+  // The threads that add up the terms of a sum over a vector: all, but in a
+  // banded block the first 128, whatever its size (one term order, and so one
+  // result, for every block size: the iterates of an infeasible QP diverge along
+  // a ray, which amplifies a change of rounding by 1e6 and more).
+  static constexpr int kSumT = FMT == kFmtBand && NT <= 1024 ? 128 : NT;
+  __device__ __forceinline__ int sum_own(int lo) const {  // first index >= lo of this thread
+    if constexpr (kSumT == NT) {
+      return own(lo);
+    } else {
+      return tid < kSumT ? lo + ((tid - lo) & (kSumT - 1)) : 0x7fffffff - kSumT;
     }
   }
 
@@ -1618,18 +1632,25 @@ struct Ipm {
     double* pkr = vec(kRS);
     double sm[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // kr.q, kr.Pkq, kq.Pkr, kr.Pkr, Px.kr
     double dummy[1] = {0.0};
-    for (int k = tid; k < N; k += NT) sm[0] = fma(kr[k], q[k], sm[0]);
+    for (int k = sum_own(0); k < N; k += kSumT) sm[0] = fma(kr[k], q[k], sm[0]);
     if (has_p) {
-      auto epi = [&](int k, double poff) {
-        const double t = fma(pi[k], kr[k], poff);
-        pkr[k] = t;
+      auto add = [&](int k, double t) {
         sm[1] = fma(kr[k], pkq[k], sm[1]);
         sm[2] = fma(kq[k], t, sm[2]);
         sm[3] = fma(kr[k], t, sm[3]);
         sm[4] = fma(px[k], kr[k], sm[4]);
       };
+      auto epi = [&](int k, double poff) {
+        const double t = fma(pi[k], kr[k], poff);
+        pkr[k] = t;
+        if constexpr (kSumT == NT) add(k, t);
+      };
       if constexpr (kSparseA) {
         for (int k = tid; k < n; k += NT) epi(k, band_poff_row(kr, k));
+        if constexpr (kSumT != NT) {
+          sync();
+          for (int k = sum_own(0); k < n; k += kSumT) add(k, pkr[k]);
+        }
       } else if (fused_ok()) {
         dense_products(nullptr, nullptr, nullptr, kr, nullptr);
         sync();
@@ -1735,12 +1756,19 @@ struct Ipm {
     const bool hp = has_p;
     const double* b0p = b0;
     const double* c0p = c0;
+    double* const xy_o = vec(kRES);
+    double* const px_o = vec(kTMP);
     auto epi_x = [&](int k, double aty_raw, double poff) {
       const double aty = aty_raw / de[k];
       const double px = hp ? fma(pi[k], xy[k], poff) / de[k] : 0.0;
       const double xo = de[k] * xy[k];
-      sm[0] = fma(c0p[k], xo, sm[0]);
-      sm[2] = fma(xo, px, sm[2]);
+      if constexpr (kSumT == NT) {
+        sm[0] = fma(c0p[k], xo, sm[0]);
+        sm[2] = fma(xo, px, sm[2]);
+      } else {  // summed below (the residual and the solve's scratch are free here)
+        xy_o[k] = xo;
+        px_o[k] = px;
+      }
       mx[1] = nanmax(mx[1], fabs((px + aty) * inv_tau + c0p[k]));
       mx[2] = nanmax(mx[2], fabs(aty));
       mx[3] = nanmax(mx[3], fabs(px));
@@ -1752,7 +1780,11 @@ struct Ipm {
       const double yo = de[kk] * xy[kk];
       const double so = s[kk] / de[kk];
       const double bo = b0p[k];
-      sm[1] = fma(bo, yo, sm[1]);
+      if constexpr (kSumT == NT) {
+        sm[1] = fma(bo, yo, sm[1]);
+      } else {
+        xy_o[kk] = yo;
+      }
       mx[0] = nanmax(mx[0], fabs((ax + so) * inv_tau - bo));
       mx[4] = nanmax(mx[4], fabs(ax + so));
       mx[5] = nanmax(mx[5], fabs(ax));
@@ -1762,6 +1794,14 @@ struct Ipm {
     if constexpr (kSparseA) {
       for (int k = tid; k < n; k += NT) epi_x(k, band_at_col(xy, k), band_poff_row(xy, k));
       for (int k = tid; k < m; k += NT) epi_y(k, band_a_row(xy, k));
+      if constexpr (kSumT != NT) {
+        sync();
+        for (int k = sum_own(0); k < n; k += kSumT) {
+          sm[0] = fma(c0p[k], xy_o[k], sm[0]);
+          sm[2] = fma(xy_o[k], px_o[k], sm[2]);
+        }
+        for (int k = sum_own(0); k < m; k += kSumT) sm[1] = fma(b0p[k], xy_o[nn + k], sm[1]);
+      }
     } else if (fused_ok()) {
       // P x, then A^T y and A x in one pass over A (the residual's vector is
       // free here).
@@ -1841,7 +1881,7 @@ struct Ipm {
       b[0] = -INFINITY;
       b[1] = -INFINITY;
       b[3] = -INFINITY;
-      for (int k = own(n); k < N; k += NT) {
+      for (int k = sum_own(n); k < N; k += kSumT) {
         const double yo = de[k] * xy[k], so = s[k] / de[k];
         a[0] = fma(yo, so, a[0]);
         if (k >= n + z) {
@@ -1859,7 +1899,7 @@ struct Ipm {
       const double mean_sy = a[1] / cnt, mean_soy = a[2] / cnt;
       double v[2] = {0, 0};
       double dummy[1] = {0};
-      for (int k = own(n + z); k < N; k += NT) {
+      for (int k = sum_own(n + z); k < N; k += kSumT) {
         const double yo = de[k] * xy[k], so = s[k] / de[k];
         const double sy = so * yo, soy = so / fmax(kEps, yo);
         v[0] += (sy - mean_sy) * (sy - mean_sy);
@@ -2153,7 +2193,7 @@ struct Ipm {
       {
         QTQP_TIC();
         double sm[2] = {0.0, 0.0};
-        for (int k = tid; k < N; k += NT) {
+        for (int k = sum_own(0); k < N; k += kSumT) {
           sm[0] = fma(xy[k], xy[k], sm[0]);
           if (k >= n) sm[1] = fma(xy[k], s[k], sm[1]);
         }
@@ -2207,22 +2247,29 @@ struct Ipm {
         double* px = vec(kXD);
         const double* pi = vec(kPI);
         double sm[5] = {0, 0, 0, 0, 0};
-        for (int k = tid; k < N; k += NT) {
+        for (int k = sum_own(0); k < N; k += kSumT) {
           sm[0] = fma(kq[k], q[k], sm[0]);
           sm[2] = fma(q[k], xy[k], sm[2]);
         }
         if (has_p) {
+          auto add = [&](int k, double a, double b) {
+            sm[1] = fma(kq[k], a, sm[1]);
+            sm[3] = fma(xy[k], b, sm[3]);
+            sm[4] = fma(b, kq[k], sm[4]);
+          };
           auto epi = [&](int k, double pq, double pxk) {
             const double a = fma(pi[k], kq[k], pq);
             const double b = fma(pi[k], xy[k], pxk);
             pkq[k] = a;
             px[k] = b;
-            sm[1] = fma(kq[k], a, sm[1]);
-            sm[3] = fma(xy[k], b, sm[3]);
-            sm[4] = fma(b, kq[k], sm[4]);
+            if constexpr (kSumT == NT) add(k, a, b);
           };
           if constexpr (kSparseA) {
             for (int k = tid; k < n; k += NT) epi(k, band_poff_row(kq, k), band_poff_row(xy, k));
+            if constexpr (kSumT != NT) {
+              sync();
+              for (int k = sum_own(0); k < n; k += kSumT) add(k, pkq[k], px[k]);
+            }
           } else if (fused_ok()) {
             dense_products(nullptr, nullptr, nullptr, kq, nullptr);
             sync();
@@ -2285,7 +2332,7 @@ struct Ipm {
       {
         double sm[3] = {0, 0, 0};
         const double dtp = tau_p - tau;
-        for (int k = tid; k < N; k += NT) {
+        for (int k = sum_own(0); k < N; k += kSumT) {
           const double va = xy[k] + alpha_p * (xyp[k] - xy[k]);
           if (k < n) {
             sm[0] = fma(va, va, sm[0]);
@@ -2405,7 +2452,7 @@ struct Ipm {
     double sm[2] = {0.0, 0.0};  // b_o . y_o, c_o . x_o
     double dummy[1] = {0.0};
     if (status == QTQP_STATUS_INFEASIBLE || status == QTQP_STATUS_UNBOUNDED) {
-      for (int k = tid; k < N; k += NT) {
+      for (int k = sum_own(0); k < N; k += kSumT) {
         if (k < n) {
           sm[1] = fma(c0[k], de[k] * xy[k], sm[1]);
         } else {
@@ -2575,9 +2622,8 @@ struct Ipm {
   // sum_{q0 <= q < q1} val[q] v[voff + idx[q]]: indices and values are
   // loaded 8 at a time, then the 8 gathers, so that several loads are in
   // flight per thread (these sparse dots are latency-bound).
-  template <typename V>
   __device__ __forceinline__ static double sparse_dot(const int* idx, const double* val,
-                                                      const V* v, int voff, int q0, int q1) {
+                                                      const double* v, int voff, int q0, int q1) {
     double t0 = 0.0, t1 = 0.0;
     int q = q0;
     for (; q + 8 <= q1; q += 8) {
@@ -2589,44 +2635,41 @@ struct Ipm {
         aa[e] = val[q + e];
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) xx[e] = double(v[voff + ii[e]]);
+      for (int e = 0; e < 8; ++e) xx[e] = v[voff + ii[e]];
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
         t0 = fma(aa[e], xx[e], t0);
         t1 = fma(aa[e + 1], xx[e + 1], t1);
       }
     }
-    for (; q < q1; ++q) t0 = fma(val[q], double(v[voff + idx[q]]), t0);
+    for (; q < q1; ++q) t0 = fma(val[q], v[voff + idx[q]], t0);
     return t0 + t1;
   }
-  // sum_{q0 <= q < q1} val[q] (scale[idx[q]] v[idx[q]]), loaded the same way.
-  __device__ __forceinline__ static double sparse_dot_scaled(const int* idx, const double* val,
-                                                             const double* v,
-                                                             const double* scale, int q0,
-                                                             int q1) {
-    double t0 = 0.0, t1 = 0.0;
+  // sum_{q0 <= q < q1} val[q] (scale[idx[q]] v[idx[q]]) (scale null: without it),
+  // loaded the same way and added up in the order of the entries.
+  template <typename V>
+  __device__ __forceinline__ static double sparse_dot_ordered(const int* idx, const double* val,
+                                                              const V* v, const double* scale,
+                                                              int q0, int q1) {
+    double t = 0.0;
     int q = q0;
     for (; q + 8 <= q1; q += 8) {
       int ii[8];
-      double aa[8], xx[8], ss[8];
+      double aa[8], xx[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         ii[e] = idx[q + e];
         aa[e] = val[q + e];
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        xx[e] = v[ii[e]];
-        ss[e] = scale[ii[e]];
-      }
+      for (int e = 0; e < 8; ++e)
+        xx[e] = scale != nullptr ? scale[ii[e]] * double(v[ii[e]]) : double(v[ii[e]]);
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        t0 = fma(aa[e], ss[e] * xx[e], t0);
-        t1 = fma(aa[e + 1], ss[e + 1] * xx[e + 1], t1);
-      }
+      for (int e = 0; e < 8; ++e) t = fma(aa[e], xx[e], t);
     }
-    for (; q < q1; ++q) t0 = fma(val[q], scale[idx[q]] * v[idx[q]], t0);
-    return t0 + t1;
+    for (; q < q1; ++q)
+      t = fma(val[q], scale != nullptr ? scale[idx[q]] * double(v[idx[q]]) : double(v[idx[q]]), t);
+    return t;
   }
   // (P_off v)_k for the owner of row k (P symmetric, so row k = column k).
   __device__ __forceinline__ double band_poff_row(const double* v, int k) const {
@@ -2642,42 +2685,52 @@ struct Ipm {
   }
 
   // The rows of A that meet each group of kGramCols columns, once per solve:
-  // grow[jp[8 g] ..) holds the rows of group g (gcnt[g] of them), each where
-  // it first meets the group.  A warp per group compacts the group's CSC
-  // entries that are their row's first in the group (the row's preceding
-  // entry, found by a binary search of its CSR columns, lies before it).
+  // grow[jp[8 g] ..) holds the rows of group g (gcnt[g] of them) in ascending
+  // order.  A warp per group marks the rows of the group's CSC entries in a bit
+  // map in shared memory (the rows between the first and the last, a window of
+  // them at a time) and lists the marked ones, so nothing depends on how the
+  // entries are ordered or whether some are stored twice.
   __device__ void band_gram_groups() {
     QTQP_BAND_LOCALS;
+    constexpr int kWarps = (NT > 1024 ? kGridBT : NT) / 32;
     const int lane = threadIdx.x & 31;
+    const int words = min(1024, int(bwin_bytes / (kWarps * sizeof(unsigned int))));
+    unsigned int* bits = reinterpret_cast<unsigned int*>(bwin) + (threadIdx.x >> 5) * words;
     const int ng = (n + kGramCols - 1) / kGramCols;
     for (int g = tid >> 5; g < ng; g += NT / 32) {
       const int j0 = g * kGramCols, q0 = jp[j0], q1 = jp[min(n, j0 + kGramCols)];
-      int cnt = 0;
-      for (int qb = q0; qb < q1; qb += 32) {
-        const int q = qb + lane;
-        bool first = false;
-        int r = 0;
-        if (q < q1) {
-          r = jx[q];
-          // Entries of row r before column j0; the entry at q is the first in
-          // the group when it stands right behind them.
-          int lo = ip[r], hi = ip[r + 1];
-          while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (ix[mid] < j0) {
-              lo = mid + 1;
-            } else {
-              hi = mid;
-            }
-          }
-          const int jc = ix[lo];  // the row's first column in the group
-          first = q >= jp[jc] && q < jp[jc + 1] && (q == jp[jc] || jx[q - 1] != r);
-        }
-        const unsigned int m = __ballot_sync(0xffffffffu, first);
-        if (first) grow[q0 + cnt + __popc(m & ((1u << lane) - 1))] = r;
-        cnt += __popc(m);
+      int lo = m, hi = -1;
+      for (int q = q0 + lane; q < q1; q += 32) {
+        lo = min(lo, jx[q]);
+        hi = max(hi, jx[q]);
       }
-      if (lane == 0) gcnt[g] = cnt;
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      hi = __reduce_max_sync(0xffffffffu, hi);
+      int at_row = q0;  // where the next row goes
+      for (int base = lo; base <= hi; base += 32 * words) {
+        const int nw = min(words, ((hi - base) >> 5) + 1);
+        for (int w = lane; w < nw; w += 32) bits[w] = 0;
+        __syncwarp();
+        for (int q = q0 + lane; q < q1; q += 32) {
+          const int r = jx[q] - base;
+          if (r >= 0 && (r >> 5) < nw) atomicOr(bits + (r >> 5), 1u << (r & 31));
+        }
+        __syncwarp();
+        for (int w0 = 0; w0 < nw; w0 += 32) {
+          unsigned int u = w0 + lane < nw ? bits[w0 + lane] : 0u;
+          const int own_rows = __popc(u);
+          int upto = own_rows;  // rows of the lanes up to this one
+          for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+          }
+          for (int p = at_row + upto - own_rows; u != 0; u &= u - 1, ++p)
+            grow[p] = base + 32 * (w0 + lane) + __ffs(u) - 1;
+          at_row += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        __syncwarp();
+      }
+      if (lane == 0) gcnt[g] = at_row - q0;
     }
     if (tid == 0) gcnt[ng] = 0;
   }
@@ -2713,6 +2766,8 @@ struct Ipm {
   // cost some 60 instructions; a group of 8 columns now shares one visit).
   // buf: the block's scratch, gram_warp_elems(bw) entries per warp.
   // dup: rows may store an entry twice; their values are added up.
+  // A tensor-core step adds its four products one after the other, and the rows
+  // come in ascending order: every entry of G is the plain sum over the rows.
   template <typename T, int NT8>
   __device__ __forceinline__ void band_gram_group(int g, T* buf, bool dup, double& dmax) const {
     QTQP_BAND_LOCALS;
@@ -2842,9 +2897,8 @@ struct Ipm {
 
   // Gram matrix in column band storage, then Cholesky.  With the shared-
   // memory window (bw <= kBandWinMaxBw) the blocked factorisation
-  // (band_chol_panel_range), whose diagonal blocks are then inverted for the
-  // solves; otherwise the global-memory variant below runs.  In grid mode the
-  // partitioned factorisation runs (band_grid.cuh).
+  // (band_chol_panel_range); otherwise the global-memory variant below runs.  In
+  // grid mode the partitioned factorisation runs (band_grid.cuh).
   template <typename T>
   __device__ int band_factorize() {
     if constexpr (FMT == kFmtSparse) {
@@ -2859,9 +2913,6 @@ struct Ipm {
       QTQP_RETIC();
       const int info = band_chol_panel_range<T, NT>(tid, 0, n, n, nullptr, 0);
       QTQP_TOC(kPhChol);
-      QTQP_RETIC();
-      if (info == 0) band_invert_diag<T, NT>(0, n);
-      QTQP_TOC(kPhInv);
       return info;
     }
   }
@@ -3079,56 +3130,6 @@ struct Ipm {
     return bad == 0 ? 0 : lo + bad;
   }
 
-  // In-place inverse of the diagonal blocks of the factor that the blocked
-  // solves use: band_solve_block(bw) columns each, from column lo on, the
-  // last one shorter.  The inverse of a lower-triangular block is lower
-  // triangular and its last row is at most bw below its first column, so it
-  // takes the block's own place in the band (whose diagonal is that of the
-  // inverse already).  A warp per block, lane c its column c, kept at (c, k)
-  // of the staged block's unused upper triangle: X_rc = -(sum_{c<=k<r} L_rk
-  // X_kc) / l_rr.  As many warps as the shared memory holds blocks.
-  template <typename T, int BT>
-  __device__ void band_invert_diag(int lo, int ne) {
-    const int bw = this->bw, ldl = bw + 1, KB = band_solve_block(bw), P = KB + 1;
-    if (KB == 1) return;
-    T* L = reinterpret_cast<T*>(Lb);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = min(BT / 32, int(bwin_bytes / (size_t(KB) * P * sizeof(T))));
-    const int nblk = (ne + KB - 1) / KB;
-    T* S = reinterpret_cast<T*>(bwin) + size_t(warp) * KB * P;
-    for (int blk = warp; blk < nblk && warp < nw; blk += nw) {
-      const int k0 = lo + blk * KB, pw = min(KB, lo + ne - k0);
-      T* Lk = L + size_t(k0) * ldl;
-#pragma unroll 8
-      for (int c = 0; c < pw; ++c)
-        if (c + lane < pw) S[(c + lane) * P + c] = Lk[size_t(c) * ldl + lane];
-      __syncwarp();
-      const T* U = S + lane * P;
-#pragma unroll 1
-      for (int r = 1; r < pw; ++r) {
-        const T* Sr = S + r * P;
-        T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
-        if (lane < r) {
-          int k = lane;
-          for (; k + 3 < r; k += 4) {
-            a0 = fma(Sr[k], U[k], a0);
-            a1 = fma(Sr[k + 1], U[k + 1], a1);
-            a2 = fma(Sr[k + 2], U[k + 2], a2);
-            a3 = fma(Sr[k + 3], U[k + 3], a3);
-          }
-          for (; k < r; ++k) a0 = fma(Sr[k], U[k], a0);
-          S[lane * P + r] = -((a0 + a1) + (a2 + a3)) * Sr[r];
-        }
-        __syncwarp();
-      }
-#pragma unroll 8
-      for (int c = 0; c < pw; ++c)
-        if (lane > 0 && c + lane < pw) Lk[size_t(c) * ldl + lane] = S[c * P + c + lane];
-      __syncwarp();
-    }
-    group_sync<BT>();
-  }
-
   // Global-memory variant (wide bands): Gram in column band storage, then
   // Cholesky with one barrier per column (the unscaled column k updates the
   // trailing band and column k-1 is finished in the same phase).
@@ -3223,176 +3224,266 @@ struct Ipm {
     }
   }
 
-  // Blocked band triangular solves, run by all BT threads of the group (lt:
-  // this thread's index), over the columns [lo, lo + ne) in the blocks whose
-  // diagonal blocks band_invert_diag inverted (X_b).  Forward, per block:
-  // z_b = X_b v_b into w, then the next bw rows of v take their updates (the
-  // rows [lo + ne, R) among them, written back at the end).  Backward, per
-  // block from the last: x_b = X_b^T (w_b - the block's columns below it
-  // times x) into v, the rows [hi, R) holding known values of x in v (the
-  // separator that follows a partition).  Both phases of a block are dot
-  // products shared by several lanes each (two barriers per block); the next
-  // three blocks' factor columns, contiguous in the band, are copied in
-  // (cp.async) meanwhile: 148 QPs' factors of 2.4 MB come from HBM.  The
-  // active vector entries live in 256 circular slots.
-  // (T = 50 MPC QP, half-bandwidth 99: blocks of 8 columns with one thread
-  // solving each diagonal block took about 0.5 ms per direction in a
-  // 128-thread block.)
-  template <typename T, int BT>
-  __device__ __forceinline__ void band_issue_block(T* dst, const T* src, int nel, int lt) {
-    constexpr int V = 16 / int(sizeof(T));
-    if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-      const int nv = nel / V;
-      for (int e = lt; e < nv; e += BT) cp_async16(dst + e * V, src + e * V);
-      if (lt < nel - nv * V) cp_async_elem(dst + nv * V + lt, src + nv * V + lt, true);
-    } else {
-      for (int e = lt; e < nel; e += BT) cp_async_elem(dst + e, src + e, true);
-    }
+  // Blocked band triangular solves over the columns [lo, lo + ne), called by all
+  // BT >= 256 threads of the group (lt: this thread's index).  Forward: z_k =
+  // (v_k - sum_c l_kc z_c) / l_kk into w, the rows [lo + ne, R) of v receiving
+  // their updates.  Backward: x_k = (w_k - sum_d l_{k+d,k} x_{k+d}) / l_kk for k
+  // in [lo, hi) into v, the rows [hi, R) holding known values of x in v (the
+  // separator that follows a partition).
+  //
+  // Plain substitution in steps of 8 columns, every term added by itself: the
+  // forward's in the order of the columns, the backward's step by step from the
+  // last column, the known values first, within a step in ascending order.  The first W =
+  // band_solve_owners(bw) threads run the steps, each with one of the rows that a
+  // step updates in a register; every one of them solves the step's 8 x 8 diagonal
+  // block for itself from eight right-hand-side values in shared memory, applies
+  // the result to its row, and publishes the row when it enters the next diagonal
+  // block.  The next W threads copy (cp.async) the factor's entries of the steps
+  // ahead into a ring of eight stages; one barrier over both lies between two
+  // steps, and the other threads wait at the end.
+  //
+  // Bound by the fetch of a step's instructions and its chain: 890 cycles per step
+  // forward and 1010 backward at half-bandwidth 99 with 148 blocks at work, 760 and
+  // 700 without the copies.  (Kept short on purpose: with the copies in the owners'
+  // threads 2800 and 1900; one thread solving each diagonal block, then a barrier
+  // and the rows, then another: about 1600.)
+  template <typename T>
+  __device__ __forceinline__ static void band_pair(const T* p, T& a, T& b) {
+    using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+    const V t = *reinterpret_cast<const V*>(p);
+    a = t.x;
+    b = t.y;
   }
-  // Lanes sharing one of `rows` dot products: a power of two up to 32.
-  template <int BT>
-  __device__ __forceinline__ static int band_lanes(int rows) {
-    int s = 1;
-    while (s < 32 && 2 * s * rows <= BT) s *= 2;
-    return s;
+  template <typename T>
+  __device__ __forceinline__ static void band_pair_put(T* p, T a, T b) {
+    using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+    V t;
+    t.x = a;
+    t.y = b;
+    *reinterpret_cast<V*>(p) = t;
+  }
+  __device__ __forceinline__ static void band_step_sync(int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
   }
 
   template <typename T, int BT>
   __device__ void band_fwd_blocked(T* v, T* w, int lo, int ne, int R, int lt) {
-    const int bw = this->bw, ldl = bw + 1, hi = lo + ne, KB = band_solve_block(bw);
+    constexpr int KB = kBandSolveBlk, NS = kBandSolveStages;
+    static_assert(BT >= 256 && (NS & (NS - 1)) == 0, "owners and copiers; ring");
+    const int bw = this->bw, ldl = bw + 1, hi = lo + ne, nb = (ne + KB - 1) / KB;
+    const int W = band_solve_owners(bw), SS = int(band_solve_stage(bw));
     const T* L = reinterpret_cast<const T*>(Lb);
-    T* win = reinterpret_cast<T*>(bwin);  // 256 slots: row r at r & 255
-    T* pan = win + 256;                   // the ring: factor columns of a block, KB ldl each
-    T* zz = pan + kBandSolveStages * KB * ldl;  // the block's values
-    const int S1 = band_lanes<BT>(KB), r1 = lt / S1, s1 = lt % S1;
-    const int S2 = band_lanes<BT>(bw), r2 = lt / S2, s2 = lt % S2;
-    int loaded = min(R, lo + bw + KB);
-    for (int r = lo + lt; r < loaded; r += BT) win[r & 255] = v[r];
-    auto issue = [&](int k, int st) {
-      if (k < hi)
-        band_issue_block<T, BT>(pan + st * KB * ldl, L + size_t(k) * ldl, min(KB, hi - k) * ldl,
-                                lt);
-      cp_async_commit();
-    };
-    for (int st = 0; st + 1 < kBandSolveStages; ++st) issue(lo + st * KB, st);
-    int buf = 0;
-    for (int k0 = lo; k0 < hi; k0 += KB, buf = (buf + 1) % kBandSolveStages) {
-      const int pw = min(KB, hi - k0);
-      // This block's columns have landed and every thread is done with the
-      // previous block, whose buffer the copies of the block three ahead fill.
-      cp_async_wait<kBandSolveStages - 2>();
-      group_sync<BT>();
-      issue(k0 + (kBandSolveStages - 1) * KB, (buf + kBandSolveStages - 1) % kBandSolveStages);
-      const int nload = min(R, k0 + 2 * KB + bw);  // rows the next block's window adds
-      const bool ld = loaded + lt < nload;
-      const T nv = ld ? v[loaded + lt] : T(0);
-      const T* pc = pan + buf * KB * ldl;  // column k0 + c: pc[c * ldl + d], d = row - column
-      {
-        T a0 = T(0), a1 = T(0);
-        if (r1 < pw) {
-          int c = s1;
-          for (; c + S1 <= r1; c += 2 * S1) {
-            a0 = fma(pc[c * ldl + r1 - c], win[(k0 + c) & 255], a0);
-            a1 = fma(pc[(c + S1) * ldl + r1 - c - S1], win[(k0 + c + S1) & 255], a1);
+    T* ring = reinterpret_cast<T*>(bwin);
+    T* rhs = ring + NS * SS;
+    T* done = rhs + 2 * KB;  // the last step's results, to w a step later
+    if (lt >= W && lt < 2 * W) {
+      // Step b: columns k0 = lo + 8 b ..; copier and owner ct have row k0 + 8 + d
+      // with d = (ct - 8 (b + 1)) mod W.  Rows from hi on are updated, not solved
+      // (columns from hi on are zero).
+      const int ct = lt - W;
+      auto issue = [&](int b) {
+        if (b < nb) {
+          T* st = ring + (b & (NS - 1)) * SS;
+          const int k0 = lo + b * KB, d = (ct - KB * (b + 1)) & (W - 1);
+          const T* src = L + size_t(k0) * ldl + KB + d;  // column k0 + c: src[c bw]
+          const int c0 = k0 + KB + d < R ? KB + d - bw : KB;
+          const int c1 = min(KB, hi - k0);
+#pragma unroll
+          for (int c = 0; c < KB; ++c) {
+            const bool ok = c >= c0 && c < c1;
+            cp_async_elem(st + c * W + ct, ok ? src + c * bw : L, ok);
           }
-          if (c <= r1) a0 = fma(pc[c * ldl + r1 - c], win[(k0 + c) & 255], a0);
+#pragma unroll 1
+          for (int e = ct; e < KB * KB; e += W) {
+            const int c = e >> 3, dd = e & 7;
+            const bool ok = c + dd < KB && dd <= bw && c < c1 && k0 + c + dd < R;
+            cp_async_elem(st + KB * W + e, ok ? L + size_t(k0 + c) * ldl + dd : L, ok);
+          }
         }
-        T z = a0 + a1;
-        for (int o = 1; o < S1; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-        if (s1 == 0 && r1 < pw) {
-          zz[r1] = z;
-          w[k0 + r1] = z;
+        cp_async_commit();
+      };
+#pragma unroll 1
+      for (int b = 0; b + 1 < NS; ++b) issue(b);
+#pragma unroll 1
+      for (int b = 0; b < nb; ++b) {
+        // Step b's entries have landed; after the barrier every owner is done with
+        // step b - 1, whose stage is filled again.
+        cp_async_wait<NS - 2>();
+        band_step_sync(2 * W);
+        issue(b + NS - 1);
+      }
+      cp_async_wait<0>();
+    } else if (lt < W) {
+      int row = lo + lt;
+      T t = row < R ? v[row] : T(0), tn = row + W < R ? v[row + W] : T(0);
+      if (lt < KB) {
+        rhs[lt] = t;
+        row += W;
+        t = tn;
+        tn = row + W < R ? v[row + W] : T(0);
+      }
+#pragma unroll 1
+      for (int b = 0; b < nb; ++b) {
+        band_step_sync(2 * W);
+        const int k0 = lo + b * KB, pw = hi - k0;
+        const T* st = ring + (b & (NS - 1)) * SS;
+        if (b > 0 && lt < KB) w[k0 - KB + lt] = done[((b - 1) & 1) * KB + lt];
+        T dg[KB][KB], z[KB], l[KB];
+        const T* rp = rhs + (b & 1) * KB;
+        const T* blk = st + KB * W;
+#pragma unroll
+        for (int c = 0; c < KB; c += 2) band_pair(rp + c, z[c], z[c + 1]);
+#pragma unroll
+        for (int c = 0; c < KB; ++c)
+#pragma unroll
+          for (int d = 0; d < KB - c; d += 2) band_pair(blk + KB * c + d, dg[c][d], dg[c][d + 1]);
+#pragma unroll
+        for (int c = 0; c < KB; ++c) l[c] = st[c * W + lt];
+#pragma unroll
+        for (int c = 0; c < KB; ++c) {
+          if (c < pw) z[c] *= dg[c][0];
+#pragma unroll
+          for (int j = c + 1; j < KB; ++j) z[j] = fma(-dg[c][j - c], z[c], z[j]);
+        }
+#pragma unroll
+        for (int c = 0; c < KB; ++c) t = fma(-l[c], z[c], t);
+        if (lt == 0) {
+#pragma unroll
+          for (int c = 0; c < KB; c += 2) band_pair_put(done + (b & 1) * KB + c, z[c], z[c + 1]);
+        }
+        const int d = (lt - KB * (b + 1)) & (W - 1);
+        if (d < KB && b + 1 < nb) {  // the row enters the next diagonal block
+          rhs[((b + 1) & 1) * KB + d] = t;
+          row += W;
+          t = tn;
+          tn = row + W < R ? v[row + W] : T(0);
         }
       }
-      group_sync<BT>();
-      const int rows = min(R, k0 + pw + bw) - (k0 + pw);
-      for (int rb = 0; rb < rows; rb += BT / S2) {
-        const int r = k0 + pw + rb + r2;
-        T a0 = T(0), a1 = T(0);
-        if (rb + r2 < rows) {
-          const T* pr = pc + (r - k0);  // entry of column c at pr[c * bw]
-          const int c0 = max(0, r - k0 - bw);
-          int c = c0 + s2;
-          for (; c + S2 < pw; c += 2 * S2) {
-            a0 = fma(pr[c * bw], zz[c], a0);
-            a1 = fma(pr[(c + S2) * bw], zz[c + S2], a1);
-          }
-          if (c < pw) a0 = fma(pr[c * bw], zz[c], a0);
-        }
-        T t = a0 + a1;
-        for (int o = 1; o < S2; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (s2 == 0 && rb + r2 < rows) win[r & 255] -= t;
-      }
-      if (ld) win[(loaded + lt) & 255] = nv;
-      loaded = max(loaded, nload);
+      if (row >= hi && row < R) v[row] = t;
     }
-    cp_async_wait<0>();
     group_sync<BT>();
-    for (int r = hi + lt; r < R; r += BT) v[r] = win[r & 255];
+    if (lt < KB && nb > 0) {
+      const int k = lo + (nb - 1) * KB + lt;
+      if (k < R) (k < hi ? w : v)[k] = done[((nb - 1) & 1) * KB + lt];
+    }
     group_sync<BT>();
   }
 
   template <typename T, int BT>
   __device__ void band_bwd_blocked(T* v, T* w, int lo, int hi, int R, int lt) {
-    const int bw = this->bw, ldl = bw + 1, KB = band_solve_block(bw);
+    constexpr int KB = kBandSolveBlk, NS = kBandSolveStages, LP = KB + 1;
+    const int bw = this->bw, ldl = bw + 1;
+    const int nb = (hi - lo + KB - 1) / KB;
+    const int W = band_solve_owners(bw), SS = int(band_solve_stage(bw));
     const T* L = reinterpret_cast<const T*>(Lb);
-    T* win = reinterpret_cast<T*>(bwin);  // 256 slots: x_r at r & 255
-    T* pan = win + 256;
-    T* uu = pan + kBandSolveStages * KB * ldl;
-    const int S1 = band_lanes<BT>(KB), c1 = lt / S1, s1 = lt % S1;
-    if (hi <= lo) return;
-    for (int r = hi + lt; r < R; r += BT) win[r & 255] = v[r];
-    int k0 = lo + (hi - 1 - lo) / KB * KB, buf = 0;
-    auto issue = [&](int k, int st) {
-      if (k >= lo)
-        band_issue_block<T, BT>(pan + st * KB * ldl, L + size_t(k) * ldl, min(KB, hi - k) * ldl,
-                                lt);
-      cp_async_commit();
-    };
-    for (int st = 0; st + 1 < kBandSolveStages; ++st) issue(k0 - st * KB, st);
-    for (; k0 >= lo; k0 -= KB, buf = (buf + 1) % kBandSolveStages) {
-      const int pw = min(KB, hi - k0);
-      const T wv = (s1 == 0 && c1 < pw) ? w[k0 + c1] : T(0);
-      // As in the forward.
-      cp_async_wait<kBandSolveStages - 2>();
+    T* ring = reinterpret_cast<T*>(bwin);
+    T* rhs = ring + NS * SS;
+    T* done = rhs + 2 * KB;
+    T* known = done + 2 * KB;
+    if (R > hi) {
+      for (int r = hi + lt; r < R; r += BT) known[r - hi] = v[r];
       group_sync<BT>();
-      issue(k0 - (kBandSolveStages - 1) * KB, (buf + kBandSolveStages - 1) % kBandSolveStages);
-      const T* pc = pan + buf * KB * ldl + c1 * ldl;  // column k0 + c1
-      {
-        T a0 = T(0), a1 = T(0);
-        if (c1 < pw) {
-          const int dmax = min(bw, R - 1 - k0 - c1), rb = k0 + c1;
-          int d = pw - c1 + s1;
-          for (; d + S1 <= dmax; d += 2 * S1) {
-            a0 = fma(pc[d], win[(rb + d) & 255], a0);
-            a1 = fma(pc[d + S1], win[(rb + d + S1) & 255], a1);
+    }
+    if (lt >= W && lt < 2 * W) {
+      // Step b: rows kb = hi - 8 (b + 1) ..; owner ct has row kb - 1 - d with d =
+      // (ct - 8 (b + 1)) mod W, whose entries L(kb + q, row) are contiguous in the
+      // band: eight neighbouring copiers copy one row's.
+      const int ct = lt - W;
+      auto issue = [&](int b) {
+        if (b < nb) {
+          T* st = ring + (b & (NS - 1)) * SS;
+          const int kb = hi - KB * (b + 1), q = ct & (KB - 1);
+#pragma unroll
+          for (int u = 0; u < KB; ++u) {
+            const int d = (ct + u * W) >> 3, i = kb - 1 - d;
+            const bool ok = q + 1 + d <= bw && i >= lo;
+            cp_async_elem(st + ((d + KB * (b + 1)) & (W - 1)) * LP + q,
+                          ok ? L + size_t(i) * ldl + (q + 1 + d) : L, ok);
           }
-          if (d <= dmax) a0 = fma(pc[d], win[(rb + d) & 255], a0);
+#pragma unroll 1
+          for (int e = ct; e < KB * KB; e += W) {
+            const int c = e >> 3, dd = e & 7;
+            const bool ok = c + dd < KB && dd <= bw && kb + c >= lo;
+            cp_async_elem(st + LP * W + e, ok ? L + size_t(kb + c) * ldl + dd : L, ok);
+          }
         }
-        T t = a0 + a1;
-        for (int o = 1; o < S1; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (s1 == 0 && c1 < pw) uu[c1] = wv - t;
+        cp_async_commit();
+      };
+#pragma unroll 1
+      for (int b = 0; b + 1 < NS; ++b) issue(b);
+#pragma unroll 1
+      for (int b = 0; b < nb; ++b) {
+        cp_async_wait<NS - 2>();
+        band_step_sync(2 * W);
+        issue(b + NS - 1);
       }
-      group_sync<BT>();
-      {
-        T a0 = T(0), a1 = T(0);
-        if (c1 < pw) {
-          int r = c1 + s1;
-          for (; r + S1 < pw; r += 2 * S1) {
-            a0 = fma(pc[r - c1], uu[r], a0);
-            a1 = fma(pc[r + S1 - c1], uu[r + S1], a1);
-          }
-          if (r < pw) a0 = fma(pc[r - c1], uu[r], a0);
+      cp_async_wait<0>();
+    } else if (lt < W) {
+      auto value = [&](int r) { return r >= lo ? w[r] : T(0); };
+      int row = hi - 1 - lt;
+      T t = value(row), tn = value(row - W);
+      // The known values that reach this row, eight entries in flight.
+      const int reach = row >= lo ? min(R, row + bw + 1) - hi : 0;
+      const T* Lr = L + size_t(max(row, lo)) * ldl + (hi - row);
+#pragma unroll 1
+      for (int r = 0; r < reach; r += 8) {
+        T l[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) l[u] = r + u < reach ? Lr[r + u] : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (r + u < reach) t = fma(-l[u], known[r + u], t);
+      }
+      if (lt < KB) {
+        rhs[KB - 1 - lt] = t;
+        row -= W;
+        t = tn;
+        tn = value(row - W);
+      }
+#pragma unroll 1
+      for (int b = 0; b < nb; ++b) {
+        band_step_sync(2 * W);
+        const int kb = hi - KB * (b + 1);
+        const T* st = ring + (b & (NS - 1)) * SS;
+        if (b > 0 && lt < KB) v[kb + KB + lt] = done[((b - 1) & 1) * KB + lt];
+        T dg[KB][KB], x[KB], l[KB];
+        const T* rp = rhs + (b & 1) * KB;
+        const T* blk = st + LP * W;
+#pragma unroll
+        for (int c = 0; c < KB; c += 2) band_pair(rp + c, x[c], x[c + 1]);
+#pragma unroll
+        for (int q = 0; q < KB; ++q) l[q] = st[lt * LP + q];
+#pragma unroll
+        for (int c = 0; c < KB; ++c)
+#pragma unroll
+          for (int d = 0; d < KB - c; d += 2) band_pair(blk + KB * c + d, dg[c][d], dg[c][d + 1]);
+#pragma unroll
+        for (int c = KB - 1; c >= 0; --c) {
+          T s = x[c];
+#pragma unroll
+          for (int j = c + 1; j < KB; ++j) s = fma(-dg[c][j - c], x[j], s);
+          x[c] = s * dg[c][0];
         }
-        T x = a0 + a1;
-        for (int o = 1; o < S1; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (s1 == 0 && c1 < pw) {
-          v[k0 + c1] = x;
-          win[(k0 + c1) & 255] = x;
+        if (lt == 0) {
+#pragma unroll
+          for (int c = 0; c < KB; c += 2) band_pair_put(done + (b & 1) * KB + c, x[c], x[c + 1]);
+        }
+#pragma unroll
+        for (int q = 0; q < KB; ++q) t = fma(-l[q], x[q], t);
+        const int d = (lt - KB * (b + 1)) & (W - 1);
+        if (d < KB && b + 1 < nb) {
+          rhs[((b + 1) & 1) * KB + KB - 1 - d] = t;
+          row -= W;
+          t = tn;
+          tn = value(row - W);
         }
       }
     }
-    cp_async_wait<0>();
+    group_sync<BT>();
+    if (lt < KB && nb > 0) {
+      const int k = hi - KB * nb + lt;
+      if (k >= lo) v[k] = done[((nb - 1) & 1) * KB + lt];
+    }
     group_sync<BT>();
   }
 
@@ -3431,7 +3522,7 @@ struct Ipm {
     double* tmp = vec(kTMP);
     float* t32 = this->t32();
     for (int j = tid; j < n; j += NT) {
-      const double g = r[j] + sparse_dot_scaled(jx, at, r + n, iry + n, jp[j], jp[j + 1]);
+      const double g = r[j] + sparse_dot_ordered(jx, at, r + n, iry + n, jp[j], jp[j + 1]);
       if (fp64) {
         tmp[j] = g;
       } else {
@@ -3439,10 +3530,15 @@ struct Ipm {
       }
     }
     sync();
-    if (fp64) {
-      band_chol_solve<double>(tmp, vec(kW));
-    } else {
-      band_chol_solve<float>(t32, t32 + n);
+    QTQP_TOC(kPhSolveCols);
+    {
+      QTQP_TIC();
+      if (fp64) {
+        band_chol_solve<double>(tmp, vec(kW));
+      } else {
+        band_chol_solve<float>(t32, t32 + n);
+      }
+      QTQP_TOC(kPhTri);
     }
     for (int k = tid; k < N; k += NT) {
       double val;
@@ -3450,8 +3546,8 @@ struct Ipm {
         val = fp64 ? tmp[k] : double(t32[k]);
       } else {
         const int i = k - n;
-        const double ax = fp64 ? sparse_dot(ix, av, tmp, 0, ip[i], ip[i + 1])
-                               : sparse_dot(ix, av, t32, 0, ip[i], ip[i + 1]);
+        const double ax = fp64 ? sparse_dot_ordered(ix, av, tmp, nullptr, ip[i], ip[i + 1])
+                               : sparse_dot_ordered(ix, av, t32, nullptr, ip[i], ip[i + 1]);
         val = iry[k] * (ax - r[k]);
       }
       out[k] = accumulate ? out[k] + val : val;
