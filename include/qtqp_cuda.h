@@ -266,7 +266,9 @@ int qtqp_dense_batch_solve_noalloc(const qtqp_dense_instance* d_inst,
  * backends factorise the full KKT; the Gram reduction follows
  * src/qtqp/solvers_dense.py:25-145 in band storage).
  * Offsets are element offsets: *_ptr/*_idx into the int32 pool, *_val into
- * the double pool. */
+ * the double pool.  The entries of a row or column may come in any order, and
+ * an entry of A stored more than once counts as the sum (ascending rows without
+ * repeats are the fast form). */
 typedef struct {
   int32_t n, m, z, has_p;
   int32_t bw, nnz_a, nnz_p, reserved;

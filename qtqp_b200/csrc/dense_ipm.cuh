@@ -2734,12 +2734,13 @@ struct Ipm {
     }
     if (tid == 0) gcnt[ng] = 0;
   }
-  // Whether a row of A stores an entry twice (sorted, so side by side), in
-  // gcnt[number of groups]; after a barrier that follows band_gram_groups.
+  // Whether some row's columns are not strictly ascending, so that an entry may
+  // be stored twice, in gcnt[number of groups]; after a barrier that follows
+  // band_gram_groups.
   __device__ void band_gram_duplicates() {
     QTQP_BAND_LOCALS;
     for (int q = 1 + tid; q < nnz_a; q += NT) {
-      if (ix[q] != ix[q - 1]) continue;
+      if (ix[q] > ix[q - 1]) continue;
       int lo = 0, hi = m;  // the row of entry q: the last i with ip[i] <= q
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
