@@ -407,6 +407,15 @@ struct Ipm {
 #pragma unroll
           for (int a = 0; a < NACC; ++a) part[u][a] = AccT(0);
         int i = s;
+        if constexpr (FMT == kFmtDense) {
+          // Eight loads in flight, in straight-line code and the order of the
+          // loop below: n > 64, whose A may come from L2 (n = 96, m = 193, one QP:
+          // 4.1 ms, 5.6 with one or two in flight).
+          for (; i + 7 * S < len; i += 8 * S) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) body(k, i + u * S, part[u % U]);
+          }
+        }
         for (; i + (U - 1) * S < len; i += U * S) {
 #pragma unroll
           for (int u = 0; u < U; ++u) body(k, i + u * S, part[u]);
@@ -1295,10 +1304,10 @@ struct Ipm {
   // + sum_{i<n} P_ik wp_i (k < n; wy, ws, wp may be null), staged per warp in
   // the panel buffer PB (PB[w * n + k]; fused_colsum adds the warps' rows after
   // a barrier); with vx, the row products (A vx)_i into rows_out[i].  A warp
-  // takes kProdRows rows at a time, lane l columns l and l + 32, their loads
-  // issued first; the row sums are reduced across the warp, the first steps
-  // sending half of the values to the partner lane and keeping the other half.
-  // Ends without a barrier.
+  // takes kProdRows rows at a time, lane l columns l and l + 32 (n <= 32: eight
+  // rows, column l), their loads issued first; the row sums are reduced across the
+  // warp, the first steps sending half of the values to the partner lane and
+  // keeping the other half.  Ends without a barrier.
   //
   // What bounds these small solves is instruction fetch: code that an
   // iteration runs once through costs about 0.4 cycles per byte whatever it
@@ -1317,65 +1326,116 @@ struct Ipm {
     const int c0 = lane, c1 = lane + 32;
     const bool ok0 = c0 < n, ok1 = c1 < n;
     double cs0 = 0.0, cs1 = 0.0;
-    if (vx != nullptr || wy != nullptr) {
-      const double x0 = ok0 && vx != nullptr ? vx[c0] : 0.0;
-      const double x1 = ok1 && vx != nullptr ? vx[c1] : 0.0;
-      const int rsel = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);  // the row a lane ends with
+    if (n <= 32) {
+      // One column per lane, eight rows at a time: half the rounds of latency of
+      // the two-column loop below, which left lone small QPs slower than row dots
+      // (n = 16, m = 33, one QP in us: row dots 632, two columns 652, this 600).
+      if (vx != nullptr || wy != nullptr) {
+        const double x0 = ok0 && vx != nullptr ? vx[c0] : 0.0;
+        const int rsel = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
 #pragma unroll 1
-      for (int base = warp * RB; base < m; base += NW * RB) {
-        double t[RB], a1[RB];
+        for (int base = warp * 8; base < m; base += NW * 8) {
+          double t[8];
 #pragma unroll
-        for (int r = 0; r < RB; ++r) {
-          const double* row = A + (base + r) * lda;
-          const bool in = base + r < m;
-          t[r] = in && ok0 ? row[c0] : 0.0;
-          a1[r] = in && ok1 ? row[c1] : 0.0;
-        }
-        if (wy != nullptr) {
+          for (int r = 0; r < 8; ++r) t[r] = base + r < m && ok0 ? A[(base + r) * lda + c0] : 0.0;
+          if (wy != nullptr) {
 #pragma unroll
-          for (int r = 0; r < RB; ++r) {
-            const int i = min(base + r, m - 1);  // rows from m on hold zeros
-            const double w = ws != nullptr ? ws[i] * wy[i] : wy[i];
-            cs0 = fma(t[r], w, cs0);
-            cs1 = fma(a1[r], w, cs1);
-          }
-        }
-        if (vx != nullptr) {
-#pragma unroll
-          for (int r = 0; r < RB; ++r) t[r] = fma(t[r], x0, a1[r] * x1);
-#pragma unroll
-          for (int half = RB / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-            const bool hi = (lane & bit) != 0;
-#pragma unroll
-            for (int j = 0; j < half; ++j) {
-              const double send = hi ? t[j] : t[j + half];
-              const double keep = hi ? t[j + half] : t[j];
-              t[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            for (int r = 0; r < 8; ++r) {
+              const int i = min(base + r, m - 1);  // rows from m on hold zeros
+              cs0 = fma(t[r], ws != nullptr ? ws[i] * wy[i] : wy[i], cs0);
             }
           }
+          if (vx != nullptr) {
 #pragma unroll
-          for (int bit = 4; bit >= 1; bit >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
-          if ((lane & 7) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
+            for (int r = 0; r < 8; ++r) t[r] *= x0;
+#pragma unroll
+            for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+              const bool hi = (lane & bit) != 0;
+#pragma unroll
+              for (int j = 0; j < half; ++j) {
+                const double send = hi ? t[j] : t[j + half];
+                const double keep = hi ? t[j + half] : t[j];
+                t[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+              }
+            }
+#pragma unroll
+            for (int bit = 2; bit >= 1; bit >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
+            if ((lane & 3) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
+          }
         }
       }
-    }
-    static_assert(RB == 4, "rsel and the full steps");
-    if (wp != nullptr) {
+      if (wp != nullptr) {
 #pragma unroll 1
-      for (int i0 = warp; i0 < n; i0 += 4 * NW) {
-        double p0[4], p1[4];
+        for (int i0 = warp; i0 < n; i0 += 8 * NW) {
+          double p0[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + u * NW;
-          const double* row = P + i * ldp;
-          p0[u] = i < n && ok0 ? row[c0] : 0.0;
-          p1[u] = i < n && ok1 ? row[c1] : 0.0;
+          for (int u = 0; u < 8; ++u)
+            p0[u] = i0 + u * NW < n && ok0 ? P[(i0 + u * NW) * ldp + c0] : 0.0;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) cs0 = fma(p0[u], wp[min(i0 + u * NW, n - 1)], cs0);
         }
+      }
+    } else {
+      if (vx != nullptr || wy != nullptr) {
+        const double x0 = ok0 && vx != nullptr ? vx[c0] : 0.0;
+        const double x1 = ok1 && vx != nullptr ? vx[c1] : 0.0;
+        const int rsel = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);  // the row a lane ends with
+#pragma unroll 1
+        for (int base = warp * RB; base < m; base += NW * RB) {
+          double t[RB], a1[RB];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const double w = wp[min(i0 + u * NW, n - 1)];
-          cs0 = fma(p0[u], w, cs0);
-          cs1 = fma(p1[u], w, cs1);
+          for (int r = 0; r < RB; ++r) {
+            const double* row = A + (base + r) * lda;
+            const bool in = base + r < m;
+            t[r] = in && ok0 ? row[c0] : 0.0;
+            a1[r] = in && ok1 ? row[c1] : 0.0;
+          }
+          if (wy != nullptr) {
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+              const int i = min(base + r, m - 1);  // rows from m on hold zeros
+              const double w = ws != nullptr ? ws[i] * wy[i] : wy[i];
+              cs0 = fma(t[r], w, cs0);
+              cs1 = fma(a1[r], w, cs1);
+            }
+          }
+          if (vx != nullptr) {
+#pragma unroll
+            for (int r = 0; r < RB; ++r) t[r] = fma(t[r], x0, a1[r] * x1);
+#pragma unroll
+            for (int half = RB / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+              const bool hi = (lane & bit) != 0;
+#pragma unroll
+              for (int j = 0; j < half; ++j) {
+                const double send = hi ? t[j] : t[j + half];
+                const double keep = hi ? t[j + half] : t[j];
+                t[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+              }
+            }
+#pragma unroll
+            for (int bit = 4; bit >= 1; bit >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
+            if ((lane & 7) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
+          }
+        }
+      }
+      static_assert(RB == 4, "rsel and the full steps");
+      if (wp != nullptr) {
+#pragma unroll 1
+        for (int i0 = warp; i0 < n; i0 += 4 * NW) {
+          double p0[4], p1[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * NW;
+            const double* row = P + i * ldp;
+            p0[u] = i < n && ok0 ? row[c0] : 0.0;
+            p1[u] = i < n && ok1 ? row[c1] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const double w = wp[min(i0 + u * NW, n - 1)];
+            cs0 = fma(p0[u], w, cs0);
+            cs1 = fma(p1[u], w, cs1);
+          }
         }
       }
     }
