@@ -209,6 +209,15 @@ struct SnUpdSmem {
   int ab[3][2];
 };
 static_assert(sizeof(SnUpdSmem) <= kArenaBytes, "update step's shared memory");
+// The slot of SnUpdSmem::ab in which entry i of a chunk counts its keys, and the
+// one that thread 0 clears after entry i's count barrier.  Counted: before that
+// barrier, of entry 0 after the chunk's start, of entry 1 after entry 0's barrier
+// (no other barrier lies between the two), of later ones after the barrier that
+// ends the step before.  So the cleared slot must be neither entry i's, which is
+// being read, nor entry i + 1's; it is entry i - 1's, whose readers have passed
+// entry i's barrier, and entry i + 1's barrier lies before its next use.
+__host__ __device__ constexpr int sn_count_slot(int i) { return i % 3; }
+__host__ __device__ constexpr int sn_clear_slot(int i) { return (i + 2) % 3; }
 static_assert(kSnMaxW <= 64 && kSnSlab == 64, "one descendant per staged pair of tiles");
 
 // Updates of rows [r0, r1) (at most kSnSlab of them) of supernode sn's block
@@ -270,7 +279,7 @@ __device__ __noinline__ void sn_update_slab(const SnFactor& F, T* L, unsigned ch
     // Finds entry i's rows in the slab, their positions, and starts its copies;
     // returns their number.
     auto prepare = [&](int i) {
-      int* ab = sm.ab[i % 3];
+      int* ab = sm.ab[sn_count_slot(i)];
       const int32_t* Rd = F.rows + sm.row[i];
       const int len = sm.len[i], cnt = sm.cnt_w[i] >> 8, wd = sm.cnt_w[i] & 255;
       auto count = [&](int key, int base) {  // keys below the slab, and up to its end
@@ -285,7 +294,7 @@ __device__ __noinline__ void sn_update_slab(const SnFactor& F, T* L, unsigned ch
         count(base + t < len ? Rd[base + t] : kNone, base);
       __syncthreads();
       const int a = ab[0], nrow = ab[1] - ab[0], s = i & 1;
-      if (t == 0) sm.ab[(i + 1) % 3][0] = sm.ab[(i + 1) % 3][1] = 0;
+      if (t == 0) sm.ab[sn_clear_slot(i)][0] = sm.ab[sn_clear_slot(i)][1] = 0;
       if (nrow > 0) {
         auto place = [&](int key, int idx) {
           if (idx >= a && idx < a + nrow) {
