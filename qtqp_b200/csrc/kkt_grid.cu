@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
   if (s.tid == 0) {
     // A wait that gave up leaves no usable factor.
     const bool gave_up = *reinterpret_cast<volatile int*>(&s.gctl->err) != 0;
-    *info = rc == 0 && gave_up ? 1 : rc;
+    *info = gave_up ? -1 : rc;
     *reinterpret_cast<int*>(ws) = 64;
   }
 }
@@ -150,13 +150,11 @@ static int coop_launch(const void* kern, void** args, cudaStream_t stream, const
                     what);
 }
 
-int kkt_grid_reset(int n, int m, void* gws, cudaStream_t stream) {
-  return cuda_check(cudaMemsetAsync(gws, 0, plan_kkt_grid(n, m).g_off, stream),
-                    "cudaMemsetAsync");
-}
-
 int kkt_grid_factorize(int n, int m, const double* diag, char* ws, size_t header, char* gws,
                        int* info, cudaStream_t stream) {
+  int rc = cuda_check(cudaMemsetAsync(gws, 0, plan_kkt_grid(n, m).g_off, stream),
+                      "cudaMemsetAsync");
+  if (rc) return rc;
   void* args[] = {&n, &m, &diag, &ws, &header, &gws, &info};
   return coop_launch(reinterpret_cast<const void*>(kkt_grid_factorize_kernel), args, stream,
                      "kkt_grid_factorize_kernel launch");

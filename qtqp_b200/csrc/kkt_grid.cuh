@@ -24,8 +24,9 @@ size_t kkt_grid_bytes(int n, int m);
 // ws: the workspace, whose header (an int32: the factor's precision, 32 or 64)
 // and single-block layout (A, P and the vectors, `header` bytes in) both forms
 // share; gws: the grid form's part.  An FP32 factor is always the single
-// block's: kkt_grid_solve then runs that form.
-int kkt_grid_reset(int n, int m, void* gws, cudaStream_t stream);
+// block's: kkt_grid_solve then runs that form.  A factorisation starts from a clean
+// barrier and clean slots, whatever an earlier call left; *info is -1 when one of
+// its waits gave up.  A solve whose waits gave up gives NaN.
 int kkt_grid_factorize(int n, int m, const double* diag, char* ws, size_t header, char* gws,
                        int* info, cudaStream_t stream);
 int kkt_grid_solve(int n, int m, const double* rhs, double* out, char* ws, size_t header,

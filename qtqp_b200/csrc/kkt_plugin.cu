@@ -140,8 +140,7 @@ extern "C" int qtqp_kkt_dense_set(int32_t n, int32_t m, const double* d_a,
                                            4 * 148));
   plugin_set_kernel<<<blocks, kPluginThreads, 0, st>>>(n, m, d_a, d_p_off, ws);
   rc = cuda_check(cudaGetLastError(), "plugin_set_kernel launch");
-  if (rc || !kkt_grid_form(n)) return rc;
-  return kkt_grid_reset(n, m, ws + grid_part(n, m), st);
+  return rc;
 }
 
 extern "C" int qtqp_kkt_dense_factorize(int32_t n, int32_t m, const double* d_diag,

@@ -133,6 +133,9 @@ class CudaDenseSolver(LinearSolver):
         self._n, self._m, self._diag.data_ptr(), self._prec, self._ws.data_ptr(),
         self._info.data_ptr(), self._stream()))
     info = int(self._info.item())
+    if info < 0:
+      raise RuntimeError("the factorisation did not run to its end: a wait between the GPU's "
+                         "blocks gave up")
     if info != 0:
       raise np.linalg.LinAlgError(f"Cholesky failed (pivot {info} not positive)")
 
