@@ -529,12 +529,14 @@ int qtqp_kkt_dense_set(int32_t n, int32_t m, const double* d_a,
  * KKT diagonal of length n+m with the dual block negative.  d_info (device
  * int32) receives 0 or the 1-based failing pivot (LAPACK dpotrf convention), or
  * -1 when a wait of the whole-GPU form gave up (nothing is known of the matrix;
- * the next factorisation starts clean). */
+ * the next factorisation starts clean).  FP64 from n = 80 on runs on the whole
+ * GPU where the current device holds its 148 blocks at once, else in one block. */
 int qtqp_kkt_dense_factorize(int32_t n, int32_t m, const double* d_diag,
                              int32_t precision, void* d_ws, int32_t* d_info,
                              void* stream);
 /* solve (solvers_dense.py:130-142): out = K_reg^{-1} rhs.  NaN when a wait of the
- * whole-GPU form gave up (factorise again). */
+ * whole-GPU form gave up (factorise again), or when the factor is that form's and
+ * the device no longer holds it. */
 int qtqp_kkt_dense_solve(int32_t n, int32_t m, const double* d_rhs,
                          double* d_out, void* d_ws, void* stream);
 /* __matmul__ (solvers_dense.py:118-128): out = K_reg x. */

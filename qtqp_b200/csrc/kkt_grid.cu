@@ -3,7 +3,7 @@
 // bring the inverse of their block back into shared memory first.
 #include "kkt_grid.cuh"
 
-#include "large_ipm.cuh"
+#include <algorithm>
 
 namespace qtqp {
 
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
     // A wait that gave up leaves no usable factor.
     const bool gave_up = *reinterpret_cast<volatile int*>(&s.gctl->err) != 0;
     *info = gave_up ? -1 : rc;
-    *reinterpret_cast<int*>(ws) = 64;
+    *reinterpret_cast<int*>(ws) = kKktFactorGrid;
   }
 }
 
@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(kGridBT, 1)
                           char* gws) {
   __shared__ double red[2 * (kGridBT / 32) * kRedMax];
   extern __shared__ __align__(16) unsigned char arena[];
-  if (*reinterpret_cast<const int*>(ws) == 32) {  // an FP32 factor: one block
+  const int factor = *reinterpret_cast<const int*>(ws);
+  if (factor != kKktFactorGrid) {  // the single block's
     if (blockIdx.x != 0) return;
     DenseIpm<kGridBT> d;
     d.bind(n, m, nullptr, ws + header, 0);
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kGridBT, 1)
     d.red = red;
     d.phase = 0;
     d.o = nullptr;
-    d.kkt_solve(rhs, out, false, false);
+    d.kkt_solve(rhs, out, false, factor != kKktFactor32);
     return;
   }
   KktGridIpm s;
@@ -140,14 +141,34 @@ __global__ void __launch_bounds__(kGridBT)
   s.kkt_matvec(x, out);
 }
 
+// (kkt_grid_resident, which every call asks first, has set the kernels' shared
+// memory.)
 static int coop_launch(const void* kern, void** args, cudaStream_t stream, const char* what) {
-  int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int(kArenaBytes)),
-                      what);
-  if (rc) return rc;
   return cuda_check(cudaLaunchCooperativeKernel(kern, dim3(kLargeBlocks), dim3(kGridBT), args,
                                                 kArenaBytes, stream),
                     what);
+}
+
+int kkt_grid_resident() {
+  int dev = 0, sms = 0, coop = 0, a = 0, b = 0;
+  for (const void* kern : {reinterpret_cast<const void*>(kkt_grid_factorize_kernel),
+                           reinterpret_cast<const void*>(kkt_grid_solve_kernel)})
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kArenaBytes)) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kkt_grid_factorize_kernel, kGridBT,
+                                                    kArenaBytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kkt_grid_solve_kernel, kGridBT,
+                                                    kArenaBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return coop ? sms * std::min(a, b) : 0;
 }
 
 int kkt_grid_factorize(int n, int m, const double* diag, char* ws, size_t header, char* gws,

@@ -12,7 +12,7 @@
 namespace qtqp {
 
 constexpr int kPluginThreads = 256;
-constexpr size_t kPluginHeader = 256;  // int32 factor precision (32 or 64)
+constexpr size_t kPluginHeader = 256;  // int32: the factor in the workspace (kKktFactor...)
 
 __host__ __device__ inline size_t plugin_bytes(int n, int m) {
   const InstLayout L = plan_layout(n, m, 0);
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kPluginThreads)
     const int i = idx / n, j = idx - i * n;
     s.P[i * s.ldp + j] = (i == j) ? 0.0 : p_off[idx];
   }
-  // The factor's precision: none yet.
+  // No factor yet.
   if (t0 == 0) *reinterpret_cast<int*>(ws) = 0;
 }
 
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kPluginThreads)
   int rc = prec == QTQP_PREC_FP64 ? s.template factorize<double>() : s.template factorize<float>();
   if (threadIdx.x == 0) {
     *info = rc;
-    *reinterpret_cast<int*>(ws) = prec == QTQP_PREC_FP64 ? 64 : 32;
+    *reinterpret_cast<int*>(ws) = prec == QTQP_PREC_FP64 ? kKktFactor64 : kKktFactor32;
   }
 }
 
@@ -66,8 +66,12 @@ __global__ void __launch_bounds__(kPluginThreads)
     plugin_solve_kernel(int n, int m, const double* rhs, double* out, char* ws) {
   DenseIpm<kPluginThreads> s;
   plugin_bind(s, n, m, ws, nullptr);
-  const bool fp64 = *reinterpret_cast<const int*>(ws) != 32;
-  s.kkt_solve(rhs, out, false, fp64);
+  const int factor = *reinterpret_cast<const int*>(ws);
+  if (factor == kKktFactorGrid) {  // made by the grid form, which no longer fits
+    for (int k = threadIdx.x; k < n + m; k += kPluginThreads) out[k] = NAN;
+    return;
+  }
+  s.kkt_solve(rhs, out, false, factor != kKktFactor32);
 }
 
 __global__ void __launch_bounds__(kPluginThreads)
@@ -154,7 +158,7 @@ extern "C" int qtqp_kkt_dense_factorize(int32_t n, int32_t m, const double* d_di
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: unknown precision");
   char* ws = static_cast<char*>(d_ws);
   // (An FP32 factor keeps the single block's plain FP32 arithmetic.)
-  if (kkt_grid_form(n) && precision == QTQP_PREC_FP64)
+  if (precision == QTQP_PREC_FP64 && kkt_grid_form(n) && kkt_grid_route(n, kkt_grid_resident()))
     return kkt_grid_factorize(n, m, d_diag, ws, kPluginHeader, ws + grid_part(n, m), d_info,
                               static_cast<cudaStream_t>(stream));
   plugin_factorize_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -169,7 +173,7 @@ extern "C" int qtqp_kkt_dense_solve(int32_t n, int32_t m, const double* d_rhs, d
   if (d_rhs == nullptr || d_out == nullptr || d_rhs == d_out)
     return fail(QTQP_ERR_BAD_ARG, "dense KKT: rhs/out must be distinct device vectors");
   char* ws = static_cast<char*>(d_ws);
-  if (kkt_grid_form(n))
+  if (kkt_grid_form(n) && kkt_grid_route(n, kkt_grid_resident()))
     return kkt_grid_solve(n, m, d_rhs, d_out, ws, kPluginHeader, ws + grid_part(n, m),
                           static_cast<cudaStream_t>(stream));
   plugin_solve_kernel<<<1, kPluginThreads, 0, static_cast<cudaStream_t>(stream)>>>(n, m, d_rhs,
