@@ -35,13 +35,14 @@ __global__ void __launch_bounds__(kPluginThreads)
     plugin_set_kernel(int n, int m, const double* a, const double* p_off, char* ws) {
   DenseIpm<kPluginThreads> s;
   plugin_bind(s, n, m, ws, nullptr);
-  const int t0 = blockIdx.x * kPluginThreads + threadIdx.x, step = gridDim.x * kPluginThreads;
-  for (int idx = t0; idx < m * n; idx += step) {
-    const int i = idx / n, j = idx - i * n;
+  // (Unsigned: the last step may pass 2^31.)
+  const uint32_t t0 = blockIdx.x * kPluginThreads + threadIdx.x, step = gridDim.x * kPluginThreads;
+  for (uint32_t idx = t0; idx < uint32_t(m) * uint32_t(n); idx += step) {
+    const int i = idx / uint32_t(n), j = idx - i * uint32_t(n);
     s.A[i * s.lda + j] = a[idx];
   }
-  for (int idx = t0; idx < n * n; idx += step) {
-    const int i = idx / n, j = idx - i * n;
+  for (uint32_t idx = t0; idx < uint32_t(n) * uint32_t(n); idx += step) {
+    const int i = idx / uint32_t(n), j = idx - i * uint32_t(n);
     s.P[i * s.ldp + j] = (i == j) ? 0.0 : p_off[idx];
   }
   // No factor yet.
