@@ -34,7 +34,8 @@
 //     the supernodes' column-major value blocks.
 // When the top levels from some level on are worth more as one dense matrix
 // (dense_level), their columns are moved to the end of the ordering (an
-// equivalent one: they are closed under ancestors) and stages 4-7 run again.
+// equivalent one: they are closed under ancestors, so the supernodes' tree and the
+// rows of 4 are only relabelled); 5 to 7 are for that ordering.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -431,8 +432,8 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   std::vector<int> perm(n);
   for (int k = 0; k < n; ++k) perm[k] = order[post[k]];
   for (int k = 0; k < n; ++k) pinv[perm[k]] = k;
-  Adj g = relabel(adj, perm, pinv);
-  std::vector<int> parent = etree(g);
+  const Adj g = relabel(adj, perm, pinv);
+  const std::vector<int> parent = etree(g);
   // Column counts of L (row subtrees).
   std::vector<int> cc(n, 0), mark(n, -1), nchild(n, 0);
   for (int k = 0; k < n; ++k) {
@@ -511,6 +512,9 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   // supernodes are above the subtrees (decided in the first pass).
   int dense_from = -1;
   std::vector<char> top(S, 0);
+  // The supernodes' parents and rows; the second pass has the first's, relabelled.
+  std::vector<int> sparent(S, -1);
+  std::vector<std::vector<int>> R(S);
   for (int pass = 0; pass < 2; ++pass) {
   P = Plan();
   P.n = n;
@@ -521,8 +525,7 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   P.colsn.assign(n, 0);
   for (int s = 0; s < S; ++s)
     for (int j = fin_first[s]; j < fin_first[s + 1]; ++j) P.colsn[j] = s;
-  std::vector<int> sparent(S, -1);
-  for (int s = 0; s < S; ++s) {
+  for (int s = 0; s < S && pass == 0; ++s) {
     const int last = fin_first[s + 1] - 1;
     sparent[s] = parent[last] >= 0 ? P.colsn[parent[last]] : -1;
   }
@@ -532,9 +535,8 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   // Row structures.
   P.rowptr.assign(S + 1, 0);
   P.valptr.assign(S + 1, 0);
-  std::vector<std::vector<int>> R(S);
   std::fill(mark.begin(), mark.end(), -1);
-  for (int s = 0; s < S; ++s) {
+  for (int s = 0; s < S && pass == 0; ++s) {
     const int f = fin_first[s], l = fin_first[s + 1];
     std::vector<int>& rs = R[s];
     for (int j = f; j < l; ++j) {
@@ -554,6 +556,10 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
           rs.push_back(r);
         }
     std::sort(rs.begin() + (l - f), rs.end());
+  }
+  for (int s = 0; s < S; ++s) {
+    const int f = fin_first[s], l = fin_first[s + 1];
+    const std::vector<int>& rs = R[s];
     P.rowptr[s + 1] = P.rowptr[s] + int64_t(rs.size());
     P.valptr[s + 1] = P.valptr[s] + int64_t(rs.size()) * (l - f);
     P.max_rows = std::max(P.max_rows, int(rs.size()));
@@ -561,45 +567,6 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   }
   P.rows.reserve(P.rowptr[S]);
   for (int s = 0; s < S; ++s) P.rows.insert(P.rows.end(), R[s].begin(), R[s].end());
-  // Left-looking update lists: for each descendant d, the runs of its rows
-  // (beyond its own columns) that fall into one supernode's column range.
-  {
-    std::vector<int32_t> cnt(S + 1, 0);
-    for (int d = 0; d < S; ++d) {
-      const int w = fin_first[d + 1] - fin_first[d];
-      const int nr = int(P.rowptr[d + 1] - P.rowptr[d]);
-      const int32_t* rd = P.rows.data() + P.rowptr[d];
-      for (int r = w; r < nr;) {
-        const int t = P.colsn[rd[r]];
-        int e = r + 1;
-        while (e < nr && P.colsn[rd[e]] == t) ++e;
-        ++cnt[t + 1];
-        r = e;
-      }
-    }
-    for (int s = 0; s < S; ++s) cnt[s + 1] += cnt[s];
-    P.upd_ptr.assign(cnt.begin(), cnt.end());
-    const int U = cnt[S];
-    P.upd_src.assign(U, 0);
-    P.upd_off.assign(U, 0);
-    P.upd_cnt.assign(U, 0);
-    std::vector<int32_t> fillp(cnt.begin(), cnt.end() - 1);
-    for (int d = 0; d < S; ++d) {
-      const int w = fin_first[d + 1] - fin_first[d];
-      const int nr = int(P.rowptr[d + 1] - P.rowptr[d]);
-      const int32_t* rd = P.rows.data() + P.rowptr[d];
-      for (int r = w; r < nr;) {
-        const int t = P.colsn[rd[r]];
-        int e = r + 1;
-        while (e < nr && P.colsn[rd[e]] == t) ++e;
-        const int u = fillp[t]++;
-        P.upd_src[u] = d;
-        P.upd_off[u] = r;
-        P.upd_cnt[u] = e - r;
-        r = e;
-      }
-    }
-  }
   // Work per supernode (multiply-adds): its updates, the Cholesky of its
   // diagonal block and the triangular solve of the rows below.
   std::vector<double> work(S, 0.0), sub(S, 0.0);
@@ -607,13 +574,17 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
   for (int s = 0; s < S; ++s) {
     const double w = fin_first[s + 1] - fin_first[s];
     const double nr = double(P.rowptr[s + 1] - P.rowptr[s]);
-    double wk = w * w * w / 6.0 + (nr - w) * w * w / 2.0;
-    for (int u = P.upd_ptr[s]; u < P.upd_ptr[s + 1]; ++u) {
-      const int d = P.upd_src[u];
-      const double wd = fin_first[d + 1] - fin_first[d];
-      const double rem = double(P.rowptr[d + 1] - P.rowptr[d]) - P.upd_off[u];
-      wk += rem * P.upd_cnt[u] * wd;
+    work[s] += w * w * w / 6.0 + (nr - w) * w * w / 2.0;
+    // Its own updates of others: the runs of its rows, as in the lists below.
+    const int32_t* rd = P.rows.data() + P.rowptr[s];
+    for (int r = int(w); r < int(nr);) {
+      const int t = P.colsn[rd[r]];
+      int e = r + 1;
+      while (e < int(nr) && P.colsn[rd[e]] == t) ++e;
+      work[t] += (nr - r) * (e - r) * w;
+      r = e;
     }
+    const double wk = work[s];  // complete: its descendants come before it
     // A supernode also costs a fixed latency (its barriers and dependent loads,
     // tens of microseconds on one block), worth about 2e5 multiply-adds of
     // a block's throughput; without it, blocks given many small supernodes
@@ -689,25 +660,77 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
     dense_from = dense_level(P, fin_first, ntl);
     if (dense_from == ntl) break;
     // The dense part's supernodes last, everything else in its order.
-    std::vector<int> seq, widths;
+    std::vector<int> seq, order_sn, newcol(n), newsn(S), nfirst(1, 0);
     std::vector<char> ntop;
     for (int part = 0; part < 2; ++part)
       for (int s = 0; s < S; ++s)
         if ((top[s] && tlev[s] >= dense_from) == (part == 1)) {
-          for (int j = fin_first[s]; j < fin_first[s + 1]; ++j) seq.push_back(perm[j]);
-          widths.push_back(fin_first[s + 1] - fin_first[s]);
+          newsn[s] = int(order_sn.size());
+          order_sn.push_back(s);
+          for (int j = fin_first[s]; j < fin_first[s + 1]; ++j) {
+            newcol[j] = int(seq.size());
+            seq.push_back(perm[j]);
+          }
+          nfirst.push_back(int(seq.size()));
           ntop.push_back(top[s]);
         }
-    perm = seq;
-    top = ntop;
-    fin_first.assign(1, 0);
-    for (int w : widths) fin_first.push_back(fin_first.back() + w);
+    std::vector<int> nparent(S, -1);
+    std::vector<std::vector<int>> nR(S);
+    for (int s = 0; s < S; ++s) {
+      const int o = order_sn[s];
+      if (sparent[o] >= 0) nparent[s] = newsn[sparent[o]];
+      nR[s].swap(R[o]);
+      for (int& r : nR[s]) r = newcol[r];
+      std::sort(nR[s].begin() + (nfirst[s + 1] - nfirst[s]), nR[s].end());
+    }
+    perm.swap(seq);
+    top.swap(ntop);
+    fin_first.swap(nfirst);
+    sparent.swap(nparent);
+    R.swap(nR);
     for (int k = 0; k < n; ++k) pinv[perm[k]] = k;
-    g = relabel(adj, perm, pinv);
-    parent = etree(g);
     continue;
   }
   P.dense_cols = n - fin_first[P.top_list[P.top_ptr[dense_from]]];
+  }
+  // Left-looking update lists: for each descendant d, the runs of its rows
+  // (beyond its own columns) that fall into one supernode's column range.
+  {
+    std::vector<int32_t> cnt(S + 1, 0);
+    for (int d = 0; d < S; ++d) {
+      const int w = fin_first[d + 1] - fin_first[d];
+      const int nr = int(P.rowptr[d + 1] - P.rowptr[d]);
+      const int32_t* rd = P.rows.data() + P.rowptr[d];
+      for (int r = w; r < nr;) {
+        const int t = P.colsn[rd[r]];
+        int e = r + 1;
+        while (e < nr && P.colsn[rd[e]] == t) ++e;
+        ++cnt[t + 1];
+        r = e;
+      }
+    }
+    for (int s = 0; s < S; ++s) cnt[s + 1] += cnt[s];
+    P.upd_ptr.assign(cnt.begin(), cnt.end());
+    const int U = cnt[S];
+    P.upd_src.assign(U, 0);
+    P.upd_off.assign(U, 0);
+    P.upd_cnt.assign(U, 0);
+    std::vector<int32_t> fillp(cnt.begin(), cnt.end() - 1);
+    for (int d = 0; d < S; ++d) {
+      const int w = fin_first[d + 1] - fin_first[d];
+      const int nr = int(P.rowptr[d + 1] - P.rowptr[d]);
+      const int32_t* rd = P.rows.data() + P.rowptr[d];
+      for (int r = w; r < nr;) {
+        const int t = P.colsn[rd[r]];
+        int e = r + 1;
+        while (e < nr && P.colsn[rd[e]] == t) ++e;
+        const int u = fillp[t]++;
+        P.upd_src[u] = d;
+        P.upd_off[u] = r;
+        P.upd_cnt[u] = e - r;
+        r = e;
+      }
+    }
   }
   // Row slabs of the top supernodes (work items of the grid), prefix counts.
   P.top_slab.assign(P.top_list.size() + 1, 0);
@@ -723,6 +746,13 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
       P.top_upd[l + 1] += P.upd_ptr[P.top_list[q] + 1] - P.upd_ptr[P.top_list[q]];
   }
   // G's lower entries (diagonal first in each column) and their positions.
+  size_t entries = 0;
+  for (const auto& row : adj) entries += row.size();
+  entries = entries / 2 + n;
+  P.gcol.reserve(entries);
+  P.grow.reserve(entries);
+  P.gpos.reserve(entries);
+  std::vector<int> low;
   for (int j = 0; j < n; ++j) {
     const int s = P.colsn[j];
     const int f = fin_first[s];
@@ -732,8 +762,11 @@ static int build_plan(int n, int m, const int32_t* ap, const int32_t* ai, const 
     P.gcol.push_back(j);
     P.grow.push_back(j);
     P.gpos.push_back(base + (j - f));
-    for (int i : g[j]) {
-      if (i <= j) continue;
+    low.clear();
+    for (int o : adj[perm[j]])
+      if (pinv[o] > j) low.push_back(pinv[o]);
+    std::sort(low.begin(), low.end());
+    for (int i : low) {
       const int32_t* hit = std::lower_bound(rs, rs + nr, i);
       if (hit == rs + nr || *hit != i)
         return fail(QTQP_ERR_BAD_ARG, "qtqp_sparse_analyze: internal error (structure)");
