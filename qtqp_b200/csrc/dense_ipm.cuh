@@ -1304,7 +1304,7 @@ struct Ipm {
   // + sum_{i<n} P_ik wp_i (k < n; wy, ws, wp may be null), staged per warp in
   // the panel buffer PB (PB[w * n + k]; fused_colsum adds the warps' rows after
   // a barrier); with vx, the row products (A vx)_i into rows_out[i].  A warp
-  // takes kProdRows rows at a time, lane l columns l and l + 32 (n <= 32: eight
+  // takes 4, 8 or 16 rows at a time, lane l columns l and l + 32 (n <= 32: eight
   // rows, column l), their loads issued first; the row sums are reduced across the
   // warp, the first steps sending half of the values to the partner lane and
   // keeping the other half.  Ends without a barrier.
@@ -1316,12 +1316,11 @@ struct Ipm {
   // short loop, in one copy, serves the residual, both products of a KKT
   // solve, the tau equations and the termination test.
   static constexpr bool kFused = FMT == kFmtDense && NT <= 1024;
-  static constexpr int kProdRows = 4;
   __device__ __forceinline__ bool fused_ok() const { return kFused && n <= 64; }
   QTQP_PHASE void dense_products(const double* vx, const double* wy, const double* ws,
                                  const double* wp, double* rows_out) const {
     QTQP_LOCALS;
-    constexpr int NW = NT / 32, RB = kProdRows;
+    constexpr int NW = NT / 32;
     const int lane = tid & 31, warp = tid >> 5;
     const int c0 = lane, c1 = lane + 32;
     const bool ok0 = c0 < n, ok1 = c1 < n;
@@ -1376,10 +1375,19 @@ struct Ipm {
         }
       }
     } else {
-      if (vx != nullptr || wy != nullptr) {
+      // RB rows per warp and round: few rows are short code, many rows few rounds of
+      // latency.  100 QPs with n = 48..50, m = 2n on four warps, mixed precision, in
+      // ms: 4 rows a round 3.07, 8 rows 2.98, 16 rows 2.78; n = 44: 2.72, 2.56, 2.66;
+      // n = 34: 4 rows 2.37 (1000 QPs of n = 8..40 lost 7 % with 16 rows for all).
+      auto rows_of_a = [&](auto rb) {
+        constexpr int RB = decltype(rb)::value;
         const double x0 = ok0 && vx != nullptr ? vx[c0] : 0.0;
         const double x1 = ok1 && vx != nullptr ? vx[c1] : 0.0;
-        const int rsel = ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);  // the row a lane ends with
+        // The row a lane ends with: its top bits, after log2(RB) halving steps.
+        int rsel = 0;
+#pragma unroll
+        for (int half = RB / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1)
+          rsel += (lane & bit) != 0 ? half : 0;
 #pragma unroll 1
         for (int base = warp * RB; base < m; base += NW * RB) {
           double t[RB], a1[RB];
@@ -1413,12 +1421,21 @@ struct Ipm {
               }
             }
 #pragma unroll
-            for (int bit = 4; bit >= 1; bit >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
-            if ((lane & 7) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
+            for (int bit = 16 / RB; bit >= 1; bit >>= 1)
+              t[0] += __shfl_xor_sync(0xffffffffu, t[0], bit);
+            if ((lane & (32 / RB - 1)) == 0 && base + rsel < m) rows_out[base + rsel] = t[0];
           }
         }
+      };
+      if (vx != nullptr || wy != nullptr) {
+        if (m > 24 * NW) {
+          rows_of_a(std::integral_constant<int, 16>());
+        } else if (m > 20 * NW) {
+          rows_of_a(std::integral_constant<int, 8>());
+        } else {
+          rows_of_a(std::integral_constant<int, 4>());
+        }
       }
-      static_assert(RB == 4, "rsel and the full steps");
       if (wp != nullptr) {
 #pragma unroll 1
         for (int i0 = warp; i0 < n; i0 += 4 * NW) {

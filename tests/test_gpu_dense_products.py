@@ -1,6 +1,6 @@
 """The dense batch kernel's matrix-vector products at the edges of their loops:
 one column per lane up to n = 32, two up to 64, row dots above (eight entries per
-lane at a time); four or eight rows per warp, with remainders; every block size.
+lane at a time); 4, 8 or 16 rows per warp, with remainders; every block size.
 
 Criteria of the other path tests: the oracle's status, the reference's acceptance
 conditions, objective relative error <= 1e-6."""
@@ -19,6 +19,7 @@ pytestmark = pytest.mark.gpu
 
 OBJ_TOL = 1e-6
 SIZES = [(1, 2), (2, 9), (7, 8), (8, 17), (16, 31), (31, 63), (32, 33), (32, 65), (33, 34),
+         (33, 45), (40, 90), (50, 97), (60, 193), (64, 190),
          (63, 64), (64, 65), (65, 66), (65, 129), (79, 80), (96, 97)]
 
 
