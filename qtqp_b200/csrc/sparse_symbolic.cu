@@ -389,12 +389,14 @@ static std::vector<int> postorder(const std::vector<int>& parent) {
 }
 
 // The top level from which on the supernodes are cheaper as one dense matrix
-// over their columns (the number of levels: none).  Measured on a B200, per
-// interior-point iteration (one factorisation, about 4.5 solves): a top level
-// costs some 250 us of grid barriers and dependent steps, whatever its size; a
-// 128-column block of the dense part some 180 us (its diagonal chain and its
-// step in the solves), the dense part 150 us once, and its trailing updates run
-// at 20 TFLOP/s.
+// over their columns (the number of levels: none).  Per interior-point iteration
+// (one factorisation, about 4.5 solves), measured on a B200 when the dense part
+// was introduced: a top level costs some 250 us of grid barriers and dependent
+// steps, whatever its size; a 128-column block of the dense part some 180 us (its
+// diagonal chain and its step in the solves), the dense part 150 us once, and its
+// trailing updates run at 20 TFLOP/s.  The diagonal chain (130 us then, 50-65 now)
+// and the solves' steps have become shorter since, to about 90 us per block, so
+// the rule leaves out levels that might now join.
 static int dense_level(const Plan& P, const std::vector<int>& first, int levels) {
   int best = levels, cols = 0;
   double best_us = 250.0 * levels;
